@@ -116,6 +116,7 @@ int upload_grid(eph_ctx *c) {
   const size_t nc = (size_t)g.ntotal;
   CUDA_TRY(c, c->T0.alloc(nc));
   CUDA_TRY(c, c->T1.alloc(nc));
+  CUDA_TRY(c, c->T2.alloc(nc));
   CUDA_TRY(c, c->kappa.alloc(nc));
   CUDA_TRY(c, c->rhoC.alloc(nc));
   CUDA_TRY(c, c->irhoC.alloc(nc));
@@ -176,6 +177,127 @@ void set_time_params(eph_ctx *c) {
   c->nsub = c->grid.substeps(&c->inner_dt);
   c->P.prescale = c->grid.dV * c->dt;
   if (c->args.coloured) c->P.zeta = 1.0 - std::exp(-c->dt / c->args.tau0);  // fix_eph_coloured_exp.cpp:190, :685
+}
+
+// ih2 per axis as the FAST substeps use it
+double3 inverse_h2(const Grid &g) {
+  return make_double3(1.0 / (g.dx * g.dx), 1.0 / (g.dy * g.dy), 1.0 / (g.dz * g.dz));
+}
+
+// The FAST substeps with precomputed coefficients run: no T-dependent cells
+// (their kappa and C_e change every step), cells counted in 32 bits
+bool fdm_fast(const eph_ctx *c) {
+  return c->mode == EPH_MODE_FAST && !c->td.tdyn && c->grid.ntotal <= 0x7fffffffL;
+}
+
+// a grid made from the fix's words: one kappa, rho_e and C_e, no source, every
+// cell DYNAMIC
+bool fdm_uniform(const eph_ctx *c) { return c->args.T_infile == "NULL"; }
+
+FdmFast fdm_args(const eph_ctx *c) {
+  const Grid &g = c->grid;
+  FdmFast F{};
+  F.nx = (int)g.nx;
+  F.ny = (int)g.ny;
+  F.nz = (int)g.nz;
+  F.nc = (int)g.ntotal;
+  const size_t nc = (size_t)g.ntotal;
+  F.uni = F.coef = c->fdm_coef.p;
+  F.src_w = c->fdm_coef.p + 6 * nc;
+  F.src0 = c->fdm_coef.p + 7 * nc;
+  return F;
+}
+
+// the FAST substeps' coefficients for the current grid constants and substep
+// length (after set_time_params; not inside a capture)
+int build_fdm_coef(eph_ctx *c) {
+  if (!fdm_fast(c)) return EPH_OK;
+  const Grid &g = c->grid;
+  const size_t nc = (size_t)g.ntotal, count = fdm_uniform(c) ? 4 : 8 * nc;
+  if (c->fdm_coef.n != count) {
+    c->buf_gen += 1;
+    CUDA_TRY(c, c->fdm_coef.alloc(count));
+  }
+  if (fdm_uniform(c)) {
+    const double3 ih2 = inverse_h2(g);
+    const double s = c->inner_dt / (g.rho[0] * g.C[0]), k = g.kappa[0] * s;
+    const double h[4] = {k * ih2.x, k * ih2.y, k * ih2.z, s};
+    CUDA_TRY(c, cudaMemcpyAsync(c->fdm_coef.p, h, sizeof(h), cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+    return EPH_OK;
+  }
+  k_fdm_coef<<<nblocks((long)nc), BLOCK, 0, c->stream>>>(fdm_args(c), inverse_h2(c->grid), c->inner_dt, c->kappa.p,
+                                                         c->irhoC.p, c->S.p, c->gflag.p, c->fdm_coef.p,
+                                                         c->fdm_coef.p + 6 * nc, c->fdm_coef.p + 7 * nc);
+  CUDA_TRY(c, cudaGetLastError());
+  return EPH_OK;
+}
+
+// the FAST substeps of one step, the first turning the deposits into dT; the
+// result ends in T0
+int launch_fdm_fast(eph_ctx *c, PhaseScope &ps) {
+  const FdmFast F = fdm_args(c);
+  const bool uni = fdm_uniform(c);
+  const size_t nc = (size_t)F.nc;
+  double *rec = c->fdm_rec;
+  // one cluster of up to 16 blocks of up to 384 cells: from there on the
+  // cells per SM make a substep's FP64 chain longer than a launch costs
+  // (measured on GB300, us per step, cluster / launches: 10^3 cells, 4
+  // substeps 9.6 / 11.9; 16^3, 11 substeps 18.3 / 25.1; 5,600 cells, 14
+  // substeps 24.6 / 29.7; 20^3, 17 substeps 37.0 / 35.8)
+  if (c->fdm_fast_cluster && c->nsub > 1 && F.nc <= FDM_CLUSTER_CELLS * c->fdm_fast_cluster) {
+    ps.launched();
+    int blocks = 1;  // a power of two, no more than there are warps of cells
+    while (2 * blocks <= c->fdm_fast_cluster && 32 * blocks < F.nc) blocks *= 2;
+    const int per = ((F.nc + blocks - 1) / blocks + 31) / 32 * 32;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)per);
+    cfg.dynamicSmemBytes = 2 * sizeof(double) * (size_t)per;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)blocks;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (uni)
+      CUDA_TRY(c, cudaLaunchKernelEx(&cfg, k_fdm_cluster_fast<true>, F, c->nsub, c->T0.p, rec, c->dT.p, c->acc.p,
+                                     c->counters.p));
+    else
+      CUDA_TRY(c, cudaLaunchKernelEx(&cfg, k_fdm_cluster_fast<false>, F, c->nsub, c->T0.p, rec, c->dT.p, c->acc.p,
+                                     c->counters.p));
+    return EPH_OK;
+  }
+  ps.launched((int)c->nsub);
+  // the last substep writes T0 where a third buffer lets it (an odd count
+  // above one would end in T1)
+  const double *src = c->T0.p;
+  const int threads = F.nc < 152 * 256 ? 64 : 128;
+  for (unsigned s = 0; s < c->nsub; ++s) {
+    double *dst = s + 1 == c->nsub && s > 0 ? c->T0.p : (src == c->T1.p ? c->T2.p : c->T1.p);
+    if (rec) dst = rec + (size_t)s * nc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)nblocks(F.nc, threads));
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = s > 0 ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (uni)
+      CUDA_TRY(c, cudaLaunchKernelEx(&cfg, k_fdm_fast<true>, F, src, dst, c->dT.p, c->acc.p, s == 0 ? 1 : 0,
+                                     c->counters.p));
+    else
+      CUDA_TRY(c, cudaLaunchKernelEx(&cfg, k_fdm_fast<false>, F, src, dst, c->dT.p, c->acc.p, s == 0 ? 1 : 0,
+                                     c->counters.p));
+    src = dst;
+  }
+  if (src != c->T0.p)
+    CUDA_TRY(c, cudaMemcpyAsync(c->T0.p, src, sizeof(double) * nc, cudaMemcpyDeviceToDevice, c->stream));
+  return EPH_OK;
 }
 
 // read back the device error word; returns EPH_OK or the matching status
@@ -659,10 +781,16 @@ int launch_end_of_step(eph_ctx *c) {
       c->nsub = g.substeps_from(c->h_bounds[0], c->h_bounds[1], c->h_bounds[2], &c->inner_dt);
       ps.launched(2);
     }
-    const double3 ih2 = make_double3(1.0 / (g.dx * g.dx), 1.0 / (g.dy * g.dy), 1.0 / (g.dz * g.dz));
+    if (fdm_fast(c)) {
+      int r = launch_fdm_fast(c, ps);
+      if (r) return r;
+      CUDA_TRY(c, cudaGetLastError());
+      return EPH_OK;
+    }
+    const double3 ih2 = inverse_h2(g);
     double *src = c->T0.p, *dst = c->T1.p;
     if (!c->td.tdyn && c->fdm_cluster && c->nsub > 1 && g.ntotal <= 2048) {
-      // a small grid: every substep in one launch of one thread-block cluster,
+      // EXACT on a small grid: every substep in one launch of one thread-block cluster,
       // the cells spread evenly over its blocks (measured on GB300: 10^3
       // cells, 17 substeps, 0.178 -> 0.169 ms per step; 16^3 cells, 11
       // substeps, 35 us per step slower than the per-substep launches, whose
@@ -681,18 +809,11 @@ int launch_end_of_step(eph_ctx *c) {
       cfg.attrs = at;
       cfg.numAttrs = 1;
       double *rec = c->fdm_rec;
-      if (c->mode == EPH_MODE_FAST)
-        CUDA_TRY(c, cudaLaunchKernelEx(&cfg, k_fdm_cluster<true>, (long)g.nx, (long)g.ny, (long)g.nz, g.dx, g.dy,
-                                       g.dz, c->inner_dt, c->nsub, c->T0.p, c->T1.p, rec, (const double *)c->kappa.p,
-                                       (const double *)c->rhoC.p, (const double *)c->S.p,
-                                       (const signed char *)c->gflag.p, c->dT.p, c->acc.p, c->counters.p, c->td, ih2,
-                                       (const double *)c->irhoC.p));
-      else
-        CUDA_TRY(c, cudaLaunchKernelEx(&cfg, k_fdm_cluster<false>, (long)g.nx, (long)g.ny, (long)g.nz, g.dx, g.dy,
-                                       g.dz, c->inner_dt, c->nsub, c->T0.p, c->T1.p, rec, (const double *)c->kappa.p,
-                                       (const double *)c->rhoC.p, (const double *)c->S.p,
-                                       (const signed char *)c->gflag.p, c->dT.p, c->acc.p, c->counters.p, c->td, ih2,
-                                       (const double *)c->irhoC.p));
+      CUDA_TRY(c, cudaLaunchKernelEx(&cfg, k_fdm_cluster, (long)g.nx, (long)g.ny, (long)g.nz, g.dx, g.dy, g.dz,
+                                     c->inner_dt, c->nsub, c->T0.p, c->T1.p, rec, (const double *)c->kappa.p,
+                                     (const double *)c->rhoC.p, (const double *)c->S.p,
+                                     (const signed char *)c->gflag.p, c->dT.p, c->acc.p, c->counters.p, c->td, ih2,
+                                     (const double *)c->irhoC.p));
       // where the last substep wrote, as with the per-substep launches below
       if (rec) src = rec + (size_t)(c->nsub - 1) * (size_t)g.ntotal;
       else if (c->nsub % 2) src = c->T1.p;
@@ -914,10 +1035,26 @@ int eph_create(int narg, const char *const *arg, const eph_md *md, eph_ctx **out
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    int n1 = 0, n2 = 0;
-    c->fdm_cluster = cudaOccupancyMaxActiveClusters(&n1, k_fdm_cluster<true>, &cfg) == cudaSuccess &&
-                     cudaOccupancyMaxActiveClusters(&n2, k_fdm_cluster<false>, &cfg) == cudaSuccess && n1 >= 1 &&
-                     n2 >= 1;
+    int n1 = 0;
+    c->fdm_cluster = cudaOccupancyMaxActiveClusters(&n1, k_fdm_cluster, &cfg) == cudaSuccess && n1 >= 1;
+    // the FAST substeps' cluster: 16 blocks where the device takes them, else 8
+    for (int size : {16, 8}) {
+      bool ok = true;
+      for (auto *kern : {(const void *)k_fdm_cluster_fast<true>, (const void *)k_fdm_cluster_fast<false>}) {
+        if (size > 8) ok = ok && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        cfg.gridDim = dim3((unsigned)size);
+        cfg.blockDim = dim3(FDM_CLUSTER_CELLS);
+        cfg.dynamicSmemBytes = 2 * FDM_CLUSTER_CELLS * sizeof(double);
+        at[0].val.clusterDim.x = (unsigned)size;
+        int most = 0;
+        ok = ok && cudaOccupancyMaxActiveClusters(&most, kern, &cfg) == cudaSuccess && most >= 1;
+      }
+      cudaGetLastError();
+      if (ok) {
+        c->fdm_fast_cluster = size;
+        break;
+      }
+    }
     cudaGetLastError();
   }
   CUDA_TRY(c, cudaMallocHost(&c->h_err, sizeof(unsigned)));
@@ -977,6 +1114,7 @@ int eph_create(int narg, const char *const *arg, const eph_md *md, eph_ctx **out
   P.coloured = c->args.coloured ? 1 : 0;
   P.step = c->step_ctr.p;
   set_time_params(c);
+  if ((r = build_fdm_coef(c))) return r;
   // bins: edge >= rc (1 + 5e-5), at least 3 per axis
   if ((r = set_bin_geometry(c, c->beta.r_cutoff))) return r;
   CUDA_TRY(c, cudaDeviceSynchronize());  // the set-up copies and memsets above ran on the default stream
@@ -1735,9 +1873,10 @@ int eph_compute_vector(eph_ctx *c, int i, double *out) {
 int eph_reset_dt(eph_ctx *c, double dt) {
   if (!c || !(dt > 0)) return EPH_ERR_ARG;
   drop_graph(c);
+  c->buf_gen += 1;  // graphs captured elsewhere hold the old step constants
   c->dt = dt;
   set_time_params(c);
-  return EPH_OK;
+  return build_fdm_coef(c);
 }
 
 int eph_save_state(eph_ctx *c, const char *path) {
@@ -1838,6 +1977,7 @@ struct eph_batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   long launches_per_step = 0;
+  std::vector<unsigned long long> gen;  // each replica's buf_gen at the capture
   std::string err;
 };
 
@@ -1953,13 +2093,17 @@ static int batch_capture(eph_batch *b) {
     return EPH_ERR_CUDA;
   }
   b->launches_per_step = launches;
+  b->gen.clear();
+  for (const eph_ctx *c : b->reps) b->gen.push_back(c->buf_gen);
   return EPH_OK;
 }
 
 int eph_batch_step(eph_batch *b, int nsteps) {
   if (!b || nsteps < 0) return EPH_ERR_ARG;
   int rc;
-  if (!b->gexec && (rc = batch_capture(b))) return rc;
+  bool stale = !b->gexec;  // no graph, or a replica's buffers or constants changed since its capture
+  for (size_t r = 0; r < b->reps.size() && !stale; ++r) stale = b->gen[r] != b->reps[r]->buf_gen;
+  if (stale && (rc = batch_capture(b))) return rc;
   for (int s = 0; s < nsteps; ++s) {
     if (cudaGraphLaunch(b->gexec, b->main) != cudaSuccess) {
       b->err = "graph launch failed";
@@ -2079,8 +2223,10 @@ int eph_set_grid_constants(eph_ctx *c, double C_e, double kappa_e) {
   CUDA_TRY(c, upload_inverse(c, rc));
   CUDA_TRY(c, cudaMemcpy(c->kappa.p, g.kappa.data(), nc * 8, cudaMemcpyHostToDevice));
   drop_graph(c);  // the substep count may change
+  const unsigned nsub = c->nsub;
   set_time_params(c);
-  return EPH_OK;
+  if (c->nsub != nsub) c->buf_gen += 1;  // graphs captured elsewhere hold the old count of substeps
+  return build_fdm_coef(c);
 }
 
 struct eph_grid {

@@ -68,7 +68,9 @@ struct eph_ctx {
   // FAST mode, one lane per atom: stage 1 folded into the density sweep
   bool fuse_w = true;
   // small grids run all their substeps as one thread-block cluster launch
+  // (EXACT: 8 blocks; FAST: the largest cluster the device takes, 0 for none)
   bool fdm_cluster = false;
+  int fdm_fast_cluster = 0;
 
   int n = 0;
   DevBuf<D4> x, v, f, xhold, f_eph, f_rng, xi, fext, A, Bw;
@@ -118,7 +120,11 @@ struct eph_ctx {
   int pair_arith = EPH_PAIRS_DF64;
   DevBuf<float4> tab_rho_df, dfrec, dfvrec;
 
-  DevBuf<double> T0, T1, kappa, rhoC, irhoC, S, dT;
+  DevBuf<double> T0, T1, T2, kappa, rhoC, irhoC, S, dT;
+  // FAST substeps (k_fdm_fast): the uniform grid's four coefficients, or 6
+  // neighbour weights, source weight and constant source per cell of a grid
+  // read from a file
+  DevBuf<double> fdm_coef;
   // temperature-dependent cells: per-cell C_e and rho_e, the parameter tables
   DevBuf<double> gC, grho, E_y, E_dy, bounds;
   DevBuf<D4> C_T, K_T;

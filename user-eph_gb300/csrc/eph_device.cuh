@@ -105,10 +105,19 @@ struct StepParams {
 // the order of their bits).
 __device__ __forceinline__ bool pos_double(double v) { return __double_as_longlong(v) > 0; }
 
+// v < 0 (false for -0 and NaN) by the bits
+__device__ __forceinline__ bool neg_double(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull;
+}
+
 // Wait until the grids this one depends on programmatically have completed
 // and their memory is visible (griddepcontrol.wait; returns at once for a
 // kernel launched without a programmatic dependency).
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Let the programmatic dependents of this grid be launched now (they wait for
+// this grid's completion in griddep_wait before they touch memory).
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ bool below(double v, double c) { return __double_as_longlong(v) < __double_as_longlong(c); }
 
 // (size_t)y for a non-negative double y, by integer work on its bits (the
@@ -166,6 +175,16 @@ __device__ __forceinline__ double recip_nr(double x) {
   const unsigned rb = __float_as_uint(rf);
   const unsigned rhi = (rb & 0x80000000u) | ((((rb >> 23) & 0xffu) + 896u) << 20) | ((rb & 0x7fffffu) >> 3);
   const double r = __longlong_as_double((long long)(((unsigned long long)rhi << 32) | (unsigned long long)(rb << 29)));
+  return fma(r, fma(-x, r, 1.0), r);
+}
+
+// 1/x for x > 0 to ~1 ulp: recip_nr's FP32-seeded Newton step and one more
+// (its 2^-44 squared is below FP64's last bit), four FP64 instructions and
+// none of them a conversion; outside the FP32 exponent range, the division.
+__device__ __forceinline__ double inv_positive(double x) {
+  const unsigned e = (unsigned)((unsigned long long)__double_as_longlong(x) >> 52);  // with the sign bit
+  if (e < 1023 - 100 || e > 1023 + 100) return 1.0 / x;
+  const double r = recip_nr(x);
   return fma(r, fma(-x, r, 1.0), r);
 }
 

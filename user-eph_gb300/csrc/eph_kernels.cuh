@@ -2194,7 +2194,7 @@ __global__ void k_fdm_substep(long nx, long ny, long nz, double dx, double dy, d
                                   ih2, irhoC);
 }
 
-// All substeps of a small grid in one launch of one thread-block cluster of
+// All substeps of a small grid (EXACT) in one launch of one thread-block cluster of
 // FDM_CLUSTER blocks (one per SM), block b holding the cells
 // [b * blockDim, (b + 1) * blockDim) (one cell per thread).  Substeps are
 // separated by a device-scope fence and the cluster's hardware barrier,
@@ -2204,7 +2204,6 @@ __global__ void k_fdm_substep(long nx, long ny, long nz, double dx, double dy, d
 // temperatures are read through L2.  Results are those of nsub launches of
 // k_fdm_substep.
 constexpr int FDM_CLUSTER = 8;
-template <bool FAST>
 __global__ void __launch_bounds__(1024, 1)
     k_fdm_cluster(long nx, long ny, long nz, double dx, double dy, double dz, double inner_dt, unsigned nsub,
                   double *__restrict__ T0, double *__restrict__ T1, double *__restrict__ rec,
@@ -2227,7 +2226,7 @@ __global__ void __launch_bounds__(1024, 1)
   for (unsigned s = 0; s < nsub; ++s) {
     if (rec) dst = rec + (size_t)s * (size_t)ntotal;
     if (mine)
-      dst[r] = fdm_cell<FAST, true>(r, nx, ny, nz, dx, dy, dz, inner_dt, src, kappa, rhoC, S, flag, dTr, counters,
+      dst[r] = fdm_cell<false, true>(r, nx, ny, nz, dx, dy, dz, inner_dt, src, kappa, rhoC, S, flag, dTr, counters,
                                     td, ih2, irhoC);
     __threadfence();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -2235,6 +2234,199 @@ __global__ void __launch_bounds__(1024, 1)
     src = dst;
     if (!rec) dst = next;
   }
+}
+
+// ------------------------------------------------ FAST grid substeps
+//
+// A FAST substep is T' = T + sum over the six neighbours c_m (T_m - T) +
+// c_s (dT + S): with the spacings, kappa, rho_e C_e and the substep length
+// fixed between steps, everything of the stencil but the temperatures is a
+// coefficient.  FP64 issue binds these kernels (2 lanes per SM and clock), so
+// what counts is FP64 instructions per cell and substep: 31 in
+// fdm_cell<true>, 14 from per-cell coefficients (k_fdm_coef, built when the
+// grid or the time step changes), 12 on a uniform grid (the fix's words, no
+// grid file), whose four coefficients are the same for every cell.  They are
+// read from device memory, so captured steps follow a change of the grid's
+// constants as they follow a change of the per-cell arrays.
+struct FdmFast {
+  int nx, ny, nz, nc;
+  // uniform grid: kappa dt' / (rho_e C_e h^2) per axis and dt' / (rho_e C_e)
+  const double *uni;
+  // per cell otherwise: 6 x nc weights (-x, +x, -y, +y, -z, +z; 0 where the
+  // stencil leaves a neighbour out or the cell does not change), the source
+  // weight and the constant source c_s S
+  const double *coef, *src_w, *src0;
+};
+
+// the neighbours of cell r in the order -x, +x, -y, +y, -z, +z (periodic)
+__device__ __forceinline__ void fdm_neighbours(const FdmFast &F, int r, int *m) {
+  const int nxy = F.nx * F.ny;
+  const int row = r / F.nx, i = r - row * F.nx, k = row / F.ny, j = row - k * F.ny;
+  m[0] = i > 0 ? r - 1 : r + (F.nx - 1);
+  m[1] = i < F.nx - 1 ? r + 1 : r - (F.nx - 1);
+  m[2] = j > 0 ? r - F.nx : r + (nxy - F.nx);
+  m[3] = j < F.ny - 1 ? r + F.nx : r - (nxy - F.nx);
+  m[4] = k > 0 ? r - nxy : r + (F.nz - 1) * nxy;
+  m[5] = k < F.nz - 1 ? r + nxy : r - (F.nz - 1) * nxy;
+}
+
+// T of a cell after one substep from its own T, its neighbours' and its
+// source term `src` (c_s dT on a uniform grid, c_s (dT + S) otherwise); w: the
+// uniform grid's three coefficients or the cell's six weights
+template <bool UNIFORM>
+__device__ __forceinline__ double fdm_next(double T, const double *Tm, const double *w, double src,
+                                           unsigned long long *__restrict__ counters) {
+  double d;
+  if (UNIFORM) {
+    d = fma(w[0], fma(-2.0, T, Tm[0] + Tm[1]), src);
+    d = fma(w[1], fma(-2.0, T, Tm[2] + Tm[3]), d);
+    d = fma(w[2], fma(-2.0, T, Tm[4] + Tm[5]), d);
+  } else {
+    d = src;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) d = fma(w[q], Tm[q] - T, d);
+  }
+  T += d;
+  if (neg_double(T)) {
+    T = 0.0;
+    atomicAdd(&counters[CNT_T_CLAMP], 1ull);
+  }
+  return T;
+}
+
+// the weights of cell r, its source weight and constant source
+template <bool UNIFORM>
+__device__ __forceinline__ void fdm_weights(const FdmFast &F, int r, double *w, double &sw, double &s0) {
+  if (UNIFORM) {
+#pragma unroll
+    for (int q = 0; q < 3; ++q) w[q] = F.uni[q];
+    sw = F.uni[3];
+    s0 = 0.0;
+  } else {
+#pragma unroll
+    for (int q = 0; q < 6; ++q) w[q] = F.coef[(size_t)q * F.nc + r];
+    sw = F.src_w[r];
+    s0 = F.src0[r];
+  }
+}
+
+// The coefficients of FdmFast per cell (eph_fdm.h:322-387: a wall neighbour is
+// replaced by the cell itself; only DYNAMIC cells change)
+__global__ void k_fdm_coef(FdmFast F, double3 ih2, double inner_dt, const double *__restrict__ kappa,
+                           const double *__restrict__ irhoC, const double *__restrict__ S,
+                           const signed char *__restrict__ flag, double *__restrict__ coef,
+                           double *__restrict__ src_w, double *__restrict__ src0) {
+  const int r = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (r >= F.nc) return;
+  int m[6];
+  fdm_neighbours(F, r, m);
+  const bool dyn = flag[r] == 1;
+  const double c = dyn ? inner_dt * irhoC[r] : 0.0, kr = kappa[r];
+  const double ih[3] = {ih2.x, ih2.y, ih2.z};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    int p = m[2 * a], q = m[2 * a + 1];
+    const bool wq = flag[q] == 2, wp = !wq && flag[p] == 2;
+    if (wq) q = r;
+    if (wp) p = r;
+    const double d = 0.25 * (kappa[q] - kappa[p]), s = c * ih[a];
+    coef[(size_t)(2 * a) * F.nc + r] = wp ? 0.0 : s * (kr - d);
+    coef[(size_t)(2 * a + 1) * F.nc + r] = wq ? 0.0 : s * (kr + d);
+  }
+  src_w[r] = c;
+  src0[r] = dyn ? c * S[r] : 0.0;
+}
+
+// One substep over the grid, one thread per cell (k_fdm_substep's contract:
+// the first substep turns the deposits into dT and clears them).  Measured on
+// GB300 (us per substep, uniform): 64^3 cells 22 -> 10.5 (FP64 issue: 5 us),
+// 26^3 cells 6.5 -> 2.2.
+template <bool UNIFORM>
+__global__ void __launch_bounds__(128)
+    k_fdm_fast(FdmFast F, const double *__restrict__ T, double *__restrict__ Tout, double *__restrict__ dT,
+               U128 *__restrict__ acc, int first, unsigned long long *__restrict__ counters) {
+  griddep_launch();
+  const int r = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  int m[6];
+  double w[6], sw, s0;
+  if (r < F.nc) {
+    fdm_neighbours(F, r, m);
+    fdm_weights<UNIFORM>(F, r, w, sw, s0);
+  }
+  griddep_wait();
+  if (r >= F.nc) return;
+  double dTr;
+  if (first) {
+    dTr = from_fixed(acc[r]);
+    dT[r] = dTr;
+    acc[r] = U128{0ull, 0ull};
+  } else {
+    dTr = dT[r];
+  }
+  double Tm[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) Tm[q] = T[m[q]];
+  Tout[r] = fdm_next<UNIFORM>(T[r], Tm, w, fma(sw, dTr, s0), counters);
+}
+
+// All substeps of a small grid in one launch of one thread-block cluster
+// (cluster size = grid size, chosen at launch), block b holding cells
+// [b * blockDim, (b + 1) * blockDim), one per thread: the temperatures live in
+// two shared-memory buffers per block and neighbours are read from the
+// owning block's buffer through distributed shared memory, so a substep is
+// one cluster barrier, six such reads and the FP64 chain.  The hardware
+// barrier is reached the same number of times by every thread (the loop
+// bound is a launch argument).  As many SMs as a cluster may have: with few
+// cells per SM the FP64 chain of a substep is short.
+// Measured on GB300 (us per step): 10^3 cells, 17 substeps 55 -> 19; 16^3
+// cells, 11 substeps 56 (11 launches) -> 18.
+constexpr int FDM_CLUSTER_CELLS = 384;  // cells per block at most
+template <bool UNIFORM>
+__global__ void __launch_bounds__(FDM_CLUSTER_CELLS)
+    k_fdm_cluster_fast(FdmFast F, unsigned nsub, double *__restrict__ T0, double *__restrict__ rec,
+                       double *__restrict__ dT, U128 *__restrict__ acc, unsigned long long *__restrict__ counters) {
+  extern __shared__ double s_T[];  // [2][blockDim]
+  const int t = (int)threadIdx.x, nt = (int)blockDim.x;
+  const int r = (int)blockIdx.x * nt + t;
+  const bool mine = r < F.nc;
+  double T = 0.0, src = 0.0, w[6];
+  unsigned at[6];  // shared::cluster addresses of the neighbours in buffer 0
+  if (mine) {
+    int m[6];
+    fdm_neighbours(F, r, m);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      const int owner = m[q] / nt;
+      const unsigned local = (unsigned)__cvta_generic_to_shared(s_T + (m[q] - owner * nt));
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at[q]) : "r"(local), "r"(owner));
+    }
+    T = T0[r];
+    s_T[t] = T;
+    double sw, s0;
+    fdm_weights<UNIFORM>(F, r, w, sw, s0);
+    const double dTr = from_fixed(acc[r]);
+    dT[r] = dTr;
+    acc[r] = U128{0ull, 0ull};
+    src = fma(sw, dTr, s0);
+  }
+  unsigned cur = 0;  // byte offset of the buffer being read
+  const unsigned half = (unsigned)(nt * sizeof(double));
+  for (unsigned s = 0; s < nsub; ++s) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (mine) {
+      double Tm[6];
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+        asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(Tm[q]) : "r"(at[q] + cur) : "memory");
+      T = fdm_next<UNIFORM>(T, Tm, w, src, counters);
+      s_T[(cur ? 0 : nt) + t] = T;
+      if (rec) rec[(size_t)s * (size_t)F.nc + r] = T;
+    }
+    cur = half - cur;
+  }
+  if (mine) T0[r] = T;
+  // no block leaves while another may still read its buffers
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Exact sum of the grid temperatures (EPH_FDM::get_T_total, eph_fdm.h:189-196).

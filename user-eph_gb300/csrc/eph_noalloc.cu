@@ -21,14 +21,17 @@
 
 #include <cuda_runtime.h>
 
+#include "eph_device.cuh"
 #include "eph_gb.h"
+
+using namespace ephgb;
 
 namespace {
 
 constexpr int kMaxDevices = 64;
 
-// [0, MAX_CELLS): second temperature buffer; [MAX_CELLS, +3): c_min, rho_min,
-// kappa_max of the stability rule.
+// [0, MAX_CELLS): second temperature buffer (before the substeps: the blocks'
+// bounds); [MAX_CELLS, +3): c_min, rho_min, kappa_max of the stability rule.
 static __device__ __align__(256) double g_fdm_scratch[EPH_NOALLOC_MAX_CELLS + 8];
 
 // Device address of g_fdm_scratch per device, filled on the first call on
@@ -37,18 +40,13 @@ static __device__ __align__(256) double g_fdm_scratch[EPH_NOALLOC_MAX_CELLS + 8]
 // address up and store the same value.
 std::atomic<double *> g_scratch_addr[kMaxDevices];
 
-__global__ void k_noalloc_bounds(long ntotal, const double *__restrict__ C, const double *__restrict__ rho,
-                                 const double *__restrict__ kappa, const signed char *__restrict__ flag,
-                                 double *__restrict__ out) {
-  // eph_fdm.h:290-300: start from cell 0 whatever its flag, then every cell
-  // that is not CONSTANT_VALUE
-  double c_min = C[0], r_min = rho[0], k_max = kappa[0];
-  for (long i = 1 + threadIdx.x; i < ntotal; i += blockDim.x)
-    if (flag[i] != 0) {
-      c_min = fmin(c_min, C[i]);
-      r_min = fmin(r_min, rho[i]);
-      k_max = fmax(k_max, kappa[i]);
-    }
+// Blocks of the bounds reduction; each leaves its three bounds in the scratch
+// grid (free until the first substep writes it), and the last kernel of the
+// two combines them.  One block over all cells took 657 us at 64^3 cells (GB300);
+// 128 blocks and a second small launch take ~8 us.
+constexpr int kBoundsBlocks = 128;
+
+__device__ __forceinline__ void block_bounds(double c_min, double r_min, double k_max, double *__restrict__ out) {
   __shared__ double s[3][256];
   s[0][threadIdx.x] = c_min;
   s[1][threadIdx.x] = r_min;
@@ -69,42 +67,78 @@ __global__ void k_noalloc_bounds(long ntotal, const double *__restrict__ C, cons
   }
 }
 
-// One substep of EPH_FDM::solve (eph_fdm.h:315-396), the reference's
-// expression order: T_out from T_in.
-__global__ void k_noalloc_substep(long nx, long ny, long nz, double dx, double dy, double dz, double inner_dt,
-                                  const double *__restrict__ T, double *__restrict__ Tout,
-                                  const double *__restrict__ kappa, const double *__restrict__ rho,
-                                  const double *__restrict__ C, const double *__restrict__ S,
-                                  const double *__restrict__ dT, const signed char *__restrict__ flag) {
-  const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long ntotal = nx * ny * nz;
-  if (r >= ntotal) return;
-  const long i = r % nx, j = (r / nx) % ny, k = r / (nx * ny);
-  double ddT = 0.0;
-  if (flag[r] != 2) {
-    long p, q;
-    p = (i > 0) ? r - 1 : r + (nx - 1);
-    q = (i < nx - 1) ? r + 1 : r - (nx - 1);
-    if (flag[q] == 2) q = r;
-    else if (flag[p] == 2) p = r;
-    ddT += (kappa[q] - kappa[p]) * (T[q] - T[p]) / dx / dx / 4.0;
-    ddT += kappa[r] * ((T[q] + T[p] - 2.0 * T[r]) / dx / dx);
-    p = (j > 0) ? r - nx : r + (ny - 1) * nx;
-    q = (j < ny - 1) ? r + nx : r - (ny - 1) * nx;
-    if (flag[q] == 2) q = r;
-    else if (flag[p] == 2) p = r;
-    ddT += (kappa[q] - kappa[p]) * (T[q] - T[p]) / dy / dy / 4.0;
-    ddT += kappa[r] * ((T[q] + T[p] - 2.0 * T[r]) / dy / dy);
-    p = (k > 0) ? r - nx * ny : r + (nz - 1) * nx * ny;
-    q = (k < nz - 1) ? r + nx * ny : r - (nz - 1) * nx * ny;
-    if (flag[q] == 2) q = r;
-    else if (flag[p] == 2) p = r;
-    ddT += (kappa[q] - kappa[p]) * (T[q] - T[p]) / dz / dz / 4.0;
-    ddT += kappa[r] * ((T[q] + T[p] - 2.0 * T[r]) / dz / dz);
+__global__ void k_noalloc_bounds(int ntotal, const double *__restrict__ C, const double *__restrict__ rho,
+                                 const double *__restrict__ kappa, const signed char *__restrict__ flag,
+                                 double *__restrict__ parts) {
+  // eph_fdm.h:290-300: start from cell 0 whatever its flag, then every cell
+  // that is not CONSTANT_VALUE
+  double c_min = C[0], r_min = rho[0], k_max = kappa[0];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ntotal; i += gridDim.x * blockDim.x)
+    if (i > 0 && flag[i] != 0) {
+      c_min = fmin(c_min, C[i]);
+      r_min = fmin(r_min, rho[i]);
+      k_max = fmax(k_max, kappa[i]);
+    }
+  block_bounds(c_min, r_min, k_max, parts + 3 * blockIdx.x);
+}
+
+__global__ void k_noalloc_bounds_of(const double *__restrict__ parts, double *__restrict__ out) {
+  const double *p = parts + 3 * threadIdx.x;  // one thread per block of k_noalloc_bounds
+  block_bounds(p[0], p[1], p[2], out);
+}
+
+// One substep of EPH_FDM::solve (eph_fdm.h:315-396): T_out from T_in.
+// Bound by FP64 issue (2 lanes per SM and clock): the reference's twelve
+// divisions by the spacings become products with 1/h^2 from the host, the
+// division by rho_e C_e one FP32-seeded Newton reciprocal (inv_positive), and
+// the cell's coordinates 32-bit divisions.  64^3 cells on GB300: 71 us per
+// substep before, 18 us now (at ~32 FP64 instructions per cell: 13 us).
+// The sum rounds within 1e-16 of itself, T itself at its own last bit as before.
+__global__ void __launch_bounds__(128)
+    k_noalloc_substep(int nx, int ny, int nz, double3 ih2, double3 ih2_4, double inner_dt, const double *__restrict__ T,
+                      double *__restrict__ Tout, const double *__restrict__ kappa, const double *__restrict__ rho,
+                      const double *__restrict__ C, const double *__restrict__ S, const double *__restrict__ dT,
+                      const signed char *__restrict__ flag) {
+  griddep_launch();
+  griddep_wait();
+  const int r = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  const int nxy = nx * ny;
+  if (r >= nxy * nz) return;
+  const int row = r / nx, i = r - row * nx, k = row / ny, j = row - k * ny;
+  const double Tr = T[r];
+  const signed char fr = flag[r];
+  double t = Tr;
+  if (fr == 1) {
+    const int p3[3] = {i > 0 ? r - 1 : r + (nx - 1), j > 0 ? r - nx : r + (nxy - nx),
+                       k > 0 ? r - nxy : r + (nz - 1) * nxy};
+    const int q3[3] = {i < nx - 1 ? r + 1 : r - (nx - 1), j < ny - 1 ? r + nx : r - (nxy - nx),
+                       k < nz - 1 ? r + nxy : r - (nz - 1) * nxy};
+    const double ih[3] = {ih2.x, ih2.y, ih2.z}, ih4[3] = {ih2_4.x, ih2_4.y, ih2_4.z};
+    // every load at once; the wall rule then selects values
+    double Tq[3], Tp[3], kq[3], kp[3];
+    bool wq[3], wp[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      wq[a] = flag[q3[a]] == 2;
+      wp[a] = flag[p3[a]] == 2;
+      Tq[a] = T[q3[a]];
+      Tp[a] = T[p3[a]];
+      kq[a] = kappa[q3[a]];
+      kp[a] = kappa[p3[a]];
+    }
+    const double kr = kappa[r], source = dT[r] + S[r], inv = inv_positive(rho[r] * C[r]);
+    double grad = 0.0, lap = 0.0;  // sum of dk dT / 4 h^2, of the second differences
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const bool sp = wp[a] && !wq[a];
+      const double uq = wq[a] ? Tr : Tq[a], up = sp ? Tr : Tp[a];
+      const double dk = (wq[a] ? kr : kq[a]) - (sp ? kr : kp[a]);
+      grad = fma(dk * (uq - up), ih4[a], grad);
+      lap = fma(ih[a], fma(-2.0, Tr, uq + up), lap);
+    }
+    t = fma((fma(kr, lap, grad) + source) * inner_dt, inv, Tr);
   }
-  double t = T[r];
-  if (flag[r] == 1) t += (ddT + dT[r] + S[r]) / (rho[r] * C[r]) * inner_dt;
-  if (t < 0.0) t = 0.0;
+  if (neg_double(t)) t = 0.0;
   Tout[r] = t;
 }
 
@@ -135,7 +169,8 @@ extern "C" int eph_fdm_solve_noalloc(long nx, long ny, long nz, const double *lo
   const double dy = (hi[1] - lo[1]) / (double)(size_t)ny;
   const double dz = (hi[2] - lo[2]) / (double)(size_t)nz;
   // stability substeps, eph_fdm.h:275-313
-  k_noalloc_bounds<<<1, 256, 0, st>>>(ntotal, C_e, rho_e, kappa, flag, scratch + EPH_NOALLOC_MAX_CELLS);
+  k_noalloc_bounds<<<kBoundsBlocks, 256, 0, st>>>((int)ntotal, C_e, rho_e, kappa, flag, scratch);
+  k_noalloc_bounds_of<<<1, kBoundsBlocks, 0, st>>>(scratch, scratch + EPH_NOALLOC_MAX_CELLS);
   double b[3];
   if (cudaMemcpyAsync(b, scratch + EPH_NOALLOC_MAX_CELLS, sizeof b, cudaMemcpyDeviceToHost, st) != cudaSuccess)
     return EPH_ERR_CUDA;
@@ -158,12 +193,25 @@ extern "C" int eph_fdm_solve_noalloc(long nx, long ny, long nz, const double *lo
     nsub = s > 1u ? s : 1u;
     inner_dt = dt / nsub;
   }
-  const int threads = 64;
-  const int blocks = (int)((ntotal + threads - 1) / threads);
+  const int threads = 128;
+  const double3 ih2 = make_double3(1.0 / (dx * dx), 1.0 / (dy * dy), 1.0 / (dz * dz));
+  const double3 ih2_4 = make_double3(0.25 * ih2.x, 0.25 * ih2.y, 0.25 * ih2.z);
   double *src = T, *dst = scratch;
   for (unsigned s = 0; s < nsub; ++s) {
-    k_noalloc_substep<<<blocks, threads, 0, st>>>(nx, ny, nz, dx, dy, dz, inner_dt, src, dst, kappa, rho_e, C_e, S,
-                                                  dT, flag);
+    // each substep a programmatic dependent of the one before: its launch
+    // overlaps that one's tail, and it waits before it touches memory
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((ntotal + threads - 1) / threads));
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = s > 0 ? 1 : 0;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, k_noalloc_substep, (int)nx, (int)ny, (int)nz, ih2, ih2_4, inner_dt, (const double *)src, dst,
+                           kappa, rho_e, C_e, S, dT, flag) != cudaSuccess)
+      return EPH_ERR_CUDA;
     double *t = src;
     src = dst;
     dst = t;
