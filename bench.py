@@ -124,15 +124,15 @@ class ClockSampler:
 
 def density_bytes(n_atoms, n_pairs):
     """Algorithmic HBM bytes of one launch of the density sweep of the bench
-    workload (k_density_list_df: FAST, one element, stage 1 folded, df64 pair
+    workload (k_density_df: FAST, one element, stage 1 folded, df64 pair
     sums over the kept candidate lists): per atom read x_i, v_i (64 B), mask,
-    state, list length (12), the atom's df64 record (32), T_e at the atom (8);
+    state, list length (12), the atom's fixed-point position (32), T_e at the atom (8);
     written pair count (4), A_i, Bw_i (64), M_i (64), G_i (48), rho, beta, T_e
     at the atom (24), cell (4); per in-cutoff pair its list entry read (4) and
-    the cached index (4), e_ij and H e as double-floats (48) written.  The
+    the cached index (4), e_ij and H as double-floats (32) written.  The
     neighbours' records, the spline table and the list entries of the shell
     beyond the cut-off are not counted."""
-    return 324 * n_atoms + 56 * n_pairs
+    return 324 * n_atoms + 40 * n_pairs
 
 
 def forces_bytes(n_atoms, n_pairs):
@@ -140,8 +140,8 @@ def forces_bytes(n_atoms, n_pairs):
     FAST, one element): per atom its record flag (16 B), pair count (4), A_i,
     Bw_i (64), M_i (64), T_e at the atom (8), f read and written (64), f_EPH
     and f_RNG written (64); per in-cutoff pair the cached index (4), e_ij and
-    H e as double-floats (48).  The neighbours' records G_j are not counted."""
-    return 284 * n_atoms + 52 * n_pairs
+    H as double-floats (32).  The neighbours' records G_j are not counted."""
+    return 284 * n_atoms + 36 * n_pairs
 
 
 # DRAM bytes of one launch (dram__bytes_read.sum + dram__bytes_write.sum) over
@@ -830,7 +830,7 @@ def main():
                    "l2": "inputs larger than L2 (pair cache ~%d MB)" % (res["n_pairs"] * 52 // 2 ** 20),
                    "mode": "fast", "pair_arithmetic": "df64", "xi": "device Philox4x32-10"},
         "gpu_launches": res["launches"],
-        "roofline": roofline("density", "k_density_list_df", density_bytes(n, res["n_pairs"]),
+        "roofline": roofline("density", "k_density_df", density_bytes(n, res["n_pairs"]),
                              DENSITY_DRAM_OVER_ALGORITHMIC, DENSITY_PIPES),
         "roofline_forces": roofline("forces", "k_forces_df", forces_bytes(n, res["n_pairs"]),
                                     FORCES_DRAM_OVER_ALGORITHMIC, FORCES_PIPES),

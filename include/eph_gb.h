@@ -244,7 +244,7 @@ int eph_autotune_list_skin(eph_ctx *ctx, const double *skins, int nskins, int st
 #define EPH_PAIRS_DF64 1
 int eph_set_pair_arithmetic(eph_ctx *ctx, int which);
 
-/* Skin s of the kept candidate lists (Angstrom; default 0.3, used from 2^15
+/* Skin s of the kept candidate lists (Angstrom; default 0.3, used from 2^14
  * atoms on with the df64 pair sums and from 2^15 to 2^20 atoms with FP64
  * ones, where it pays; a skin set here applies at any size, 0 turns
  * the lists off).  The reference takes its pairs from the engine's Verlet list

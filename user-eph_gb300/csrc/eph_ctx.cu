@@ -30,10 +30,13 @@ bool df_active(const eph_ctx *c);
 // pg rows per pair: {rho_j(r^2), rho_i(r^2)} in EXACT mode, {rho_i(r^2)/r^2, 0}
 // in FAST mode with several elements, the y and z of H e with one element
 // when stage 1 is folded into the density sweep (the force sweep then needs
-// no H per pair); none otherwise
+// no H per pair).  The df64 sweeps need none; below 16,384 atoms, where the
+// lanes per atom decide which sweeps run, the rows are there anyway.
 cudaError_t alloc_pg(eph_ctx *c) {
-  if (c->mode == EPH_MODE_EXACT || c->multi || fused_friction(c))
-    return c->pg.alloc((size_t)c->kcap * (size_t)c->n);
+  const size_t rows = (size_t)c->kcap * (size_t)c->n;
+  const bool df = fused_friction(c) && c->pair_arith == EPH_PAIRS_DF64 && c->n >= 16384;
+  if (c->mode == EPH_MODE_EXACT || ((c->multi || fused_friction(c)) && !df))
+    return c->pg.n == rows ? cudaSuccess : c->pg.alloc(rows);
   c->pg.free();
   return cudaSuccess;
 }
@@ -369,11 +372,80 @@ bool fused_friction(const eph_ctx *c) {
 
 // FAST pair sums in df64: the one-lane density sweep with stage 1 folded,
 // over the bin search (k_density_df) or the kept lists (k_density_list_df),
-// then k_forces_df at any lanes per atom; bins of at most 1022 per axis
-// (the records pack them in 10 bits each)
+// then k_forces_df at any lanes per atom
 bool df_active(const eph_ctx *c) {
   return c->pair_arith == EPH_PAIRS_DF64 && c->mode == EPH_MODE_FAST && fused_friction(c) &&
-         !(c->tpa > 1 && c->n < 16384) && c->P.nb[0] <= 1022 && c->P.nb[1] <= 1022 && c->P.nb[2] <= 1022;
+         !(c->tpa > 1 && c->n < 16384);
+}
+
+// Lanes per atom of the df64 density sweep: more lanes while one lane per
+// atom leaves the SMs short of warps; the bin search also splits its 27 bins
+// over them (measured on GB300, us per launch with 1 / 2 / 4 lanes.  Kept lists:
+// 16,384 atoms 53 / 39 / 36, 32,000 62 / 52 / 51, 62,500 88 / 75 / 94, 131,072
+// 127 / 137 / 174.  Bin search: 16,384 atoms 136 / 98 / 70, 23,328 167 / 111 /
+// 80, 32,000 161 / 116 / 125, 131,072 363 / 326 / 340, 256,000 566 / 558 / 621,
+// 500,000 960 / 1,021 / 1,171.  From the EAM list: 16,384 atoms 102 / 70 / 52,
+// 62,500 132 / 104 / 120, 256,000 390 / 392 / 486)
+int density_lanes(const eph_ctx *c) {
+  if (c->reuse) return c->n <= 40000 ? 4 : (c->n <= 98304 ? 2 : 1);
+  if (c->eam) return c->n <= 32768 ? 4 : (c->n <= 196608 ? 2 : 1);
+  return c->n <= 28000 ? 4 : (c->n <= 300000 ? 2 : 1);
+}
+
+template <bool MULTI, int LANES>
+void launch_density_df_l(eph_ctx *c, const DensityArgs &D) {
+  const int nb = nblocks((long)c->n * LANES);
+  if (c->reuse) k_density_df<MULTI, LANES, DF_LIST><<<nb, BLOCK, 0, c->stream>>>(c->P, D);
+  else if (D.elist) k_density_df<MULTI, LANES, DF_EAM><<<nb, BLOCK, 0, c->stream>>>(c->P, D);
+  else k_density_df<MULTI, LANES, DF_BINS><<<nb, BLOCK, 0, c->stream>>>(c->P, D);
+}
+
+template <bool MULTI>
+void launch_density_df(eph_ctx *c, int xi_mode) {
+  DensityArgs D{};
+  D.mask = c->mask.p;
+  D.bin_count = c->bin_count.p;
+  D.bins = c->bins.p;
+  D.atom_bin = c->atom_bin.p;
+  D.atom_off = c->atom_off.p;
+  D.rec = c->dfrec.p;
+  D.x = c->x.p;
+  D.v = c->v.p;
+  D.xi_given = c->xi.p;
+  D.xi_mode = xi_mode;
+  D.T_e = c->T0.p;
+  D.pj = c->pj.p;
+  D.pe = reinterpret_cast<float4 *>(c->pe.p);
+  D.nshort = c->nshort.p;
+  D.A = c->A.p;
+  D.Bw = c->Bw.p;
+  D.rho = c->rho.p;
+  D.beta = c->beta_i.p;
+  D.cell = c->cell.p;
+  D.Te_i = c->Te_i.p;
+  D.wrapflag = c->wrapflag.p;
+  D.err = c->d_err.p;
+  D.counters = c->counters.p;
+  D.Mm = c->Mm.p;
+  D.G = c->G.p;
+  if (c->reuse) {
+    D.cl = c->cl.p;
+    D.cl_n = c->cl_n.p;
+    D.state = c->state.p;
+    D.rb = c->rb.p;
+    D.flist = c->flist.p;
+    D.xref = c->xref.p;
+  } else {
+    // with the standalone engine's EAM force the candidates come from its
+    // pair list of this step (the same bins and order; no bin scan)
+    if (!(c->eam_list_fresh && eam_pair_list(c, &D.elist, &D.ens))) D.elist = nullptr, D.ens = nullptr;
+    c->eam_list_fresh = false;
+  }
+  switch (density_lanes(c)) {
+    case 1: launch_density_df_l<MULTI, 1>(c, D); break;
+    case 2: launch_density_df_l<MULTI, 2>(c, D); break;
+    default: launch_density_df_l<MULTI, 4>(c, D); break;
+  }
 }
 
 template <bool FAST, bool MULTI, bool FUSE>
@@ -401,13 +473,8 @@ void launch_density_f(eph_ctx *c, int xi_mode) {
     }
   }
   if constexpr (FAST && FUSE) {
-    if (c->reuse && df_active(c)) {
-      float4 *pa = reinterpret_cast<float4 *>(c->pe.p), *pb = pa + (size_t)c->kcap * c->n;
-      k_density_list_df<MULTI><<<nblocks(c->n), BLOCK, 0, c->stream>>>(
-          c->P, c->x.p, c->mask.p, c->bin_count.p, c->bins.p, c->atom_bin.p, c->atom_off.p, c->dfrec.p, c->dfvrec.p,
-          c->xi.p, xi_mode, c->T0.p, c->pj.p, pa, pb, reinterpret_cast<float4 *>(c->pg.p), c->nshort.p, c->A.p,
-          c->Bw.p, c->rho.p, c->beta_i.p, c->cell.p, c->Te_i.p, c->wrapflag.p, c->d_err.p, c->counters.p, c->v.p,
-          c->Mm.p, c->G.p, c->cl.p, c->cl_n.p, c->state.p, c->rb.p, c->flist.p);
+    if (df_active(c)) {
+      launch_density_df<MULTI>(c, xi_mode);
       return;
     }
     if (c->reuse) {
@@ -416,23 +483,6 @@ void launch_density_f(eph_ctx *c, int xi_mode) {
           c->T0.p, c->pj.p, c->pe.p, c->pg.p, c->nshort.p, c->A.p, c->Bw.p, c->rho.p, c->beta_i.p, c->cell.p,
           c->Te_i.p, c->wrapflag.p, c->d_err.p, c->counters.p, c->v.p, c->Mm.p, c->G.p, c->cl.p, c->cl_n.p,
           c->state.p, c->rb.p, c->flist.p);
-      return;
-    }
-  }
-  if constexpr (FAST && FUSE) {
-    if (df_active(c)) {
-      float4 *pa = reinterpret_cast<float4 *>(c->pe.p), *pb = pa + (size_t)c->kcap * c->n;
-      // with the standalone engine's EAM force the candidates come from its
-      // pair list of this step (the same bins and order; no bin scan)
-      const unsigned *elist = nullptr;
-      const int *ens = nullptr;
-      if (!(c->eam_list_fresh && eam_pair_list(c, &elist, &ens))) elist = nullptr, ens = nullptr;
-      k_density_df<MULTI><<<nblocks(c->n), BLOCK, 0, c->stream>>>(
-          c->P, c->mask.p, c->bin_count.p, c->bins.p, c->atom_bin.p, c->atom_off.p, c->dfrec.p, c->dfvrec.p, c->x.p,
-          c->xi.p, xi_mode, c->T0.p, c->pj.p, pa, pb, reinterpret_cast<float4 *>(c->pg.p), c->nshort.p, c->A.p,
-          c->Bw.p, c->rho.p, c->beta_i.p, c->cell.p, c->Te_i.p, c->wrapflag.p, c->d_err.p, c->counters.p, c->v.p,
-          c->Mm.p, c->G.p, elist, ens);
-      c->eam_list_fresh = false;
       return;
     }
   }
@@ -452,12 +502,10 @@ template <bool FAST, bool MULTI, bool FRIC, bool RAND>
 void launch_forces_t(eph_ctx *c) {
   const int tpa = FAST ? c->tpa : 1;
   if (FAST && FRIC && df_active(c)) {
-    const float4 *pa = reinterpret_cast<const float4 *>(c->pe.p), *pb = pa + (size_t)c->kcap * c->n;
 #define EPH_FORCES_DF(T)                                                                                          \
   k_forces_df<MULTI, RAND, T><<<nblocks((long)c->n * T), BLOCK, 0, c->stream>>>(                                   \
-      c->P, c->pj.p, pa, pb, reinterpret_cast<const float4 *>(c->pg.p), c->nshort.p, c->Mm.p,                    \
-      reinterpret_cast<const float4 *>(c->G.p), c->A.p, c->Bw.p, c->Te_i.p, c->f.p, c->f_eph.p, c->f_rng.p,       \
-      c->f_dis.p, c->f_sto.p)
+      c->P, c->pj.p, reinterpret_cast<const float4 *>(c->pe.p), c->nshort.p, c->Mm.p,                             \
+      reinterpret_cast<const float4 *>(c->G.p), c->A.p, c->Bw.p, c->Te_i.p, c->f.p, c->f_eph.p, c->f_rng.p, c->f_dis.p, c->f_sto.p, c->dfrec.p, c->d_err.p)
     if (tpa == 1) EPH_FORCES_DF(1);
     else if (tpa == 2) EPH_FORCES_DF(2);
     else if (tpa == 4) EPH_FORCES_DF(4);
@@ -513,9 +561,13 @@ int set_bin_geometry(eph_ctx *c, double r) {
     c->P.w[k] = c->prd[k] / nb[k];
     c->P.inv_w[k] = 1.0 / c->P.w[k];
     c->P.wf[k] = (float)c->P.w[k];
-    c->P.w_hi[k] = (float)c->P.w[k];
-    c->P.w_lo[k] = (float)(c->P.w[k] - (double)c->P.w_hi[k]);
   }
+  // fixed-point unit of the df64 sweeps' positions: the range 2^(63 - q) A is at
+  // least twice the bins' radius r
+  c->P.fix_q = 63 - (int)std::ceil(std::log2(2.0 * r));
+  c->P.fix_hi = (float)std::ldexp(1.0, 32 - c->P.fix_q);
+  c->P.fix_lo = (float)std::ldexp(1.0, 8 - c->P.fix_q);
+  for (int k = 0; k < 3; ++k) c->P.fix_prd[k] = to_fixed_coord(c->prd[k], c->P.fix_q);
   c->nbins = nb[0] * nb[1] * nb[2];
   return EPH_OK;
 }
@@ -529,8 +581,8 @@ int auto_bcap(const eph_ctx *c) {
 
 // Kept candidate lists: FAST mode, model 4 with friction, the one-lane
 // density sweep (one lane per atom, or 16,384 atoms and more), no pair force
-// of the engine (it needs bins every step) and no adjoint.  By default from
-// 2^15 to 2^20 atoms: the lists save the bin search, which the density
+// of the engine (it needs bins every step) and no adjoint.  With FP64 pair
+// sums by default from 2^15 to 2^20 atoms: the lists save the bin search, which the density
 // sweep's FP64 pass hides less well in small systems, and cost four small
 // launches a step plus the atoms near moved ones (measured on GB300 with a
 // 0.3 A skin, step time: 16,384 atoms +18 %, 62,500 atoms -8 %, 131,072 atoms
@@ -539,11 +591,12 @@ int auto_bcap(const eph_ctx *c) {
 // limit); a skin set through eph_set_list_skin applies at any size.
 bool want_list(const eph_ctx *c) {
   // with the df64 pair sums (whose pass 2 no longer hides the bin search) the
-  // lists pay at every size from 2^15 atoms on (measured on GB300, step time
-  // bin search -> lists: 131,072 atoms 0.543 -> 0.482 ms, 500,000 atoms
-  // 1.447 -> 1.112 ms, 1,000,188 atoms 2.663 -> 2.007 ms, 2,048,000 atoms
-  // 5.133 -> 3.849 ms)
-  const bool size_ok = c->lskin_user || (c->n >= (1 << 15) && (c->n <= (1 << 20) || c->pair_arith == EPH_PAIRS_DF64));
+  // lists pay at every size that runs them, from 2^14 atoms on (measured on
+  // GB300, bins and density sweep of a step, bin search -> lists: 16,384 atoms
+  // 86 -> 66 us, 32,000 atoms 136 -> 80, 131,072 atoms 354 -> 163, 500,000
+  // atoms 1,031 -> 446)
+  const bool df = c->pair_arith == EPH_PAIRS_DF64;
+  const bool size_ok = c->lskin_user || (df ? c->n >= (1 << 14) : c->n >= (1 << 15) && c->n <= (1 << 20));
   if (c->mode != EPH_MODE_FAST || c->lskin <= 0.0 || c->list_block || c->eam || c->n <= 0 ||
       !(c->tpa == 1 || c->n >= 16384) || !fused_friction(c) || !size_ok)
     return false;
@@ -658,14 +711,14 @@ int launch_bin(eph_ctx *c) {
     const bool df = df_active(c);
     k_list_check<<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->xref.p, c->state.p, rb,
                                               c->flist.p, c->counters.p, df ? c->dfrec.p : nullptr,
-                                              df ? c->dfvrec.p : nullptr, c->v.p);
+                                              c->v.p);
     k_list_decide<<<1, 32, 0, c->stream>>>(rb, c->flist.p, c->counters.p);
     k_list_mark<<<LIST_FMAX, BLOCK, 0, c->stream>>>(c->P, c->x.p, rb, c->flist.p, c->bin_count.p, c->bins.p,
                                                     c->state.p);
     k_zero_if<<<nblocks(c->nbins), BLOCK, 0, c->stream>>>(c->bin_count.p, c->nbins, rb + 2);
     k_bin<<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->bin_count.p, c->bins.p,
                                        c->atom_bin.p, c->atom_off.p, c->d_err.p, c->counters.p, 0, rb + 2,
-                                       c->xref.p);
+                                       c->xref.p, df ? c->dfrec.p : nullptr, c->v.p);
     if (c->bcap <= 64 && c->nbins < 32768)
       k_bin_sort_warp<<<nblocks((long)c->nbins * 32), BLOCK, 0, c->stream>>>(c->nbins, c->bcap, c->bin_count.p,
                                                                               c->bins.p, rb + 2);
@@ -680,7 +733,7 @@ int launch_bin(eph_ctx *c) {
   const bool df = df_active(c);
   k_bin<<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->bin_count.p, c->bins.p,
                                      c->atom_bin.p, c->atom_off.p, c->d_err.p, c->counters.p, 1, nullptr, nullptr,
-                                     df ? c->dfrec.p : nullptr, df ? c->dfvrec.p : nullptr, c->v.p);
+                                     df ? c->dfrec.p : nullptr, c->v.p);
   ps.launched();
   // a warp per bin where the bins are few (the sort's latency shows), a
   // thread per bin where they are many (measured on GB300: 343 bins 20 ->
@@ -1110,6 +1163,9 @@ int eph_create(int narg, const char *const *arg, const eph_md *md, eph_ctx **out
   P.gdx = g.dx;
   P.gdy = g.dy;
   P.gdz = g.dz;
+  P.inv_gd[0] = 1.0 / g.dx;
+  P.inv_gd[1] = 1.0 / g.dy;
+  P.inv_gd[2] = 1.0 / g.dz;
   P.seed = (unsigned)c->args.seed;
   P.coloured = c->args.coloured ? 1 : 0;
   P.step = c->step_ctr.p;
@@ -1178,6 +1234,10 @@ int eph_set_pair_arithmetic(eph_ctx *c, int which) {
   drop_graph(c);
   c->buf_gen += 1;  // graphs captured elsewhere hold the old kernels
   c->pair_arith = which;
+  if (c->n > 0) {
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));  // alloc_pg may free rows a kernel still reads
+    CUDA_TRY(c, alloc_pg(c));
+  }
   return c->n > 0 ? configure_list(c) : EPH_OK;  // the lists' default range depends on it
 }
 
@@ -1460,8 +1520,7 @@ int eph_set_atoms(eph_ctx *c, int n, const double *hx, const double *hv, const i
     CUDA_TRY(c, c->stage.alloc(8 * N));
     CUDA_TRY(c, c->atom_bin.alloc(N));
     CUDA_TRY(c, c->atom_off.alloc(N));
-    CUDA_TRY(c, c->dfrec.alloc(2 * N));
-    CUDA_TRY(c, c->dfvrec.alloc(2 * N));
+    CUDA_TRY(c, c->dfrec.alloc(4 * N));
     CUDA_TRY(c, c->part.alloc((size_t)nblocks(n, 256)));
     if (c->fext.p) CUDA_TRY(c, c->fext.alloc(N));
     // capacities from the number density: a bin holds ~density*w^3 atoms, the

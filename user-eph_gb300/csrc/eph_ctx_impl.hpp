@@ -115,10 +115,10 @@ struct eph_ctx {
   DevBuf<D4> tab_rho_r_sq, tab_beta, tab_alpha;
   // FAST pair sums in df64 (eph_set_pair_arithmetic, on by default): the
   // rho(r^2) tables in local form (two float4 per knot) and the per-atom
-  // records k_bin writes for them (bin offset and bin, velocity: two float4
-  // each per atom)
+  // records k_bin or k_list_check writes for them (df_record: 64 B per atom)
   int pair_arith = EPH_PAIRS_DF64;
-  DevBuf<float4> tab_rho_df, dfrec, dfvrec;
+  DevBuf<float4> tab_rho_df;
+  DevBuf<int4> dfrec;
 
   DevBuf<double> T0, T1, T2, kappa, rhoC, irhoC, S, dT;
   // FAST substeps (k_fdm_fast): the uniform grid's four coefficients, or 6

@@ -132,8 +132,20 @@ DF_FN df mul(df a, df b) {
   return r;
 }
 
-// a * b + c
-DF_FN df fma(df a, df b, df c) { return add(mul(a, b), c); }
+// a * b + c: add(mul(a, b), c) without normalising the product in between
+// (TwoSum needs no order, and the product's low part joins the error term)
+DF_FN df fma(df a, df b, df c) {
+  float p, e;
+  two_prod(a.hi, b.hi, p, e);
+  e = fmaf(a.hi, b.lo, e);
+  e = fmaf(a.lo, b.hi, e);
+  float s, se;
+  two_sum(p, c.hi, s, se);
+  se += e + c.lo;
+  df r;
+  fast_two_sum(s, se, r.hi, r.lo);
+  return r;
+}
 
 // a < b for normalised values
 DF_FN bool lt(df a, df b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
@@ -267,8 +279,10 @@ DF_FN df bsum_value(bsum s) { return add(s.tot, acc_value(s.blk)); }
 
 // a . b of two df64 3-vectors, normalised
 DF_FN df dot3(df ax, df ay, df az, df bx, df by, df bz) {
-  acc s = acc_zero();
-  acc_fma(s, ax, bx);
+  acc s;  // the first product starts the sum
+  two_prod(ax.hi, bx.hi, s.hi, s.lo);
+  s.lo = fmaf(ax.hi, bx.lo, s.lo);
+  s.lo = fmaf(ax.lo, bx.hi, s.lo);
   acc_fma(s, ay, by);
   acc_fma(s, az, bz);
   return acc_value(s);

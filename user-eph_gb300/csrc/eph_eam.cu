@@ -265,28 +265,27 @@ __device__ __forceinline__ void herm_df(const float4 *__restrict__ t, int n, df6
     if (!lt(p, one)) p = one;
   }
   if (m < 0) m = 0;
-  const float4 hi = t[2 * (size_t)m], lo = t[2 * (size_t)m + 1];
+  float4 hi, lo;
+  load_row(t + 2 * (size_t)m, hi, lo);
   const df c0{hi.x, lo.x}, c1{hi.y, lo.y}, c2{hi.z, lo.z}, c3{hi.w, lo.w};
   v = horner(c0, c1, c2, c3, p);
   dv = fma(p, fma(p, mul(df{3.0f, 0.0f}, c3), mul(df{2.0f, 0.0f}, c2)), c1);
 }
 
-// A pair's displacement as double-floats: from the atoms' df64 records of
-// this step's bins when there are any (the bin difference with the periodic
-// image plus the offsets in the bins, no FP64 work), else from the FP64
-// positions as k_eam_density forms it
-__device__ __forceinline__ void pair_e_df(const StepParams &P, const float4 *__restrict__ rec, int4 Bi, float4 oi,
-                                          float4 ol, const D4 &xi, const D4 *__restrict__ x, unsigned j,
-                                          unsigned code, df64::df &ex, df64::df &ey, df64::df &ez) {
+// A pair's displacement as double-floats: from the atoms' fixed-point records
+// of this step when there are any (xf: atom i's; no FP64 work), else from the
+// FP64 positions as k_eam_density forms it
+__device__ __forceinline__ void pair_e_df(const StepParams &P, const int4 *__restrict__ rec, const long long *xf,
+                                          const D4 &xi, const D4 *__restrict__ x, unsigned j, unsigned code,
+                                          df64::df &ex, df64::df &ey, df64::df &ez) {
   if (rec) {
-    const float4 R0 = rec[2 * (size_t)j], R1 = rec[2 * (size_t)j + 1];
-    const unsigned pk = __float_as_uint(R0.w);
-    const int dx = (int)(pk & 1023u) - 1 + ((int)(code % 3u) - 1) * P.nb[0] - Bi.x;
-    const int dy = (int)((pk >> 10) & 1023u) - 1 + ((int)((code / 3u) % 3u) - 1) * P.nb[1] - Bi.y;
-    const int dz = (int)((pk >> 20) & 1023u) - 1 + ((int)(code / 9u) - 1) * P.nb[2] - Bi.z;
-    ex = pair_disp(dx, R0.x, R1.x, oi.x, ol.x, P.w_hi[0], P.w_lo[0]);
-    ey = pair_disp(dy, R0.y, R1.y, oi.y, ol.y, P.w_hi[1], P.w_lo[1]);
-    ez = pair_disp(dz, R0.z, R1.z, oi.z, ol.z, P.w_hi[2], P.w_lo[2]);
+    long long e[3];
+    int4 ra, rb;
+    load_record(rec + 4 * (size_t)j, ra, rb);
+    pair_fixed(P, ra, rb, code, xf, e);
+    ex = fixed_df(e[0], P.fix_hi, P.fix_lo);
+    ey = fixed_df(e[1], P.fix_hi, P.fix_lo);
+    ez = fixed_df(e[2], P.fix_hi, P.fix_lo);
   } else {
     double a, b, c;
     image_vector(P, xi, x[j], code, a, b, c);
@@ -294,6 +293,14 @@ __device__ __forceinline__ void pair_e_df(const StepParams &P, const float4 *__r
     ey = df64::from_double(b);
     ez = df64::from_double(c);
   }
+}
+
+// atom i's fixed-point position from its record
+__device__ __forceinline__ void own_fixed(const int4 *__restrict__ rec, int i, long long *xf) {
+  const int4 a = rec[4 * (size_t)i], b = rec[4 * (size_t)i + 1];
+  xf[0] = ((long long)a.y << 32) | (unsigned)a.x;
+  xf[1] = ((long long)a.w << 32) | (unsigned)a.z;
+  xf[2] = ((long long)b.y << 32) | (unsigned)b.x;
 }
 
 // k_eam_density with the pair arithmetic in double-float: e from the FP64
@@ -306,7 +313,7 @@ __global__ void __launch_bounds__(128)
                      const int4 *__restrict__ atom_bin, const float4 *__restrict__ atom_off,
                      unsigned *__restrict__ epj, int *__restrict__ ens, int kcap, double *__restrict__ fp,
                      float2 *__restrict__ fpd, double *__restrict__ energy, unsigned *__restrict__ err,
-                     const float4 *__restrict__ rec) {
+                     const int4 *__restrict__ rec) {
   using namespace df64;
   __shared__ unsigned s_cand[CAND_SMEM * 128];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -328,11 +335,8 @@ __global__ void __launch_bounds__(128)
   }
   const int nc = eam_candidates(P, E, i, valid, Bi, oi, bin_count, bins, kcap, err, cset);
   __syncwarp();
-  float4 rh = make_float4(0.f, 0.f, 0.f, 0.f), rl = rh;
-  if (rec && valid) {
-    rh = rec[2 * (size_t)i];
-    rl = rec[2 * (size_t)i + 1];
-  }
+  long long xf[3] = {0, 0, 0};
+  if (rec && valid) own_fixed(rec, i, xf);
   const df rc2{E.rc2_hi, E.rc2_lo}, inv_dr{E.inv_dr_hi, E.inv_dr_lo};
   bsum rs = bsum_zero();
   int ns = 0;
@@ -342,7 +346,7 @@ __global__ void __launch_bounds__(128)
     const unsigned u = cget(k);
     const unsigned j = u & IDX_MASK;
     df dx, dy, dz;
-    pair_e_df(P, rec, Bi, rh, rl, xi, x, j, u >> IDX_BITS, dx, dy, dz);
+    pair_e_df(P, rec, xf, xi, x, j, u >> IDX_BITS, dx, dy, dz);
     const df r2 = dot3(dx, dy, dz, dx, dy, dz);
     if (lt(r2, rc2)) {
       epj[(size_t)ns * P.n + i] = u;  // ns <= k: the candidate there is consumed
@@ -375,18 +379,13 @@ __global__ void __launch_bounds__(128)
     k_eam_force_df(StepParams P, EamParams E, const D4 *__restrict__ x, const int *__restrict__ type,
                    const unsigned *__restrict__ epj, const int *__restrict__ ens, const float2 *__restrict__ fpd,
                    const D4 *__restrict__ fext, D4 *__restrict__ f, double *__restrict__ energy,
-                   const float4 *__restrict__ rec, const int4 *__restrict__ atom_bin) {
+                   const int4 *__restrict__ rec) {
   using namespace df64;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.n) return;
   const D4 xi = x[i];
-  int4 Bi = make_int4(0, 0, 0, 0);
-  float4 rh = make_float4(0.f, 0.f, 0.f, 0.f), rl = rh;
-  if (rec) {
-    Bi = atom_bin[i];
-    rh = rec[2 * (size_t)i];
-    rl = rec[2 * (size_t)i + 1];
-  }
+  long long xf[3] = {0, 0, 0};
+  if (rec) own_fixed(rec, i, xf);
   const int a = E.map[type[i]];
   const float2 gi = fpd[i];
   const df fpi{gi.x, gi.y}, inv_dr{E.inv_dr_hi, E.inv_dr_lo};
@@ -396,7 +395,7 @@ __global__ void __launch_bounds__(128)
     const unsigned u = epj[(size_t)k * P.n + i];
     const unsigned j = u & IDX_MASK;
     df dx, dy, dz;
-    pair_e_df(P, rec, Bi, rh, rl, xi, x, j, u >> IDX_BITS, dx, dy, dz);
+    pair_e_df(P, rec, xf, xi, x, j, u >> IDX_BITS, dx, dy, dz);
     const df r2 = dot3(dx, dy, dz, dx, dy, dz);
     const df r = df64::sqrt(r2, rsqrt_estimate(r2.hi));
     const df rinv = recip(r, rcp_estimate(r.hi));
@@ -550,12 +549,12 @@ int launch_eam(eph_ctx *c) {
   const D4 *fext = c->have_fext ? c->fext.p : nullptr;
   if (c->mode == EPH_MODE_FAST && c->pair_arith == EPH_PAIRS_DF64) {
     // the atoms' df64 records of this step's bins, where k_bin wrote them
-    const float4 *rec = ctxi::df_active(c) ? c->dfrec.p : nullptr;
+    const int4 *rec = ctxi::df_active(c) ? c->dfrec.p : nullptr;
     k_eam_density_df<<<nb, BLOCK, 0, c->stream>>>(c->P, E, c->x.p, c->type.p, c->bin_count.p, c->bins.p,
                                                    c->atom_bin.p, c->atom_off.p, d->pj.p, d->ns.p, d->kcap, d->fp.p,
                                                    d->fpd.p, d->energy.p, c->d_err.p, rec);
     k_eam_force_df<<<nb, BLOCK, 0, c->stream>>>(c->P, E, c->x.p, c->type.p, d->pj.p, d->ns.p, d->fpd.p, fext,
-                                                 c->f.p, d->energy.p, rec, c->atom_bin.p);
+                                                 c->f.p, d->energy.p, rec);
   } else {
     k_eam_density<<<nb, BLOCK, 0, c->stream>>>(c->P, E, c->x.p, c->type.p, c->bin_count.p, c->bins.p,
                                                 c->atom_bin.p, c->atom_off.p, d->pj.p, d->ns.p, d->kcap, d->fp.p,

@@ -175,39 +175,13 @@ __device__ __forceinline__ void wrap_into_box(const StepParams &P, D4 &xi) {
 // (unwrapped) bin corner.
 // With a gate (candidate-list reuse): nothing unless *gate (a build step),
 // no wrap (k_list_check did it), and the positions are kept in xref.
-// The records of atom i for the df64 pair sums (k_density_df,
-// k_density_list_df) in bins B of the current geometry: rec[2i] = {offset
-// x - lo - B w, hi parts; B + 1 packed 10 bits per axis}, rec[2i+1] =
-// {offset, lo parts; element}, vrec[2i], vrec[2i+1] = velocity, hi and lo.
-// The offset is formed with one rounding; a pair's displacement is then
-// d w + (o_j - o_i), d its bin difference.
-__device__ __forceinline__ void df_records(const StepParams &P, int i, const D4 &xi, const int *B,
-                                           const D4 *__restrict__ v, float4 *__restrict__ rec,
-                                           float4 *__restrict__ vrec) {
-  const double p[3] = {xi.x, xi.y, xi.z};
-  df64::df o[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) o[k] = df64::from_double(fma(-(double)B[k], P.w[k], p[k] - P.lo[k]));
-  const unsigned packed = (unsigned)(B[0] + 1) | ((unsigned)(B[1] + 1) << 10) | ((unsigned)(B[2] + 1) << 20);
-  rec[2 * (size_t)i] = make_float4(o[0].hi, o[1].hi, o[2].hi, __uint_as_float(packed));
-  rec[2 * (size_t)i + 1] = make_float4(o[0].lo, o[1].lo, o[2].lo, __int_as_float((int)xi.w));
-  const D4 vi = v[i];
-  const df64::df vx = df64::from_double(vi.x), vy = df64::from_double(vi.y), vz = df64::from_double(vi.z);
-  vrec[2 * (size_t)i] = make_float4(vx.hi, vy.hi, vz.hi, 0.f);
-  vrec[2 * (size_t)i + 1] = make_float4(vx.lo, vy.lo, vz.lo, 0.f);
-}
-
-// With rec (the df64 pair sums), also the atom's records for them: rec[2i] =
-// {offset in its bin, hi parts; bin + 1 packed 10 bits per axis},
-// rec[2i+1] = {offset, lo parts; element}, vrec[2i], vrec[2i+1] = velocity,
-// hi and lo parts.  The offset is x - lo - b w with one rounding; a pair's
-// displacement is then d w + (o_j - o_i), d the bin difference.
+// With rec (the df64 pair sums), also the atom's record for them (df_record).
 __global__ void k_bin(StepParams P, D4 *__restrict__ x, D4 *__restrict__ xhold, const int *__restrict__ wrapflag,
                       int *__restrict__ bin_count, BinEntry *__restrict__ bins, int4 *__restrict__ atom_bin,
                       float4 *__restrict__ atom_off, unsigned *__restrict__ err,
                       unsigned long long *__restrict__ counters, int bump_step, const int *__restrict__ gate = nullptr,
-                      D4 *__restrict__ xref = nullptr, float4 *__restrict__ rec = nullptr,
-                      float4 *__restrict__ vrec = nullptr, const D4 *__restrict__ v = nullptr) {
+                      D4 *__restrict__ xref = nullptr, int4 *__restrict__ rec = nullptr,
+                      const D4 *__restrict__ v = nullptr) {
   if (gate && !*gate) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0 && bump_step) *P.step += 1ull;  // read by the density sweep that follows
@@ -251,10 +225,37 @@ __global__ void k_bin(StepParams P, D4 *__restrict__ x, D4 *__restrict__ xhold, 
   }
   atom_bin[i] = make_int4(B[0], B[1], B[2], flat);
   atom_off[i] = make_float4(o[0], o[1], o[2], 0.f);
-  if (rec) df_records(P, i, xi, B, v, rec, vrec);
+  if (rec) {
+    const int none[3] = {0, 0, 0};
+    df_record(P, i, xi, none, false, v[i], rec);
+  }
 }
 
 // -------------------------------------------------------- density sweep
+
+// Append u to the candidate list of the lane's atom where `take`: with one
+// lane per atom after the lane's own nc entries; with LANES lanes, which share
+// the atom's list and all call this together, in lane order (nc, the list's
+// length, stays the same on the atom's lanes).  At most cap entries.
+template <int LANES, class Set>
+__device__ __forceinline__ void append_candidate(bool take, unsigned u, int &nc, int cap, Set cset,
+                                                 unsigned *__restrict__ err) {
+  int pos = nc;
+  if (LANES == 1) {
+    if (take && nc < cap) ++nc;
+  } else {
+    const int lane = threadIdx.x & 31;
+    const unsigned mine = (LANES == 32 ? 0xffffffffu : ((1u << LANES) - 1u) << (lane & ~(LANES - 1)));
+    const unsigned who = __ballot_sync(0xffffffffu, take) & mine;
+    pos += __popc(who & ((1u << lane) - 1u));
+    nc += __popc(who);
+    nc = nc < cap ? nc : cap;
+  }
+  if (take) {
+    if (pos < cap) cset(pos, u);
+    else atomicOr(err, ERR_PAIR_OVERFLOW);
+  }
+}
 
 // Candidates of atom i in the bin at stencil offset (dx, dy, dz) from its
 // own: the entries whose FP32 distance passes the widened cut-off, appended
@@ -319,6 +320,56 @@ __device__ __forceinline__ void bin_candidates(const StepParams &P, int i, bool 
   }
 }
 
+// bin_candidates (FAST) over all 27 bins with LANES lanes per atom: lane g
+// takes bins g, g + LANES, ... of the stencil and the lanes append to the
+// atom's one list.  Every lane of the warp calls it.
+template <int LANES, bool SKIP = false, class Set>
+__device__ __forceinline__ void shared_candidates(const StepParams &P, int i, bool active, int4 Bi, float4 oi,
+                                                  const int *__restrict__ bin_count,
+                                                  const BinEntry *__restrict__ bins, unsigned *__restrict__ err,
+                                                  int &nc, int cap, Set cset, float r2band,
+                                                  const int *__restrict__ skip = nullptr, float r2lo = -1.f) {
+  const int g = (int)threadIdx.x & (LANES - 1);
+  for (int m = 0; m < (27 + LANES - 1) / LANES; ++m) {
+    const int b = g + m * LANES;
+    const bool look = active && b < 27;
+    const int bb = b < 27 ? b : 13, dx = bb % 3 - 1, dy = (bb / 3) % 3 - 1, dz = bb / 9 - 1;
+    const int Tz = Bi.z + dz, tz = Tz < 0 ? Tz + P.nb[2] : (Tz >= P.nb[2] ? Tz - P.nb[2] : Tz);
+    const int Ty = Bi.y + dy, ty = Ty < 0 ? Ty + P.nb[1] : (Ty >= P.nb[1] ? Ty - P.nb[1] : Ty);
+    const int Tx = Bi.x + dx, tx = Tx < 0 ? Tx + P.nb[0] : (Tx >= P.nb[0] ? Tx - P.nb[0] : Tx);
+    const int kz = Tz < 0 ? -1 : (Tz >= P.nb[2] ? 1 : 0), ky = Ty < 0 ? -1 : (Ty >= P.nb[1] ? 1 : 0),
+              kx = Tx < 0 ? -1 : (Tx >= P.nb[0] ? 1 : 0);
+    const float bx = (float)dx * P.wf[0] - oi.x, by = (float)dy * P.wf[1] - oi.y, bz = (float)dz * P.wf[2] - oi.z;
+    const int flat = tx + P.nb[0] * (ty + P.nb[1] * tz);
+    int cnt = 0;
+    if (look) {
+      cnt = bin_count[flat];
+      cnt = cnt < P.bcap ? cnt : P.bcap;
+    }
+    const int cmax = __reduce_max_sync(0xffffffffu, cnt);
+    const BinEntry *be = bins + (size_t)flat * P.bcap;
+    for (int s = 0; s < cmax; ++s) {
+      bool take = false;
+      unsigned u = 0;
+      if (s < cnt) {
+        const BinEntry e = be[s];
+        const unsigned j = e.idx & IDX_MASK;
+        const float ex = bx + e.ox, ey = by + e.oy, ez = bz + e.oz;
+        const float r2 = ex * ex + ey * ey + ez * ez;
+        if (j != (unsigned)i && r2 < r2band && r2 >= r2lo && !(SKIP && (skip[j] & 2))) {
+          const unsigned wc = e.idx >> IDX_BITS;
+          const int mx = kx - ((int)(wc % 3u) - 1), my = ky - ((int)((wc / 3u) % 3u) - 1),
+                    mz = kz - ((int)(wc / 9u) - 1);
+          take = mx >= -1 && mx <= 1 && my >= -1 && my <= 1 && mz >= -1 && mz <= 1;
+          if (!take) atomicOr(err, ERR_DRIFT);
+          u = j | ((unsigned)((mx + 1) + 3 * (my + 1) + 9 * (mz + 1)) << IDX_BITS);
+        }
+      }
+      append_candidate<LANES>(take, u, nc, cap, cset, err);
+    }
+  }
+}
+
 // Pass 1 of the density sweep for atom i: the candidates of the 27 bins
 // around its own within the FP32 thresholds r2lo <= r^2 < r2band, appended
 // after the first nc0 (at most cap in all).  Returns their number.
@@ -339,43 +390,34 @@ __device__ __forceinline__ int collect_candidates(const StepParams &P, int i, bo
 }
 
 // Pass 1 from the standalone engine's EAM pair list of this step
-// (k_eam_density's rows: the same bins, the same stencil order, every pair
-// within the EAM cut-off, which exceeds r2band): its entries within the
-// FP32 threshold r2band, tested with bin_candidates' arithmetic on the
-// neighbours' bins and offsets -- the candidates of the bin search, in its
-// order, without scanning the bins.  Returns their number.
-template <class Set>
-__device__ __forceinline__ int list_candidates(const StepParams &P, int i, bool active, int4 Bi, float4 oi,
-                                               const unsigned *__restrict__ elist, const int *__restrict__ ens,
-                                               const int4 *__restrict__ atom_bin, const float4 *__restrict__ atom_off,
-                                               unsigned *__restrict__ err, Set cset, float r2band, int cap) {
-  int nc = 0;
+// (k_eam_density's rows: every pair within the EAM cut-off, which exceeds
+// r2band): its entries within the FP32 threshold r2band, from the high words
+// of the fixed-point positions -- the candidates of the bin search, without
+// scanning the bins.  Lane g of the atom's LANES takes entries g, g + LANES,
+// ....
+template <int LANES, class Set>
+__device__ __forceinline__ void list_candidates(const StepParams &P, int i, bool active, const long long *xi,
+                                                const unsigned *__restrict__ elist, const int *__restrict__ ens,
+                                                const int4 *__restrict__ rec, unsigned *__restrict__ err, int &nc,
+                                                int cap, Set cset, float r2band) {
+  const int g = (int)threadIdx.x & (LANES - 1);
   const int ne = active ? ens[i] : 0;
   const int nmax = __reduce_max_sync(0xffffffffu, ne);
-  for (int k = 0; k < nmax; ++k) {
-    if (k >= ne) continue;
-    const unsigned u = elist[(size_t)k * P.n + i];
-    const unsigned j = u & IDX_MASK, code = u >> IDX_BITS;
-    const int4 Bj = atom_bin[j];
-    const float4 oj = atom_off[j];
-    // the stencil cell of the pair: j's (unwrapped) bin moved by its image
-    const int dx = Bj.x + ((int)(code % 3u) - 1) * P.nb[0] - Bi.x;
-    const int dy = Bj.y + ((int)((code / 3u) % 3u) - 1) * P.nb[1] - Bi.y;
-    const int dz = Bj.z + ((int)(code / 9u) - 1) * P.nb[2] - Bi.z;
-    if (dx < -1 || dx > 1 || dy < -1 || dy > 1 || dz < -1 || dz > 1) {
-      atomicOr(err, ERR_DRIFT);
-      continue;
+  for (int k = g; k - g < nmax; k += LANES) {
+    bool take = false;
+    unsigned u = 0;
+    if (k < ne) {
+      u = elist[(size_t)k * P.n + i];
+      long long e[3];
+      int4 ra, rb;
+      load_record(rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
+      pair_fixed(P, ra, rb, u >> IDX_BITS, xi, e);
+      const float ex = (float)(int)(e[0] >> 32) * P.fix_hi, ey = (float)(int)(e[1] >> 32) * P.fix_hi,
+                  ez = (float)(int)(e[2] >> 32) * P.fix_hi;
+      take = ex * ex + ey * ey + ez * ez < r2band;
     }
-    const float bx = (float)dx * P.wf[0] - oi.x, by = (float)dy * P.wf[1] - oi.y, bz = (float)dz * P.wf[2] - oi.z;
-    const float ex = bx + oj.x, ey = by + oj.y, ez = bz + oj.z;
-    if (ex * ex + ey * ey + ez * ez < r2band) {
-      if (nc >= cap)
-        atomicOr(err, ERR_PAIR_OVERFLOW);
-      else
-        cset(nc++, u);
-    }
+    append_candidate<LANES>(take, u, nc, cap, cset, err);
   }
-  return nc;
 }
 
 // The same sort with one warp per bin, for bins of at most 64 entries: lane l
@@ -497,8 +539,8 @@ __device__ __forceinline__ void density_vector(const StepParams &P, const D4 &xi
 // The end of the density sweep for atom i (its pairs summed): alpha, beta,
 // the deviates, its grid cell and T_e, and the per-atom records.
 // With DFG (the df64 force sweep follows) the gathered records go to G as
-// double-floats, three float4 per atom: {W hi, X_x hi}, {W lo, X_x lo},
-// {X_y hi, X_z hi, X_y lo, X_z lo} (W = a_i w_i, X = a_i xi_i); an atom the
+// double-floats, 64 B per atom of which 48 are used: {W hi, X_x hi}, {W lo,
+// X_x lo}, {X_y hi, X_z hi, X_y lo, X_z lo} (W = a_i w_i, X = a_i xi_i); an atom the
 // reference skips as a neighbour (rho <= 0 or outside the group) is marked
 // by a NaN in its first word.
 template <bool FAST, bool FUSE_W, bool DFG = false>
@@ -559,7 +601,7 @@ __device__ __forceinline__ void density_epilogue(
       const df64::df X[3] = {df64::from_double(alpha * xi3[0]), df64::from_double(alpha * xi3[1]),
                              df64::from_double(alpha * xi3[2])};
       const bool live = active && pos_double(rho);
-      float4 *g = reinterpret_cast<float4 *>(G) + 3 * (size_t)i;
+      float4 *g = reinterpret_cast<float4 *>(G) + 4 * (size_t)i;
       g[0] = make_float4(live ? W[0].hi : __int_as_float(0x7fc00000), W[1].hi, W[2].hi, X[0].hi);
       g[1] = make_float4(W[0].lo, W[1].lo, W[2].lo, X[0].lo);
       g[2] = make_float4(X[1].hi, X[2].hi, X[1].lo, X[2].lo);
@@ -667,161 +709,14 @@ __global__ void __launch_bounds__(128) k_density(
 
 // resident blocks of 128 threads per SM the df64 sweeps are compiled for
 // (their register budget: 65,536 / (128 x blocks)); measured on GB300 at
-// 2,048,000 atoms: density 6 and 7 alike, 8 spills and is 17 % slower;
-// forces 6 / 7 / 8: 1.51 / 1.36 / 1.50 ms
+// 2,048,000 atoms: density 6 / 7 / 8 blocks 1.44 / 1.36 / 1.69 ms (8 spills),
+// forces 7 / 8 / 9 blocks 0.84 / 0.84 / 0.89 ms (9 spills)
 #ifndef EPH_DF_DENSITY_BLOCKS
-#define EPH_DF_DENSITY_BLOCKS 6
+#define EPH_DF_DENSITY_BLOCKS 7
 #endif
 #ifndef EPH_DF_FORCES_BLOCKS
-#define EPH_DF_FORCES_BLOCKS 7
+#define EPH_DF_FORCES_BLOCKS 8
 #endif
-// candidates per iteration of the df64 density sweep's pass 2 (measured on
-// GB300 at 2,048,000 atoms: 1 -> 3.89 ms, 2 -> 3.91 ms; the sweep waits on
-// the neighbours' records and its pair-cache writes more than on its chains)
-#ifndef DF_UNROLL
-#define DF_UNROLL 1
-#endif
-
-// The FAST density sweep of k_density<true, MULTI, true> (one lane per atom,
-// stage 1 and M_i folded) with every per-pair operation in df64 on the FP32
-// pipe: pass 1 is k_density's; pass 2 forms e = d w + (o_j - o_i) from the
-// atoms' bin offsets (k_bin's records, 48 significant bits), r^2, the exact
-// cut-off test, rho_j(r^2) (spline_rho_df), H = rho_j(r^2) / r^2 (a df64
-// Newton reciprocal), H e, and the sums of M_i and S_i (blocked df64 sums,
-// folded every 8 candidates); the epilogue is k_density's in FP64 and writes
-// the records G for k_forces_df.  Pair cache (row k of atom i at k*n + i):
-// pa = {e hi, (H e)_x hi | H_ji hi}, pb = the lo parts, pc = {(H e)_y, (H e)_z}
-// hi, hi, lo, lo with one element, {H_ij hi, H_ij lo} with several.
-template <bool MULTI>
-__global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(
-    StepParams P, const int *__restrict__ mask, const int *__restrict__ bin_count, const BinEntry *__restrict__ bins,
-    const int4 *__restrict__ atom_bin, const float4 *__restrict__ atom_off, const float4 *__restrict__ rec,
-    const float4 *__restrict__ vrec, const D4 *__restrict__ x, const D4 *__restrict__ xi_given, int xi_mode,
-    const double *__restrict__ T_e, unsigned *__restrict__ pj, float4 *__restrict__ pa, float4 *__restrict__ pb,
-    float4 *__restrict__ pc, int *__restrict__ nshort, D4 *__restrict__ A, D4 *__restrict__ Bw,
-    double *__restrict__ rho_out, double *__restrict__ beta_out, int *__restrict__ cell, double *__restrict__ Te_i,
-    int *__restrict__ wrapflag, unsigned *__restrict__ err, unsigned long long *__restrict__ counters,
-    const D4 *__restrict__ v, D4 *__restrict__ Mm, D4 *__restrict__ G, const unsigned *__restrict__ elist = nullptr,
-    const int *__restrict__ ens = nullptr) {
-  using namespace df64;
-  __shared__ unsigned s_cand[CAND_SMEM * 128];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t = threadIdx.x, nt = blockDim.x;
-  if (i == 0) *wrapflag = 0;  // the binning kernel has read it
-  const bool valid = i < P.n;
-  const bool active = valid && (mask[i] & P.groupbit) != 0;
-  auto cget = [&](int k) -> unsigned { return k < CAND_SMEM ? s_cand[k * nt + t] : pj[(size_t)k * P.n + i]; };
-  auto cset = [&](int k, unsigned u) {
-    if (k < CAND_SMEM)
-      s_cand[k * nt + t] = u;
-    else
-      pj[(size_t)k * P.n + i] = u;
-  };
-  int4 Bi = make_int4(0, 0, 0, 0);
-  float4 oi = make_float4(0.f, 0.f, 0.f, 0.f), Ri1 = make_float4(0.f, 0.f, 0.f, 0.f);
-  int ns = 0, nc = 0;
-  if (valid) {
-    Bi = atom_bin[i];
-    oi = rec[2 * (size_t)i];
-    Ri1 = rec[2 * (size_t)i + 1];
-  }
-  const int ei = __float_as_int(Ri1.w);
-  // pass 1: candidates, FP32/integer work only, warp-uniform loop bounds;
-  // from the EAM pair list when the standalone engine made one this step
-  {
-    float4 of = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (active) of = atom_off[i];
-    if (elist)
-      nc = list_candidates(P, i, active, Bi, of, elist, ens, atom_bin, atom_off, err, cset, P.rc2_band, P.kcap);
-    else
-      nc = collect_candidates<true>(P, i, active, Bi, of, bin_count, bins, err, cget, cset, P.rc2_band, P.kcap);
-  }
-  __syncwarp();
-  // pass 2 in df64: M_i (xx, xy, xz, yy, yz, zz) and S_i (x, y, z), DF_UNROLL
-  // candidates per iteration with no branch around their arithmetic: a
-  // candidate outside the cut-off (or past the lane's list) is evaluated at
-  // r^2 = 1 with H forced to 0, so its terms add exact zeros and it writes no
-  // pair.
-  bsum sm[9];
-#pragma unroll
-  for (int q = 0; q < 9; ++q) sm[q] = bsum_zero();
-  const df rc2{P.rc2_hi, P.rc2_lo};
-  const int nmax = __reduce_max_sync(0xffffffffu, nc);
-  for (int k = 0; k < nmax; k += DF_UNROLL) {
-    unsigned uu[DF_UNROLL];
-    df ex[DF_UNROLL], ey[DF_UNROLL], ez[DF_UNROLL], r2[DF_UNROLL];
-    int ej[DF_UNROLL];
-    bool in[DF_UNROLL];
-#pragma unroll
-    for (int c = 0; c < DF_UNROLL; ++c) {
-      const bool have = k + c < nc;
-      const unsigned u = have ? cget(k + c) : 0u;
-      const unsigned j = u & IDX_MASK, code = have ? u >> IDX_BITS : CODE_NOSHIFT;
-      const float4 R0 = rec[2 * (size_t)j], R1 = rec[2 * (size_t)j + 1];
-      const unsigned pk = __float_as_uint(R0.w);
-      // bin difference of the pair: j's bin + its periodic image - i's bin
-      const int dx = (int)(pk & 1023u) - 1 + ((int)(code % 3u) - 1) * P.nb[0] - Bi.x;
-      const int dy = (int)((pk >> 10) & 1023u) - 1 + ((int)((code / 3u) % 3u) - 1) * P.nb[1] - Bi.y;
-      const int dz = (int)((pk >> 20) & 1023u) - 1 + ((int)(code / 9u) - 1) * P.nb[2] - Bi.z;
-      ex[c] = pair_disp(dx, R0.x, R1.x, oi.x, Ri1.x, P.w_hi[0], P.w_lo[0]);
-      ey[c] = pair_disp(dy, R0.y, R1.y, oi.y, Ri1.y, P.w_hi[1], P.w_lo[1]);
-      ez[c] = pair_disp(dz, R0.z, R1.z, oi.z, Ri1.z, P.w_hi[2], P.w_lo[2]);
-      r2[c] = dot3(ex[c], ey[c], ez[c], ex[c], ey[c], ez[c]);
-      in[c] = have && lt(r2[c], rc2);
-      if (!in[c]) r2[c] = df{1.0f, 0.0f};
-      ej[c] = __float_as_int(R1.w);
-      uu[c] = u;
-    }
-#pragma unroll
-    for (int c = 0; c < DF_UNROLL; ++c) {
-      const df rji = spline_rho_df(P, ej[c], r2[c], err);
-      const df inv = recip(r2[c], rcp_estimate(r2[c].hi));
-      df H = mul(rji, inv);
-      if (!in[c]) H = df{0.0f, 0.0f};
-      const df hx = mul(H, ex[c]), hy = mul(H, ey[c]), hz = mul(H, ez[c]);
-      if (in[c]) {
-        const size_t slot = (size_t)ns * P.n + i;
-        pj[slot] = uu[c];
-        if (MULTI) {
-          const df rij = ej[c] != ei ? spline_rho_df(P, ei, r2[c], err) : rji;
-          const df Hji = mul(rij, inv);
-          pa[slot] = make_float4(ex[c].hi, ey[c].hi, ez[c].hi, Hji.hi);
-          pb[slot] = make_float4(ex[c].lo, ey[c].lo, ez[c].lo, Hji.lo);
-          pc[slot] = make_float4(H.hi, H.lo, 0.f, 0.f);
-        } else {
-          pa[slot] = make_float4(ex[c].hi, ey[c].hi, ez[c].hi, hx.hi);
-          pb[slot] = make_float4(ex[c].lo, ey[c].lo, ez[c].lo, hx.lo);
-          pc[slot] = make_float4(hy.hi, hz.hi, hy.lo, hz.lo);
-        }
-        ++ns;
-      }
-      acc_fma(sm[0].blk, hx, ex[c]);
-      acc_fma(sm[1].blk, hx, ey[c]);
-      acc_fma(sm[2].blk, hx, ez[c]);
-      acc_fma(sm[3].blk, hy, ey[c]);
-      acc_fma(sm[4].blk, hy, ez[c]);
-      acc_fma(sm[5].blk, hz, ez[c]);
-      const unsigned j = uu[c] & IDX_MASK;
-      const float4 V0 = vrec[2 * (size_t)j], V1 = vrec[2 * (size_t)j + 1];
-      const df d = dot3(ex[c], ey[c], ez[c], df{V0.x, V1.x}, df{V0.y, V1.y}, df{V0.z, V1.z});
-      acc_fma(sm[6].blk, d, hx);
-      acc_fma(sm[7].blk, d, hy);
-      acc_fma(sm[8].blk, d, hz);
-    }
-    if ((k & 7) == 8 - DF_UNROLL) {
-#pragma unroll
-      for (int q = 0; q < 9; ++q) bsum_fold(sm[q]);
-    }
-  }
-  if (!valid) return;
-  double mq[9];
-#pragma unroll
-  for (int q = 0; q < 9; ++q) mq[q] = to_double(bsum_value(sm[q]));
-  const D4 xi = x[i];
-  density_epilogue<true, true, true>(P, i, active, xi, ei, 0.0, ns, mq[0], mq[1], mq[2], mq[3], mq[4], mq[5], mq[6],
-                                     mq[7], mq[8], xi_given, xi_mode, T_e, nshort, A, Bw, rho_out, beta_out, cell,
-                                     Te_i, err, counters, v, Mm, G);
-}
 
 // The FAST density sweep with TPA lanes per atom (TPA = 2, 4, 8) for small
 // systems, where one lane per atom leaves the SMs a few warps each and the
@@ -957,6 +852,9 @@ __device__ __forceinline__ double min_image(double d, double L, double h) {
   return d > h ? d - L : (d < -h ? d + L : d);
 }
 
+// the boxes min_image adds to d
+__device__ __forceinline__ int image_count(double d, double h) { return d > h ? -1 : (d < -h ? 1 : 0); }
+
 // The 3x3x3 image code of x_j seen from x_i: the image of x_j within half a
 // box of x_i on every axis, decided in FP32 (the box is at least three list
 // radii wide, so a pair within the list radius is far from the threshold).
@@ -971,15 +869,18 @@ __device__ __forceinline__ unsigned image_code(const StepParams &P, float xi, fl
 }
 
 // The bin and FP32 offset of a position wrapped into the box (an atom whose
-// bins entry is stale: it moved since the build)
-__device__ __forceinline__ void current_bin(const StepParams &P, const D4 &xi, int4 &B, float4 &o) {
+// bins entry is stale: it moved since the build), and by how many boxes
+__device__ __forceinline__ void current_bin(const StepParams &P, const D4 &xi, int4 &B, float4 &o,
+                                            int *image = nullptr) {
   const double p[3] = {xi.x, xi.y, xi.z};
   int b[3];
   float of[3];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     double q = p[k] - P.lo[k];
-    q -= floor(q / P.prd[k]) * P.prd[k];
+    const double turns = floor(q / P.prd[k]);
+    q -= turns * P.prd[k];
+    if (image) image[k] = -(int)turns - (q >= P.prd[k] ? 1 : 0);  // boxes added to p
     if (q >= P.prd[k]) q -= P.prd[k];
     if (q < 0.0) q = 0.0;
     int bb = (int)floor(q * P.inv_w[k]);
@@ -994,13 +895,13 @@ __device__ __forceinline__ void current_bin(const StepParams &P, const D4 &xi, i
 // First kernel of a step with list reuse: the engine's wrap (as k_bin does
 // it), then each atom's displacement since the list build; moved atoms get
 // state 2 and join the list of moved atoms (state 0 otherwise).  With rec
-// (the df64 density sweep), also every atom's records for it from its
-// current position, in the bins of the current geometry (df_records).
+// (the df64 density sweep), also every atom's record for it: its position
+// continued from the build (the image next to xref, so the image codes of the
+// lists' entries stay what they were) and whether it moved.
 __global__ void k_list_check(StepParams P, D4 *__restrict__ x, D4 *__restrict__ xhold,
                              const int *__restrict__ wrapflag, const D4 *__restrict__ xref, int *__restrict__ state,
                              int *__restrict__ rb, int *__restrict__ flist, unsigned long long *__restrict__ counters,
-                             float4 *__restrict__ rec = nullptr, float4 *__restrict__ vrec = nullptr,
-                             const D4 *__restrict__ v = nullptr) {
+                             int4 *__restrict__ rec = nullptr, const D4 *__restrict__ v = nullptr) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *P.step += 1ull;  // read by the density sweep that follows
   bool moved = false;
@@ -1012,22 +913,18 @@ __global__ void k_list_check(StepParams P, D4 *__restrict__ x, D4 *__restrict__ 
       xhold[i] = xi;
       if (i == 0) atomicAdd(&counters[CNT_WRAP], 1ull);
     }
-    if (rec) {
-      const double p[3] = {xi.x, xi.y, xi.z};
-      int B[3];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const int b = (int)floor((p[k] - P.lo[k]) * P.inv_w[k]);
-        B[k] = b < -1 ? -1 : (b > P.nb[k] ? P.nb[k] : b);
-      }
-      df_records(P, i, xi, B, v, rec, vrec);
-    }
     const D4 r = xref[i];
-    const double dx = min_image(xi.x - r.x, P.prd[0], P.half_prd[0]);
-    const double dy = min_image(xi.y - r.y, P.prd[1], P.half_prd[1]);
-    const double dz = min_image(xi.z - r.z, P.prd[2], P.half_prd[2]);
-    moved = dx * dx + dy * dy + dz * dz >= P.lslow2;
+    const double d0[3] = {xi.x - r.x, xi.y - r.y, xi.z - r.z};
+    int m[3];
+    double d[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      m[k] = image_count(d0[k], P.half_prd[k]);
+      d[k] = m[k] < 0 ? d0[k] - P.prd[k] : (m[k] > 0 ? d0[k] + P.prd[k] : d0[k]);
+    }
+    moved = d[0] * d[0] + d[1] * d[1] + d[2] * d[2] >= P.lslow2;
     state[i] = moved ? 2 : 0;
+    if (rec) df_record(P, i, xi, m, moved, v[i], rec);
   }
   // one atomic per warp (after a long run without a build most atoms move)
   const unsigned mv = __ballot_sync(0xffffffffu, moved);
@@ -1237,195 +1134,350 @@ __global__ void __maxnreg__(64) k_density_list(
                                xi_mode, T_e, nshort, A, Bw, rho_out, beta_out, cell, Te_i, err, counters, v, Mm, G);
 }
 
-// k_density_list with k_density_df's pass 2: the candidates come from the
-// kept lists as there (build steps search the bins, atoms flagged near moved
-// ones search afresh), then every pair term and sum in df64 from the records
-// k_list_check wrote this step (bins of the current positions); the periodic
-// image of a candidate comes from FP32 positions rebuilt from those records
-// (B w + o, good to ~1e-6 of the box: the image test has a margin of
-// tens of angstroms).
-template <bool MULTI>
-__global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_list_df(
-    StepParams P, const D4 *__restrict__ x, const int *__restrict__ mask, const int *__restrict__ bin_count,
-    const BinEntry *__restrict__ bins, const int4 *__restrict__ atom_bin, const float4 *__restrict__ atom_off,
-    const float4 *__restrict__ rec, const float4 *__restrict__ vrec, const D4 *__restrict__ xi_given, int xi_mode,
-    const double *__restrict__ T_e, unsigned *__restrict__ pj, float4 *__restrict__ pa, float4 *__restrict__ pb,
-    float4 *__restrict__ pc, int *__restrict__ nshort, D4 *__restrict__ A, D4 *__restrict__ Bw,
-    double *__restrict__ rho_out, double *__restrict__ beta_out, int *__restrict__ cell, double *__restrict__ Te_i,
-    int *__restrict__ wrapflag, unsigned *__restrict__ err, unsigned long long *__restrict__ counters,
-    const D4 *__restrict__ v, D4 *__restrict__ Mm, D4 *__restrict__ G, unsigned *__restrict__ cl,
-    int *__restrict__ cl_n, const int *__restrict__ state, const int *__restrict__ rb,
-    const int *__restrict__ flist) {
+// ------------------------------------------- FAST density sweep in df64
+//
+// calculate_environment (fix_eph.cpp:431-466), stage 1 and M_i in one pass
+// (the FAST density sweep of k_density<true, MULTI, true>) with every
+// per-pair operation in df64 on the FP32 pipe and LANES lanes per atom.
+//   pass 1 gathers the atom's candidates into shared memory (its lanes share
+//     one list): DF_BINS searches the 27 bins of the step, DF_EAM takes them
+//     from the EAM engine's pair list, DF_LIST keeps lists (build steps search
+//     the bins within r_cutoff + s and write them; atoms flagged by
+//     k_list_check / k_list_mark search the bins of the build afresh, leave
+//     moved atoms' entries out and add the moved atoms);
+//   pass 2 forms e from the fixed-point positions (pair_fixed, fixed_df), r^2,
+//     the cut-off test, rho_j(r^2) (spline_rho_df), H = rho_j(r^2) / r^2 and the
+//     sums of M_i and S_i (blocked df64 sums: 8 products, then a Dekker
+//     addition into the totals in shared memory), lane g taking candidates g,
+//     g + LANES, ...; a candidate outside the cut-off is evaluated at r^2 = 1
+//     with H forced to 0, so its terms add exact zeros and it writes no pair;
+//   the epilogue (density_epilogue, FP64) runs on one thread per atom in the
+//     block's first warps, whatever LANES is.
+// Pair cache (row k of atom i at k*n + i): pj = neighbour | image code << 27,
+// pe = {e hi, H_ji hi}, {the lo parts} (H_ji = rho_i(r^2) / r^2, the weight
+// of the neighbour's term in the force sweep): 36 B per pair.  H e, which the
+// cache used to hold too (52 B), costs the force sweep two multiplications.
+//
+// What bounds it on GB300, in the order it was taken away (2,048,000 atoms,
+// kept lists, ms per launch): 1.98 at the start, with the L1 at 68 % of its
+// wavefront rate (every 16-byte load of a scattered record touches a line per
+// lane), 500 instructions per candidate and little L1 left beside the
+// candidates in shared memory.  Fixed-point positions whose image the list
+// keeps (no bins to unpack, no image test) and 36 B instead of 52 B per cached
+// pair: 420 instructions, but 2.03 until the loads changed; 256-bit loads of
+// record halves and table rows: 1.84; lists read from global memory two
+// candidates ahead, so that the L1 keeps the table and records: 1.47; the
+// division-free grid cell: 1.44; 7 blocks per SM, which the totals' place in
+// shared memory allows: 1.36.  Now the issue slots, the L1 and (in the
+// epilogues) the FP64 pipe are each 60-65 % busy.  Cooperative asynchronous
+// copies of whole records to shared memory took 1.69 and were not kept.
+enum : int { DF_BINS = 0, DF_LIST = 1, DF_EAM = 2 };
+
+// what the sweep reads and writes besides the step constants
+struct DensityArgs {
+  const int *mask, *bin_count;
+  const BinEntry *bins;
+  const int4 *atom_bin;
+  const float4 *atom_off;
+  const int4 *rec;
+  const D4 *x, *v, *xi_given;
+  int xi_mode;
+  const double *T_e;
+  unsigned *pj;
+  float4 *pe;
+  int *nshort;
+  D4 *A, *Bw;
+  double *rho, *beta;
+  int *cell;
+  double *Te_i;
+  int *wrapflag;
+  unsigned *err;
+  unsigned long long *counters;
+  D4 *Mm, *G;
+  // DF_LIST
+  unsigned *cl;
+  int *cl_n;
+  const int *state, *rb, *flist;
+  const D4 *xref;
+  // DF_EAM
+  const unsigned *elist;
+  const int *ens;
+};
+
+template <bool MULTI, int LANES, int SRC>
+__global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepParams P, DensityArgs D) {
   using namespace df64;
-  __shared__ unsigned s_cand[CAND_SMEM * 128];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t = threadIdx.x, nt = blockDim.x;
-  if (i == 0) *wrapflag = 0;  // k_list_check has read it
+  constexpr int NA = 128 / LANES;                    // atoms per block
+  // The bin search keeps its candidates in shared memory: candidate k of atom
+  // a at k * 128 + t with one lane per atom, else in the atom's own run of an
+  // odd length (its lanes read neighbouring words).  Lists are read row by
+  // row from global memory, two candidates ahead: what shared memory they
+  // would take is L1 that the spline table and the records need.
+  constexpr int CAP = SRC != DF_BINS ? 0 : (LANES == 1 ? CAND_SMEM : CAND_SMEM * LANES - 1);
+  __shared__ unsigned s_cand[CAP ? CAND_SMEM * 128 : 1];
+  __shared__ float2 s_tot[9 * 128];
+  const int t = threadIdx.x, a = t / LANES, g = t % LANES;
+  const int i = blockIdx.x * NA + a;
+  if (i == 0 && g == 0) *D.wrapflag = 0;  // the kernels before have read it
   const bool valid = i < P.n;
-  const bool active = valid && (mask[i] & P.groupbit) != 0;
+  const bool active = valid && (D.mask[i] & P.groupbit) != 0;
   const size_t n = (size_t)P.n;
-  auto sget = [&](int k) -> unsigned { return k < CAND_SMEM ? s_cand[k * nt + t] : pj[(size_t)k * n + i]; };
-  auto sset = [&](int k, unsigned u) {
-    if (k < CAND_SMEM)
-      s_cand[k * nt + t] = u;
-    else
-      pj[(size_t)k * n + i] = u;
+  auto at = [&](int k) -> unsigned & { return s_cand[LANES == 1 ? k * 128 + t : a * CAP + k]; };
+  unsigned *__restrict__ pj = D.pj;
+  // candidates past the shared rows: the atom's rows of pj (their slots are
+  // written only after the candidates there are read) or, for a kept list,
+  // the list itself
+  auto set = [&](int k, unsigned u) {
+    if (k < CAP) at(k) = u;
+    else pj[(size_t)k * n + i] = u;
   };
-  auto lset = [&](int k, unsigned u) {
-    if (k < CAND_SMEM) s_cand[k * nt + t] = u;
-    cl[(size_t)k * n + i] = u;
-  };
-  auto lget = [&](int k) -> unsigned { return cl[(size_t)k * n + i]; };
-  D4 xi = D4{0.0, 0.0, 0.0, 0.0};
-  if (valid) xi = x[i];
-  const bool build = rb[2] != 0;
+#pragma unroll
+  for (int q = 0; q < 9; ++q) s_tot[q * 128 + t] = make_float2(0.f, 0.f);
+  long long xi[3] = {0, 0, 0};
+  int ei = 0;
+  if (valid) {
+    int4 ra, rb;
+    load_record(D.rec + 4 * (size_t)i, ra, rb);
+    xi[0] = ((long long)ra.y << 32) | (unsigned)ra.x;
+    xi[1] = ((long long)ra.w << 32) | (unsigned)ra.z;
+    xi[2] = ((long long)rb.y << 32) | (unsigned)rb.x;
+    ei = rb.z;
+  }
   int nc = 0;
-  bool fresh = false;
-  if (build) {
+  bool fresh = true;  // the candidates are of this step's positions
+  const unsigned *tail = pj;
+  if (SRC == DF_LIST) {
+    const bool build = D.rb[2] != 0;
+    if (build) {
+      int4 Bi = make_int4(0, 0, 0, 0);
+      float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (active) {
+        Bi = D.atom_bin[i];
+        oi = D.atom_off[i];
+      }
+      auto lset = [&](int k, unsigned u) {
+        if (k < CAP) at(k) = u;
+        D.cl[(size_t)k * n + i] = u;
+      };
+      // the candidates inside the cut-off first, the shell out to r_list after
+      // them: the shell's pairs mostly fail the exact test, and at the end of
+      // the lists whole warps skip them
+      if (LANES == 1) {
+        auto lget = [&](int k) -> unsigned { return D.cl[(size_t)k * n + i]; };
+        nc = collect_candidates<true>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, lget, lset, P.rc2_band, P.lcap);
+        nc = collect_candidates<true>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, lget, lset, P.rl2_band, P.lcap,
+                                      nullptr, P.rc2_band, nc);
+      } else {
+        shared_candidates<LANES>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, nc, P.lcap, lset, P.rc2_band);
+        shared_candidates<LANES>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, nc, P.lcap, lset, P.rl2_band,
+                                 nullptr, P.rc2_band);
+      }
+      tail = D.cl;
+      if (valid && g == 0) D.cl_n[i] = nc;
+    } else {
+      const int st = active ? D.state[i] : 0;
+      fresh = st != 0;
+      if (__any_sync(0xffffffffu, fresh)) {
+        int4 Bi = make_int4(0, 0, 0, 0);
+        float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
+        double base[3] = {0.0, 0.0, 0.0};  // the position the image codes below refer to
+        if (fresh) {
+          const D4 x = D.x[i];
+          if (st & 2) {  // a moved atom: from its wrapped position, not continued from the build
+            int image[3];
+            current_bin(P, x, Bi, oi, image);
+            const double p[3] = {x.x, x.y, x.z};
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+              base[k] = p[k] + image[k] * P.prd[k];
+              xi[k] = to_fixed_coord(p[k], P.fix_q) + (long long)image[k] * P.fix_prd[k];
+            }
+          } else {
+            Bi = D.atom_bin[i];
+            oi = D.atom_off[i];
+            const D4 r = D.xref[i];
+            base[0] = r.x + min_image(x.x - r.x, P.prd[0], P.half_prd[0]);
+            base[1] = r.y + min_image(x.y - r.y, P.prd[1], P.half_prd[1]);
+            base[2] = r.z + min_image(x.z - r.z, P.prd[2], P.half_prd[2]);
+          }
+        }
+        if (LANES == 1) {
+          auto get = [&](int k) -> unsigned { return k < CAP ? at(k) : pj[(size_t)k * n + i]; };
+          nc = collect_candidates<true, true>(P, i, fresh, Bi, oi, D.bin_count, D.bins, D.err, get, set, P.rl2_band,
+                                              P.kcap, D.state);
+        } else {
+          shared_candidates<LANES, true>(P, i, fresh, Bi, oi, D.bin_count, D.bins, D.err, nc, P.kcap, set, P.rl2_band,
+                                         D.state);
+        }
+        // the moved atoms near enough (a widened test; pass 2 decides), their
+        // image next to the position above
+        const int nf = D.rb[1];  // <= LIST_FMAX on a step without a build
+        for (int q = 0; q < nf; ++q) {
+          const int f = D.flist[q];
+          bool take = false;
+          unsigned u = 0;
+          if (fresh && f != i && g == 0) {
+            const D4 xf = D.x[f], r = D.xref[f];
+            const double d[3] = {r.x + min_image(xf.x - r.x, P.prd[0], P.half_prd[0]) - base[0],
+                                 r.y + min_image(xf.y - r.y, P.prd[1], P.half_prd[1]) - base[1],
+                                 r.z + min_image(xf.z - r.z, P.prd[2], P.half_prd[2]) - base[2]};
+            double r2 = 0.0;
+            unsigned code = 0, place = 1;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+              const int m = image_count(d[k], P.half_prd[k]);
+              const double c = min_image(d[k], P.prd[k], P.half_prd[k]);
+              r2 += c * c;
+              code += (unsigned)(m + 1) * place;
+              place *= 3u;
+            }
+            take = r2 < P.rc2 * (1.0 + 1e-4);
+            u = (unsigned)f | (code << IDX_BITS);
+          }
+          append_candidate<LANES>(take, u, nc, P.kcap, set, D.err);
+        }
+      }
+      if (!fresh) {
+        tail = D.cl;
+        nc = active ? D.cl_n[i] : 0;
+      }
+      if (!active) fresh = true;
+    }
+  } else if (SRC == DF_EAM) {
+    list_candidates<LANES>(P, i, active, xi, D.elist, D.ens, D.rec, D.err, nc, P.kcap, set, P.rc2_band);
+  } else {
     int4 Bi = make_int4(0, 0, 0, 0);
     float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
     if (active) {
-      Bi = atom_bin[i];
-      oi = atom_off[i];
+      Bi = D.atom_bin[i];
+      oi = D.atom_off[i];
     }
-    nc = collect_candidates<true>(P, i, active, Bi, oi, bin_count, bins, err, lget, lset, P.rc2_band, P.lcap);
-    nc = collect_candidates<true>(P, i, active, Bi, oi, bin_count, bins, err, lget, lset, P.rl2_band, P.lcap,
-                                  nullptr, P.rc2_band, nc);
-    if (valid) cl_n[i] = nc;
-  } else {
-    const int st = active ? state[i] : 0;
-    fresh = st != 0;
-    if (__any_sync(0xffffffffu, fresh)) {
-      int4 Bi = make_int4(0, 0, 0, 0);
-      float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (fresh) {
-        if (st & 2) {
-          current_bin(P, xi, Bi, oi);
-        } else {
-          Bi = atom_bin[i];
-          oi = atom_off[i];
-        }
-      }
-      nc = collect_candidates<true, true>(P, i, fresh, Bi, oi, bin_count, bins, err, sget, sset, P.rl2_band, P.kcap,
-                                          state);
-      const int nf = rb[1];  // <= LIST_FMAX on a step without a build
-      for (int q = 0; q < nf; ++q) {
-        const int f = flist[q];
-        if (fresh && f != i) {
-          const D4 xf = x[f];
-          const double dx = min_image(xf.x - xi.x, P.prd[0], P.half_prd[0]);
-          const double dy = min_image(xf.y - xi.y, P.prd[1], P.half_prd[1]);
-          const double dz = min_image(xf.z - xi.z, P.prd[2], P.half_prd[2]);
-          if (dx * dx + dy * dy + dz * dz < P.rc2 * (1.0 + 1e-4)) {
-            if (nc < P.kcap)
-              sset(nc++, (unsigned)f | (CODE_NOSHIFT << IDX_BITS));
-            else
-              atomicOr(err, ERR_PAIR_OVERFLOW);
-          }
-        }
-      }
-    }
-    if (active && !fresh) {
-      nc = cl_n[i];
-      const int nh = nc < CAND_SMEM ? nc : CAND_SMEM;
-#pragma unroll 8
-      for (int k = 0; k < nh; ++k) s_cand[k * nt + t] = __ldcs(cl + (size_t)k * n + i);  // read once a step
+    if (LANES == 1) {
+      auto get = [&](int k) -> unsigned { return k < CAP ? at(k) : pj[(size_t)k * n + i]; };
+      nc = collect_candidates<true>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, get, set, P.rc2_band, P.kcap);
+    } else {
+      shared_candidates<LANES>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, nc, P.kcap, set, P.rc2_band);
     }
   }
   __syncwarp();
-  const unsigned *__restrict__ tail = fresh ? pj : cl;
-  // atom i's records; its FP32 position B w + o for the image test
-  float4 oi = make_float4(0.f, 0.f, 0.f, 0.f), Ri1 = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (valid) {
-    oi = rec[2 * (size_t)i];
-    Ri1 = rec[2 * (size_t)i + 1];
-  }
-  const unsigned pki = __float_as_uint(oi.w);
-  const int bix = (int)(pki & 1023u) - 1, biy = (int)((pki >> 10) & 1023u) - 1, biz = (int)((pki >> 20) & 1023u) - 1;
-  const float pix = (float)bix * P.wf[0] + oi.x, piy = (float)biy * P.wf[1] + oi.y, piz = (float)biz * P.wf[2] + oi.z;
-  const int ei = __float_as_int(Ri1.w);
-  bsum sm[9];
+  // pass 2; the next candidate's position is loaded while this one is summed,
+  // each half of a record in one 256-bit load (load_row)
+  acc sm[9];
 #pragma unroll
-  for (int q = 0; q < 9; ++q) sm[q] = bsum_zero();
+  for (int q = 0; q < 9; ++q) sm[q] = acc_zero();
   const df rc2{P.rc2_hi, P.rc2_lo};
-  int ns = 0;
   const int nmax = __reduce_max_sync(0xffffffffu, nc);
-  for (int k = 0; k < nmax; ++k) {
-    const bool have = k < nc;
-    const unsigned j = have ? (k < CAND_SMEM ? s_cand[k * nt + t] : __ldcs(tail + (size_t)k * n + i)) & IDX_MASK : 0u;
-    const float4 R0 = rec[2 * (size_t)j], R1 = rec[2 * (size_t)j + 1];
-    const unsigned pk = __float_as_uint(R0.w);
-    const int bjx = (int)(pk & 1023u) - 1, bjy = (int)((pk >> 10) & 1023u) - 1, bjz = (int)((pk >> 20) & 1023u) - 1;
-    const float qx = (float)bjx * P.wf[0] + R0.x - pix, qy = (float)bjy * P.wf[1] + R0.y - piy,
-                qz = (float)bjz * P.wf[2] + R0.z - piz;
-    const int mx = qx > P.half_prdf[0] ? -1 : (qx < -P.half_prdf[0] ? 1 : 0);
-    const int my = qy > P.half_prdf[1] ? -1 : (qy < -P.half_prdf[1] ? 1 : 0);
-    const int mz = qz > P.half_prdf[2] ? -1 : (qz < -P.half_prdf[2] ? 1 : 0);
-    const unsigned code = (unsigned)((mx + 1) + 3 * (my + 1) + 9 * (mz + 1));
-    const df ex = pair_disp(bjx + mx * P.nb[0] - bix, R0.x, R1.x, oi.x, Ri1.x, P.w_hi[0], P.w_lo[0]);
-    const df ey = pair_disp(bjy + my * P.nb[1] - biy, R0.y, R1.y, oi.y, Ri1.y, P.w_hi[1], P.w_lo[1]);
-    const df ez = pair_disp(bjz + mz * P.nb[2] - biz, R0.z, R1.z, oi.z, Ri1.z, P.w_hi[2], P.w_lo[2]);
+  int ns = 0;
+  auto cand = [&](int k) -> unsigned {
+    if (k >= nc) return CODE_NOSHIFT << IDX_BITS;  // atom 0, not counted
+    return k < CAP ? at(k) : tail[(size_t)k * n + i];
+  };
+  unsigned u = cand(g), u2 = cand(g + LANES);
+  int4 ra, rb;
+  load_record(D.rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
+  for (int k = g, m = 0; k - g < nmax; k += LANES, ++m) {
+    const unsigned uc = u;
+    const int4 ca = ra, cb = rb;
+    int4 V0, V1;
+    load_record(D.rec + 4 * (size_t)(uc & IDX_MASK) + 2, V0, V1);
+    u = u2;
+    u2 = cand(k + 2 * LANES);
+    load_record(D.rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
+    long long ef[3];
+    pair_fixed(P, ca, cb, uc >> IDX_BITS, xi, ef);
+    const df ex = fixed_df(ef[0], P.fix_hi, P.fix_lo), ey = fixed_df(ef[1], P.fix_hi, P.fix_lo),
+             ez = fixed_df(ef[2], P.fix_hi, P.fix_lo);
     df r2 = dot3(ex, ey, ez, ex, ey, ez);
-    const bool in = have && lt(r2, rc2);
+    // a moved atom in a kept list is out of the cut-off of every atom that
+    // reads its list (it may even be outside the integers' range)
+    bool in = k < nc && lt(r2, rc2);
+    if (SRC == DF_LIST) in = in && (fresh || cb.w == 0);
     // the shell beyond the cut-off sits at the end of the lists: where no
     // lane of the warp has a pair inside, the iteration would add only zeros
-    if (!__any_sync(0xffffffffu, in)) {
-      if ((k & 7) == 7) {
-#pragma unroll
-        for (int q = 0; q < 9; ++q) bsum_fold(sm[q]);
-      }
-      continue;
-    }
-    if (!in) r2 = df{1.0f, 0.0f};
-    const int ej = __float_as_int(R1.w);
-    const df rji = spline_rho_df(P, ej, r2, err);
-    const df inv = recip(r2, rcp_estimate(r2.hi));
-    df H = mul(rji, inv);
-    if (!in) H = df{0.0f, 0.0f};
-    const df hx = mul(H, ex), hy = mul(H, ey), hz = mul(H, ez);
-    if (in) {
-      if (ns < P.kcap) {
-        const size_t slot = (size_t)ns * n + i;
-        pj[slot] = j | (code << IDX_BITS);
-        if (MULTI) {
-          const df rij = ej != ei ? spline_rho_df(P, ei, r2, err) : rji;
-          const df Hji = mul(rij, inv);
-          pa[slot] = make_float4(ex.hi, ey.hi, ez.hi, Hji.hi);
-          pb[slot] = make_float4(ex.lo, ey.lo, ez.lo, Hji.lo);
-          pc[slot] = make_float4(H.hi, H.lo, 0.f, 0.f);
-        } else {
-          pa[slot] = make_float4(ex.hi, ey.hi, ez.hi, hx.hi);
-          pb[slot] = make_float4(ex.lo, ey.lo, ez.lo, hx.lo);
-          pc[slot] = make_float4(hy.hi, hz.hi, hy.lo, hz.lo);
-        }
+    const unsigned who = __ballot_sync(0xffffffffu, in);
+    if (who != 0u) {
+      if (!in) r2 = df{1.0f, 0.0f};
+      const int ej = cb.z;
+      const df rji = spline_rho_df(P, ej, r2, D.err);
+      const df inv = recip(r2, rcp_estimate(r2.hi));
+      df H = mul(rji, inv);
+      if (!in) H = df{0.0f, 0.0f};
+      const df hx = mul(H, ex), hy = mul(H, ey), hz = mul(H, ez);
+      int slot = ns;
+      if (LANES > 1) {  // the atom's pairs in lane order
+        const int lane = t & 31;
+        const unsigned mine = who & (((1u << LANES) - 1u) << (lane & ~(LANES - 1)));
+        slot += __popc(mine & ((1u << lane) - 1u));
+        ns += __popc(mine);
       } else {
-        atomicOr(err, ERR_PAIR_OVERFLOW);
+        ns += in;
       }
-      ++ns;
+      if (in) {
+        if (slot < P.kcap) {
+          const size_t row = (size_t)slot * n + i;
+          pj[row] = uc;
+          df Hji = H;
+          if (MULTI && ej != ei) Hji = mul(spline_rho_df(P, ei, r2, D.err), inv);
+          store_row(D.pe + 2 * row, make_float4(ex.hi, ey.hi, ez.hi, Hji.hi),
+                    make_float4(ex.lo, ey.lo, ez.lo, Hji.lo));
+        } else {
+          atomicOr(D.err, ERR_PAIR_OVERFLOW);
+        }
+      }
+      acc_fma(sm[0], hx, ex);
+      acc_fma(sm[1], hx, ey);
+      acc_fma(sm[2], hx, ez);
+      acc_fma(sm[3], hy, ey);
+      acc_fma(sm[4], hy, ez);
+      acc_fma(sm[5], hz, ez);
+      const df d = dot3(ex, ey, ez, df{__int_as_float(V0.x), __int_as_float(V1.x)},
+                        df{__int_as_float(V0.y), __int_as_float(V1.y)}, df{__int_as_float(V0.z), __int_as_float(V1.z)});
+      acc_fma(sm[6], d, hx);
+      acc_fma(sm[7], d, hy);
+      acc_fma(sm[8], d, hz);
     }
-    acc_fma(sm[0].blk, hx, ex);
-    acc_fma(sm[1].blk, hx, ey);
-    acc_fma(sm[2].blk, hx, ez);
-    acc_fma(sm[3].blk, hy, ey);
-    acc_fma(sm[4].blk, hy, ez);
-    acc_fma(sm[5].blk, hz, ez);
-    const float4 V0 = vrec[2 * (size_t)j], V1 = vrec[2 * (size_t)j + 1];
-    const df d = dot3(ex, ey, ez, df{V0.x, V1.x}, df{V0.y, V1.y}, df{V0.z, V1.z});
-    acc_fma(sm[6].blk, d, hx);
-    acc_fma(sm[7].blk, d, hy);
-    acc_fma(sm[8].blk, d, hz);
-    if ((k & 7) == 7) {
+    if ((m & 7) == 7) {
 #pragma unroll
-      for (int q = 0; q < 9; ++q) bsum_fold(sm[q]);
+      for (int q = 0; q < 9; ++q) {
+        const float2 w = s_tot[q * 128 + t];
+        const df sum = add(df{w.x, w.y}, acc_value(sm[q]));
+        s_tot[q * 128 + t] = make_float2(sum.hi, sum.lo);
+        sm[q] = acc_zero();
+      }
     }
   }
-  if (!valid) return;
+#pragma unroll
+  for (int q = 0; q < 9; ++q) {
+    const float2 w = s_tot[q * 128 + t];
+    const df sum = add(df{w.x, w.y}, acc_value(sm[q]));
+    s_tot[q * 128 + t] = make_float2(sum.hi, sum.lo);
+  }
+  // one thread per atom: thread t of the first NA finishes atom blockIdx.x * NA + t
+  int o = i, ns_o = ns;
+  if (LANES > 1) {
+    __shared__ int s_ns[NA];
+    if (g == 0) s_ns[a] = ns;
+    __syncthreads();
+    if (t >= NA) return;
+    o = blockIdx.x * NA + t;
+    ns_o = s_ns[t];
+  }
+  if (o >= P.n) return;
   double mq[9];
 #pragma unroll
-  for (int q = 0; q < 9; ++q) mq[q] = to_double(bsum_value(sm[q]));
-  density_epilogue<true, true, true>(P, i, active, xi, ei, 0.0, ns < P.kcap ? ns : P.kcap, mq[0], mq[1], mq[2],
-                                     mq[3], mq[4], mq[5], mq[6], mq[7], mq[8], xi_given, xi_mode, T_e, nshort, A,
-                                     Bw, rho_out, beta_out, cell, Te_i, err, counters, v, Mm, G);
+  for (int q = 0; q < 9; ++q) {
+    const float2 *w = s_tot + q * 128 + (LANES > 1 ? t * LANES : t);
+    double sum = to_double(df{w[0].x, w[0].y});
+#pragma unroll
+    for (int l = 1; l < LANES; ++l) sum += to_double(df{w[l].x, w[l].y});
+    mq[q] = sum;
+  }
+  const D4 xo = D.x[o];
+  const bool act = LANES > 1 ? (D.mask[o] & P.groupbit) != 0 : active;
+  density_epilogue<true, true, true>(P, o, act, xo, LANES > 1 ? (int)xo.w : ei, 0.0, ns_o < P.kcap ? ns_o : P.kcap,
+                                     mq[0], mq[1], mq[2], mq[3], mq[4], mq[5], mq[6], mq[7], mq[8], D.xi_given,
+                                     D.xi_mode, D.T_e, D.nshort, D.A, D.Bw, D.rho, D.beta, D.cell, D.Te_i, D.err,
+                                     D.counters, D.v, D.Mm, D.G);
 }
 
 // -------------------------------------------------------- friction sweep 1
@@ -1716,82 +1768,93 @@ __global__ void __launch_bounds__(128) k_forces_m(StepParams P, const unsigned *
 }
 
 // k_forces_m over the df64 pair cache and records of k_density_df: per pair
-// (e.W_j) H e and (e.X_j) H e (several elements: H_ji (e.W_j) e) in df64
-// with blocked sums; the per-atom part (-M_i W_i, the pairs the reference
-// skips, eta sqrt(T_e), the force update) in FP64 as k_forces_m does it, with
-// W_i = a_i w_i and X_i = a_i xi_i formed from A and Bw exactly as the FP64
-// records are.  A neighbour the reference skips (rho_j <= 0 or outside the
-// group) carries a NaN in its record's first word.
+// H_ji (e.W_j) e and H_ji (e.X_j) e in df64 with blocked sums; the per-atom
+// part (-M_i W_i, the pairs the reference skips, eta sqrt(T_e), the force
+// update) in FP64 as k_forces_m does it, with W_i = a_i w_i and X_i = a_i xi_i
+// formed from A and Bw exactly as the FP64 records are.  A neighbour the
+// reference skips (rho_j <= 0 or outside the group) carries a NaN in its
+// record's first word.
+// It streams the pair cache (36 B per pair) and gathers a 48 B record per pair
+// from L2; on GB300 the latency of those loads bounds it, so the totals live
+// in shared memory (64 registers, 8 blocks per SM) and the next neighbour's
+// index is loaded one pair ahead.  2,048,000 atoms: 1.18 ms with 52 B per pair
+// and 16-byte loads; 1.10 with 36 B; 0.84 with 256-bit loads and 8 blocks.
 template <bool MULTI, bool RAND, int TPA = 1>
 __global__ void __launch_bounds__(128, EPH_DF_FORCES_BLOCKS)
-    k_forces_df(StepParams P, const unsigned *__restrict__ pj, const float4 *__restrict__ pa,
-                const float4 *__restrict__ pb, const float4 *__restrict__ pc, const int *__restrict__ nshort,
-                const D4 *__restrict__ Mm, const float4 *__restrict__ Gf, const D4 *__restrict__ A,
-                const D4 *__restrict__ Bw, const double *__restrict__ Te_i, D4 *__restrict__ f,
-                D4 *__restrict__ f_eph, D4 *__restrict__ f_rng, D4 *__restrict__ f_dis, D4 *__restrict__ f_sto) {
+    k_forces_df(StepParams P, const unsigned *__restrict__ pj, const float4 *__restrict__ pe,
+                const int *__restrict__ nshort, const D4 *__restrict__ Mm, const float4 *__restrict__ Gf,
+                const D4 *__restrict__ A, const D4 *__restrict__ Bw, const double *__restrict__ Te_i,
+                D4 *__restrict__ f, D4 *__restrict__ f_eph, D4 *__restrict__ f_rng, D4 *__restrict__ f_dis,
+                D4 *__restrict__ f_sto, const int4 *__restrict__ rec, unsigned *__restrict__ err) {
   using namespace df64;
+  __shared__ float2 s_tot[6 * 128];  // the sums' totals; the blocks of 8 are in registers
+  const int t = threadIdx.x;
   const long gt = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const int i = (int)(gt / TPA), g = (int)(gt % TPA);
   if (TPA == 1 && i >= P.n) return;  // with TPA > 1 every lane joins the butterfly
-  bsum se[3], sr[3];
+  constexpr int NS = RAND ? 6 : 3;
+  acc sm[NS];
 #pragma unroll
-  for (int q = 0; q < 3; ++q) se[q] = sr[q] = bsum_zero();
+  for (int q = 0; q < NS; ++q) {
+    sm[q] = acc_zero();
+    s_tot[q * 128 + t] = make_float2(0.f, 0.f);
+  }
   bool live = false;
   int ns = 0, skipped = 0;
   if (i < P.n) {
-    const float g0 = Gf[3 * (size_t)i].x;
+    const float g0 = Gf[4 * (size_t)i].x;
     live = g0 == g0;  // not NaN: rho_i > 0 and in the group
     if (live) ns = nshort[i];
   }
+  auto fold = [&]() {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      const float2 w = s_tot[q * 128 + t];
+      const df sum = add(df{w.x, w.y}, acc_value(sm[q]));
+      s_tot[q * 128 + t] = make_float2(sum.hi, sum.lo);
+      sm[q] = acc_zero();
+    }
+  };
   int m = 0;
+  unsigned jn = g < ns ? pj[(size_t)g * P.n + i] & IDX_MASK : 0u;
   for (int k = g; k < ns; k += TPA, ++m) {
     const size_t slot = (size_t)k * P.n + i;
-    const unsigned j = pj[slot] & IDX_MASK;
-    const float4 G0 = Gf[3 * (size_t)j];
+    const unsigned j = jn;
+    if (k + TPA < ns) jn = pj[slot + (size_t)TPA * P.n] & IDX_MASK;
+    float4 a, b, G0, G1;
+    load_row(Gf + 4 * (size_t)j, G0, G1);
+    load_row_once(pe + 2 * slot, a, b);
     if (G0.x != G0.x) {  // a pair the reference skips (handled below)
       skipped = 1;
     } else {
-      const float4 a = pa[slot], b = pb[slot];
-      const float4 G1 = Gf[3 * (size_t)j + 1];
-      const df ex{a.x, b.x}, ey{a.y, b.y}, ez{a.z, b.z};
-      df hx, hy, hz;
-      if (MULTI) {
-        const df Hji{a.w, b.w};
-        hx = mul(Hji, ex);
-        hy = mul(Hji, ey);
-        hz = mul(Hji, ez);
-      } else {
-        const float4 c = pc[slot];
-        hx = df{a.w, b.w};
-        hy = df{c.x, c.z};
-        hz = df{c.y, c.w};
-      }
-      const df sw = dot3(ex, ey, ez, df{G0.x, G1.x}, df{G0.y, G1.y}, df{G0.z, G1.z});
-      acc_fma(se[0].blk, sw, hx);
-      acc_fma(se[1].blk, sw, hy);
-      acc_fma(se[2].blk, sw, hz);
+      const df ex{a.x, b.x}, ey{a.y, b.y}, ez{a.z, b.z}, Hji{a.w, b.w};
+      const df sw = mul(Hji, dot3(ex, ey, ez, df{G0.x, G1.x}, df{G0.y, G1.y}, df{G0.z, G1.z}));
+      acc_fma(sm[0], sw, ex);
+      acc_fma(sm[1], sw, ey);
+      acc_fma(sm[2], sw, ez);
       if (RAND) {
-        const float4 G2 = Gf[3 * (size_t)j + 2];
-        const df sx = dot3(ex, ey, ez, df{G0.w, G1.w}, df{G2.x, G2.z}, df{G2.y, G2.w});
-        acc_fma(sr[0].blk, sx, hx);
-        acc_fma(sr[1].blk, sx, hy);
-        acc_fma(sr[2].blk, sx, hz);
+        const float4 G2 = Gf[4 * (size_t)j + 2];
+        const df sx = mul(Hji, dot3(ex, ey, ez, df{G0.w, G1.w}, df{G2.x, G2.z}, df{G2.y, G2.w}));
+        acc_fma(sm[NS - 3], sx, ex);
+        acc_fma(sm[NS - 2], sx, ey);
+        acc_fma(sm[NS - 1], sx, ez);
       }
     }
-    if ((m & 7) == 7) {
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        bsum_fold(se[q]);
-        if (RAND) bsum_fold(sr[q]);
-      }
-    }
+    if ((m & 7) == 7) fold();
   }
-  double fex = to_double(bsum_value(se[0])), fey = to_double(bsum_value(se[1])), fez = to_double(bsum_value(se[2]));
+  fold();
+  double tot[6];
+#pragma unroll
+  for (int q = 0; q < NS; ++q) {
+    const float2 w = s_tot[q * 128 + t];
+    tot[q] = to_double(df{w.x, w.y});
+  }
+  double fex = tot[0], fey = tot[1], fez = tot[2];
   double frx = 0.0, fry = 0.0, frz = 0.0;
   if (RAND) {
-    frx = to_double(bsum_value(sr[0]));
-    fry = to_double(bsum_value(sr[1]));
-    frz = to_double(bsum_value(sr[2]));
+    frx = tot[3];
+    fry = tot[4];
+    frz = tot[5];
   }
   if (TPA > 1) {
 #pragma unroll
@@ -1818,29 +1881,26 @@ __global__ void __launch_bounds__(128, EPH_DF_FORCES_BLOCKS)
       for (int k = 0; k < ns; ++k) {
         const size_t slot = (size_t)k * P.n + i;
         const unsigned j = pj[slot] & IDX_MASK;
-        const float g0 = Gf[3 * (size_t)j].x;
+        const float g0 = Gf[4 * (size_t)j].x;
         if (g0 == g0) continue;
-        const float4 pa4 = pa[slot], pb4 = pb[slot], pc4 = pc[slot];
-        const double ex = to_double(df{pa4.x, pb4.x}), ey = to_double(df{pa4.y, pb4.y}),
-                     ez = to_double(df{pa4.z, pb4.z});
-        double hx, hy, hz, H;
-        if (MULTI) {  // H_ij e
-          H = to_double(df{pc4.x, pc4.y});
-          hx = ex;
-          hy = ey;
-          hz = ez;
-        } else {
-          hx = to_double(df{pa4.w, pb4.w});
-          hy = to_double(df{pc4.x, pc4.z});
-          hz = to_double(df{pc4.y, pc4.w});
-          H = 1.0;
+        const float4 hi = pe[2 * slot], lo = pe[2 * slot + 1];
+        const df dx{hi.x, lo.x}, dy{hi.y, lo.y}, dz{hi.z, lo.z};
+        df H{hi.w, lo.w};  // H_ij: the cached H_ji with one element
+        if (MULTI) {
+          const int ej = rec[4 * (size_t)j + 1].z;
+          if (ej != rec[4 * (size_t)i + 1].z) {
+            const df r2 = dot3(dx, dy, dz, dx, dy, dz);
+            H = mul(spline_rho_df(P, ej, r2, err), recip(r2, rcp_estimate(r2.hi)));
+          }
         }
-        const double sw = H * dot3_fma(ex, ey, ez, Wx, Wy, Wz);
+        const double ex = to_double(dx), ey = to_double(dy), ez = to_double(dz);
+        const double hx = to_double(mul(H, dx)), hy = to_double(mul(H, dy)), hz = to_double(mul(H, dz));
+        const double sw = dot3_fma(ex, ey, ez, Wx, Wy, Wz);
         cex = fma(sw, hx, cex);
         cey = fma(sw, hy, cey);
         cez = fma(sw, hz, cez);
         if (RAND) {
-          const double sx = H * dot3_fma(ex, ey, ez, Xx, Xy, Xz);
+          const double sx = dot3_fma(ex, ey, ez, Xx, Xy, Xz);
           crx = fma(sx, hx, crx);
           cry = fma(sx, hy, cry);
           crz = fma(sx, hz, crz);
