@@ -448,6 +448,17 @@ void launch_density_df(eph_ctx *c, int xi_mode) {
   }
 }
 
+// Lanes per atom of k_density_tpa, unless the caller chose them: enough warps
+// for the chip, few enough that a warp's FP64 instructions stay full (measured
+// on GB300, us per launch with 4 / 8 / 16 / 32 lanes: 500 atoms 62 / 40 / 26 /
+// 20, 2,048 atoms 49 / 33 / 25 / 26, 4,000 atoms 52 / 39 / 33 / 49, 6,912
+// atoms 59 / 45 / 61 / 71, 10,976 atoms 72 / 63 / 67 / 94, 13,500 atoms 72 /
+// 92 / 91 / 117)
+int density_tpa(const eph_ctx *c) {
+  if (!c->tpa_auto) return c->tpa;
+  return c->n <= 1500 ? 32 : (c->n <= 5400 ? 16 : (c->n <= 12000 ? 8 : 4));
+}
+
 template <bool FAST, bool MULTI, bool FUSE>
 void launch_density_f(eph_ctx *c, int xi_mode) {
   // several lanes per atom in the density sweep too below 16,384 atoms, where
@@ -461,13 +472,17 @@ void launch_density_f(eph_ctx *c, int xi_mode) {
     // shared-memory column (the one-lane sweeps spill to the pair rows)
     if (c->tpa > 1 && c->n < 16384 && !c->eam) {
 #define EPH_DENSITY_TPA(T)                                                                                         \
-  k_density_tpa<MULTI, FUSE, T><<<nblocks((long)c->n * T), BLOCK, 0, c->stream>>>(                                  \
+  k_density_tpa<MULTI, FUSE, T><<<nblocks((long)c->n * T), tpa_threads(T), 0, c->stream>>>(                                  \
       c->P, c->x.p, c->mask.p, c->bin_count.p, c->bins.p, c->atom_bin.p, c->atom_off.p, c->xi.p, xi_mode, c->T0.p, \
       c->pj.p, c->pe.p, c->pg.p, c->nshort.p, c->A.p, c->Bw.p, c->rho.p, c->beta_i.p, c->cell.p, c->Te_i.p,        \
       c->wrapflag.p, c->d_err.p, c->counters.p, c->v.p, c->Mm.p, c->G.p)
-      if (c->tpa == 2) EPH_DENSITY_TPA(2);
-      else if (c->tpa == 4) EPH_DENSITY_TPA(4);
-      else EPH_DENSITY_TPA(8);
+      switch (density_tpa(c)) {
+        case 2: EPH_DENSITY_TPA(2); break;
+        case 4: EPH_DENSITY_TPA(4); break;
+        case 8: EPH_DENSITY_TPA(8); break;
+        case 16: EPH_DENSITY_TPA(16); break;
+        default: EPH_DENSITY_TPA(32);
+      }
 #undef EPH_DENSITY_TPA
       return;
     }

@@ -322,13 +322,19 @@ __device__ __forceinline__ void bin_candidates(const StepParams &P, int i, bool 
 
 // bin_candidates (FAST) over all 27 bins with LANES lanes per atom: lane g
 // takes bins g, g + LANES, ... of the stencil and the lanes append to the
-// atom's one list.  Every lane of the warp calls it.
-template <int LANES, bool SKIP = false, class Set>
+// atom's one list what `keep` does not refuse (a candidate and its FP32 r^2).
+// Every lane of the warp calls it.
+struct KeepAll {
+  __device__ bool operator()(unsigned, float) const { return true; }
+};
+template <int LANES, bool SKIP = false, class Set, class Keep = KeepAll>
 __device__ __forceinline__ void shared_candidates(const StepParams &P, int i, bool active, int4 Bi, float4 oi,
                                                   const int *__restrict__ bin_count,
                                                   const BinEntry *__restrict__ bins, unsigned *__restrict__ err,
                                                   int &nc, int cap, Set cset, float r2band,
-                                                  const int *__restrict__ skip = nullptr, float r2lo = -1.f) {
+                                                  const int *__restrict__ skip = nullptr, float r2lo = -1.f,
+                                                  Keep keep = Keep()) {
+  constexpr int CHUNK = 4;
   const int g = (int)threadIdx.x & (LANES - 1);
   for (int m = 0; m < (27 + LANES - 1) / LANES; ++m) {
     const int b = g + m * LANES;
@@ -341,31 +347,44 @@ __device__ __forceinline__ void shared_candidates(const StepParams &P, int i, bo
               kx = Tx < 0 ? -1 : (Tx >= P.nb[0] ? 1 : 0);
     const float bx = (float)dx * P.wf[0] - oi.x, by = (float)dy * P.wf[1] - oi.y, bz = (float)dz * P.wf[2] - oi.z;
     const int flat = tx + P.nb[0] * (ty + P.nb[1] * tz);
+    const BinEntry *be = bins + (size_t)flat * P.bcap;
+    // entries CHUNK at a time, the first ones beside the count (slots past it
+    // are read, not used): one memory latency per chunk instead of per entry
+    BinEntry e[CHUNK];
+#pragma unroll
+    for (int c = 0; c < CHUNK; ++c) e[c] = be[c < P.bcap ? c : 0];
     int cnt = 0;
     if (look) {
       cnt = bin_count[flat];
       cnt = cnt < P.bcap ? cnt : P.bcap;
     }
     const int cmax = __reduce_max_sync(0xffffffffu, cnt);
-    const BinEntry *be = bins + (size_t)flat * P.bcap;
-    for (int s = 0; s < cmax; ++s) {
-      bool take = false;
-      unsigned u = 0;
-      if (s < cnt) {
-        const BinEntry e = be[s];
-        const unsigned j = e.idx & IDX_MASK;
-        const float ex = bx + e.ox, ey = by + e.oy, ez = bz + e.oz;
-        const float r2 = ex * ex + ey * ey + ez * ez;
-        if (j != (unsigned)i && r2 < r2band && r2 >= r2lo && !(SKIP && (skip[j] & 2))) {
-          const unsigned wc = e.idx >> IDX_BITS;
-          const int mx = kx - ((int)(wc % 3u) - 1), my = ky - ((int)((wc / 3u) % 3u) - 1),
-                    mz = kz - ((int)(wc / 9u) - 1);
-          take = mx >= -1 && mx <= 1 && my >= -1 && my <= 1 && mz >= -1 && mz <= 1;
-          if (!take) atomicOr(err, ERR_DRIFT);
-          u = j | ((unsigned)((mx + 1) + 3 * (my + 1) + 9 * (mz + 1)) << IDX_BITS);
-        }
+    for (int s0 = 0; s0 < cmax; s0 += CHUNK) {
+      if (s0) {
+#pragma unroll
+        for (int c = 0; c < CHUNK; ++c)
+          if (s0 + c < cnt) e[c] = be[s0 + c];
       }
-      append_candidate<LANES>(take, u, nc, cap, cset, err);
+#pragma unroll
+      for (int c = 0; c < CHUNK; ++c) {
+        bool take = false;
+        unsigned u = 0;
+        if (s0 + c < cnt) {
+          const unsigned j = e[c].idx & IDX_MASK;
+          const float ex = bx + e[c].ox, ey = by + e[c].oy, ez = bz + e[c].oz;
+          const float r2 = ex * ex + ey * ey + ez * ez;
+          if (j != (unsigned)i && r2 < r2band && r2 >= r2lo && !(SKIP && (skip[j] & 2))) {
+            const unsigned wc = e[c].idx >> IDX_BITS;
+            const int mx = kx - ((int)(wc % 3u) - 1), my = ky - ((int)((wc / 3u) % 3u) - 1),
+                      mz = kz - ((int)(wc / 9u) - 1);
+            take = mx >= -1 && mx <= 1 && my >= -1 && my <= 1 && mz >= -1 && mz <= 1;
+            if (!take) atomicOr(err, ERR_DRIFT);
+            u = j | ((unsigned)((mx + 1) + 3 * (my + 1) + 9 * (mz + 1)) << IDX_BITS);
+            take = take && keep(u, r2);
+          }
+        }
+        append_candidate<LANES>(take, u, nc, cap, cset, err);
+      }
     }
   }
 }
@@ -536,6 +555,26 @@ __device__ __forceinline__ void density_vector(const StepParams &P, const D4 &xi
   ez = cz - xi.z;
 }
 
+// atom i's deviates of this step: the device generator's or those given
+__device__ __forceinline__ void atom_deviates(const StepParams &P, int i, const D4 *__restrict__ xi_given, int xi_mode,
+                                              double *xi3) {
+  if (xi_mode == 0) {
+    gaussian3(P.seed, *P.step, (unsigned)i, xi3);
+  } else {
+    const D4 g = xi_given[i];
+    xi3[0] = g.x;
+    xi3[1] = g.y;
+    xi3[2] = g.z;
+  }
+}
+
+// what an atom's epilogue needs that does not depend on its pairs, where
+// another warp of the block made it meanwhile
+struct ReadyAtom {
+  double xi[3], Te;
+  int cell;
+};
+
 // The end of the density sweep for atom i (its pairs summed): alpha, beta,
 // the deviates, its grid cell and T_e, and the per-atom records.
 // With DFG (the df64 force sweep follows) the gathered records go to G as
@@ -551,7 +590,7 @@ __device__ __forceinline__ void density_epilogue(
     D4 *__restrict__ A, D4 *__restrict__ Bw, double *__restrict__ rho_out, double *__restrict__ beta_out,
     int *__restrict__ cell, double *__restrict__ Te_i, unsigned *__restrict__ err,
     unsigned long long *__restrict__ counters, const D4 *__restrict__ v, D4 *__restrict__ Mm,
-    D4 *__restrict__ G) {
+    D4 *__restrict__ G, const ReadyAtom *ready = nullptr) {
   nshort[i] = ns;
   // FAST with M_i: rho_i = trace M_i = sum_j rho_j(r^2) / r^2 * r^2, within
   // the reciprocal's error (~6e-14) of the sum of rho_j(r^2)
@@ -567,18 +606,17 @@ __device__ __forceinline__ void density_epilogue(
     }
     if (FAST && rho > 0) alpha = alpha / rho;
     if (P.flags & 0x02) {
-      if (xi_mode == 0) {
-        gaussian3(P.seed, *P.step, (unsigned)i, xi3);
+      if (ready) {
+        xi3[0] = ready->xi[0];
+        xi3[1] = ready->xi[1];
+        xi3[2] = ready->xi[2];
       } else {
-        const D4 g = xi_given[i];
-        xi3[0] = g.x;
-        xi3[1] = g.y;
-        xi3[2] = g.z;
+        atom_deviates(P, i, xi_given, xi_mode, xi3);
       }
     }
-    const long c = grid_index(P, xi.x, xi.y, xi.z);
-    cell[i] = (int)c;
-    Te_i[i] = T_e[c];
+    const int c = ready ? ready->cell : (int)grid_index(P, xi.x, xi.y, xi.z);
+    cell[i] = c;
+    Te_i[i] = ready ? ready->Te : T_e[c];
   }
   A[i] = D4{rho, alpha, xi3[0], xi3[1]};
   if (FUSE_W) {
@@ -718,17 +756,25 @@ __global__ void __launch_bounds__(128) k_density(
 #define EPH_DF_FORCES_BLOCKS 8
 #endif
 
-// The FAST density sweep with TPA lanes per atom (TPA = 2, 4, 8) for small
-// systems, where one lane per atom leaves the SMs a few warps each and the
-// sweep waits on its loads.  Lane g of an atom searches bins g, g + TPA, ...
-// of the 27 (its candidates in its own shared-memory column, at most
-// CAND_SMEM), tests them exactly, and after a prefix sum over the atom's
-// lanes writes its in-cutoff pairs to rows [offset_g, offset_g + count_g)
-// of the pair cache; rho (and with FUSE_W, M_i and S_i) are summed over the
-// lanes by a butterfly and lane 0 finishes the atom.  Sums in a fixed order
-// (the same every run), within rounding of the one-lane sweep.
+// The FAST density sweep with TPA lanes per atom for small systems (FP64 pair
+// terms), where one lane per atom leaves the SMs a few warps each.  The
+// lanes search the 27 bins together and leave the atom's pairs -- the
+// candidates sure to be inside the cut-off by their FP32 distance, and those
+// within its error of the cut-off that pass the FP64 test -- in one list in
+// shared memory, whose entry k is row k of the pair cache; then lane g sums
+// rows g, g + TPA, ....  Meanwhile the block's last warps draw the atoms'
+// deviates and find their grid cells; the lanes' sums meet in shared memory
+// and one thread per atom, in the block's first threads, finishes the atom.
+// Sums in a fixed order (the same every run), within rounding of the one-lane
+// sweep.
+// FP64 issue and latency bound it: a warp FP64 instruction takes 16 cycles of
+// the SM's pipe however few lanes are active, so what counts is full warps
+// and short chains.  GB300, us per launch at 4,000 atoms: 90 with the lanes'
+// own candidates (half the iterations idle, an extra pass for the exact
+// test) and everything per atom on every eighth lane; 33 now (16 lanes).
+constexpr int tpa_threads(int tpa) { return 128 + (128 / tpa + 31) / 32 * 32; }
 template <bool MULTI, bool FUSE_W, int TPA>
-__global__ void __launch_bounds__(128) k_density_tpa(
+__global__ void __launch_bounds__(tpa_threads(TPA)) k_density_tpa(
     StepParams P, const D4 *__restrict__ x, const int *__restrict__ mask, const int *__restrict__ bin_count,
     const BinEntry *__restrict__ bins, const int4 *__restrict__ atom_bin, const float4 *__restrict__ atom_off,
     const D4 *__restrict__ xi_given, int xi_mode, const double *__restrict__ T_e, unsigned *__restrict__ pj,
@@ -737,21 +783,37 @@ __global__ void __launch_bounds__(128) k_density_tpa(
     double *__restrict__ Te_i, int *__restrict__ wrapflag, unsigned *__restrict__ err,
     unsigned long long *__restrict__ counters, const D4 *__restrict__ v, D4 *__restrict__ Mm,
     D4 *__restrict__ G) {
-  static_assert(CAND_SMEM <= 64, "candidate masks are 64 bits");
-  __shared__ unsigned s_cand[CAND_SMEM * 128];
-  const long gt = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = (int)(gt / TPA), g = (int)(gt % TPA);
-  const int t = threadIdx.x, nt = blockDim.x;
-  if (gt == 0) *wrapflag = 0;  // the binning kernel has read it
+  constexpr int NA = 128 / TPA;  // atoms per block
+  constexpr int NSUM = FUSE_W ? 9 : 1;
+  __shared__ __align__(16) unsigned s_cand[NA * (KMAX + 1)];
+  __shared__ double s_sum[NSUM * 128];
+  double *s_tot = reinterpret_cast<double *>(s_cand);  // [NSUM][NA], once the lists are read
+  __shared__ ReadyAtom s_ready[NA];
+  __shared__ int s_ns[NA];
+  const int t = threadIdx.x, a = t / TPA, g = t % TPA;
+  if (blockIdx.x == 0 && t == 0) *wrapflag = 0;  // the binning kernel has read it
+  if (t >= 128) {  // the last warps: what does not depend on the pairs
+    const int r = t - 128, o = blockIdx.x * NA + r;
+    if (r < NA && o < P.n && (mask[o] & P.groupbit)) {
+      ReadyAtom w{{0.0, 0.0, 0.0}, 0.0, 0};
+      const D4 xo = x[o];
+      w.cell = (int)grid_index(P, xo.x, xo.y, xo.z);
+      w.Te = T_e[w.cell];
+      if (P.flags & 0x02) atom_deviates(P, o, xi_given, xi_mode, w.xi);
+      s_ready[r] = w;
+    }
+    __syncthreads();
+    __syncthreads();
+    return;
+  }
+  const int i = blockIdx.x * NA + a;
   const bool valid = i < P.n;
   const bool active = valid && (mask[i] & P.groupbit) != 0;
-  auto cget = [&](int k) -> unsigned { return s_cand[k * nt + t]; };
-  auto cset = [&](int k, unsigned u) { s_cand[k * nt + t] = u; };
+  unsigned *list = s_cand + a * (KMAX + 1);
   D4 xi = D4{0.0, 0.0, 0.0, 0.0};
   if (valid) xi = x[i];
   const int ei = (int)xi.w;
-  // pass 1: this lane's bins (the same number of rounds on every lane)
-  int nc = 0;
+  int ns = 0;
   {
     int4 Bi = make_int4(0, 0, 0, 0);
     float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -759,75 +821,64 @@ __global__ void __launch_bounds__(128) k_density_tpa(
       Bi = atom_bin[i];
       oi = atom_off[i];
     }
-    for (int m = 0; m < (27 + TPA - 1) / TPA; ++m) {
-      const int b = g + m * TPA;  // (dz + 1) * 9 + (dy + 1) * 3 + (dx + 1)
-      const bool look = active && b < 27;
-      const int bb = b < 27 ? b : 13;
-      bin_candidates<true>(P, i, look, Bi, oi, bb % 3 - 1, (bb / 3) % 3 - 1, bb / 9 - 1, bin_count, bins, err, nc,
-                           CAND_SMEM, cget, cset, P.rc2_band);
-    }
+    const float sure = (float)(P.rc2 * (1.0 - 1e-4));
+    shared_candidates<TPA>(
+        P, i, active, Bi, oi, bin_count, bins, err, ns, P.kcap, [&](int k, unsigned u) { list[k] = u; }, P.rc2_band,
+        nullptr, -1.f, [&](unsigned u, float r2) {
+          if (r2 < sure) return true;
+          double ex, ey, ez;
+          density_vector(P, xi, x[u & IDX_MASK], u >> IDX_BITS, ex, ey, ez);
+          return below(dot3_fma(ex, ey, ez, ex, ey, ez), P.rc2);
+        });
   }
   __syncwarp();
-  // pass 2a: the exact test of this lane's candidates
-  unsigned long long keep = 0ull;
-  const int nmax = __reduce_max_sync(0xffffffffu, nc);
-  for (int k = 0; k < nmax; ++k) {
-    if (k < nc) {
-      const unsigned u = cget(k);
-      double ex, ey, ez;
-      density_vector(P, xi, x[u & IDX_MASK], u >> IDX_BITS, ex, ey, ez);
-      if (below(dot3_fma(ex, ey, ez, ex, ey, ez), P.rc2)) keep |= 1ull << k;
-    }
-  }
-  // rows of this lane's pairs: an exclusive prefix sum over the atom's lanes
-  const int count = __popcll(keep);
-  int incl = count;
-#pragma unroll
-  for (int d = 1; d < TPA; d <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, d);
-    if (g >= d) incl += y;
-  }
-  const int ns = __shfl_sync(0xffffffffu, incl, (int)(threadIdx.x & 31) | (TPA - 1));
-  const int off = incl - count;
-  if (ns > P.kcap && g == 0 && valid) atomicOr(err, ERR_PAIR_OVERFLOW);
-  // pass 2b: the kept pairs
   double rho = 0.0, Sx = 0.0, Sy = 0.0, Sz = 0.0;
   double mxx = 0.0, mxy = 0.0, mxz = 0.0, myy = 0.0, myz = 0.0, mzz = 0.0;
-  unsigned long long rest = keep;
-  const int n2 = __reduce_max_sync(0xffffffffu, count);
-  for (int m = 0; m < n2; ++m) {
-    if (m < count) {
-      const int k = __ffsll((long long)rest) - 1;
-      rest &= rest - 1ull;
-      const unsigned u = cget(k);
-      const D4 xj = x[u & IDX_MASK];
-      double ex, ey, ez;
-      density_vector(P, xi, xj, u >> IDX_BITS, ex, ey, ez);
-      const double r2 = dot3_fma(ex, ey, ez, ex, ey, ez);
-      if (off + m < P.kcap)
-        density_pair<true, MULTI, FUSE_W>(P, ei, u, (int)xj.w, ex, ey, ez, r2, (size_t)(off + m) * P.n + i, pj, pe,
-                                          pg, v, err, rho, mxx, mxy, mxz, myy, myz, mzz, Sx, Sy, Sz);
+  unsigned u_next = g < ns ? list[g] : 0u;
+  D4 x_next = xi;
+  if (g < ns) x_next = x[u_next & IDX_MASK];
+  for (int k = g; k < ns; k += TPA) {
+    const unsigned u = u_next;
+    const D4 xj = x_next;
+    if (k + TPA < ns) {  // the next neighbour's position while this pair is summed
+      u_next = list[k + TPA];
+      x_next = x[u_next & IDX_MASK];
     }
+    double ex, ey, ez;
+    density_vector(P, xi, xj, u >> IDX_BITS, ex, ey, ez);
+    const double r2 = dot3_fma(ex, ey, ez, ex, ey, ez);
+    density_pair<true, MULTI, FUSE_W>(P, ei, u, (int)xj.w, ex, ey, ez, r2, (size_t)k * P.n + i, pj, pe, pg, v, err,
+                                      rho, mxx, mxy, mxz, myy, myz, mzz, Sx, Sy, Sz);
   }
+  // sum q of the atom's lane l at q * 128 + l * NA + (atom): the finishing
+  // threads read neighbouring words
+  const int at = g * NA + a;
+  if (FUSE_W) {
+    const double m[9] = {mxx, mxy, mxz, myy, myz, mzz, Sx, Sy, Sz};
 #pragma unroll
-  for (int o = TPA / 2; o > 0; o >>= 1) {
-    if (!FUSE_W) rho += __shfl_xor_sync(0xffffffffu, rho, o);  // with M_i: its trace
-    if (FUSE_W) {
-      mxx += __shfl_xor_sync(0xffffffffu, mxx, o);
-      mxy += __shfl_xor_sync(0xffffffffu, mxy, o);
-      mxz += __shfl_xor_sync(0xffffffffu, mxz, o);
-      myy += __shfl_xor_sync(0xffffffffu, myy, o);
-      myz += __shfl_xor_sync(0xffffffffu, myz, o);
-      mzz += __shfl_xor_sync(0xffffffffu, mzz, o);
-      Sx += __shfl_xor_sync(0xffffffffu, Sx, o);
-      Sy += __shfl_xor_sync(0xffffffffu, Sy, o);
-      Sz += __shfl_xor_sync(0xffffffffu, Sz, o);
-    }
+    for (int q = 0; q < NSUM; ++q) s_sum[q * 128 + at] = m[q];
+  } else {
+    s_sum[at] = rho;
   }
-  if (!valid || g != 0) return;
-  density_epilogue<true, FUSE_W>(P, i, active, xi, ei, rho, ns < P.kcap ? ns : P.kcap, mxx, mxy, mxz, myy, myz, mzz,
-                                 Sx, Sy, Sz, xi_given, xi_mode, T_e, nshort, A, Bw, rho_out, beta_out, cell, Te_i,
-                                 err, counters, v, Mm, G);
+  if (g == 0) s_ns[a] = ns;
+  __syncthreads();
+  for (int q = t; q < NSUM * NA; q += 128) {  // sum q / NA of atom q % NA
+    const double *w = s_sum + q / NA * 128 + q % NA;
+    double sum = w[0];
+#pragma unroll
+    for (int l = 1; l < TPA; ++l) sum += w[l * NA];
+    s_tot[q] = sum;
+  }
+  __syncthreads();
+  const int o = blockIdx.x * NA + t;
+  if (t >= NA || o >= P.n) return;
+  double m[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q) m[q] = q < NSUM ? s_tot[q * NA + t] : 0.0;
+  const D4 xo = x[o];
+  density_epilogue<true, FUSE_W>(P, o, (mask[o] & P.groupbit) != 0, xo, (int)xo.w, m[0], s_ns[t], m[0], m[1], m[2],
+                                 m[3], m[4], m[5], m[6], m[7], m[8], xi_given, xi_mode, T_e, nshort, A, Bw, rho_out,
+                                 beta_out, cell, Te_i, err, counters, v, Mm, G, s_ready + t);
 }
 
 // ------------------------------------------------ candidate-list reuse
@@ -1663,8 +1714,9 @@ __global__ void __launch_bounds__(128) k_forces_m(StepParams P, const unsigned *
                                                   D4 *__restrict__ f, D4 *__restrict__ f_eph, D4 *__restrict__ f_rng,
                                                   D4 *__restrict__ f_dis, D4 *__restrict__ f_sto) {
   const long gt = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = (int)(gt / TPA), g = (int)(gt % TPA);
-  if (TPA == 1 && i >= P.n) return;  // with TPA > 1 every lane joins the butterfly
+  int i = (int)(gt / TPA);
+  const int g = (int)(gt % TPA);
+  if (TPA == 1 && i >= P.n) return;  // with TPA > 1 every lane joins the sums
   double fex = 0.0, fey = 0.0, fez = 0.0, frx = 0.0, fry = 0.0, frz = 0.0;
   bool live = false;
   int ns = 0, skipped = 0;
@@ -1672,9 +1724,11 @@ __global__ void __launch_bounds__(128) k_forces_m(StepParams P, const unsigned *
     live = pos_double(G[2 * (size_t)i + 1].z);  // rho_i > 0 (0 outside the group)
     if (live) ns = nshort[i];
   }
+  unsigned j_next = g < ns ? pj[(size_t)g * P.n + i] & IDX_MASK : 0u;
   for (int k = g; k < ns; k += TPA) {
     const size_t slot = (size_t)k * P.n + i;
-    const unsigned j = pj[slot] & IDX_MASK;
+    const unsigned j = j_next;
+    if (k + TPA < ns) j_next = pj[slot + (size_t)TPA * P.n] & IDX_MASK;
     const D4 e = pe[slot];
     const D4 Gj1 = G[2 * (size_t)j], Gj2 = G[2 * (size_t)j + 1];
     if (!pos_double(Gj2.z)) {  // a pair the reference skips (handled below)
@@ -1708,19 +1762,45 @@ __global__ void __launch_bounds__(128) k_forces_m(StepParams P, const unsigned *
     }
   }
   if (TPA > 1) {
-#pragma unroll
-    for (int o = TPA / 2; o > 0; o >>= 1) {
-      fex += __shfl_xor_sync(0xffffffffu, fex, o);
-      fey += __shfl_xor_sync(0xffffffffu, fey, o);
-      fez += __shfl_xor_sync(0xffffffffu, fez, o);
-      if (RAND) {
-        frx += __shfl_xor_sync(0xffffffffu, frx, o);
-        fry += __shfl_xor_sync(0xffffffffu, fry, o);
-        frz += __shfl_xor_sync(0xffffffffu, frz, o);
-      }
-      skipped |= __shfl_xor_sync(0xffffffffu, skipped, o);
+    // the lanes' sums meet in shared memory; the block's first threads finish
+    // an atom each
+    constexpr int NA = 128 / TPA, NSUM = RAND ? 6 : 3;
+    __shared__ double s_sum[NSUM * 128], s_tot[NSUM * NA];
+    __shared__ int s_skip[128];
+    const int t = threadIdx.x, at = g * NA + t / TPA;
+    s_sum[at] = fex;
+    s_sum[128 + at] = fey;
+    s_sum[256 + at] = fez;
+    if (RAND) {
+      s_sum[(NSUM - 3) * 128 + at] = frx;
+      s_sum[(NSUM - 2) * 128 + at] = fry;
+      s_sum[(NSUM - 1) * 128 + at] = frz;
     }
-    if (i >= P.n || g != 0) return;
+    s_skip[at] = skipped;
+    __syncthreads();
+    for (int q = t; q < NSUM * NA; q += 128) {
+      const double *w = s_sum + q / NA * 128 + q % NA;
+      double sum = w[0];
+#pragma unroll
+      for (int l = 1; l < TPA; ++l) sum += w[l * NA];
+      s_tot[q] = sum;
+    }
+    __syncthreads();
+    i = blockIdx.x * NA + t;
+    if (t >= NA || i >= P.n) return;
+    fex = s_tot[t];
+    fey = s_tot[NA + t];
+    fez = s_tot[2 * NA + t];
+    if (RAND) {
+      frx = s_tot[(NSUM - 3) * NA + t];
+      fry = s_tot[(NSUM - 2) * NA + t];
+      frz = s_tot[(NSUM - 1) * NA + t];
+    }
+    skipped = 0;
+#pragma unroll
+    for (int l = 0; l < TPA; ++l) skipped |= s_skip[l * NA + t];
+    live = pos_double(G[2 * (size_t)i + 1].z);
+    ns = live ? nshort[i] : 0;
   }
   if (live) {
     double cex = 0.0, cey = 0.0, cez = 0.0, crx = 0.0, cry = 0.0, crz = 0.0;
