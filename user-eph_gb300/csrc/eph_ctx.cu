@@ -384,8 +384,9 @@ bool df_active(const eph_ctx *c) {
 // 16,384 atoms 53 / 39 / 36, 32,000 62 / 52 / 51, 62,500 88 / 75 / 94, 131,072
 // 127 / 137 / 174.  Bin search: 16,384 atoms 136 / 98 / 70, 23,328 167 / 111 /
 // 80, 32,000 161 / 116 / 125, 131,072 363 / 326 / 340, 256,000 566 / 558 / 621,
-// 500,000 960 / 1,021 / 1,171.  From the EAM list: 16,384 atoms 102 / 70 / 52,
-// 62,500 132 / 104 / 120, 256,000 390 / 392 / 486)
+// 500,000 960 / 1,021 / 1,171.  From an EAM list that does not have the fix's
+// pairs apart: 16,384 atoms 102 / 70 / 52, 62,500 132 / 104 / 120, 256,000 390
+// / 392 / 486; from one that has, as the kept lists)
 int density_lanes(const eph_ctx *c) {
   if (c->reuse) return c->n <= 40000 ? 4 : (c->n <= 98304 ? 2 : 1);
   if (c->eam) return c->n <= 32768 ? 4 : (c->n <= 196608 ? 2 : 1);
@@ -395,26 +396,37 @@ int density_lanes(const eph_ctx *c) {
 template <bool MULTI, int LANES>
 void launch_density_df_l(eph_ctx *c, const DensityArgs &D) {
   const int nb = nblocks((long)c->n * LANES);
-  if (c->reuse) k_density_df<MULTI, LANES, DF_LIST><<<nb, BLOCK, 0, c->stream>>>(c->P, D);
-  else if (D.elist) k_density_df<MULTI, LANES, DF_EAM><<<nb, BLOCK, 0, c->stream>>>(c->P, D);
+  if (D.elist) k_density_df<MULTI, LANES, DF_EAM><<<nb, BLOCK, 0, c->stream>>>(c->P, D);
+  else if (c->reuse) k_density_df<MULTI, LANES, DF_LIST><<<nb, BLOCK, 0, c->stream>>>(c->P, D);
   else k_density_df<MULTI, LANES, DF_BINS><<<nb, BLOCK, 0, c->stream>>>(c->P, D);
 }
 
 template <bool MULTI>
 void launch_density_df(eph_ctx *c, int xi_mode) {
   DensityArgs D{};
+  CandidateArgs &C = D.C;
+  C.bin_count = c->bin_count.p;
+  C.bins = c->bins.p;
+  C.atom_bin = c->atom_bin.p;
+  C.atom_off = c->atom_off.p;
+  C.rec = c->dfrec.p;
+  C.x = c->x.p;
+  C.err = c->d_err.p;
+  C.pj = c->pj.p;
+  C.kcap = c->P.kcap;
+  C.band = c->P.rc2_band;
+  C.rc2 = c->P.rc2;
+  C.cl = c->cl.p;
+  C.cl_n = c->cl_n.p;
+  C.state = c->state.p;
+  C.rb = c->rb.p;
+  C.flist = c->flist.p;
+  C.xref = c->xref.p;
   D.mask = c->mask.p;
-  D.bin_count = c->bin_count.p;
-  D.bins = c->bins.p;
-  D.atom_bin = c->atom_bin.p;
-  D.atom_off = c->atom_off.p;
-  D.rec = c->dfrec.p;
-  D.x = c->x.p;
   D.v = c->v.p;
   D.xi_given = c->xi.p;
   D.xi_mode = xi_mode;
   D.T_e = c->T0.p;
-  D.pj = c->pj.p;
   D.pe = reinterpret_cast<float4 *>(c->pe.p);
   D.nshort = c->nshort.p;
   D.A = c->A.p;
@@ -424,23 +436,13 @@ void launch_density_df(eph_ctx *c, int xi_mode) {
   D.cell = c->cell.p;
   D.Te_i = c->Te_i.p;
   D.wrapflag = c->wrapflag.p;
-  D.err = c->d_err.p;
   D.counters = c->counters.p;
   D.Mm = c->Mm.p;
   D.G = c->G.p;
-  if (c->reuse) {
-    D.cl = c->cl.p;
-    D.cl_n = c->cl_n.p;
-    D.state = c->state.p;
-    D.rb = c->rb.p;
-    D.flist = c->flist.p;
-    D.xref = c->xref.p;
-  } else {
-    // with the standalone engine's EAM force the candidates come from its
-    // pair list of this step (the same bins and order; no bin scan)
-    if (!(c->eam_list_fresh && eam_pair_list(c, &D.elist, &D.ens))) D.elist = nullptr, D.ens = nullptr;
-    c->eam_list_fresh = false;
-  }
+  // with the standalone engine's EAM force the candidates come from its pair
+  // list of this step (no bin scan)
+  if (!(c->eam_list_fresh && eam_pair_list(c, &D.elist, &D.ens, &D.ens_in))) D.elist = nullptr;
+  c->eam_list_fresh = false;
   switch (density_lanes(c)) {
     case 1: launch_density_df_l<MULTI, 1>(c, D); break;
     case 2: launch_density_df_l<MULTI, 2>(c, D); break;
@@ -459,6 +461,10 @@ int density_tpa(const eph_ctx *c) {
   return c->n <= 1500 ? 32 : (c->n <= 5400 ? 16 : (c->n <= 12000 ? 8 : 4));
 }
 
+bool df_records_wanted(const eph_ctx *c) {
+  return df_active(c) || (c->eam && c->mode == EPH_MODE_FAST && c->pair_arith == EPH_PAIRS_DF64);
+}
+
 template <bool FAST, bool MULTI, bool FUSE>
 void launch_density_f(eph_ctx *c, int xi_mode) {
   // several lanes per atom in the density sweep too below 16,384 atoms, where
@@ -467,15 +473,16 @@ void launch_density_f(eph_ctx *c, int xi_mode) {
   // and lane sums cost more than they hide: 32,000 atoms 71 -> 81 ms per 200
   // steps, so the one-lane sweep stays there)
   if constexpr (FAST) {
-    // not over the EAM engine's bins: they are sized for its cut-off, and a
-    // lane's share of 27 such bins can hold more candidates than its
-    // shared-memory column (the one-lane sweeps spill to the pair rows)
-    if (c->tpa > 1 && c->n < 16384 && !c->eam) {
+    if (c->tpa > 1 && c->n < 16384) {
+      // with the EAM engine the pairs come from its list of this step
+      const unsigned *elist = nullptr;
+      const int *ens = nullptr, *inner = nullptr;
+      if (!(df_records_wanted(c) && c->eam_list_fresh && eam_pair_list(c, &elist, &ens, &inner))) elist = nullptr;
 #define EPH_DENSITY_TPA(T)                                                                                         \
   k_density_tpa<MULTI, FUSE, T><<<nblocks((long)c->n * T), tpa_threads(T), 0, c->stream>>>(                                  \
       c->P, c->x.p, c->mask.p, c->bin_count.p, c->bins.p, c->atom_bin.p, c->atom_off.p, c->xi.p, xi_mode, c->T0.p, \
       c->pj.p, c->pe.p, c->pg.p, c->nshort.p, c->A.p, c->Bw.p, c->rho.p, c->beta_i.p, c->cell.p, c->Te_i.p,        \
-      c->wrapflag.p, c->d_err.p, c->counters.p, c->v.p, c->Mm.p, c->G.p)
+      c->wrapflag.p, c->d_err.p, c->counters.p, c->v.p, c->Mm.p, c->G.p, elist, ens, c->dfrec.p)
       switch (density_tpa(c)) {
         case 2: EPH_DENSITY_TPA(2); break;
         case 4: EPH_DENSITY_TPA(4); break;
@@ -587,6 +594,9 @@ int set_bin_geometry(eph_ctx *c, double r) {
   return EPH_OK;
 }
 
+// the radius the pair sweeps search: the fix's cut-off, or the EAM engine's
+double pair_radius(const eph_ctx *c) { return std::max(c->beta.r_cutoff, eam_cutoff(c)); }
+
 // a bin's capacity from the number density: ~density * w^3 atoms
 int auto_bcap(const eph_ctx *c) {
   const double dens = c->n / (c->prd[0] * c->prd[1] * c->prd[2]);
@@ -605,18 +615,18 @@ int auto_bcap(const eph_ctx *c) {
 // 2,048,000 atoms +0.2 %, where both sweeps already run at the FP64 issue
 // limit); a skin set through eph_set_list_skin applies at any size.
 bool want_list(const eph_ctx *c) {
+  const bool df = c->pair_arith == EPH_PAIRS_DF64;
   // with the df64 pair sums (whose pass 2 no longer hides the bin search) the
   // lists pay at every size that runs them, from 2^14 atoms on (measured on
   // GB300, bins and density sweep of a step, bin search -> lists: 16,384 atoms
   // 86 -> 66 us, 32,000 atoms 136 -> 80, 131,072 atoms 354 -> 163, 500,000
   // atoms 1,031 -> 446)
-  const bool df = c->pair_arith == EPH_PAIRS_DF64;
   const bool size_ok = c->lskin_user || (df ? c->n >= (1 << 14) : c->n >= (1 << 15) && c->n <= (1 << 20));
-  if (c->mode != EPH_MODE_FAST || c->lskin <= 0.0 || c->list_block || c->eam || c->n <= 0 ||
-      !(c->tpa == 1 || c->n >= 16384) || !fused_friction(c) || !size_ok)
+  if (c->mode != EPH_MODE_FAST || c->lskin <= 0.0 || c->list_block || c->n <= 0 ||
+      (c->eam && !df) || !(c->tpa == 1 || c->n >= 16384) || !fused_friction(c) || !size_ok)
     return false;
   for (int k = 0; k < 3; ++k)
-    if ((int)(c->prd[k] / ((c->beta.r_cutoff + c->lskin) * (1.0 + 5e-5))) < 3) return false;
+    if ((int)(c->prd[k] / ((pair_radius(c) + c->lskin) * (1.0 + 5e-5))) < 3) return false;
   return true;
 }
 
@@ -634,7 +644,7 @@ void drop_list(eph_ctx *c) {
 int configure_list(eph_ctx *c) {
   const bool want = want_list(c);
   if (!want && !c->reuse) return EPH_OK;
-  const double rc = c->beta.r_cutoff;
+  const double rc = pair_radius(c);
   const int nbins_was = c->nbins, bcap_was = c->bcap;
   int r = set_bin_geometry(c, want ? rc + c->lskin : rc);
   if (r) return r;
@@ -654,7 +664,7 @@ int configure_list(eph_ctx *c) {
   const size_t N = (size_t)c->n;
   const double rl = rc + c->lskin, rm = rc + 0.5 * c->lskin;
   const double dens = c->n / (c->prd[0] * c->prd[1] * c->prd[2]);
-  const int lcap = std::min(256, ((int)std::ceil(2.0 * dens * 4.18879020478639 * rl * rl * rl + 24.0) + 7) / 8 * 8);
+  const int lcap = std::min(c->eam ? 512 : 256, ((int)std::ceil(2.0 * dens * 4.18879020478639 * rl * rl * rl + 24.0) + 7) / 8 * 8);
   if (lcap != c->lcap || c->cl.n != (size_t)lcap * N) CUDA_TRY(c, c->cl.alloc((size_t)lcap * N));
   c->lcap = lcap;
   for (DevBuf<int> *b : {&c->cl_n, &c->state})
@@ -714,6 +724,24 @@ int launch_post_force(eph_ctx *c, int xi_mode) {
   return launch_pair_sweeps(c, xi_mode);
 }
 
+// A warp per bin where the bins are few (the sort's latency shows) or hold
+// more than a few entries (a thread's insertion sort is quadratic), a thread
+// per bin where there are many small ones (measured on GB300: 343 bins 20 -> 2
+// us; 226,981 bins of 9 atoms 60 us by thread, 100 us by warp; bins of 28 atoms, the
+// whole binning of 16,384 atoms 125 us by thread, 17 us by warp)
+void launch_bin_sort(eph_ctx *c, const int *gate) {
+  const int nb = nblocks((long)c->nbins * 32);
+  const bool small = c->bcap <= 40;
+  if (c->bcap <= SORT_WARP_MAX && (c->nbins < 32768 || !small)) {
+    if (c->bcap <= 64)
+      k_bin_sort_warp<2><<<nb, BLOCK, 0, c->stream>>>(c->nbins, c->bcap, c->bin_count.p, c->bins.p, gate);
+    else
+      k_bin_sort_warp<4><<<nb, BLOCK, 0, c->stream>>>(c->nbins, c->bcap, c->bin_count.p, c->bins.p, gate);
+  } else {
+    k_bin_sort<<<nblocks(c->nbins), BLOCK, 0, c->stream>>>(c->nbins, c->bcap, c->bin_count.p, c->bins.p, gate);
+  }
+}
+
 int launch_bin(eph_ctx *c) {
   const int nb = nblocks(c->n);
   PhaseScope ps(c, EPH_PHASE_BIN);
@@ -723,7 +751,7 @@ int launch_bin(eph_ctx *c) {
     // flags the atoms near moved ones and leaves the bins as they are
     int *rb = c->rb.p;
     CUDA_TRY(c, cudaMemsetAsync(rb + 1, 0, sizeof(int), c->stream));
-    const bool df = df_active(c);
+    const bool df = df_records_wanted(c);
     k_list_check<<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->xref.p, c->state.p, rb,
                                               c->flist.p, c->counters.p, df ? c->dfrec.p : nullptr,
                                               c->v.p);
@@ -734,30 +762,19 @@ int launch_bin(eph_ctx *c) {
     k_bin<<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->bin_count.p, c->bins.p,
                                        c->atom_bin.p, c->atom_off.p, c->d_err.p, c->counters.p, 0, rb + 2,
                                        c->xref.p, df ? c->dfrec.p : nullptr, c->v.p);
-    if (c->bcap <= 64 && c->nbins < 32768)
-      k_bin_sort_warp<<<nblocks((long)c->nbins * 32), BLOCK, 0, c->stream>>>(c->nbins, c->bcap, c->bin_count.p,
-                                                                              c->bins.p, rb + 2);
-    else
-      k_bin_sort<<<nblocks(c->nbins), BLOCK, 0, c->stream>>>(c->nbins, c->bcap, c->bin_count.p, c->bins.p, rb + 2);
+    launch_bin_sort(c, rb + 2);
     ps.launched(6);
     CUDA_TRY(c, cudaGetLastError());
     return EPH_OK;
   }
   ps.launched();
   CUDA_TRY(c, cudaMemsetAsync(c->bin_count.p, 0, sizeof(int) * (size_t)c->nbins, c->stream));
-  const bool df = df_active(c);
+  const bool df = df_records_wanted(c);
   k_bin<<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->bin_count.p, c->bins.p,
                                      c->atom_bin.p, c->atom_off.p, c->d_err.p, c->counters.p, 1, nullptr, nullptr,
                                      df ? c->dfrec.p : nullptr, c->v.p);
   ps.launched();
-  // a warp per bin where the bins are few (the sort's latency shows), a
-  // thread per bin where they are many (measured on GB300: 343 bins 20 ->
-  // ~2 µs; 226,981 bins 0.06 ms by thread, 0.10 ms by warp)
-  if (c->bcap <= 64 && c->nbins < 32768)
-    k_bin_sort_warp<<<nblocks((long)c->nbins * 32), BLOCK, 0, c->stream>>>(c->nbins, c->bcap, c->bin_count.p,
-                                                                            c->bins.p);
-  else
-    k_bin_sort<<<nblocks(c->nbins), BLOCK, 0, c->stream>>>(c->nbins, c->bcap, c->bin_count.p, c->bins.p);
+  launch_bin_sort(c, nullptr);
   CUDA_TRY(c, cudaGetLastError());
   return EPH_OK;
 }
@@ -1269,7 +1286,7 @@ int apply_list_skin(eph_ctx *c, double skin, bool user) {
   int r = configure_list(c);
   if (r) return r;
   if (was && !c->reuse) {  // back to the cutoff's bins
-    if ((r = set_bin_geometry(c, c->beta.r_cutoff))) return r;
+    if ((r = set_bin_geometry(c, pair_radius(c)))) return r;
     if (!c->bcap_user) c->bcap = auto_bcap(c);
     c->P.bcap = c->bcap;
     CUDA_TRY(c, c->bins.alloc((size_t)c->nbins * c->bcap));
@@ -1374,7 +1391,7 @@ int eph_autotune_list_skin(eph_ctx *c, const double *skins, int nskins, int step
     const double keep_s = c->lskin;
     const bool keep_u = c->lskin_user;
     c->lskin_user = true;
-    for (int k = 0; k < nskins && !applies; ++k) {
+    for (int k = 0; k < nskins && !applies && !c->eam; ++k) {
       c->lskin = skins[k];
       applies = skins[k] > 0.0 && want_list(c);
     }

@@ -198,12 +198,17 @@ int launch_pair_sweeps(eph_ctx *c, int xi_mode);
 // the engine's pair force for this step into f (plus the external force)
 // bins of edge >= r (1 + 5e-5), at least three per axis (all of P's bin geometry)
 int set_bin_geometry(eph_ctx *c, double r);
-// the df64 pair sums run (and k_bin writes the atoms' df64 records)
+// the df64 pair sums run
 bool df_active(const eph_ctx *c);
+// k_bin (or k_list_check) writes the atoms' df64 records: for those sums or
+// for the EAM engine's
+bool df_records_wanted(const eph_ctx *c);
 int launch_eam(eph_ctx *c);
 // the EAM pair list of the step (rows k * n + i, counts) if it holds every
-// candidate of the fix's density sweep
-bool eam_pair_list(const eph_ctx *c, const unsigned **pj, const int **ns);
+// candidate of the fix's density sweep; inner: the counts of those at the
+// front of the rows, where the list puts them apart (else null)
+bool eam_pair_list(const eph_ctx *c, const unsigned **pj, const int **ns, const int **inner);
+double eam_cutoff(const eph_ctx *c);  // its cut-off, 0 without one
 int eam_resize(eph_ctx *c);  // per-atom buffers of the pair force for c->n atoms
 void eam_free(eph_ctx *c);
 

@@ -188,6 +188,20 @@ DF_FN float rsqrt_estimate(float x) {
 #endif
 }
 
+// 1/sqrt(a) for a > 0 in the FP32 normal range from y ~ 1/sqrt(a.hi): one
+// Newton-Raphson step with its second-order term, y + y (t/2 + 3 t^2/8), t = 1 -
+// a y^2 with the products formed exactly (1 - p is exact, p being 1 within a
+// few ulps): what is left is the rounding of t and of the correction, ~2^-47
+DF_FN df rsqrt(df a, float y) {
+  float yy, ye, p, pe;
+  two_prod(y, y, yy, ye);
+  two_prod(a.hi, yy, p, pe);
+  const float t = ((1.0f - p) - pe) - fmaf(a.hi, ye, a.lo * yy);
+  df r;
+  fast_two_sum(y, y * fmaf(0.375f * t, t, 0.5f * t), r.hi, r.lo);
+  return r;
+}
+
 // sqrt(a) for a > 0 in the FP32 normal range from y ~ 1/sqrt(a.hi): the
 // estimate s0 = a.hi y, then twice s + y (a - s^2) / 2 (Karp and Markstein's
 // form of Newton's iteration, "High-precision division and square root",

@@ -178,6 +178,15 @@ __device__ __forceinline__ void pair_fixed(const StepParams &P, int4 a, int4 b, 
   }
 }
 
+// atom i's fixed-point position from its record
+__device__ __forceinline__ void own_fixed(const int4 *__restrict__ rec, int i, long long *xf) {
+  int4 a, b;
+  load_record(rec + 4 * (size_t)i, a, b);
+  xf[0] = ((long long)a.y << 32) | (unsigned)a.x;
+  xf[1] = ((long long)a.w << 32) | (unsigned)a.z;
+  xf[2] = ((long long)b.y << 32) | (unsigned)b.x;
+}
+
 // The record of atom i for the df64 pair sums, one 64-byte line half: {x lo,
 // x hi, y lo, y hi}, {z lo, z hi, element, moved}, velocity hi parts, velocity
 // lo parts.  Position in fixed point plus `image` boxes.

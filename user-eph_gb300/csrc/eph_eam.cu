@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "eph_candidates.cuh"
 #include "eph_ctx_impl.hpp"
 #include "eph_df64.cuh"
 #include "eph_df_pair.cuh"
@@ -28,7 +29,7 @@ struct EamDevice {
   DevBuf<float2> fpd;  // F'(rho_i) / dr as a double-float, gathered per pair
   DevBuf<double> fp, energy, esum;
   DevBuf<unsigned> pj;    // pair list, [kcap][n]
-  DevBuf<int> ns;         // pairs per atom
+  DevBuf<int> ns, ns_in;  // pairs per atom; with kept lists, those at the front of its rows
   int kcap = 0;
   int map[65] = {0};      // LAMMPS type -> setfl element
   double rc2_band = 0.0;  // FP32 candidate threshold
@@ -46,6 +47,7 @@ struct EamParams {
   float rc2_band;
   float inv_dr_hi, inv_dr_lo, rc2_hi, rc2_lo;  // 1/dr and rc^2 as double-floats
   int map[65];
+  int one;  // the one element of every type, or -1
 };
 
 // value and d/d(index) of a Hermite table at x (in units of the knot spacing)
@@ -239,213 +241,285 @@ __global__ void __launch_bounds__(128)
 
 // ---------------------------------------------- df64 pair sums (FAST mode)
 
-// herm() on a double-float table at q >= 0 (knot units): the interval from
-// the FP32 part of q settled by the sign of the double-float remainder, the
-// same clamps (at most the last interval, p at most 1), the value and the
-// derivative per knot unit
-__device__ __forceinline__ void herm_df(const float4 *__restrict__ t, int n, df64::df q, df64::df &v,
-                                        df64::df &dv) {
+// The interval m of a Hermite table of n knots at q >= 0 (knot units) and the
+// offset p in it: m from the FP32 part of q settled by the sign of the
+// double-float remainder, with herm()'s clamps (at most the last interval, p
+// at most 1)
+__device__ __forceinline__ void herm_place(int n, df64::df q, int &m, df64::df &p) {
   using namespace df64;
   const df one{1.0f, 0.0f};
   const float kr = floor_estimate(q.hi);
-  int m = floor_estimate_int(kr);
+  m = floor_estimate_int(kr);
   float th, te;
   two_sum(q.hi, -kr, th, te);
-  df p = make(th, te + q.lo);
-  if (lt(p, df{0.0f, 0.0f})) {
-    m -= 1;
-    p = add(p, one);
-  } else if (!lt(p, one)) {
-    m += 1;
-    p = sub(p, one);
+  p = make(th, te + q.lo);
+  if (!(p.hi >= 0.0f && p.hi < 1.0f) || (unsigned)m > (unsigned)(n - 2)) {  // rarely: at a knot or past the table
+    if (lt(p, df{0.0f, 0.0f})) {
+      m -= 1;
+      p = add(p, one);
+    } else if (!lt(p, one)) {
+      m += 1;
+      p = sub(p, one);
+    }
+    if (m > n - 2) {
+      p = add(p, df{(float)(m - (n - 2)), 0.0f});
+      m = n - 2;
+      if (!lt(p, one)) p = one;
+    }
+    if (m < 0) m = 0;
   }
-  if (m > n - 2) {
-    p = add(p, df{(float)(m - (n - 2)), 0.0f});
-    m = n - 2;
-    if (!lt(p, one)) p = one;
-  }
-  if (m < 0) m = 0;
+}
+
+// value of the table at (m, p)
+__device__ __forceinline__ df64::df herm_value(const float4 *__restrict__ t, int m, df64::df p) {
+  using namespace df64;
   float4 hi, lo;
   load_row(t + 2 * (size_t)m, hi, lo);
-  const df c0{hi.x, lo.x}, c1{hi.y, lo.y}, c2{hi.z, lo.z}, c3{hi.w, lo.w};
-  v = horner(c0, c1, c2, c3, p);
-  dv = fma(p, fma(p, mul(df{3.0f, 0.0f}, c3), mul(df{2.0f, 0.0f}, c2)), c1);
+  return horner(df{hi.x, lo.x}, df{hi.y, lo.y}, df{hi.z, lo.z}, df{hi.w, lo.w}, p);
 }
 
-// A pair's displacement as double-floats: from the atoms' fixed-point records
-// of this step when there are any (xf: atom i's; no FP64 work), else from the
-// FP64 positions as k_eam_density forms it
-__device__ __forceinline__ void pair_e_df(const StepParams &P, const int4 *__restrict__ rec, const long long *xf,
-                                          const D4 &xi, const D4 *__restrict__ x, unsigned j, unsigned code,
-                                          df64::df &ex, df64::df &ey, df64::df &ez) {
-  if (rec) {
-    long long e[3];
-    int4 ra, rb;
-    load_record(rec + 4 * (size_t)j, ra, rb);
-    pair_fixed(P, ra, rb, code, xf, e);
-    ex = fixed_df(e[0], P.fix_hi, P.fix_lo);
-    ey = fixed_df(e[1], P.fix_hi, P.fix_lo);
-    ez = fixed_df(e[2], P.fix_hi, P.fix_lo);
-  } else {
-    double a, b, c;
-    image_vector(P, xi, x[j], code, a, b, c);
-    ex = df64::from_double(a);
-    ey = df64::from_double(b);
-    ez = df64::from_double(c);
-  }
-}
-
-// atom i's fixed-point position from its record
-__device__ __forceinline__ void own_fixed(const int4 *__restrict__ rec, int i, long long *xf) {
-  const int4 a = rec[4 * (size_t)i], b = rec[4 * (size_t)i + 1];
-  xf[0] = ((long long)a.y << 32) | (unsigned)a.x;
-  xf[1] = ((long long)a.w << 32) | (unsigned)a.z;
-  xf[2] = ((long long)b.y << 32) | (unsigned)b.x;
-}
-
-// k_eam_density with the pair arithmetic in double-float: e from the FP64
-// positions (the periodic image added as k_eam_density adds it), then r^2,
-// the cut-off test, r and f_b(r) in df64, rho_i in blocked sums; F and F'
-// per atom in FP64; F' / dr also as a double-float for k_eam_force_df
-__global__ void __launch_bounds__(128)
-    k_eam_density_df(StepParams P, EamParams E, const D4 *__restrict__ x, const int *__restrict__ type,
-                     const int *__restrict__ bin_count, const BinEntry *__restrict__ bins,
-                     const int4 *__restrict__ atom_bin, const float4 *__restrict__ atom_off,
-                     unsigned *__restrict__ epj, int *__restrict__ ens, int kcap, double *__restrict__ fp,
-                     float2 *__restrict__ fpd, double *__restrict__ energy, unsigned *__restrict__ err,
-                     const int4 *__restrict__ rec) {
+// value and derivative per knot unit: Horner's scheme and, from its partial
+// sums, Horner's scheme of the derivative (synthetic division)
+__device__ __forceinline__ void herm_both(const float4 *__restrict__ t, int m, df64::df p, df64::df &v, df64::df &dv) {
   using namespace df64;
-  __shared__ unsigned s_cand[CAND_SMEM * 128];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t = threadIdx.x, nt = blockDim.x;
+  float4 hi, lo;
+  load_row(t + 2 * (size_t)m, hi, lo);
+  const df b3{hi.w, lo.w};
+  const df b2 = fma(p, b3, df{hi.z, lo.z});
+  const df b1 = fma(p, b2, df{hi.y, lo.y});
+  v = fma(p, b1, df{hi.x, lo.x});
+  dv = fma(p, fma(p, b3, b2), b1);
+}
+
+// resident blocks of 128 threads per SM the df64 sweeps are compiled for (GB300,
+// both sweeps at 256,000 atoms with 7 + 6 / 8 + 7 / 10 + 8 blocks: 655 / 645 / 671 us)
+#ifndef EPH_EAM_DENSITY_BLOCKS
+#define EPH_EAM_DENSITY_BLOCKS 8
+#endif
+#ifndef EPH_EAM_FORCE_BLOCKS
+#define EPH_EAM_FORCE_BLOCKS 7
+#endif
+
+// rho_i = sum_j f_b(r_ij) with the pair arithmetic in double-float and LANES
+// lanes per atom: the candidates from the bins of the step or the kept lists
+// (pair_candidates), e from the fixed-point positions, r^2, the cut-off test,
+// the in-cut-off pairs to the EAM pair list (row k at k * n + i), r and f_b(r)
+// in df64, rho_i in blocked sums; F and F' per atom in FP64; F' / dr also as a
+// double-float for k_eam_force_df.  ONE: every type is the same setfl element.
+// What bounds it: the candidates.  The 27 bins of 6.5 A hold 675 of them per
+// atom, of which 78-85 are pairs; the bins' search took two thirds of the
+// instructions (73,000 a warp), the kept lists leave 121 per atom.
+// GB300, 256,000 atoms: 989 us -> 285 (kept lists); where the bins are searched
+// every step, 16,384 atoms took both sweeps 536 us, now 100 (8 lanes).
+template <bool ONE, int LANES, bool LIST>
+__global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
+    k_eam_density_df(StepParams P, EamParams E, CandidateArgs C, const int *__restrict__ type, int *__restrict__ ens,
+                     int *__restrict__ ens_in, double *__restrict__ fp, float2 *__restrict__ fpd, double *__restrict__ energy) {
+  using namespace df64;
+  constexpr int CAP = LIST ? 0 : (LANES == 1 ? CAND_SMEM : CAND_SMEM * LANES - 1);
+  __shared__ unsigned s_cand[CAP ? CAND_SMEM * 128 : 1];
+  const int t = threadIdx.x, a = t / LANES, g = t % LANES;
+  const int i = blockIdx.x * (128 / LANES) + a;
   const bool valid = i < P.n;
-  auto cget = [&](int k) -> unsigned { return k < CAND_SMEM ? s_cand[k * nt + t] : epj[(size_t)k * P.n + i]; };
-  auto cset = [&](int k, unsigned u) {
-    if (k < CAND_SMEM)
-      s_cand[k * nt + t] = u;
-    else
-      epj[(size_t)k * P.n + i] = u;
-  };
-  const D4 xi = valid ? x[i] : D4{0.0, 0.0, 0.0, 0.0};
-  int4 Bi = make_int4(0, 0, 0, 0);
-  float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (valid) {
-    Bi = atom_bin[i];
-    oi = atom_off[i];
-  }
-  const int nc = eam_candidates(P, E, i, valid, Bi, oi, bin_count, bins, kcap, err, cset);
+  const size_t n = (size_t)P.n;
+  auto at = [&](int k) -> unsigned & { return s_cand[LANES == 1 ? k * 128 + t : a * CAP + k]; };
+  long long xi[3] = {0, 0, 0};
+  if (valid) own_fixed(C.rec, i, xi);
+  const unsigned *tail;
+  bool fresh;
+  const int nc = pair_candidates<LANES, LIST, CAP>(P, C, i, g, valid, valid, at, tail, fresh);
   __syncwarp();
-  long long xf[3] = {0, 0, 0};
-  if (rec && valid) own_fixed(rec, i, xf);
   const df rc2{E.rc2_hi, E.rc2_lo}, inv_dr{E.inv_dr_hi, E.inv_dr_lo};
   bsum rs = bsum_zero();
-  int ns = 0;
+  int ns = 0, far = 0;
   const int nmax = __reduce_max_sync(FULL, nc);
-  for (int k = 0; k < nmax; ++k) {
-    if (k >= nc) continue;
-    const unsigned u = cget(k);
-    const unsigned j = u & IDX_MASK;
-    df dx, dy, dz;
-    pair_e_df(P, rec, xf, xi, x, j, u >> IDX_BITS, dx, dy, dz);
-    const df r2 = dot3(dx, dy, dz, dx, dy, dz);
-    if (lt(r2, rc2)) {
-      epj[(size_t)ns * P.n + i] = u;  // ns <= k: the candidate there is consumed
-      ++ns;
-      df v, dv;
-      const df q = mul(df64::sqrt(r2, rsqrt_estimate(r2.hi)), inv_dr);
-      herm_df(E.fd + 2 * (size_t)E.map[type[j]] * E.nr, E.nr, q, v, dv);
-      acc_add(rs.blk, v);
-      if ((ns & 7) == 0) bsum_fold(rs);
+  auto cand = [&](int k) -> unsigned {
+    if (k >= nc) return CODE_NOSHIFT << IDX_BITS;  // atom 0, not counted
+    return k < CAP ? at(k) : tail[(size_t)k * n + i];
+  };
+  unsigned u = cand(g), u2 = cand(g + LANES);
+  int4 ra, rb;
+  load_record(C.rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
+  for (int k = g, m = 0; k - g < nmax; k += LANES, ++m) {
+    const unsigned uc = u;
+    const int4 ca = ra, cb = rb;
+    u = u2;
+    u2 = cand(k + 2 * LANES);
+    load_record(C.rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
+    long long ef[3];
+    pair_fixed(P, ca, cb, uc >> IDX_BITS, xi, ef);
+    const df ex = fixed_df(ef[0], P.fix_hi, P.fix_lo), ey = fixed_df(ef[1], P.fix_hi, P.fix_lo),
+             ez = fixed_df(ef[2], P.fix_hi, P.fix_lo);
+    const df r2 = dot3(ex, ey, ez, ex, ey, ez);
+    bool in = k < nc && lt(r2, rc2);
+    if (LIST) in = in && (fresh || cb.w == 0);  // a moved atom in a kept list is out of reach
+    const unsigned who = __ballot_sync(FULL, in);
+    if (who == 0u) continue;  // the lists' shell, together at their ends
+    // the pair's row: from the front, in lane order; with kept lists the pairs
+    // the fix's density sweep does not need go to the row's back
+    const bool out = LIST && in && !(r2.hi < P.rc2_band);
+    int slot = ns, back = far;
+    if (LANES > 1) {
+      const unsigned lane = t & 31, below = (1u << lane) - 1u;
+      const unsigned group = ((1u << LANES) - 1u) << (lane & ~(LANES - 1));
+      const unsigned outs = LIST ? __ballot_sync(FULL, out) & group : 0u, ins = who & group & ~outs;
+      slot += __popc(ins & below);
+      ns += __popc(ins);
+      if (LIST) {
+        back += __popc(outs & below);
+        far += __popc(outs);
+      }
+    } else {
+      ns += in && !out;
+      far += out;
     }
+    if (in) {
+      const int row = out ? C.kcap - 1 - back : slot;
+      if (ns + far <= C.kcap) C.pj[(size_t)row * n + i] = uc;  // front rows <= k: the candidate there is consumed
+      else atomicOr(C.err, ERR_PAIR_OVERFLOW);
+      const df r = mul(r2, rsqrt(r2, rsqrt_estimate(r2.hi)));
+      int mk;
+      df p;
+      herm_place(E.nr, mul(r, inv_dr), mk, p);
+      const int b = ONE ? E.one : E.map[type[uc & IDX_MASK]];
+      acc_add(rs.blk, herm_value(E.fd + 2 * (size_t)b * E.nr, mk, p));
+    }
+    if ((m & 7) == 7) bsum_fold(rs);
   }
-  if (!valid) return;
-  const double rho = to_double(bsum_value(rs));
-  ens[i] = ns;
-  const int a = E.map[type[i]];
+  double rho = to_double(bsum_value(rs));
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1) rho += __shfl_xor_sync(FULL, rho, o);
+  if (!valid || g != 0) return;
+  ns = ns < C.kcap ? ns : C.kcap;
+  ens[i] = LIST ? (ns + far < C.kcap ? ns + far : C.kcap) : ns;
+  if (LIST) ens_in[i] = ns;
+  const int el = ONE ? E.one : E.map[type[i]];
   double F, dF;
-  herm(E.F + (size_t)a * E.nrho, E.nrho, rho * E.inv_drho, F, dF);
+  herm(E.F + (size_t)el * E.nrho, E.nrho, rho * E.inv_drho, F, dF);
   dF *= E.inv_drho;
   if (rho > E.rho_max) F += dF * (rho - E.rho_max);
   fp[i] = dF;
-  const df g = from_double(dF * E.inv_dr);
-  fpd[i] = make_float2(g.hi, g.lo);
+  const df gd = from_double(dF * E.inv_dr);
+  fpd[i] = make_float2(gd.hi, gd.lo);
   energy[i] = F;
 }
 
-// k_eam_force with the pair arithmetic in double-float: per pair r, 1/r,
-// the Hermite tables f_b, f_a and z2r = r phi, dE/dr and (dE/dr / r) e in
-// df64, the force and 1/2 sum phi in blocked sums
-__global__ void __launch_bounds__(128)
-    k_eam_force_df(StepParams P, EamParams E, const D4 *__restrict__ x, const int *__restrict__ type,
-                   const unsigned *__restrict__ epj, const int *__restrict__ ens, const float2 *__restrict__ fpd,
-                   const D4 *__restrict__ fext, D4 *__restrict__ f, double *__restrict__ energy,
-                   const int4 *__restrict__ rec) {
+// k_eam_force with the pair arithmetic in double-float and LANES lanes per
+// atom: per pair 1/r (a Newton step on the FP32 estimate), r = r^2 / r, the
+// Hermite tables f_b, f_a and z2r = r phi at one interval and offset, dE/dr and
+// (dE/dr / r) e in df64, the force and 1/2 sum phi in blocked sums.  Bound by
+// FP32 issue: ~700 instructions per pair before (an interval and a scaled
+// derivative per table, square root and reciprocal apart), ~430 now.
+// GB300, 256,000 atoms: 596 -> 361 us.
+template <bool ONE, int LANES>
+__global__ void __launch_bounds__(128, EPH_EAM_FORCE_BLOCKS)
+    k_eam_force_df(StepParams P, EamParams E, const int *__restrict__ type, const unsigned *__restrict__ epj,
+                   const int *__restrict__ ens, const int *__restrict__ ens_in, int kcap,
+                   const float2 *__restrict__ fpd, const D4 *__restrict__ fext, D4 *__restrict__ f,
+                   double *__restrict__ energy, const int4 *__restrict__ rec) {
   using namespace df64;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P.n) return;
-  const D4 xi = x[i];
-  long long xf[3] = {0, 0, 0};
-  if (rec) own_fixed(rec, i, xf);
-  const int a = E.map[type[i]];
-  const float2 gi = fpd[i];
-  const df fpi{gi.x, gi.y}, inv_dr{E.inv_dr_hi, E.inv_dr_lo};
-  bsum sx = bsum_zero(), sy = bsum_zero(), sz = bsum_zero(), se = bsum_zero();
-  const int ns = ens[i];
-  for (int k = 0; k < ns; ++k) {
-    const unsigned u = epj[(size_t)k * P.n + i];
-    const unsigned j = u & IDX_MASK;
-    df dx, dy, dz;
-    pair_e_df(P, rec, xf, xi, x, j, u >> IDX_BITS, dx, dy, dz);
-    const df r2 = dot3(dx, dy, dz, dx, dy, dz);
-    const df r = df64::sqrt(r2, rsqrt_estimate(r2.hi));
-    const df rinv = recip(r, rcp_estimate(r.hi));
-    const df q = mul(r, inv_dr);
-    const int b = E.map[type[j]];
-    df fb, dfb, fa, dfa, z, dzz;
-    herm_df(E.fd + 2 * (size_t)b * E.nr, E.nr, q, fb, dfb);
-    dfa = dfb;
-    if (a != b) herm_df(E.fd + 2 * (size_t)a * E.nr, E.nr, q, fa, dfa);
-    const int hi = a > b ? a : b, lo = a > b ? b : a;
-    herm_df(E.zd + 2 * (size_t)(hi * (hi + 1) / 2 + lo) * E.nr, E.nr, q, z, dzz);
+  const int t = threadIdx.x, g = t % LANES;
+  const int i = blockIdx.x * (128 / LANES) + t / LANES;
+  const bool valid = i < P.n;
+  if (LANES == 1 && !valid) return;
+  long long xi[3] = {0, 0, 0};
+  int el = ONE ? E.one : 0, ns = 0, front = 0;
+  df fpi{0.0f, 0.0f};
+  if (valid) {
+    own_fixed(rec, i, xi);
+    if (!ONE) el = E.map[type[i]];
+    const float2 gi = fpd[i];
+    fpi = df{gi.x, gi.y};
+    ns = front = ens[i];
+    if (ens_in) front = ens_in[i];  // the others from the row's back
+  }
+  const df inv_dr{E.inv_dr_hi, E.inv_dr_lo};
+  bsum s[4] = {bsum_zero(), bsum_zero(), bsum_zero(), bsum_zero()};
+  const size_t n = (size_t)P.n;
+  auto pair = [&](int k) -> unsigned {
+    if (k >= ns) return CODE_NOSHIFT << IDX_BITS;
+    return epj[(size_t)(k < front ? k : kcap - 1 - (k - front)) * n + i];
+  };
+  unsigned u = pair(g), u2 = pair(g + LANES);
+  int4 ra, rb;
+  load_record(rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
+  float2 gn = fpd[u & IDX_MASK];
+  for (int k = g, m = 0; k < ns; k += LANES, ++m) {
+    const unsigned uc = u;
+    const int4 ca = ra, cb = rb;
+    const float2 gj = gn;
+    u = u2;
+    u2 = pair(k + 2 * LANES);
+    load_record(rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
+    gn = fpd[u & IDX_MASK];
+    long long ef[3];
+    pair_fixed(P, ca, cb, uc >> IDX_BITS, xi, ef);
+    const df ex = fixed_df(ef[0], P.fix_hi, P.fix_lo), ey = fixed_df(ef[1], P.fix_hi, P.fix_lo),
+             ez = fixed_df(ef[2], P.fix_hi, P.fix_lo);
+    const df r2 = dot3(ex, ey, ez, ex, ey, ez);
+    const df rinv = rsqrt(r2, rsqrt_estimate(r2.hi));
+    int mk;
+    df p;
+    herm_place(E.nr, mul(mul(r2, rinv), inv_dr), mk, p);
+    const int b = ONE ? el : E.map[type[uc & IDX_MASK]];
+    df fb, dfb, z, dz;
+    herm_both(E.fd + 2 * (size_t)b * E.nr, mk, p, fb, dfb);
+    const int hi = el > b ? el : b, lo = el > b ? b : el;
+    herm_both(E.zd + 2 * (size_t)(hi * (hi + 1) / 2 + lo) * E.nr, mk, p, z, dz);
+    // F'_a(rho_i) f_b' + F'_b(rho_j) f_a'
+    df emb;
+    if (ONE || el == b) {
+      emb = mul(add(fpi, df{gj.x, gj.y}), dfb);
+    } else {
+      df fa, dfa;
+      herm_both(E.fd + 2 * (size_t)el * E.nr, mk, p, fa, dfa);
+      emb = add(mul(fpi, dfb), mul(df{gj.x, gj.y}, dfa));
+    }
     const df phi = mul(z, rinv);
-    const df dphi = mul(sub(mul(dzz, inv_dr), phi), rinv);
-    const float2 gj = fpd[j];
-    const df dEdr = add(add(mul(fpi, dfb), mul(df{gj.x, gj.y}, dfa)), dphi);
-    const df s = mul(dEdr, rinv);
-    acc_fma(sx.blk, s, dx);
-    acc_fma(sy.blk, s, dy);
-    acc_fma(sz.blk, s, dz);
-    acc_add(se.blk, df{0.5f * phi.hi, 0.5f * phi.lo});
-    if ((k & 7) == 7) {
-      bsum_fold(sx);
-      bsum_fold(sy);
-      bsum_fold(sz);
-      bsum_fold(se);
+    const df dphi = mul(fma(dz, inv_dr, neg(phi)), rinv);
+    const df sc = mul(add(emb, dphi), rinv);
+    acc_fma(s[0].blk, sc, ex);
+    acc_fma(s[1].blk, sc, ey);
+    acc_fma(s[2].blk, sc, ez);
+    acc_add(s[3].blk, df{0.5f * phi.hi, 0.5f * phi.lo});
+    if ((m & 7) == 7) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) bsum_fold(s[q]);
     }
   }
-  D4 out{to_double(bsum_value(sx)), to_double(bsum_value(sy)), to_double(bsum_value(sz)), 0.0};
+  double w[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    w[q] = to_double(bsum_value(s[q]));
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) w[q] += __shfl_xor_sync(FULL, w[q], o);
+  }
+  if (!valid || g != 0) return;
+  D4 out{w[0], w[1], w[2], 0.0};
   if (fext) {
-    const D4 g = fext[i];
-    out.x += g.x;
-    out.y += g.y;
-    out.z += g.z;
+    const D4 e = fext[i];
+    out.x += e.x;
+    out.y += e.y;
+    out.z += e.z;
   }
   f[i] = out;
-  energy[i] += to_double(bsum_value(se));
+  energy[i] += w[3];
 }
 
-// sum of the per-atom energies, one block, fixed order
+// sum of the per-atom energies in a fixed order: ENERGY_BLOCKS partial sums,
+// then theirs (one block over all atoms took 478 us at 256,000 atoms, GB300)
+constexpr int ENERGY_BLOCKS = 256;
 __global__ void k_eam_energy_sum(const double *__restrict__ e, int n, double *__restrict__ out) {
   __shared__ double s[256];
   double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) acc += e[i];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) acc += e[i];
   s[threadIdx.x] = acc;
   __syncthreads();
   for (int h = blockDim.x / 2; h > 0; h >>= 1) {
     if ((int)threadIdx.x < h) s[threadIdx.x] += s[threadIdx.x + h];
     __syncthreads();
   }
-  if (threadIdx.x == 0) *out = s[0];
+  if (threadIdx.x == 0) out[blockIdx.x] = s[0];
 }
 
 EamParams eam_params(const eph_ctx *c) {
@@ -470,6 +544,9 @@ EamParams eam_params(const eph_ctx *c) {
   E.rc2_hi = rc2.hi;
   E.rc2_lo = rc2.lo;
   std::memcpy(E.map, d->map, sizeof(E.map));
+  E.one = d->map[1];
+  for (int t = 2; t <= c->ntypes; ++t)
+    if (d->map[t] != E.one) E.one = -1;
   return E;
 }
 
@@ -501,10 +578,37 @@ int upload_table(eph_ctx *c, DevBuf<D4> &dst, const std::vector<std::vector<doub
   return EPH_OK;
 }
 
+// Lanes per atom of the df64 EAM sweeps (measured on GB300, both sweeps, us
+// with 2 / 4 / 8 / 16 lanes: 2,048 atoms 212 / 117 / 71 / 49, 6,912 atoms 218 /
+// 126 / 83 / 68, 16,384 atoms 122 / 80 / 66 / 76, 32,000 atoms 143 / 115 / 114 /
+// 125, 131,072 atoms 364 / 351 / 362 / 417, 256,000 atoms 649 / 642 / 671 / 789,
+// 500,000 atoms 1,173 / 1,210 / 1,280 / 1,518; one lane 1,219 there)
+int eam_lanes(const eph_ctx *c) {
+  return c->n <= 10000 ? 16 : (c->n <= 32000 ? 8 : (c->n <= 360000 ? 4 : 2));
+}
+
+template <bool ONE, int LANES>
+void launch_eam_df(eph_ctx *c, const EamParams &E, const CandidateArgs &C, const D4 *fext) {
+  EamDevice *d = c->eam;
+  const int nb = nblocks((long)c->n * LANES);
+  if (c->reuse)
+    k_eam_density_df<ONE, LANES, true><<<nb, BLOCK, 0, c->stream>>>(c->P, E, C, c->type.p, d->ns.p, d->ns_in.p,
+                                                                    d->fp.p, d->fpd.p,
+                                                                    d->energy.p);
+  else
+    k_eam_density_df<ONE, LANES, false><<<nb, BLOCK, 0, c->stream>>>(c->P, E, C, c->type.p, d->ns.p, nullptr, d->fp.p,
+                                                                     d->fpd.p, d->energy.p);
+  k_eam_force_df<ONE, LANES><<<nb, BLOCK, 0, c->stream>>>(c->P, E, c->type.p, d->pj.p, d->ns.p,
+                                                          c->reuse ? d->ns_in.p : nullptr, d->kcap, d->fpd.p, fext,
+                                                          c->f.p, d->energy.p, c->dfrec.p);
+}
+
 }  // namespace
 
 namespace ephgb {
 namespace ctxi {
+
+double eam_cutoff(const eph_ctx *c) { return c->eam ? c->eam->host.rc : 0.0; }
 
 void eam_free(eph_ctx *c) {
   delete c->eam;
@@ -518,6 +622,7 @@ int eam_resize(eph_ctx *c) {
   CUDA_TRY(c, d->fp.alloc(N));
   CUDA_TRY(c, d->energy.alloc(N));
   CUDA_TRY(c, d->ns.alloc(N));
+  CUDA_TRY(c, d->ns_in.alloc(N));
   CUDA_TRY(c, d->fpd.alloc(N));
   CUDA_TRY(c, cudaMemset(d->energy.p, 0, sizeof(double) * N));
   // pair rows from the number density: twice the cut-off sphere, plus slack
@@ -528,7 +633,7 @@ int eam_resize(eph_ctx *c) {
   return EPH_OK;
 }
 
-bool eam_pair_list(const eph_ctx *c, const unsigned **pj, const int **ns) {
+bool eam_pair_list(const eph_ctx *c, const unsigned **pj, const int **ns, const int **inner) {
   const EamDevice *d = c->eam;
   if (!d || !d->pj.p || !d->ns.p || d->ns.n < (size_t)c->n) return false;
   // every pair within the fix's FP32 candidate threshold must be in the list
@@ -536,6 +641,7 @@ bool eam_pair_list(const eph_ctx *c, const unsigned **pj, const int **ns) {
   if (!((double)c->P.rc2_band * (1.0 + 1e-5) < d->host.rc * d->host.rc)) return false;
   *pj = d->pj.p;
   *ns = d->ns.p;
+  *inner = c->reuse ? d->ns_in.p : nullptr;
   return true;
 }
 
@@ -548,13 +654,36 @@ int launch_eam(eph_ctx *c) {
   ps.launched(2);
   const D4 *fext = c->have_fext ? c->fext.p : nullptr;
   if (c->mode == EPH_MODE_FAST && c->pair_arith == EPH_PAIRS_DF64) {
-    // the atoms' df64 records of this step's bins, where k_bin wrote them
-    const int4 *rec = ctxi::df_active(c) ? c->dfrec.p : nullptr;
-    k_eam_density_df<<<nb, BLOCK, 0, c->stream>>>(c->P, E, c->x.p, c->type.p, c->bin_count.p, c->bins.p,
-                                                   c->atom_bin.p, c->atom_off.p, d->pj.p, d->ns.p, d->kcap, d->fp.p,
-                                                   d->fpd.p, d->energy.p, c->d_err.p, rec);
-    k_eam_force_df<<<nb, BLOCK, 0, c->stream>>>(c->P, E, c->x.p, c->type.p, d->pj.p, d->ns.p, d->fpd.p, fext,
-                                                 c->f.p, d->energy.p, rec);
+    CandidateArgs C{};
+    C.bin_count = c->bin_count.p;
+    C.bins = c->bins.p;
+    C.atom_bin = c->atom_bin.p;
+    C.atom_off = c->atom_off.p;
+    C.rec = c->dfrec.p;
+    C.x = c->x.p;
+    C.err = c->d_err.p;
+    C.pj = d->pj.p;
+    C.kcap = d->kcap;
+    C.band = E.rc2_band;
+    C.rc2 = E.rc2;
+    C.cl = c->cl.p;
+    C.cl_n = c->cl_n.p;
+    C.state = c->state.p;
+    C.rb = c->rb.p;
+    C.flist = c->flist.p;
+    C.xref = c->xref.p;
+    const int lanes = eam_lanes(c);
+    if (E.one >= 0) {
+      if (lanes == 2) launch_eam_df<true, 2>(c, E, C, fext);
+      else if (lanes == 4) launch_eam_df<true, 4>(c, E, C, fext);
+      else if (lanes == 8) launch_eam_df<true, 8>(c, E, C, fext);
+      else launch_eam_df<true, 16>(c, E, C, fext);
+    } else {
+      if (lanes == 2) launch_eam_df<false, 2>(c, E, C, fext);
+      else if (lanes == 4) launch_eam_df<false, 4>(c, E, C, fext);
+      else if (lanes == 8) launch_eam_df<false, 8>(c, E, C, fext);
+      else launch_eam_df<false, 16>(c, E, C, fext);
+    }
   } else {
     k_eam_density<<<nb, BLOCK, 0, c->stream>>>(c->P, E, c->x.p, c->type.p, c->bin_count.p, c->bins.p,
                                                 c->atom_bin.p, c->atom_off.p, d->pj.p, d->ns.p, d->kcap, d->fp.p,
@@ -594,14 +723,14 @@ int eph_set_pair_eam(eph_ctx *c, const char *path, int ntypes, const char *const
     d->map[t] = m;
   }
   ctxi::eam_free(c);
-  ctxi::drop_list(c);  // the pair force needs this step's bins every step
+  ctxi::drop_list(c);  // a larger radius: configured with the atoms
   c->eam = d;
   int r;
   CUDA_TRY(c, cudaSetDevice(c->device));
   if ((r = upload_table(c, d->F, d->host.F)) || (r = upload_table(c, d->f, d->host.f, &d->fd)) ||
       (r = upload_table(c, d->z2r, d->host.z2r, &d->zd)))
     return r;
-  CUDA_TRY(c, d->esum.alloc(1));
+  CUDA_TRY(c, d->esum.alloc(1 + ENERGY_BLOCKS));
   d->rc2_band = d->host.rc * d->host.rc * (1.0 + 1e-4);
   // the bins must hold every pair within the larger of the two cutoffs (all
   // of their geometry: the FP64, FP32 and double-float bin edges)
@@ -618,7 +747,9 @@ int eph_pair_energy(eph_ctx *c, double *E) {
   if (!c || !E) return EPH_ERR_ARG;
   *E = 0.0;
   if (!c->eam || !c->eam->energy.p) return EPH_OK;
-  k_eam_energy_sum<<<1, 256, 0, c->stream>>>(c->eam->energy.p, c->n, c->eam->esum.p);
+  double *part = c->eam->esum.p + 1;
+  k_eam_energy_sum<<<ENERGY_BLOCKS, 256, 0, c->stream>>>(c->eam->energy.p, c->n, part);
+  k_eam_energy_sum<<<1, 256, 0, c->stream>>>(part, ENERGY_BLOCKS, c->eam->esum.p);
   CUDA_TRY(c, cudaMemcpyAsync(E, c->eam->esum.p, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   return ctxi::check_device(c);
 }

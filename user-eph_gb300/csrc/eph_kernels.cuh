@@ -14,6 +14,7 @@
 // explicitly.
 #pragma once
 
+#include "eph_candidates.cuh"
 #include "eph_device.cuh"
 #include "eph_df64.cuh"
 #include "eph_df_pair.cuh"
@@ -233,216 +234,13 @@ __global__ void k_bin(StepParams P, D4 *__restrict__ x, D4 *__restrict__ xhold, 
 
 // -------------------------------------------------------- density sweep
 
-// Append u to the candidate list of the lane's atom where `take`: with one
-// lane per atom after the lane's own nc entries; with LANES lanes, which share
-// the atom's list and all call this together, in lane order (nc, the list's
-// length, stays the same on the atom's lanes).  At most cap entries.
-template <int LANES, class Set>
-__device__ __forceinline__ void append_candidate(bool take, unsigned u, int &nc, int cap, Set cset,
-                                                 unsigned *__restrict__ err) {
-  int pos = nc;
-  if (LANES == 1) {
-    if (take && nc < cap) ++nc;
-  } else {
-    const int lane = threadIdx.x & 31;
-    const unsigned mine = (LANES == 32 ? 0xffffffffu : ((1u << LANES) - 1u) << (lane & ~(LANES - 1)));
-    const unsigned who = __ballot_sync(0xffffffffu, take) & mine;
-    pos += __popc(who & ((1u << lane) - 1u));
-    nc += __popc(who);
-    nc = nc < cap ? nc : cap;
-  }
-  if (take) {
-    if (pos < cap) cset(pos, u);
-    else atomicOr(err, ERR_PAIR_OVERFLOW);
-  }
-}
-
-// Candidates of atom i in the bin at stencil offset (dx, dy, dz) from its
-// own: the entries whose FP32 distance passes the widened cut-off, appended
-// through cset (FAST: in bin order; EXACT: kept in ascending neighbour index
-// by insertion) while nc < cap.  Contains a warp-wide max: every lane of the
-// warp calls it the same number of times (look = false for a lane with
-// nothing to search).  r2band is the FP32 threshold (the cutoff's, or the
-// candidate list's); with SKIP, entries of atoms flagged as moved (skip[j] &
-// 2) are left out.
-template <bool FAST, bool SKIP = false, class Get, class Set>
-__device__ __forceinline__ void bin_candidates(const StepParams &P, int i, bool look, int4 Bi, float4 oi, int dx,
-                                               int dy, int dz, const int *__restrict__ bin_count,
-                                               const BinEntry *__restrict__ bins, unsigned *__restrict__ err,
-                                               int &nc, int cap, Get cget, Set cset, float r2band,
-                                               const int *__restrict__ skip = nullptr, float r2lo = -1.f) {
-  const int Tz = Bi.z + dz, tz = Tz < 0 ? Tz + P.nb[2] : (Tz >= P.nb[2] ? Tz - P.nb[2] : Tz);
-  const int kz = Tz < 0 ? -1 : (Tz >= P.nb[2] ? 1 : 0);
-  const float bz = (float)dz * P.wf[2] - oi.z;
-  const int Ty = Bi.y + dy, ty = Ty < 0 ? Ty + P.nb[1] : (Ty >= P.nb[1] ? Ty - P.nb[1] : Ty);
-  const int ky = Ty < 0 ? -1 : (Ty >= P.nb[1] ? 1 : 0);
-  const float by = (float)dy * P.wf[1] - oi.y;
-  const int Tx = Bi.x + dx, tx = Tx < 0 ? Tx + P.nb[0] : (Tx >= P.nb[0] ? Tx - P.nb[0] : Tx);
-  const int kx = Tx < 0 ? -1 : (Tx >= P.nb[0] ? 1 : 0);
-  const float bx = (float)dx * P.wf[0] - oi.x;
-  const int flat = tx + P.nb[0] * (ty + P.nb[1] * tz);
-  int cnt = 0;
-  if (look) {
-    cnt = bin_count[flat];
-    cnt = cnt < P.bcap ? cnt : P.bcap;
-  }
-  const int cmax = __reduce_max_sync(0xffffffffu, cnt);
-  const BinEntry *be = bins + (size_t)flat * P.bcap;
-  for (int s = 0; s < cmax; ++s) {
-    if (s < cnt) {
-      const BinEntry b = be[s];
-      const unsigned j = b.idx & IDX_MASK;
-      const float ex = bx + b.ox, ey = by + b.oy, ez = bz + b.oz;
-      const float r2 = ex * ex + ey * ey + ez * ez;
-      if (j != (unsigned)i && r2 < r2band && r2 >= r2lo && !(SKIP && (skip[j] & 2))) {
-        const unsigned wc = b.idx >> IDX_BITS;
-        const int mx = kx - ((int)(wc % 3u) - 1), my = ky - ((int)((wc / 3u) % 3u) - 1),
-                  mz = kz - ((int)(wc / 9u) - 1);
-        if (mx < -1 || mx > 1 || my < -1 || my > 1 || mz < -1 || mz > 1) {
-          atomicOr(err, ERR_DRIFT);
-        } else if (nc >= cap) {
-          atomicOr(err, ERR_PAIR_OVERFLOW);
-        } else {
-          const unsigned u = j | ((unsigned)((mx + 1) + 3 * (my + 1) + 9 * (mz + 1)) << IDX_BITS);
-          int pos = nc++;
-          if (!FAST) {  // ascending neighbour index
-            while (pos > 0) {
-              const unsigned prev = cget(pos - 1);
-              if ((prev & IDX_MASK) <= j) break;
-              cset(pos, prev);
-              --pos;
-            }
-          }
-          cset(pos, u);
-        }
-      }
-    }
-  }
-}
-
-// bin_candidates (FAST) over all 27 bins with LANES lanes per atom: lane g
-// takes bins g, g + LANES, ... of the stencil and the lanes append to the
-// atom's one list what `keep` does not refuse (a candidate and its FP32 r^2).
-// Every lane of the warp calls it.
-struct KeepAll {
-  __device__ bool operator()(unsigned, float) const { return true; }
-};
-template <int LANES, bool SKIP = false, class Set, class Keep = KeepAll>
-__device__ __forceinline__ void shared_candidates(const StepParams &P, int i, bool active, int4 Bi, float4 oi,
-                                                  const int *__restrict__ bin_count,
-                                                  const BinEntry *__restrict__ bins, unsigned *__restrict__ err,
-                                                  int &nc, int cap, Set cset, float r2band,
-                                                  const int *__restrict__ skip = nullptr, float r2lo = -1.f,
-                                                  Keep keep = Keep()) {
-  constexpr int CHUNK = 4;
-  const int g = (int)threadIdx.x & (LANES - 1);
-  for (int m = 0; m < (27 + LANES - 1) / LANES; ++m) {
-    const int b = g + m * LANES;
-    const bool look = active && b < 27;
-    const int bb = b < 27 ? b : 13, dx = bb % 3 - 1, dy = (bb / 3) % 3 - 1, dz = bb / 9 - 1;
-    const int Tz = Bi.z + dz, tz = Tz < 0 ? Tz + P.nb[2] : (Tz >= P.nb[2] ? Tz - P.nb[2] : Tz);
-    const int Ty = Bi.y + dy, ty = Ty < 0 ? Ty + P.nb[1] : (Ty >= P.nb[1] ? Ty - P.nb[1] : Ty);
-    const int Tx = Bi.x + dx, tx = Tx < 0 ? Tx + P.nb[0] : (Tx >= P.nb[0] ? Tx - P.nb[0] : Tx);
-    const int kz = Tz < 0 ? -1 : (Tz >= P.nb[2] ? 1 : 0), ky = Ty < 0 ? -1 : (Ty >= P.nb[1] ? 1 : 0),
-              kx = Tx < 0 ? -1 : (Tx >= P.nb[0] ? 1 : 0);
-    const float bx = (float)dx * P.wf[0] - oi.x, by = (float)dy * P.wf[1] - oi.y, bz = (float)dz * P.wf[2] - oi.z;
-    const int flat = tx + P.nb[0] * (ty + P.nb[1] * tz);
-    const BinEntry *be = bins + (size_t)flat * P.bcap;
-    // entries CHUNK at a time, the first ones beside the count (slots past it
-    // are read, not used): one memory latency per chunk instead of per entry
-    BinEntry e[CHUNK];
-#pragma unroll
-    for (int c = 0; c < CHUNK; ++c) e[c] = be[c < P.bcap ? c : 0];
-    int cnt = 0;
-    if (look) {
-      cnt = bin_count[flat];
-      cnt = cnt < P.bcap ? cnt : P.bcap;
-    }
-    const int cmax = __reduce_max_sync(0xffffffffu, cnt);
-    for (int s0 = 0; s0 < cmax; s0 += CHUNK) {
-      if (s0) {
-#pragma unroll
-        for (int c = 0; c < CHUNK; ++c)
-          if (s0 + c < cnt) e[c] = be[s0 + c];
-      }
-#pragma unroll
-      for (int c = 0; c < CHUNK; ++c) {
-        bool take = false;
-        unsigned u = 0;
-        if (s0 + c < cnt) {
-          const unsigned j = e[c].idx & IDX_MASK;
-          const float ex = bx + e[c].ox, ey = by + e[c].oy, ez = bz + e[c].oz;
-          const float r2 = ex * ex + ey * ey + ez * ez;
-          if (j != (unsigned)i && r2 < r2band && r2 >= r2lo && !(SKIP && (skip[j] & 2))) {
-            const unsigned wc = e[c].idx >> IDX_BITS;
-            const int mx = kx - ((int)(wc % 3u) - 1), my = ky - ((int)((wc / 3u) % 3u) - 1),
-                      mz = kz - ((int)(wc / 9u) - 1);
-            take = mx >= -1 && mx <= 1 && my >= -1 && my <= 1 && mz >= -1 && mz <= 1;
-            if (!take) atomicOr(err, ERR_DRIFT);
-            u = j | ((unsigned)((mx + 1) + 3 * (my + 1) + 9 * (mz + 1)) << IDX_BITS);
-            take = take && keep(u, r2);
-          }
-        }
-        append_candidate<LANES>(take, u, nc, cap, cset, err);
-      }
-    }
-  }
-}
-
-// Pass 1 of the density sweep for atom i: the candidates of the 27 bins
-// around its own within the FP32 thresholds r2lo <= r^2 < r2band, appended
-// after the first nc0 (at most cap in all).  Returns their number.
-template <bool FAST, bool SKIP = false, class Get, class Set>
-__device__ __forceinline__ int collect_candidates(const StepParams &P, int i, bool active, int4 Bi, float4 oi,
-                                                  const int *__restrict__ bin_count,
-                                                  const BinEntry *__restrict__ bins, unsigned *__restrict__ err,
-                                                  Get cget, Set cset, float r2band, int cap,
-                                                  const int *__restrict__ skip = nullptr, float r2lo = -1.f,
-                                                  int nc0 = 0) {
-  int nc = nc0;
-  for (int dz = -1; dz <= 1; ++dz)
-    for (int dy = -1; dy <= 1; ++dy)
-      for (int dx = -1; dx <= 1; ++dx)
-        bin_candidates<FAST, SKIP>(P, i, active, Bi, oi, dx, dy, dz, bin_count, bins, err, nc, cap, cget, cset,
-                                   r2band, skip, r2lo);
-  return nc;
-}
-
-// Pass 1 from the standalone engine's EAM pair list of this step
-// (k_eam_density's rows: every pair within the EAM cut-off, which exceeds
-// r2band): its entries within the FP32 threshold r2band, from the high words
-// of the fixed-point positions -- the candidates of the bin search, without
-// scanning the bins.  Lane g of the atom's LANES takes entries g, g + LANES,
-// ....
-template <int LANES, class Set>
-__device__ __forceinline__ void list_candidates(const StepParams &P, int i, bool active, const long long *xi,
-                                                const unsigned *__restrict__ elist, const int *__restrict__ ens,
-                                                const int4 *__restrict__ rec, unsigned *__restrict__ err, int &nc,
-                                                int cap, Set cset, float r2band) {
-  const int g = (int)threadIdx.x & (LANES - 1);
-  const int ne = active ? ens[i] : 0;
-  const int nmax = __reduce_max_sync(0xffffffffu, ne);
-  for (int k = g; k - g < nmax; k += LANES) {
-    bool take = false;
-    unsigned u = 0;
-    if (k < ne) {
-      u = elist[(size_t)k * P.n + i];
-      long long e[3];
-      int4 ra, rb;
-      load_record(rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
-      pair_fixed(P, ra, rb, u >> IDX_BITS, xi, e);
-      const float ex = (float)(int)(e[0] >> 32) * P.fix_hi, ey = (float)(int)(e[1] >> 32) * P.fix_hi,
-                  ez = (float)(int)(e[2] >> 32) * P.fix_hi;
-      take = ex * ex + ey * ey + ez * ez < r2band;
-    }
-    append_candidate<LANES>(take, u, nc, cap, cset, err);
-  }
-}
-
-// The same sort with one warp per bin, for bins of at most 64 entries: lane l
-// holds entries l and l + 32, each entry's place is the number of entries
-// with a smaller atom index (indices are distinct), found by broadcasting
-// every entry's key across the warp; all loads happen before any store.
+// Sorts every bin's entries by atom index with one warp per bin, for bins of
+// at most 32 R entries: lane l holds entries l, l + 32, ..., each entry's place
+// is the number of entries with a smaller atom index (indices are distinct),
+// found by broadcasting every entry's key across the warp; all loads happen
+// before any store.
+constexpr int SORT_WARP_MAX = 128;
+template <int R>
 __global__ void k_bin_sort_warp(int nbins, int bcap, const int *__restrict__ bin_count, BinEntry *__restrict__ bins,
                                 const int *__restrict__ gate = nullptr) {
   if (gate && !*gate) return;
@@ -452,24 +250,32 @@ __global__ void k_bin_sort_warp(int nbins, int bcap, const int *__restrict__ bin
   int cnt = bin_count[w];
   cnt = cnt < bcap ? cnt : bcap;
   BinEntry *e = bins + (size_t)w * bcap;
-  const bool h0 = lane < cnt, h1 = lane + 32 < cnt;
-  BinEntry a{}, b{};
-  if (h0) a = e[lane];
-  if (h1) b = e[lane + 32];
-  const unsigned ka = h0 ? (a.idx & IDX_MASK) : 0xffffffffu, kb = h1 ? (b.idx & IDX_MASK) : 0xffffffffu;
-  int ra = 0, rb = 0;
-  for (int s = 0; s < 32; ++s) {
-    const unsigned k0 = __shfl_sync(0xffffffffu, ka, s), k1 = __shfl_sync(0xffffffffu, kb, s);
-    ra += (k0 < ka) + (k1 < ka);
-    rb += (k0 < kb) + (k1 < kb);
+  BinEntry b[R];
+  unsigned key[R];
+  int place[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    b[r] = BinEntry{};
+    if (lane + 32 * r < cnt) b[r] = e[lane + 32 * r];
+    key[r] = lane + 32 * r < cnt ? (b[r].idx & IDX_MASK) : 0xffffffffu;
+    place[r] = 0;
+  }
+  const int most = cnt < 32 ? cnt : 32;
+  for (int s = 0; s < most; ++s) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const unsigned k = __shfl_sync(0xffffffffu, key[r], s);
+#pragma unroll
+      for (int q = 0; q < R; ++q) place[q] += k < key[q];
+    }
   }
   __syncwarp();
-  if (h0) e[ra] = a;
-  if (h1) e[rb] = b;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (lane + 32 * r < cnt) e[place[r]] = b[r];
 }
 
-// Sort every bin's entries by atom index (one thread per bin, a handful of
-// entries each), so the candidate order below is fixed run to run.
+// The same with one thread per bin (a handful of entries each), so the candidate order below is fixed run to run.
 __global__ void k_bin_sort(int nbins, int bcap, const int *__restrict__ bin_count, BinEntry *__restrict__ bins,
                            const int *__restrict__ gate = nullptr) {
   if (gate && !*gate) return;
@@ -782,7 +588,8 @@ __global__ void __launch_bounds__(tpa_threads(TPA)) k_density_tpa(
     D4 *__restrict__ Bw, double *__restrict__ rho_out, double *__restrict__ beta_out, int *__restrict__ cell,
     double *__restrict__ Te_i, int *__restrict__ wrapflag, unsigned *__restrict__ err,
     unsigned long long *__restrict__ counters, const D4 *__restrict__ v, D4 *__restrict__ Mm,
-    D4 *__restrict__ G) {
+    D4 *__restrict__ G, const unsigned *__restrict__ elist, const int *__restrict__ ens,
+    const int4 *__restrict__ rec) {
   constexpr int NA = 128 / TPA;  // atoms per block
   constexpr int NSUM = FUSE_W ? 9 : 1;
   __shared__ __align__(16) unsigned s_cand[NA * (KMAX + 1)];
@@ -822,14 +629,21 @@ __global__ void __launch_bounds__(tpa_threads(TPA)) k_density_tpa(
       oi = atom_off[i];
     }
     const float sure = (float)(P.rc2 * (1.0 - 1e-4));
-    shared_candidates<TPA>(
-        P, i, active, Bi, oi, bin_count, bins, err, ns, P.kcap, [&](int k, unsigned u) { list[k] = u; }, P.rc2_band,
-        nullptr, -1.f, [&](unsigned u, float r2) {
-          if (r2 < sure) return true;
-          double ex, ey, ez;
-          density_vector(P, xi, x[u & IDX_MASK], u >> IDX_BITS, ex, ey, ez);
-          return below(dot3_fma(ex, ey, ez, ex, ey, ez), P.rc2);
-        });
+    auto set = [&](int k, unsigned u) { list[k] = u; };
+    auto inside = [&](unsigned u, float r2) {
+      if (r2 < sure) return true;
+      double ex, ey, ez;
+      density_vector(P, xi, x[u & IDX_MASK], u >> IDX_BITS, ex, ey, ez);
+      return below(dot3_fma(ex, ey, ez, ex, ey, ez), P.rc2);
+    };
+    if (elist) {  // the engine's EAM pair list of this step
+      long long xf[3] = {0, 0, 0};
+      if (valid) own_fixed(rec, i, xf);
+      list_candidates<TPA>(P, i, active, xf, elist, ens, rec, err, ns, P.kcap, set, P.rc2_band, inside);
+    } else {
+      shared_candidates<TPA>(P, i, active, Bi, oi, bin_count, bins, err, ns, P.kcap, set, P.rc2_band, nullptr, -1.f,
+                             inside);
+    }
   }
   __syncwarp();
   double rho = 0.0, Sx = 0.0, Sy = 0.0, Sz = 0.0;
@@ -899,56 +713,11 @@ __global__ void __launch_bounds__(tpa_threads(TPA)) k_density_tpa(
 // cutoff), and e = (x_j +- L) - x_i rounds as the engine's ghost atoms give
 // it.
 
-__device__ __forceinline__ double min_image(double d, double L, double h) {
-  return d > h ? d - L : (d < -h ? d + L : d);
-}
-
-// the boxes min_image adds to d
-__device__ __forceinline__ int image_count(double d, double h) { return d > h ? -1 : (d < -h ? 1 : 0); }
-
-// The 3x3x3 image code of x_j seen from x_i: the image of x_j within half a
-// box of x_i on every axis, decided in FP32 (the box is at least three list
-// radii wide, so a pair within the list radius is far from the threshold).
-// The pair vector then comes from density_vector, the rounding of the bin
-// search path.
-__device__ __forceinline__ unsigned image_code(const StepParams &P, float xi, float yi, float zi, const D4 &xj) {
-  const float dx = float_bits(xj.x) - xi, dy = float_bits(xj.y) - yi, dz = float_bits(xj.z) - zi;
-  const int mx = dx > P.half_prdf[0] ? -1 : (dx < -P.half_prdf[0] ? 1 : 0);
-  const int my = dy > P.half_prdf[1] ? -1 : (dy < -P.half_prdf[1] ? 1 : 0);
-  const int mz = dz > P.half_prdf[2] ? -1 : (dz < -P.half_prdf[2] ? 1 : 0);
-  return (unsigned)((mx + 1) + 3 * (my + 1) + 9 * (mz + 1));
-}
-
-// The bin and FP32 offset of a position wrapped into the box (an atom whose
-// bins entry is stale: it moved since the build), and by how many boxes
-__device__ __forceinline__ void current_bin(const StepParams &P, const D4 &xi, int4 &B, float4 &o,
-                                            int *image = nullptr) {
-  const double p[3] = {xi.x, xi.y, xi.z};
-  int b[3];
-  float of[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    double q = p[k] - P.lo[k];
-    const double turns = floor(q / P.prd[k]);
-    q -= turns * P.prd[k];
-    if (image) image[k] = -(int)turns - (q >= P.prd[k] ? 1 : 0);  // boxes added to p
-    if (q >= P.prd[k]) q -= P.prd[k];
-    if (q < 0.0) q = 0.0;
-    int bb = (int)floor(q * P.inv_w[k]);
-    bb = bb < 0 ? 0 : (bb >= P.nb[k] ? P.nb[k] - 1 : bb);
-    b[k] = bb;
-    of[k] = (float)(q - (double)bb * P.w[k]);
-  }
-  B = make_int4(b[0], b[1], b[2], b[0] + P.nb[0] * (b[1] + P.nb[1] * b[2]));
-  o = make_float4(of[0], of[1], of[2], 0.f);
-}
-
 // First kernel of a step with list reuse: the engine's wrap (as k_bin does
 // it), then each atom's displacement since the list build; moved atoms get
 // state 2 and join the list of moved atoms (state 0 otherwise).  With rec
-// (the df64 density sweep), also every atom's record for it: its position
-// continued from the build (the image next to xref, so the image codes of the
-// lists' entries stay what they were) and whether it moved.
+// (the df64 sweeps), also every atom's record for them (record_image) and
+// whether it moved.
 __global__ void k_list_check(StepParams P, D4 *__restrict__ x, D4 *__restrict__ xhold,
                              const int *__restrict__ wrapflag, const D4 *__restrict__ xref, int *__restrict__ state,
                              int *__restrict__ rb, int *__restrict__ flist, unsigned long long *__restrict__ counters,
@@ -965,17 +734,16 @@ __global__ void k_list_check(StepParams P, D4 *__restrict__ x, D4 *__restrict__ 
       if (i == 0) atomicAdd(&counters[CNT_WRAP], 1ull);
     }
     const D4 r = xref[i];
-    const double d0[3] = {xi.x - r.x, xi.y - r.y, xi.z - r.z};
-    int m[3];
-    double d[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      m[k] = image_count(d0[k], P.half_prd[k]);
-      d[k] = m[k] < 0 ? d0[k] - P.prd[k] : (m[k] > 0 ? d0[k] + P.prd[k] : d0[k]);
-    }
-    moved = d[0] * d[0] + d[1] * d[1] + d[2] * d[2] >= P.lslow2;
+    const double d[3] = {xi.x - r.x, xi.y - r.y, xi.z - r.z};
+    const double dx = min_image(d[0], P.prd[0], P.half_prd[0]), dy = min_image(d[1], P.prd[1], P.half_prd[1]),
+                 dz = min_image(d[2], P.prd[2], P.half_prd[2]);
+    moved = dx * dx + dy * dy + dz * dz >= P.lslow2;
     state[i] = moved ? 2 : 0;
-    if (rec) df_record(P, i, xi, m, moved, v[i], rec);
+    if (rec) {
+      int image[3];
+      record_image(P, xi, d, moved, image);
+      df_record(P, i, xi, image, moved, v[i], rec);
+    }
   }
   // one atomic per warp (after a long run without a build most atoms move)
   const unsigned mv = __ballot_sync(0xffffffffu, moved);
@@ -1226,15 +994,11 @@ enum : int { DF_BINS = 0, DF_LIST = 1, DF_EAM = 2 };
 
 // what the sweep reads and writes besides the step constants
 struct DensityArgs {
-  const int *mask, *bin_count;
-  const BinEntry *bins;
-  const int4 *atom_bin;
-  const float4 *atom_off;
-  const int4 *rec;
-  const D4 *x, *v, *xi_given;
+  CandidateArgs C;
+  const int *mask;
+  const D4 *v, *xi_given;
   int xi_mode;
   const double *T_e;
-  unsigned *pj;
   float4 *pe;
   int *nshort;
   D4 *A, *Bw;
@@ -1242,17 +1006,11 @@ struct DensityArgs {
   int *cell;
   double *Te_i;
   int *wrapflag;
-  unsigned *err;
   unsigned long long *counters;
   D4 *Mm, *G;
-  // DF_LIST
-  unsigned *cl;
-  int *cl_n;
-  const int *state, *rb, *flist;
-  const D4 *xref;
   // DF_EAM
   const unsigned *elist;
-  const int *ens;
+  const int *ens, *ens_in;
 };
 
 template <bool MULTI, int LANES, int SRC>
@@ -1274,141 +1032,30 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
   const bool active = valid && (D.mask[i] & P.groupbit) != 0;
   const size_t n = (size_t)P.n;
   auto at = [&](int k) -> unsigned & { return s_cand[LANES == 1 ? k * 128 + t : a * CAP + k]; };
-  unsigned *__restrict__ pj = D.pj;
-  // candidates past the shared rows: the atom's rows of pj (their slots are
-  // written only after the candidates there are read) or, for a kept list,
-  // the list itself
-  auto set = [&](int k, unsigned u) {
-    if (k < CAP) at(k) = u;
-    else pj[(size_t)k * n + i] = u;
-  };
+  unsigned *__restrict__ pj = D.C.pj;
 #pragma unroll
   for (int q = 0; q < 9; ++q) s_tot[q * 128 + t] = make_float2(0.f, 0.f);
   long long xi[3] = {0, 0, 0};
   int ei = 0;
   if (valid) {
     int4 ra, rb;
-    load_record(D.rec + 4 * (size_t)i, ra, rb);
+    load_record(D.C.rec + 4 * (size_t)i, ra, rb);
     xi[0] = ((long long)ra.y << 32) | (unsigned)ra.x;
     xi[1] = ((long long)ra.w << 32) | (unsigned)ra.z;
     xi[2] = ((long long)rb.y << 32) | (unsigned)rb.x;
     ei = rb.z;
   }
   int nc = 0;
-  bool fresh = true;  // the candidates are of this step's positions
+  bool fresh = true;
   const unsigned *tail = pj;
-  if (SRC == DF_LIST) {
-    const bool build = D.rb[2] != 0;
-    if (build) {
-      int4 Bi = make_int4(0, 0, 0, 0);
-      float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (active) {
-        Bi = D.atom_bin[i];
-        oi = D.atom_off[i];
-      }
-      auto lset = [&](int k, unsigned u) {
-        if (k < CAP) at(k) = u;
-        D.cl[(size_t)k * n + i] = u;
-      };
-      // the candidates inside the cut-off first, the shell out to r_list after
-      // them: the shell's pairs mostly fail the exact test, and at the end of
-      // the lists whole warps skip them
-      if (LANES == 1) {
-        auto lget = [&](int k) -> unsigned { return D.cl[(size_t)k * n + i]; };
-        nc = collect_candidates<true>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, lget, lset, P.rc2_band, P.lcap);
-        nc = collect_candidates<true>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, lget, lset, P.rl2_band, P.lcap,
-                                      nullptr, P.rc2_band, nc);
-      } else {
-        shared_candidates<LANES>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, nc, P.lcap, lset, P.rc2_band);
-        shared_candidates<LANES>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, nc, P.lcap, lset, P.rl2_band,
-                                 nullptr, P.rc2_band);
-      }
-      tail = D.cl;
-      if (valid && g == 0) D.cl_n[i] = nc;
-    } else {
-      const int st = active ? D.state[i] : 0;
-      fresh = st != 0;
-      if (__any_sync(0xffffffffu, fresh)) {
-        int4 Bi = make_int4(0, 0, 0, 0);
-        float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
-        double base[3] = {0.0, 0.0, 0.0};  // the position the image codes below refer to
-        if (fresh) {
-          const D4 x = D.x[i];
-          if (st & 2) {  // a moved atom: from its wrapped position, not continued from the build
-            int image[3];
-            current_bin(P, x, Bi, oi, image);
-            const double p[3] = {x.x, x.y, x.z};
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-              base[k] = p[k] + image[k] * P.prd[k];
-              xi[k] = to_fixed_coord(p[k], P.fix_q) + (long long)image[k] * P.fix_prd[k];
-            }
-          } else {
-            Bi = D.atom_bin[i];
-            oi = D.atom_off[i];
-            const D4 r = D.xref[i];
-            base[0] = r.x + min_image(x.x - r.x, P.prd[0], P.half_prd[0]);
-            base[1] = r.y + min_image(x.y - r.y, P.prd[1], P.half_prd[1]);
-            base[2] = r.z + min_image(x.z - r.z, P.prd[2], P.half_prd[2]);
-          }
-        }
-        if (LANES == 1) {
-          auto get = [&](int k) -> unsigned { return k < CAP ? at(k) : pj[(size_t)k * n + i]; };
-          nc = collect_candidates<true, true>(P, i, fresh, Bi, oi, D.bin_count, D.bins, D.err, get, set, P.rl2_band,
-                                              P.kcap, D.state);
-        } else {
-          shared_candidates<LANES, true>(P, i, fresh, Bi, oi, D.bin_count, D.bins, D.err, nc, P.kcap, set, P.rl2_band,
-                                         D.state);
-        }
-        // the moved atoms near enough (a widened test; pass 2 decides), their
-        // image next to the position above
-        const int nf = D.rb[1];  // <= LIST_FMAX on a step without a build
-        for (int q = 0; q < nf; ++q) {
-          const int f = D.flist[q];
-          bool take = false;
-          unsigned u = 0;
-          if (fresh && f != i && g == 0) {
-            const D4 xf = D.x[f], r = D.xref[f];
-            const double d[3] = {r.x + min_image(xf.x - r.x, P.prd[0], P.half_prd[0]) - base[0],
-                                 r.y + min_image(xf.y - r.y, P.prd[1], P.half_prd[1]) - base[1],
-                                 r.z + min_image(xf.z - r.z, P.prd[2], P.half_prd[2]) - base[2]};
-            double r2 = 0.0;
-            unsigned code = 0, place = 1;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-              const int m = image_count(d[k], P.half_prd[k]);
-              const double c = min_image(d[k], P.prd[k], P.half_prd[k]);
-              r2 += c * c;
-              code += (unsigned)(m + 1) * place;
-              place *= 3u;
-            }
-            take = r2 < P.rc2 * (1.0 + 1e-4);
-            u = (unsigned)f | (code << IDX_BITS);
-          }
-          append_candidate<LANES>(take, u, nc, P.kcap, set, D.err);
-        }
-      }
-      if (!fresh) {
-        tail = D.cl;
-        nc = active ? D.cl_n[i] : 0;
-      }
-      if (!active) fresh = true;
-    }
+  if (SRC == DF_EAM && D.ens_in) {  // the list has them apart
+    tail = D.elist;
+    nc = active ? D.ens_in[i] : 0;
   } else if (SRC == DF_EAM) {
-    list_candidates<LANES>(P, i, active, xi, D.elist, D.ens, D.rec, D.err, nc, P.kcap, set, P.rc2_band);
+    auto set = [&](int k, unsigned u) { pj[(size_t)k * n + i] = u; };
+    list_candidates<LANES>(P, i, active, xi, D.elist, D.ens, D.C.rec, D.C.err, nc, P.kcap, set, P.rc2_band);
   } else {
-    int4 Bi = make_int4(0, 0, 0, 0);
-    float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (active) {
-      Bi = D.atom_bin[i];
-      oi = D.atom_off[i];
-    }
-    if (LANES == 1) {
-      auto get = [&](int k) -> unsigned { return k < CAP ? at(k) : pj[(size_t)k * n + i]; };
-      nc = collect_candidates<true>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, get, set, P.rc2_band, P.kcap);
-    } else {
-      shared_candidates<LANES>(P, i, active, Bi, oi, D.bin_count, D.bins, D.err, nc, P.kcap, set, P.rc2_band);
-    }
+    nc = pair_candidates<LANES, SRC == DF_LIST, CAP>(P, D.C, i, g, valid, active, at, tail, fresh);
   }
   __syncwarp();
   // pass 2; the next candidate's position is loaded while this one is summed,
@@ -1425,15 +1072,15 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
   };
   unsigned u = cand(g), u2 = cand(g + LANES);
   int4 ra, rb;
-  load_record(D.rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
+  load_record(D.C.rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
   for (int k = g, m = 0; k - g < nmax; k += LANES, ++m) {
     const unsigned uc = u;
     const int4 ca = ra, cb = rb;
     int4 V0, V1;
-    load_record(D.rec + 4 * (size_t)(uc & IDX_MASK) + 2, V0, V1);
+    load_record(D.C.rec + 4 * (size_t)(uc & IDX_MASK) + 2, V0, V1);
     u = u2;
     u2 = cand(k + 2 * LANES);
-    load_record(D.rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
+    load_record(D.C.rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
     long long ef[3];
     pair_fixed(P, ca, cb, uc >> IDX_BITS, xi, ef);
     const df ex = fixed_df(ef[0], P.fix_hi, P.fix_lo), ey = fixed_df(ef[1], P.fix_hi, P.fix_lo),
@@ -1449,7 +1096,7 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
     if (who != 0u) {
       if (!in) r2 = df{1.0f, 0.0f};
       const int ej = cb.z;
-      const df rji = spline_rho_df(P, ej, r2, D.err);
+      const df rji = spline_rho_df(P, ej, r2, D.C.err);
       const df inv = recip(r2, rcp_estimate(r2.hi));
       df H = mul(rji, inv);
       if (!in) H = df{0.0f, 0.0f};
@@ -1468,11 +1115,11 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
           const size_t row = (size_t)slot * n + i;
           pj[row] = uc;
           df Hji = H;
-          if (MULTI && ej != ei) Hji = mul(spline_rho_df(P, ei, r2, D.err), inv);
+          if (MULTI && ej != ei) Hji = mul(spline_rho_df(P, ei, r2, D.C.err), inv);
           store_row(D.pe + 2 * row, make_float4(ex.hi, ey.hi, ez.hi, Hji.hi),
                     make_float4(ex.lo, ey.lo, ez.lo, Hji.lo));
         } else {
-          atomicOr(D.err, ERR_PAIR_OVERFLOW);
+          atomicOr(D.C.err, ERR_PAIR_OVERFLOW);
         }
       }
       acc_fma(sm[0], hx, ex);
@@ -1523,11 +1170,11 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
     for (int l = 1; l < LANES; ++l) sum += to_double(df{w[l].x, w[l].y});
     mq[q] = sum;
   }
-  const D4 xo = D.x[o];
+  const D4 xo = D.C.x[o];
   const bool act = LANES > 1 ? (D.mask[o] & P.groupbit) != 0 : active;
   density_epilogue<true, true, true>(P, o, act, xo, LANES > 1 ? (int)xo.w : ei, 0.0, ns_o < P.kcap ? ns_o : P.kcap,
                                      mq[0], mq[1], mq[2], mq[3], mq[4], mq[5], mq[6], mq[7], mq[8], D.xi_given,
-                                     D.xi_mode, D.T_e, D.nshort, D.A, D.Bw, D.rho, D.beta, D.cell, D.Te_i, D.err,
+                                     D.xi_mode, D.T_e, D.nshort, D.A, D.Bw, D.rho, D.beta, D.cell, D.Te_i, D.C.err,
                                      D.counters, D.v, D.Mm, D.G);
 }
 
