@@ -262,6 +262,119 @@ __global__ void k_adj_fdm_back(GridArgs G, const double *__restrict__ W, const d
     Tb[r] = lam;
 }
 
+// What the reverse substeps of a step need of the forward's temperatures, for
+// every substep and cell at once: the source rate, the kappa derivative (lap)
+// and whether the cell kept its value (not clamped at T = 0), substep_reverse's
+// expressions.  Substep k = blockIdx.y starts from T0 (k = 0) or
+// Tsub + (k - 1) nc; the cell's coordinates take two 32-bit divisions (the six
+// 64-bit ones of axis_pq were most of its time).
+__global__ void k_adj_fdm_rates(GridArgs G, const double *__restrict__ T0, const double *__restrict__ Tsub,
+                                const double *__restrict__ src, double2 *__restrict__ rates,
+                                unsigned char *__restrict__ kept) {
+  const int r = (int)(blockIdx.x * blockDim.x + threadIdx.x), nc = (int)G.nc;
+  if (r >= nc) return;
+  const double *T = blockIdx.y ? Tsub + (size_t)(blockIdx.y - 1) * G.nc : T0;
+  const int n[3] = {(int)G.n[0], (int)G.n[1], (int)G.n[2]};
+  const int row = r / n[0], k = row / n[1];
+  const int at[3] = {r - row * n[0], row - k * n[1], k};
+  const signed char flag = G.flag[r];
+  double ddT = 0.0, lap = 0.0;
+  if (flag != 2) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const int st = a == 0 ? 1 : (a == 1 ? n[0] : n[0] * n[1]);
+      int p = at[a] > 0 ? r - st : r + (n[a] - 1) * st, q = at[a] < n[a] - 1 ? r + st : r - (n[a] - 1) * st;
+      if (G.flag[q] == 2) q = r;
+      else if (G.flag[p] == 2) p = r;
+      const double ih2 = G.ih2[a];
+      const double l = (T[q] + T[p] - 2.0 * T[r]) * ih2;
+      ddT += (G.kappa[q] - G.kappa[p]) * (T[q] - T[p]) * 0.25 * ih2 + G.kappa[r] * l;
+      lap += l;
+    }
+  }
+  const double rate = ddT + src[r] + G.S[r];
+  const double pre = flag == 1 ? T[r] + rate * G.irhoC[r] * G.inner_dt : T[r];
+  const size_t out = (size_t)blockIdx.y * G.nc + r;
+  rates[out] = make_double2(rate, lap);
+  kept[out] = pre >= 0.0 ? 1 : 0;
+}
+
+// The whole reverse of a step's grid solve in one cluster launch (one cell per
+// thread; the cotangents in two shared-memory buffers per block, neighbours
+// read through distributed shared memory as in the forward's
+// k_fdm_cluster_fast): k_adj_fdm_first and every k_adj_fdm_back with their
+// expressions, the temperatures' part from k_adj_fdm_rates.  16^3 cells and 11
+// substeps on GB300: 12 launches, ~80 us; 27 + 8 us in two.
+constexpr int ADJ_CLUSTER_CELLS = 384;
+__global__ void __launch_bounds__(ADJ_CLUSTER_CELLS)
+    k_adj_fdm_cluster(GridArgs G, const double *__restrict__ W, int ns, const double2 *__restrict__ rates,
+                      const unsigned char *__restrict__ kept, const double *__restrict__ tau, double *__restrict__ Tb,
+                      double *__restrict__ srcbar, double *__restrict__ gC, double *__restrict__ gK) {
+  extern __shared__ double s_u[];  // [2][blockDim]
+  const int t = (int)threadIdx.x, nt = (int)blockDim.x;
+  const int r = (int)blockIdx.x * nt + t;
+  const bool mine = r < (int)G.nc;
+  double w[7], u = 0.0, lam = 0.0, sb = 0.0, C = 0.0, K = 0.0, irhoC = 0.0, rho = 0.0;
+  bool dyn = false;
+  unsigned at[6];
+  if (mine) {
+    const int nx = (int)G.n[0], ny = (int)G.n[1], nz = (int)G.n[2], nxy = nx * ny;
+    const int row = r / nx, i = r - row * nx, k = row / ny, j = row - k * ny;
+    const int m[6] = {i > 0 ? r - 1 : r + (nx - 1), i < nx - 1 ? r + 1 : r - (nx - 1),
+                      j > 0 ? r - nx : r + (nxy - nx), j < ny - 1 ? r + nx : r - (nxy - nx),
+                      k > 0 ? r - nxy : r + (nz - 1) * nxy, k < nz - 1 ? r + nxy : r - (nz - 1) * nxy};
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      const int owner = m[q] / nt;
+      const unsigned local = (unsigned)__cvta_generic_to_shared(s_u + (m[q] - owner * nt));
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at[q]) : "r"(local), "r"(owner));
+    }
+#pragma unroll
+    for (int q = 0; q < 7; ++q) w[q] = W[(size_t)q * G.nc + r];
+    dyn = G.flag[r] == 1;
+    irhoC = G.irhoC[r];
+    rho = G.rho_e[r];
+    C = gC[r];
+    K = gK[r];
+    lam = Tb[r] + *tau;
+  }
+  unsigned cur = 0;
+  const unsigned half = (unsigned)(nt * sizeof(double));
+  for (int k = ns - 1; k >= 0; --k) {
+    if (mine) {  // substep_reverse
+      const double2 q = rates[(size_t)k * G.nc + r];
+      u = kept[(size_t)k * G.nc + r] ? lam : 0.0;
+      double v = 0.0;
+      if (dyn) {
+        v = u * G.inner_dt * irhoC;
+        C -= v * q.x * rho * irhoC;
+        K += v * q.y;
+      }
+      sb = k == ns - 1 ? v : sb + v;
+      s_u[(cur ? nt : 0) + t] = u;
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (mine) {
+      double un[6];
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+        asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(un[q]) : "r"(at[q] + cur) : "memory");
+      lam = fma(w[0], u, u);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) lam = fma(w[q + 1], un[q], lam);
+    }
+    cur = half - cur;
+  }
+  if (mine) {
+    Tb[r] = lam;
+    srcbar[r] = sb;
+    gC[r] = C;
+    gK[r] = K;
+  }
+  // no block leaves while another may still read its buffers
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 __global__ void k_adj_add(double *__restrict__ a, long n, const double *__restrict__ v) {
   const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (r < n) a[r] += *v;
@@ -613,6 +726,7 @@ __global__ void __launch_bounds__(ABLOCK)
 // parts carry them to ~1e-13 A); the spline is the forward's local-form df64
 // table (value and derivative from the same interval, whose knot receives the
 // coefficient gradient).  Results agree with the FP64 sweeps to ~1e-12.
+// (rows 2k and 2k + 1 share a 32-byte sector: the loops read such pairs)
 constexpr int R_X = 0, R_V = 2, R_WX = 4, R_C = 7, R_W = 10, R_N = 12;
 
 // rows R_X (x, a_i = alpha_i / rho_i or 0), R_V (v, element, live flag),
@@ -706,17 +820,29 @@ __global__ void __launch_bounds__(ABLOCK)
     const float4 ih = ri[R_X], il = ri[R_X + 1];
     const df3 cei = df3_of(ri[R_C], ri[R_C + 1]), cri = df3_split(ri[R_C], ri[R_C + 1], ri[R_C + 2]);
     const int ns = S.ns[i];
+    // the next neighbour's position and flags are loaded while this pair is
+    // summed, each pair of rows in one 256-bit load
+    unsigned u_next = ns > 0 ? S.pj[i] : 0u;
+    float4 xh_n, xl_n, vh_n, vl_n;
+    load_row(rec + (size_t)R_N * (u_next & IDX_MASK) + R_X, xh_n, xl_n);
+    load_row(rec + (size_t)R_N * (u_next & IDX_MASK) + R_V, vh_n, vl_n);
     for (int k = 0; k < ns; ++k) {
-      const unsigned u = S.pj[(size_t)k * P.n + i];
-      const unsigned j = u & IDX_MASK;
-      const float4 *rj = rec + (size_t)R_N * j;
-      const float4 vl = rj[R_V + 1];
+      const unsigned u = u_next;
+      const float4 xh = xh_n, xl = xl_n, vh = vh_n, vl = vl_n;
+      const float4 *rj = rec + (size_t)R_N * (u & IDX_MASK);
+      float4 wx2, ch, cl, c2;  // rows R_C - 1 .. R_C + 2
+      load_row(rj + R_C - 1, wx2, ch);
+      load_row(rj + R_C + 1, cl, c2);
+      if (k + 1 < ns) {
+        u_next = S.pj[(size_t)(k + 1) * P.n + i];
+        load_row(rec + (size_t)R_N * (u_next & IDX_MASK) + R_X, xh_n, xl_n);
+        load_row(rec + (size_t)R_N * (u_next & IDX_MASK) + R_V, vh_n, vl_n);
+      }
       if (!(vl.w > 0.0f)) continue;  // rho_j <= 0
-      const df3 e = adj_disp(P, rj[R_X], rj[R_X + 1], ih, il, u >> IDX_BITS);
+      const df3 e = adj_disp(P, xh, xl, ih, il, u >> IDX_BITS);
       const df r2 = ddot(e, e);
-      const df H = mul(spline_rho_df(P, __float_as_int(rj[R_V].w), r2, err), recip(r2, rcp_estimate(r2.hi)));
-      const float4 ch = rj[R_C], cl = rj[R_C + 1];
-      const df3 cej = df3_of(ch, cl), crj = df3_split(ch, cl, rj[R_C + 2]);
+      const df H = mul(spline_rho_df(P, __float_as_int(vh.w), r2, err), recip(r2, rcp_estimate(r2.hi)));
+      const df3 cej = df3_of(ch, cl), crj = df3_split(ch, cl, c2);
       const df dE = mul(H, ddot(e, dsub(cei, cej)));
       const df dR = mul(H, ddot(e, dsub(cri, crj)));
       acc_fma(U[0], dE, e.x);
@@ -779,6 +905,12 @@ __global__ void __launch_bounds__(ABLOCK)
 // k_adj_sweep2 with the pair loop in df64 (the same terms, in the same
 // grouping; rows of k_adj_split and R_W of k_adj_sweep1_df).  RMODE 0 keeps
 // its per-thread coefficient accumulators as df64 pairs in shared memory.
+// Both sweeps read the neighbours' rows with 256-bit loads, two 16-byte halves
+// a request, and ask for the next neighbour's while this one's are computed:
+// sweep 2 is bound by issue (1560 instructions per 32 pairs; 250 blocks at
+// 32 000 atoms put two on 98 SMs and one on 54), sweep 1 by the latency of its
+// scattered rows.  GB300, 32 000 atoms: sweep 2 149 -> 109 us, sweep 1 81 -> 58.
+// Two lanes per atom, at 2 to 4 blocks per SM, gave 1% to -2% of the pass.
 template <bool FAST, bool MULTI, int RMODE>
 __global__ void __launch_bounds__(ABLOCK)
     k_adj_sweep2_df(StepParams P, Slot S, const int *__restrict__ mask, const int *__restrict__ type,
@@ -808,11 +940,20 @@ __global__ void __launch_bounds__(ABLOCK)
     const df Wwi{Oh.w, Ol.w};
     acc gx[3] = {acc_zero(), acc_zero(), acc_zero()}, gv[3] = {acc_zero(), acc_zero(), acc_zero()};
     const int ns = S.ns[i];
+    unsigned u_next = ns > 0 ? S.pj[i] : 0u;
+    float4 xh_n, xl_n;
+    load_row(rec + (size_t)R_N * (u_next & IDX_MASK) + R_X, xh_n, xl_n);
     for (int k = 0; k < ns; ++k) {
-      const unsigned u = S.pj[(size_t)k * P.n + i];
-      const unsigned j = u & IDX_MASK;
-      const float4 *rj = rec + (size_t)R_N * j;
-      const float4 jxh = rj[R_X], jxl = rj[R_X + 1], jvh = rj[R_V], jvl = rj[R_V + 1];
+      const unsigned u = u_next;
+      const float4 jxh = xh_n, jxl = xl_n;
+      const float4 *rj = rec + (size_t)R_N * (u & IDX_MASK);
+      float4 jvh, jvl, jOh, jOl;
+      load_row(rj + R_V, jvh, jvl);
+      load_row(rj + R_W, jOh, jOl);
+      if (k + 1 < ns) {
+        u_next = S.pj[(size_t)(k + 1) * P.n + i];
+        load_row(rec + (size_t)R_N * (u_next & IDX_MASK) + R_X, xh_n, xl_n);
+      }
       const df3 e = adj_disp(P, jxh, jxl, ih, il, u >> IDX_BITS);
       const df r2 = ddot(e, e);
       const df rinv = recip(r2, rcp_estimate(r2.hi));
@@ -831,7 +972,6 @@ __global__ void __launch_bounds__(ABLOCK)
       }
       const bool live_j = jvl.w > 0.0f;
       const df aj{jxh.w, jxl.w};
-      const float4 jOh = rj[R_W], jOl = rj[R_W + 1];
       const df3 Wj = df3_of(jOh, jOl);
       const df Wwj{jOh.w, jOl.w};
       const df3 dv = dsub(vi, df3_of(jvh, jvl));
@@ -843,9 +983,12 @@ __global__ void __launch_bounds__(ABLOCK)
       df3 Vi = dscale(e_dv, Wi), Vj = dscale(e_dv, Wj);
       df3 g = dscale(eOd, dv);
       if (live_i && live_j) {
-        const float4 jwh = rj[R_WX], jwl = rj[R_WX + 1], jch = rj[R_C], jcl = rj[R_C + 1];
-        const df3 wj = df3_of(jwh, jwl), xij = df3_split(jwh, jwl, rj[R_WX + 2]);
-        const df3 dE = dsub(cei, df3_of(jch, jcl)), dR = dsub(cri, df3_split(jch, jcl, rj[R_C + 2]));
+        float4 jwh, jwl, jw2, jch, jcl, jc2;
+        load_row(rj + R_WX, jwh, jwl);
+        load_row(rj + R_WX + 2, jw2, jch);
+        load_row(rj + R_C + 1, jcl, jc2);
+        const df3 wj = df3_of(jwh, jwl), xij = df3_split(jwh, jwl, jw2);
+        const df3 dE = dsub(cei, df3_of(jch, jcl)), dR = dsub(cri, df3_split(jch, jcl, jc2));
         const df e_dE = ddot(e, dE), e_dR = ddot(e, dR);
         const df ewi = ddot(e, wi), ewj = ddot(e, wj), exi = ddot(e, xii), exj = ddot(e, xij);
         Bi_ = add(Bi_, add(mul(ewi, e_dE), mul(exi, e_dR)));
@@ -904,25 +1047,52 @@ __global__ void __launch_bounds__(ABLOCK)
     fb[i] = D4{dtfm * vbx, dtfm * vby, dtfm * vbz, 0.0};
   }
   if (RMODE == 0) {
+    // A warp takes 16 columns: a lane adds four of a column's 128 pairs, then
+    // the 32 lanes' sums in FP64, halving the columns a lane holds at every
+    // exchange (16 additions for 16 columns; a thread per column took 128 x 3
+    // FP64 instructions of 16 cycles each)
     __syncthreads();
-    for (int q = t; q < nt4; q += nt) {
-      double sum = 0.0;
-      for (int tt = 0; tt < nt; ++tt) {
-        const float2 cell = s_pf[q * nt + tt];
-        sum += to_double(df64::df{cell.x, cell.y});
+    const int lane = t & 31;
+    for (int q0 = 16 * (t >> 5); q0 < nt4; q0 += 16 * (nt >> 5)) {
+      double v[16];
+#pragma unroll
+      for (int m = 0; m < 16; ++m) {
+        df64::df sum{0.0f, 0.0f};
+        if (q0 + m < nt4) {
+#pragma unroll
+          for (int w = 0; w < ABLOCK / 32; ++w) {
+            const float2 cell = s_pf[(q0 + m) * nt + 32 * w + lane];
+            sum = df64::add(sum, df64::df{cell.x, cell.y});
+          }
+        }
+        v[m] = df64::to_double(sum);
       }
-      gpart[(size_t)blockIdx.x * nt4 + q] += sum;
+#pragma unroll
+      for (int h = 8; h > 0; h >>= 1) {
+        const bool up = lane & (2 * h);
+#pragma unroll
+        for (int m = 0; m < h; ++m) {
+          const double keep = up ? v[m + h] : v[m], give = up ? v[m] : v[m + h];
+          v[m] = keep + __shfl_xor_sync(FULL, give, 2 * h);
+        }
+      }
+      v[0] += __shfl_xor_sync(FULL, v[0], 1);
+      const int q = q0 + (lane >> 1);
+      if (!(lane & 1) && q < nt4) gpart[(size_t)blockIdx.x * nt4 + q] += v[0];
     }
   }
 }
 
-// sum of the blocks' partial rows, in block order
+// sum of the blocks' partial rows: a warp per column (250 rows of 64 columns
+// on GB300: one thread per column 34 us, 7 us now)
 __global__ void k_adj_reduce(const double *__restrict__ gpart, int nparts, int nt4, double *__restrict__ acc) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  const int q = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (q >= nt4) return;
   double s = 0.0;
-  for (int b = 0; b < nparts; ++b) s += gpart[(size_t)b * nt4 + q];
-  acc[q] += s;
+  for (int b = lane; b < nparts; b += 32) s += gpart[(size_t)b * nt4 + q];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+  if (lane == 0) acc[q] += s;
 }
 
 }  // namespace
@@ -959,6 +1129,8 @@ struct eph_adjoint {
   DevBuf<D4> xb, vb, fb, cE, cR, W;
   DevBuf<float4> dfr;  // df64 rows of the reverse sweeps (R_N per atom), the pair arithmetic is df64
   DevBuf<double> Tb, u0, u1, srcbar, gC, gK, rho_e;
+  DevBuf<double2> fdm_rates;  // per substep and cell of the step being reversed, see k_adj_fdm_rates
+  DevBuf<unsigned char> fdm_kept;
   DevBuf<double> fdmW;  // [7][ncells]: transposed substep stencil, see k_adj_fdm_weights
   DevBuf<double> g_rho, g_alpha, part_rho, part_alpha;
   DevBuf<double> tbc;     // per atom: contribution to the grid's cotangent
@@ -1050,6 +1222,57 @@ int load_state(eph_adjoint *a, const D4 *x, const D4 *v, const D4 *f, const D4 *
   return EPH_OK;
 }
 
+// What the reverse sweeps of a step read of it, copied to its slot by two
+// kernels: after the density and friction sweeps, and at the end of the step.
+// Bound by the memory they move; of the neighbour rows only the filled ones
+// (the 13 copy nodes they took the place of moved every slot), split over
+// gridDim.y threads per atom since one thread per atom leaves the rows a
+// serial chain of loads.
+struct RecordMid {
+  const D4 *x, *v, *A, *Bw;
+  const double *Te, *T0;
+  const int *cell, *ns;
+  const unsigned *pj;
+  D4 *rx, *rv, *rA, *rBw;
+  double *rTe, *rT0;
+  int *rcell, *rns;
+  unsigned *rpj;
+};
+
+__global__ void __launch_bounds__(ABLOCK) k_adj_record_mid(RecordMid R, int n, long nc, int kcap) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int y = (int)blockIdx.y;
+  if (y == 0 && i < nc) R.rT0[i] = R.T0[i];
+  if (i >= n) return;
+  if (y == 0) {
+    R.rx[i] = R.x[i];
+    R.rv[i] = R.v[i];
+    R.rA[i] = R.A[i];
+    R.rBw[i] = R.Bw[i];
+    R.rTe[i] = R.Te[i];
+    R.rcell[i] = R.cell[i];
+    R.rns[i] = R.ns[i];
+  }
+  const int ns = min(R.ns[i], kcap);
+  for (int k = y; k < ns; k += (int)gridDim.y) R.rpj[(size_t)k * n + i] = R.pj[(size_t)k * n + i];
+}
+
+struct RecordEnd {
+  const D4 *v, *fE, *fR;
+  const double *src;
+  D4 *rv, *rfE, *rfR;
+  double *rsrc;
+};
+
+__global__ void __launch_bounds__(ABLOCK) k_adj_record_end(RecordEnd R, int n, long nc) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nc) R.rsrc[i] = R.src[i];
+  if (i >= n) return;
+  R.rv[i] = R.v[i];
+  R.rfE[i] = R.fE[i];
+  R.rfR[i] = R.fR[i];
+}
+
 // the plain engine step (the sequence of eph_step), optionally recording slot s
 int run_step(eph_adjoint *a, int s) {
   eph_ctx *c = a->c;
@@ -1062,30 +1285,25 @@ int run_step(eph_adjoint *a, int s) {
   else
     ADJ_TRY(a, cudaMemsetAsync(c->f.p, 0, sizeof(D4) * N, c->stream));
   if ((r = ctxi::launch_post_force(c, 0))) return from_ctx(a, r);
+  const size_t o = (size_t)std::max(s, 0) * N, og = (size_t)std::max(s, 0) * (size_t)a->nc;
+  const int rb = nb_of(std::max((long)a->n, a->nc));
   if (s >= 0) {
-    const size_t o = (size_t)s * N;
-    ADJ_TRY(a, d2d(a->r_x1.p + o, c->x.p, N, c->stream));
-    ADJ_TRY(a, d2d(a->r_v1.p + o, c->v.p, N, c->stream));
-    ADJ_TRY(a, d2d(a->r_A.p + o, c->A.p, N, c->stream));
-    ADJ_TRY(a, d2d(a->r_Bw.p + o, c->Bw.p, N, c->stream));
-    ADJ_TRY(a, d2d(a->r_Te.p + o, c->Te_i.p, N, c->stream));
-    ADJ_TRY(a, d2d(a->r_cell.p + o, c->cell.p, N, c->stream));
-    ADJ_TRY(a, d2d(a->r_ns.p + o, c->nshort.p, N, c->stream));
-    ADJ_TRY(a, d2d(a->r_pj.p + (size_t)s * a->kcap * N, c->pj.p, (size_t)a->kcap * N, c->stream));
-    ADJ_TRY(a, d2d(a->r_T0.p + (size_t)s * a->nc, c->T0.p, (size_t)a->nc, c->stream));
+    RecordMid R{c->x.p, c->v.p, c->A.p, c->Bw.p, c->Te_i.p, c->T0.p, c->cell.p, c->nshort.p, c->pj.p,
+                a->r_x1.p + o, a->r_v1.p + o, a->r_A.p + o, a->r_Bw.p + o, a->r_Te.p + o, a->r_T0.p + og,
+                a->r_cell.p + o, a->r_ns.p + o, a->r_pj.p + o * (size_t)a->kcap};
+    k_adj_record_mid<<<dim3((unsigned)rb, 8), ABLOCK, 0, c->stream>>>(R, a->n, a->nc, a->kcap);
+    a->launches += 1;
   }
   if ((r = ctxi::launch_final(c))) return from_ctx(a, r);
-  if (s >= 0) {
-    const size_t o = (size_t)s * N;
-    ADJ_TRY(a, d2d(a->r_v2.p + o, c->v.p, N, c->stream));
-    ADJ_TRY(a, d2d(a->r_fE.p + o, c->f_eph.p, N, c->stream));
-    ADJ_TRY(a, d2d(a->r_fR.p + o, c->f_rng.p, N, c->stream));
-    if (a->fdm) c->fdm_rec = a->r_Tsub.p + (size_t)s * a->nsub * (size_t)a->nc;
-  }
+  if (s >= 0 && a->fdm) c->fdm_rec = a->r_Tsub.p + (size_t)s * a->nsub * (size_t)a->nc;
   r = ctxi::launch_end_of_step(c);
   c->fdm_rec = nullptr;
   if (r) return from_ctx(a, r);
-  if (s >= 0 && a->fdm) ADJ_TRY(a, d2d(a->r_src.p + (size_t)s * a->nc, c->dT.p, (size_t)a->nc, c->stream));
+  if (s >= 0) {
+    RecordEnd R{c->v.p, c->f_eph.p, c->f_rng.p, c->dT.p, a->r_v2.p + o, a->r_fE.p + o, a->r_fR.p + o, a->r_src.p + og};
+    k_adj_record_end<<<rb, ABLOCK, 0, c->stream>>>(R, a->n, a->fdm ? a->nc : 0);
+    a->launches += 1;
+  }
   a->launches += c->launches - before;
   c->launches = before;
   return EPH_OK;
@@ -1204,18 +1422,42 @@ int reverse_step(eph_adjoint *a, int s, const double *eb, const double *tau) {
     auto Tat = [&](unsigned m) -> const double * {
       return m == 0 ? a->r_T0.p + (size_t)s * nc : a->r_Tsub.p + ((size_t)s * ns + (m - 1)) * (size_t)nc;
     };
-    double *ub[2] = {a->u0.p, a->u1.p};
-    const int gb32 = nb_of(nc, 32);  // small grids: spread the cells over more SMs
-    k_adj_fdm_first<<<gb32, 32, 0, c->stream>>>(G, Tat(ns - 1), src, a->Tb.p, tau, ub[0], a->srcbar.p, a->gC.p,
-                                                a->gK.p);
-    a->launches += 1;
-    int cur = 0;
-    for (int k = (int)ns - 1; k >= 0; --k) {
-      const double *Tprev = k >= 1 ? Tat((unsigned)k - 1) : nullptr;
-      k_adj_fdm_back<<<gb32, 32, 0, c->stream>>>(G, a->fdmW.p, ub[cur], Tprev, src, ub[cur ^ 1], a->Tb.p,
-                                                 a->srcbar.p, a->gC.p, a->gK.p);
+    if (c->fdm_fast_cluster && nc <= (long)ADJ_CLUSTER_CELLS * c->fdm_fast_cluster && ns <= 65535u) {
+      k_adj_fdm_rates<<<dim3((unsigned)nb_of(nc, 64), ns), 64, 0, c->stream>>>(
+          G, Tat(0), a->r_Tsub.p + (size_t)s * ns * nc, src, a->fdm_rates.p, a->fdm_kept.p);
+      int blocks = 1;
+      while (2 * blocks <= c->fdm_fast_cluster && 32 * blocks < nc) blocks *= 2;
+      const int per = (int)(((nc + blocks - 1) / blocks + 31) / 32 * 32);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)blocks);
+      cfg.blockDim = dim3((unsigned)per);
+      cfg.dynamicSmemBytes = 2 * sizeof(double) * (size_t)per;
+      cfg.stream = c->stream;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = (unsigned)blocks;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      ADJ_TRY(a, cudaLaunchKernelEx(&cfg, k_adj_fdm_cluster, G, (const double *)a->fdmW.p, (int)ns,
+                                    (const double2 *)a->fdm_rates.p, (const unsigned char *)a->fdm_kept.p, tau,
+                                    a->Tb.p, a->srcbar.p, a->gC.p, a->gK.p));
+      a->launches += 2;
+    } else {
+      double *ub[2] = {a->u0.p, a->u1.p};
+      const int gb32 = nb_of(nc, 32);  // small grids: spread the cells over more SMs
+      k_adj_fdm_first<<<gb32, 32, 0, c->stream>>>(G, Tat(ns - 1), src, a->Tb.p, tau, ub[0], a->srcbar.p, a->gC.p,
+                                                  a->gK.p);
       a->launches += 1;
-      cur ^= 1;
+      int cur = 0;
+      for (int k = (int)ns - 1; k >= 0; --k) {
+        const double *Tprev = k >= 1 ? Tat((unsigned)k - 1) : nullptr;
+        k_adj_fdm_back<<<gb32, 32, 0, c->stream>>>(G, a->fdmW.p, ub[cur], Tprev, src, ub[cur ^ 1], a->Tb.p,
+                                                   a->srcbar.p, a->gC.p, a->gK.p);
+        a->launches += 1;
+        cur ^= 1;
+      }
     }
   } else {
     k_adj_add<<<gb, 64, 0, c->stream>>>(a->Tb.p, nc, tau);
@@ -1334,11 +1576,11 @@ int issue_backward(eph_adjoint *a, bool skip_last) {
   }
   // the blocks' partial rows of the table-coefficient gradients, once per pass
   if (a->amode == 0) {
-    k_adj_reduce<<<nb_of(a->nt4_alpha), ABLOCK, 0, c->stream>>>(a->part_alpha.p, nb, a->nt4_alpha, a->g_alpha.p);
+    k_adj_reduce<<<nb_of(a->nt4_alpha, ABLOCK / 32), ABLOCK, 0, c->stream>>>(a->part_alpha.p, nb, a->nt4_alpha, a->g_alpha.p);
     a->launches += 1;
   }
   if (a->rmode == 0) {
-    k_adj_reduce<<<nb_of(a->nt4_rho), ABLOCK, 0, c->stream>>>(a->part_rho.p, nb, a->nt4_rho, a->g_rho.p);
+    k_adj_reduce<<<nb_of(a->nt4_rho, ABLOCK / 32), ABLOCK, 0, c->stream>>>(a->part_rho.p, nb, a->nt4_rho, a->g_rho.p);
     a->launches += 1;
   }
   ADJ_TRY(a, cudaGetLastError());
@@ -1412,6 +1654,9 @@ int ensure_records(eph_adjoint *a) {
   if ((r = ensure(a, a->r_pj, K * (size_t)a->kcap * N))) return r;
   if ((r = ensure(a, a->r_T0, K * (size_t)a->nc)) || (r = ensure(a, a->r_src, K * (size_t)a->nc))) return r;
   if ((r = ensure(a, a->r_Tsub, K * (size_t)a->nsub * (size_t)a->nc))) return r;
+  if ((r = ensure(a, a->fdm_rates, (size_t)a->nsub * (size_t)a->nc)) ||
+      (r = ensure(a, a->fdm_kept, (size_t)a->nsub * (size_t)a->nc)))
+    return r;
   return EPH_OK;
 }
 
@@ -1588,6 +1833,8 @@ int eph_adjoint_create(eph_ctx *c, int checkpoint_every, eph_adjoint **out) {
     ADJ_TRY(a, cudaFuncSetAttribute(k_adj_sweep2_df<false, true, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     sh));
   }
+  if (c->fdm_fast_cluster > 8)
+    ADJ_TRY(a, cudaFuncSetAttribute(k_adj_fdm_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   for (cudaEvent_t &e : a->ev) ADJ_TRY(a, cudaEventCreate(&e));
   // the start of every trajectory: the context as it is now
   int r = save_state(a, a->s_x.p, a->s_v.p, a->s_f.p, a->s_xh.p, a->s_T.p, a->s_step.p);
