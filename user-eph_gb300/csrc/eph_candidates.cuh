@@ -105,17 +105,16 @@ __device__ __forceinline__ void append_candidate(bool take, unsigned u, int &nc,
 
 // Candidates of atom i in the bin at stencil offset (dx, dy, dz) from its
 // own: the entries whose FP32 distance passes the widened cut-off, appended
-// through cset (FAST: in bin order; EXACT: kept in ascending neighbour index
-// by insertion) while nc < cap.  Contains a warp-wide max: every lane of the
+// through cset in bin order while nc < cap.  Contains a warp-wide max: every lane of the
 // warp calls it the same number of times (look = false for a lane with
 // nothing to search).  r2band is the FP32 threshold (the cutoff's, or the
 // candidate list's); with SKIP, entries of atoms flagged as moved (skip[j] &
 // 2) are left out.
-template <bool FAST, bool SKIP = false, class Get, class Set>
+template <bool SKIP = false, class Set>
 __device__ __forceinline__ void bin_candidates(const StepParams &P, int i, bool look, int4 Bi, float4 oi, int dx,
                                                int dy, int dz, const int *__restrict__ bin_count,
                                                const BinEntry *__restrict__ bins, unsigned *__restrict__ err,
-                                               int &nc, int cap, Get cget, Set cset, float r2band,
+                                               int &nc, int cap, Set cset, float r2band,
                                                const int *__restrict__ skip = nullptr, float r2lo = -1.f) {
   const int Tz = Bi.z + dz, tz = Tz < 0 ? Tz + P.nb[2] : (Tz >= P.nb[2] ? Tz - P.nb[2] : Tz);
   const int kz = Tz < 0 ? -1 : (Tz >= P.nb[2] ? 1 : 0);
@@ -150,23 +149,14 @@ __device__ __forceinline__ void bin_candidates(const StepParams &P, int i, bool 
           atomicOr(err, ERR_PAIR_OVERFLOW);
         } else {
           const unsigned u = j | ((unsigned)((mx + 1) + 3 * (my + 1) + 9 * (mz + 1)) << IDX_BITS);
-          int pos = nc++;
-          if (!FAST) {  // ascending neighbour index
-            while (pos > 0) {
-              const unsigned prev = cget(pos - 1);
-              if ((prev & IDX_MASK) <= j) break;
-              cset(pos, prev);
-              --pos;
-            }
-          }
-          cset(pos, u);
+          cset(nc++, u);
         }
       }
     }
   }
 }
 
-// bin_candidates (FAST) over all 27 bins with LANES lanes per atom: lane g
+// bin_candidates over all 27 bins with LANES lanes per atom: lane g
 // takes bins g, g + LANES, ... of the stencil and the lanes append to the
 // atom's one list what `keep` does not refuse (a candidate and its FP32 r^2).
 // Every lane of the warp calls it.
@@ -238,18 +228,18 @@ __device__ __forceinline__ void shared_candidates(const StepParams &P, int i, bo
 // Pass 1 of the density sweep for atom i: the candidates of the 27 bins
 // around its own within the FP32 thresholds r2lo <= r^2 < r2band, appended
 // after the first nc0 (at most cap in all).  Returns their number.
-template <bool FAST, bool SKIP = false, class Get, class Set>
+template <bool SKIP = false, class Set>
 __device__ __forceinline__ int collect_candidates(const StepParams &P, int i, bool active, int4 Bi, float4 oi,
                                                   const int *__restrict__ bin_count,
                                                   const BinEntry *__restrict__ bins, unsigned *__restrict__ err,
-                                                  Get cget, Set cset, float r2band, int cap,
+                                                  Set cset, float r2band, int cap,
                                                   const int *__restrict__ skip = nullptr, float r2lo = -1.f,
                                                   int nc0 = 0) {
   int nc = nc0;
   for (int dz = -1; dz <= 1; ++dz)
     for (int dy = -1; dy <= 1; ++dy)
       for (int dx = -1; dx <= 1; ++dx)
-        bin_candidates<FAST, SKIP>(P, i, active, Bi, oi, dx, dy, dz, bin_count, bins, err, nc, cap, cget, cset,
+        bin_candidates<SKIP>(P, i, active, Bi, oi, dx, dy, dz, bin_count, bins, err, nc, cap, cset,
                                    r2band, skip, r2lo);
   return nc;
 }
@@ -329,7 +319,6 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
     if (k < CAP) at(k) = u;
     else C.pj[(size_t)k * n + i] = u;
   };
-  auto get = [&](int k) -> unsigned { return k < CAP ? at(k) : C.pj[(size_t)k * n + i]; };
   if (!LIST) {
     int4 Bi = make_int4(0, 0, 0, 0);
     float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -338,7 +327,7 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
       oi = C.atom_off[i];
     }
     if (LANES == 1)
-      nc = collect_candidates<true>(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, get, set, C.band, C.kcap);
+      nc = collect_candidates(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, set, C.band, C.kcap);
     else
       shared_candidates<LANES>(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, nc, C.kcap, set, C.band);
     return nc;
@@ -358,9 +347,8 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
     // them: the shell's pairs mostly fail the exact test, and at the end of
     // the lists whole warps skip them
     if (LANES == 1) {
-      auto lget = [&](int k) -> unsigned { return C.cl[(size_t)k * n + i]; };
-      nc = collect_candidates<true>(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, lget, lset, C.band, P.lcap);
-      nc = collect_candidates<true>(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, lget, lset, P.rl2_band, P.lcap,
+      nc = collect_candidates(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, lset, C.band, P.lcap);
+      nc = collect_candidates(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, lset, P.rl2_band, P.lcap,
                                     nullptr, C.band, nc);
     } else {
       shared_candidates<LANES>(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, nc, P.lcap, lset, C.band);
@@ -391,7 +379,7 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
       }
     }
     if (LANES == 1)
-      nc = collect_candidates<true, true>(P, i, fresh, Bi, oi, C.bin_count, C.bins, C.err, get, set, P.rl2_band, C.kcap,
+      nc = collect_candidates<true>(P, i, fresh, Bi, oi, C.bin_count, C.bins, C.err, set, P.rl2_band, C.kcap,
                                           C.state);
     else
       shared_candidates<LANES, true>(P, i, fresh, Bi, oi, C.bin_count, C.bins, C.err, nc, C.kcap, set, P.rl2_band,

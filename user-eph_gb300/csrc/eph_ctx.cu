@@ -236,6 +236,26 @@ int build_fdm_coef(eph_ctx *c) {
   return EPH_OK;
 }
 
+// launch of one cluster of at most `most` blocks over nc cells, a cell per
+// thread: a power of two of blocks, no more than there are warps of cells
+cudaLaunchConfig_t grid_cluster(int nc, int most, cudaStream_t stream, cudaLaunchAttribute *at) {
+  int blocks = 1;
+  while (2 * blocks <= most && 32 * blocks < nc) blocks *= 2;
+  const int per = ((nc + blocks - 1) / blocks + 31) / 32 * 32;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)per);
+  cfg.dynamicSmemBytes = 2 * sizeof(double) * (size_t)per;
+  cfg.stream = stream;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)blocks;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
 // the FAST substeps of one step, the first turning the deposits into dT; the
 // result ends in T0
 int launch_fdm_fast(eph_ctx *c, PhaseScope &ps) {
@@ -250,21 +270,8 @@ int launch_fdm_fast(eph_ctx *c, PhaseScope &ps) {
   // substeps 24.6 / 29.7; 20^3, 17 substeps 37.0 / 35.8)
   if (c->fdm_fast_cluster && c->nsub > 1 && F.nc <= FDM_CLUSTER_CELLS * c->fdm_fast_cluster) {
     ps.launched();
-    int blocks = 1;  // a power of two, no more than there are warps of cells
-    while (2 * blocks <= c->fdm_fast_cluster && 32 * blocks < F.nc) blocks *= 2;
-    const int per = ((F.nc + blocks - 1) / blocks + 31) / 32 * 32;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3((unsigned)per);
-    cfg.dynamicSmemBytes = 2 * sizeof(double) * (size_t)per;
-    cfg.stream = c->stream;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)blocks;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    const cudaLaunchConfig_t cfg = grid_cluster(F.nc, c->fdm_fast_cluster, c->stream, at);
     if (uni)
       CUDA_TRY(c, cudaLaunchKernelEx(&cfg, k_fdm_cluster_fast<true>, F, c->nsub, c->T0.p, rec, c->dT.p, c->acc.p,
                                      c->counters.p));
@@ -465,6 +472,14 @@ bool df_records_wanted(const eph_ctx *c) {
   return df_active(c) || (c->eam && c->mode == EPH_MODE_FAST && c->pair_arith == EPH_PAIRS_DF64);
 }
 
+// atoms below which the EXACT sweeps take more lanes per atom (density 16
+// instead of 4, friction and forces 8 instead of 4): fewer lanes leave fewer
+// idle, more hide latency where the warps are few (GB300, us per step, more /
+// fewer lanes: density 2,048 atoms 31 / 62, 8,788 atoms 48 / 64, 16,384 atoms
+// 85 / 82, 62,500 atoms 268 / 205; friction and forces 500 atoms 47 / 65,
+// 16,384 atoms 106 / 105, 62,500 atoms 357 / 308)
+constexpr int EXACT_WIDE = 16384;
+
 template <bool FAST, bool MULTI, bool FUSE>
 void launch_density_f(eph_ctx *c, int xi_mode) {
   // several lanes per atom in the density sweep too below 16,384 atoms, where
@@ -508,7 +523,18 @@ void launch_density_f(eph_ctx *c, int xi_mode) {
       return;
     }
   }
-  k_density<FAST, MULTI, FUSE><<<nblocks(c->n), BLOCK, 0, c->stream>>>(
+  if constexpr (!FAST) {
+#define EPH_DENSITY_EXACT(L)                                                                                         \
+  k_density_exact<MULTI, L><<<nblocks((long)c->n * L, EXD_THREADS), EXD_THREADS, 0, c->stream>>>(                      \
+      c->P, c->x.p, c->mask.p, c->bin_count.p, c->bins.p, c->atom_bin.p, c->atom_off.p, c->xi.p, xi_mode, c->T0.p,     \
+      c->pj.p, c->pe.p, c->pg.p, c->nshort.p, c->A.p, c->Bw.p, c->rho.p, c->beta_i.p, c->cell.p, c->Te_i.p,            \
+      c->wrapflag.p, c->d_err.p, c->counters.p)
+    if (c->n < EXACT_WIDE) EPH_DENSITY_EXACT(16);
+    else EPH_DENSITY_EXACT(4);
+#undef EPH_DENSITY_EXACT
+    return;
+  }
+  k_density<MULTI, FUSE><<<nblocks(c->n), BLOCK, 0, c->stream>>>(
       c->P, c->x.p, c->mask.p, c->bin_count.p, c->bins.p, c->atom_bin.p, c->atom_off.p, c->xi.p, xi_mode, c->T0.p,
       c->pj.p, c->pe.p, c->pg.p, c->nshort.p, c->A.p, c->Bw.p, c->rho.p, c->beta_i.p, c->cell.p, c->Te_i.p,
       c->wrapflag.p, c->d_err.p, c->counters.p, c->v.p, c->Mm.p, c->G.p);
@@ -522,7 +548,7 @@ void launch_density_t(eph_ctx *c, int xi_mode) {
 
 template <bool FAST, bool MULTI, bool FRIC, bool RAND>
 void launch_forces_t(eph_ctx *c) {
-  const int tpa = FAST ? c->tpa : 1;
+  const int tpa = c->tpa;
   if (FAST && FRIC && df_active(c)) {
 #define EPH_FORCES_DF(T)                                                                                          \
   k_forces_df<MULTI, RAND, T><<<nblocks((long)c->n * T), BLOCK, 0, c->stream>>>(                                   \
@@ -547,8 +573,18 @@ void launch_forces_t(eph_ctx *c) {
 #undef EPH_FORCES_M
     return;
   }
+  if (!FAST) {
+#define EPH_FORCES_EXACT(L)                                                                                          \
+  k_forces_exact<MULTI, FRIC, RAND, L><<<nblocks((long)c->n * L, EX_THREADS), EX_THREADS, 0, c->stream>>>(           \
+      c->P, c->mask.p, c->pj.p, c->pe.p, c->pg.p, c->nshort.p, c->A.p, c->Bw.p, c->Te_i.p, c->f.p, c->f_eph.p,       \
+      c->f_rng.p, c->f_dis.p, c->f_sto.p)
+    if (c->n < EXACT_WIDE) EPH_FORCES_EXACT(8);
+    else EPH_FORCES_EXACT(4);
+#undef EPH_FORCES_EXACT
+    return;
+  }
   if (tpa == 1) {
-    k_forces<FAST, MULTI, FRIC, RAND><<<nblocks(c->n), BLOCK, 0, c->stream>>>(
+    k_forces<MULTI, FRIC, RAND><<<nblocks(c->n), BLOCK, 0, c->stream>>>(
         c->P, c->mask.p, c->pj.p, c->pe.p, c->pg.p, c->nshort.p, c->A.p, c->Bw.p, c->Te_i.p, c->f.p, c->f_eph.p,
         c->f_rng.p, c->f_dis.p, c->f_sto.p);
     return;
@@ -688,8 +724,12 @@ int configure_list(eph_ctx *c) {
 
 // stage 1 as its own sweep: EXACT mode (FAST mode folds it into the density sweep)
 void launch_friction_w(eph_ctx *c) {
-  k_friction_w<<<nblocks(c->n), BLOCK, 0, c->stream>>>(c->P, c->mask.p, c->v.p, c->pj.p, c->pe.p, c->pg.p,
-                                                       c->nshort.p, c->A.p, c->Bw.p);
+#define EPH_FRICTION_W(L)                                                                                        \
+  k_friction_w<L><<<nblocks((long)c->n * L, EX_THREADS), EX_THREADS, 0, c->stream>>>(                             \
+      c->P, c->mask.p, c->v.p, c->pj.p, c->pe.p, c->pg.p, c->nshort.p, c->A.p, c->Bw.p)
+  if (c->n < EXACT_WIDE) EPH_FRICTION_W(8);
+  else EPH_FRICTION_W(4);
+#undef EPH_FRICTION_W
 }
 
 template <bool FAST, bool FRIC, bool RAND>
@@ -874,37 +914,18 @@ int launch_end_of_step(eph_ctx *c) {
     }
     const double3 ih2 = inverse_h2(g);
     double *src = c->T0.p, *dst = c->T1.p;
-    if (!c->td.tdyn && c->fdm_cluster && c->nsub > 1 && g.ntotal <= 2048) {
-      // EXACT on a small grid: every substep in one launch of one thread-block cluster,
-      // the cells spread evenly over its blocks (measured on GB300: 10^3
-      // cells, 17 substeps, 0.178 -> 0.169 ms per step; 16^3 cells, 11
-      // substeps, 35 us per step slower than the per-substep launches, whose
-      // FP64 work then spreads over more SMs)
+    if (!c->td.tdyn && c->mode != EPH_MODE_FAST && c->fdm_exact_cluster && c->nsub > 1 &&
+        g.ntotal <= (long)FDM_EXACT_CELLS * c->fdm_exact_cluster) {
+      // EXACT on a small grid: every substep in one launch of one cluster
+      // (measured on GB300, us per step, cluster / a launch per substep: 4^3
+      // cells 31 / 53, 13^3 29 / 59, 16^3 45 / 69, 20^3 73 / 73)
       ps.launched(1);
-      const long per_block = ((g.ntotal + FDM_CLUSTER - 1) / FDM_CLUSTER + 31) / 32 * 32;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(FDM_CLUSTER);
-      cfg.blockDim = dim3((unsigned)per_block);
-      cfg.stream = c->stream;
       cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = FDM_CLUSTER;
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      double *rec = c->fdm_rec;
-      CUDA_TRY(c, cudaLaunchKernelEx(&cfg, k_fdm_cluster, (long)g.nx, (long)g.ny, (long)g.nz, g.dx, g.dy, g.dz,
-                                     c->inner_dt, c->nsub, c->T0.p, c->T1.p, rec, (const double *)c->kappa.p,
+      const cudaLaunchConfig_t cfg = grid_cluster((int)g.ntotal, c->fdm_exact_cluster, c->stream, at);
+      CUDA_TRY(c, cudaLaunchKernelEx(&cfg, k_fdm_cluster_exact, fdm_args(c), make_double3(g.dx, g.dy, g.dz),
+                                     c->inner_dt, c->nsub, c->T0.p, c->fdm_rec, (const double *)c->kappa.p,
                                      (const double *)c->rhoC.p, (const double *)c->S.p,
-                                     (const signed char *)c->gflag.p, c->dT.p, c->acc.p, c->counters.p, c->td, ih2,
-                                     (const double *)c->irhoC.p));
-      // where the last substep wrote, as with the per-substep launches below
-      if (rec) src = rec + (size_t)(c->nsub - 1) * (size_t)g.ntotal;
-      else if (c->nsub % 2) src = c->T1.p;
-      if (src != c->T0.p)
-        CUDA_TRY(c, cudaMemcpyAsync(c->T0.p, src, sizeof(double) * (size_t)g.ntotal, cudaMemcpyDeviceToDevice,
-                                    c->stream));
+                                     (const signed char *)c->gflag.p, c->dT.p, c->acc.p, c->counters.p));
       CUDA_TRY(c, cudaGetLastError());
       return EPH_OK;
     }
@@ -1109,39 +1130,26 @@ int eph_create(int narg, const char *const *arg, const eph_md *md, eph_ctx **out
   CUDA_TRY(c, cudaSetDevice(c->device));
   CUDA_TRY(c, cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   c->own_stream = true;
-  {  // can a cluster of the small-grid solve be resident (a query; nothing is launched)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(FDM_CLUSTER);
-    cfg.blockDim = dim3(1024);
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = FDM_CLUSTER;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int n1 = 0;
-    c->fdm_cluster = cudaOccupancyMaxActiveClusters(&n1, k_fdm_cluster, &cfg) == cudaSuccess && n1 >= 1;
-    // the FAST substeps' cluster: 16 blocks where the device takes them, else 8
+  // the largest cluster of the small-grid solves that can be resident (a
+  // query; nothing is launched): 16 blocks where the device takes them, else 8
+  auto cluster_of = [](std::initializer_list<const void *> kernels, int cells) {
     for (int size : {16, 8}) {
       bool ok = true;
-      for (auto *kern : {(const void *)k_fdm_cluster_fast<true>, (const void *)k_fdm_cluster_fast<false>}) {
+      for (const void *kern : kernels) {
         if (size > 8) ok = ok && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-        cfg.gridDim = dim3((unsigned)size);
-        cfg.blockDim = dim3(FDM_CLUSTER_CELLS);
-        cfg.dynamicSmemBytes = 2 * FDM_CLUSTER_CELLS * sizeof(double);
-        at[0].val.clusterDim.x = (unsigned)size;
+        cudaLaunchAttribute at[1];
+        const cudaLaunchConfig_t cfg = grid_cluster(size * cells, size, nullptr, at);
         int most = 0;
         ok = ok && cudaOccupancyMaxActiveClusters(&most, kern, &cfg) == cudaSuccess && most >= 1;
       }
       cudaGetLastError();
-      if (ok) {
-        c->fdm_fast_cluster = size;
-        break;
-      }
+      if (ok) return size;
     }
-    cudaGetLastError();
-  }
+    return 0;
+  };
+  c->fdm_fast_cluster = cluster_of({(const void *)k_fdm_cluster_fast<true>, (const void *)k_fdm_cluster_fast<false>},
+                                   FDM_CLUSTER_CELLS);
+  c->fdm_exact_cluster = cluster_of({(const void *)k_fdm_cluster_exact}, FDM_EXACT_CELLS);
   CUDA_TRY(c, cudaMallocHost(&c->h_err, sizeof(unsigned)));
   CUDA_TRY(c, c->d_err.alloc(1));
   CUDA_TRY(c, c->counters.alloc(NCOUNTERS));

@@ -67,10 +67,9 @@ struct eph_ctx {
   bool tpa_auto = true;
   // FAST mode, one lane per atom: stage 1 folded into the density sweep
   bool fuse_w = true;
-  // small grids run all their substeps as one thread-block cluster launch
-  // (EXACT: 8 blocks; FAST: the largest cluster the device takes, 0 for none)
-  bool fdm_cluster = false;
-  int fdm_fast_cluster = 0;
+  // small grids run all their substeps as one thread-block cluster launch:
+  // the blocks of the largest cluster the device takes, 0 for none
+  int fdm_fast_cluster = 0, fdm_exact_cluster = 0;
 
   int n = 0;
   DevBuf<D4> x, v, f, xhold, f_eph, f_rng, xi, fext, A, Bw;

@@ -17,6 +17,7 @@
 #include "eph_candidates.cuh"
 #include "eph_device.cuh"
 #include "eph_df64.cuh"
+#include "eph_softfp.cuh"
 #include "eph_df_pair.cuh"
 
 namespace ephgb {
@@ -298,50 +299,45 @@ __global__ void k_bin_sort(int nbins, int bcap, const int *__restrict__ bin_coun
 
 // One in-cutoff pair (i, j) of the density sweep: rho_j(r^2) into rho_i, the
 // pair cache row at `slot`, and with FUSE_W the sums of M_i and S_i.
-template <bool FAST, bool MULTI, bool FUSE_W>
+template <bool MULTI, bool FUSE_W>
 __device__ __forceinline__ void density_pair(const StepParams &P, int ei, unsigned u, int ej, double ex, double ey,
                                              double ez, double r2, size_t slot, unsigned *__restrict__ pj,
                                              D4 *__restrict__ pe, double2 *__restrict__ pg,
                                              const D4 *__restrict__ v, unsigned *__restrict__ err, double &rho,
                                              double &mxx, double &mxy, double &mxz, double &myy, double &myz,
                                              double &mzz, double &Sx, double &Sy, double &Sz) {
-  const double rji = spline_eval<FAST>(P.tab_rho_r_sq + (size_t)ej * P.n_rho, P.inv_dr_sq, P.n_rho, r2, err);
+  const double rji = spline_eval<true>(P.tab_rho_r_sq + (size_t)ej * P.n_rho, P.inv_dr_sq, P.n_rho, r2, err);
   double rij = rji;
   if (MULTI && ej != ei)
-    rij = spline_eval<FAST>(P.tab_rho_r_sq + (size_t)ei * P.n_rho, P.inv_dr_sq, P.n_rho, r2, err);
-  // with M_i summed (FAST, FUSE_W) rho_i is its trace, sum_j H_ij r^2
+    rij = spline_eval<true>(P.tab_rho_r_sq + (size_t)ei * P.n_rho, P.inv_dr_sq, P.n_rho, r2, err);
+  // with M_i summed (FUSE_W) rho_i is its trace, sum_j H_ij r^2
   // (density_epilogue): one FP64 add per pair less
-  if (!(FAST && FUSE_W)) rho += rji;
+  if (!FUSE_W) rho += rji;
   pj[slot] = u;
-  if (FAST) {
-    const double inv_r2 = recip_nr(r2);
-    const double H = rji * inv_r2;
-    const double hx = H * ex, hy = H * ey, hz = H * ez;
-    if (FUSE_W && !MULTI) {
-      // one element: H_ij = H_ji, and the force sweep takes the pair's
-      // H e from here instead of multiplying by H per pair
-      pe[slot] = D4{ex, ey, ez, hx};
-      pg[slot] = make_double2(hy, hz);
-    } else {
-      pe[slot] = D4{ex, ey, ez, H};
-      if (MULTI) pg[slot] = make_double2(rij * inv_r2, 0.0);
-    }
-    if (FUSE_W) {
-      const D4 vj = v[u & IDX_MASK];
-      mxx = fma(hx, ex, mxx);
-      mxy = fma(hx, ey, mxy);
-      mxz = fma(hx, ez, mxz);
-      myy = fma(hy, ey, myy);
-      myz = fma(hy, ez, myz);
-      mzz = fma(hz, ez, mzz);
-      const double d = dot3_fma(ex, ey, ez, vj.x, vj.y, vj.z);
-      Sx = fma(d, hx, Sx);
-      Sy = fma(d, hy, Sy);
-      Sz = fma(d, hz, Sz);
-    }
+  const double inv_r2 = recip_nr(r2);
+  const double H = rji * inv_r2;
+  const double hx = H * ex, hy = H * ey, hz = H * ez;
+  if (FUSE_W && !MULTI) {
+    // one element: H_ij = H_ji, and the force sweep takes the pair's
+    // H e from here instead of multiplying by H per pair
+    pe[slot] = D4{ex, ey, ez, hx};
+    pg[slot] = make_double2(hy, hz);
   } else {
-    pe[slot] = D4{ex, ey, ez, r2};
-    pg[slot] = make_double2(rji, rij);
+    pe[slot] = D4{ex, ey, ez, H};
+    if (MULTI) pg[slot] = make_double2(rij * inv_r2, 0.0);
+  }
+  if (FUSE_W) {
+    const D4 vj = v[u & IDX_MASK];
+    mxx = fma(hx, ex, mxx);
+    mxy = fma(hx, ey, mxy);
+    mxz = fma(hx, ez, mxz);
+    myy = fma(hy, ey, myy);
+    myz = fma(hy, ez, myz);
+    mzz = fma(hz, ez, mzz);
+    const double d = dot3_fma(ex, ey, ez, vj.x, vj.y, vj.z);
+    Sx = fma(d, hx, Sx);
+    Sy = fma(d, hy, Sy);
+    Sz = fma(d, hz, Sz);
   }
 }
 
@@ -486,7 +482,7 @@ __device__ __forceinline__ void density_epilogue(
 // M_i = sum_j H_ij e e^T and S_i = sum_j H_ij (e.v_j) e (H_ij = rho_j(r^2)/r^2),
 // then w_i = (alpha_i / rho_i) (M_i v_i - S_i).  It also leaves M_i and the
 // records G_i = {a_i w_i, a_i xi_i, rho_i} for k_forces_m.
-template <bool FAST, bool MULTI, bool FUSE_W = false>
+template <bool MULTI, bool FUSE_W = false>
 __global__ void __launch_bounds__(128) k_density(
     StepParams P, const D4 *__restrict__ x, const int *__restrict__ mask, const int *__restrict__ bin_count,
     const BinEntry *__restrict__ bins, const int4 *__restrict__ atom_bin, const float4 *__restrict__ atom_off,
@@ -522,7 +518,7 @@ __global__ void __launch_bounds__(128) k_density(
       Bi = atom_bin[i];
       oi = atom_off[i];
     }
-    nc = collect_candidates<FAST>(P, i, active, Bi, oi, bin_count, bins, err, cget, cset, P.rc2_band, P.kcap);
+    nc = collect_candidates(P, i, active, Bi, oi, bin_count, bins, err, cset, P.rc2_band, P.kcap);
   }
   __syncwarp();
   // pass 2: exact FP64 test, density and pair cache, in lockstep
@@ -536,17 +532,130 @@ __global__ void __launch_bounds__(128) k_density(
       const D4 xj = x[u & IDX_MASK];
       double ex, ey, ez;
       density_vector(P, xi, xj, u >> IDX_BITS, ex, ey, ez);
-      const double r2 = FAST ? dot3_fma(ex, ey, ez, ex, ey, ez) : dot3(ex, ey, ez, ex, ey, ez);
+      const double r2 = dot3_fma(ex, ey, ez, ex, ey, ez);
       if (below(r2, P.rc2)) {  // r2 >= 0
-        density_pair<FAST, MULTI, FUSE_W>(P, ei, u, (int)xj.w, ex, ey, ez, r2, (size_t)ns * P.n + i, pj, pe, pg,
+        density_pair<MULTI, FUSE_W>(P, ei, u, (int)xj.w, ex, ey, ez, r2, (size_t)ns * P.n + i, pj, pe, pg,
                                           v, err, rho, mxx, mxy, mxz, myy, myz, mzz, Sx, Sy, Sz);
         ++ns;
       }
     }
   }
   if (!valid) return;
-  density_epilogue<FAST, FUSE_W>(P, i, active, xi, ei, rho, ns, mxx, mxy, mxz, myy, myz, mzz, Sx, Sy, Sz, xi_given,
+  density_epilogue<true, FUSE_W>(P, i, active, xi, ei, rho, ns, mxx, mxy, mxz, myy, myz, mzz, Sx, Sy, Sz, xi_given,
                                  xi_mode, T_e, nshort, A, Bw, rho_out, beta_out, cell, Te_i, err, counters, v, Mm, G);
+}
+
+// The density sweep of EXACT mode, L lanes per atom: the lanes search
+// the 27 bins together, sort the atom's candidates by neighbour index (each
+// counts the smaller ones of its own, then writes them to their places), test
+// and cache the pairs, compacted in that order; one thread per atom, in the
+// block's first threads, then adds the densities in the same order and
+// finishes the atom.  Candidate k is kept in shared memory for k < EXD_CAP;
+// further ones wait in the atom's rows of pj, and in order in the first word
+// of its rows of pe: row k is read, in step, before the pair rows up to k are
+// written.
+// Latency and issue bind it (FP64 pipe half busy).  One lane per atom inserted
+// each candidate into its place through shared memory, a serial chain.
+// GB300, us per step: 2,048 atoms 377 -> 31, 62,500 atoms 424 -> 205.
+constexpr int EXD_THREADS = 256;
+constexpr int EXD_CAP = 72;  // a row stride of 8 banks: the lanes of 4 atoms in distinct banks
+template <bool MULTI, int L>
+__global__ void __launch_bounds__(EXD_THREADS, 4) k_density_exact(
+    StepParams P, const D4 *__restrict__ x, const int *__restrict__ mask, const int *__restrict__ bin_count,
+    const BinEntry *__restrict__ bins, const int4 *__restrict__ atom_bin, const float4 *__restrict__ atom_off,
+    const D4 *__restrict__ xi_given, int xi_mode, const double *__restrict__ T_e, unsigned *__restrict__ pj,
+    D4 *__restrict__ pe, double2 *__restrict__ pg, int *__restrict__ nshort, D4 *__restrict__ A,
+    D4 *__restrict__ Bw, double *__restrict__ rho_out, double *__restrict__ beta_out, int *__restrict__ cell,
+    double *__restrict__ Te_i, int *__restrict__ wrapflag, unsigned *__restrict__ err,
+    unsigned long long *__restrict__ counters) {
+  constexpr int NA = EXD_THREADS / L, CAP = EXD_CAP;
+  __shared__ unsigned s_found[NA * CAP], s_sorted[NA * CAP];
+  __shared__ int s_ns[NA];
+  const int t = threadIdx.x, a = t / L, g = t & (L - 1), lane = t & 31;
+  const int i = blockIdx.x * NA + a;
+  if (blockIdx.x == 0 && t == 0) *wrapflag = 0;  // the binning kernel has read it
+  const bool active = i < P.n && (mask[i] & P.groupbit) != 0;
+  unsigned *found = s_found + a * CAP, *sorted = s_sorted + a * CAP;
+  auto place = [&](int k) -> unsigned & { return k < CAP ? found[k] : pj[(size_t)k * P.n + i]; };
+  auto in_order = [&](int k) -> unsigned & {
+    return k < CAP ? sorted[k] : *reinterpret_cast<unsigned *>(pe + (size_t)k * P.n + i);
+  };
+  int nc = 0;
+  {
+    int4 Bi = make_int4(0, 0, 0, 0);
+    float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (active) {
+      Bi = atom_bin[i];
+      oi = atom_off[i];
+    }
+    auto set = [&](int k, unsigned u) { place(k) = u; };
+    shared_candidates<L>(P, i, active, Bi, oi, bin_count, bins, err, nc, P.kcap, set, P.rc2_band);
+  }
+  __syncwarp();
+  const int nmax = __reduce_max_sync(0xffffffffu, nc);
+  // an atom's candidates are distinct atoms: a box has at least three bins
+  // along every axis
+  for (int m = g; m - g < nmax; m += 4 * L) {
+    unsigned u[4], key[4];
+    int rank[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      u[q] = m + q * L < nc ? place(m + q * L) : 0u;
+      key[q] = u[q] & IDX_MASK;
+    }
+    for (int k = 0; k < nc; ++k) {
+      const unsigned other = place(k) & IDX_MASK;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) rank[q] += other < key[q] ? 1 : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (m + q * L < nc) in_order(rank[q]) = u[q];
+  }
+  __syncwarp();
+  D4 xi = D4{0.0, 0.0, 0.0, 0.0};
+  if (active) xi = x[i];
+  const int ei = (int)xi.w;
+  int ns = 0;
+  for (int k = g; k - g < nmax; k += L) {
+    bool in = false;
+    unsigned u = 0;
+    D4 xj = D4{0.0, 0.0, 0.0, 0.0};
+    double ex = 0.0, ey = 0.0, ez = 0.0, r2 = 0.0;
+    if (k < nc) {
+      u = in_order(k);
+      xj = x[u & IDX_MASK];
+      density_vector(P, xi, xj, u >> IDX_BITS, ex, ey, ez);
+      r2 = dot3(ex, ey, ez, ex, ey, ez);
+      in = below(r2, P.rc2);  // r2 >= 0
+    }
+    const unsigned who = (__ballot_sync(0xffffffffu, in) >> (lane & ~(L - 1))) & ((1u << L) - 1u);
+    if (in) {
+      const size_t slot = (size_t)(ns + __popc(who & ((1u << g) - 1u))) * P.n + i;
+      const int ej = (int)xj.w;
+      const double rji = spline_eval<false>(P.tab_rho_r_sq + (size_t)ej * P.n_rho, P.inv_dr_sq, P.n_rho, r2, err);
+      double rij = rji;
+      if (MULTI && ej != ei)
+        rij = spline_eval<false>(P.tab_rho_r_sq + (size_t)ei * P.n_rho, P.inv_dr_sq, P.n_rho, r2, err);
+      pj[slot] = u;
+      pe[slot] = D4{ex, ey, ez, r2};
+      pg[slot] = make_double2(rji, rij);
+    }
+    ns += __popc(who);
+  }
+  if (g == 0) s_ns[a] = ns;
+  __syncthreads();
+  if (t >= NA) return;
+  const int o = blockIdx.x * NA + t;
+  if (o >= P.n) return;
+  ns = s_ns[t];
+  double rho = 0.0;
+#pragma unroll 8
+  for (int k = 0; k < ns; ++k) rho += pg[(size_t)k * P.n + o].x;
+  const D4 xo = x[o];
+  density_epilogue<false, false>(P, o, (mask[o] & P.groupbit) != 0, xo, (int)xo.w, rho, ns, 0.0, 0.0, 0.0, 0.0, 0.0,
+                                 0.0, 0.0, 0.0, 0.0, xi_given, xi_mode, T_e, nshort, A, Bw, rho_out, beta_out, cell,
+                                 Te_i, err, counters, nullptr, nullptr, nullptr);
 }
 
 // ------------------------------------------- FAST pair sweeps in df64
@@ -661,7 +770,7 @@ __global__ void __launch_bounds__(tpa_threads(TPA)) k_density_tpa(
     double ex, ey, ez;
     density_vector(P, xi, xj, u >> IDX_BITS, ex, ey, ez);
     const double r2 = dot3_fma(ex, ey, ez, ex, ey, ez);
-    density_pair<true, MULTI, FUSE_W>(P, ei, u, (int)xj.w, ex, ey, ez, r2, (size_t)k * P.n + i, pj, pe, pg, v, err,
+    density_pair<MULTI, FUSE_W>(P, ei, u, (int)xj.w, ex, ey, ez, r2, (size_t)k * P.n + i, pj, pe, pg, v, err,
                                       rho, mxx, mxy, mxz, myy, myz, mzz, Sx, Sy, Sz);
   }
   // sum q of the atom's lane l at q * 128 + l * NA + (atom): the finishing
@@ -842,7 +951,6 @@ __global__ void __maxnreg__(64) k_density_list(
   const bool valid = i < P.n;
   const bool active = valid && (mask[i] & P.groupbit) != 0;
   const size_t n = (size_t)P.n;
-  auto sget = [&](int k) -> unsigned { return k < CAND_SMEM ? s_cand[k * nt + t] : pj[(size_t)k * n + i]; };
   auto sset = [&](int k, unsigned u) {
     if (k < CAND_SMEM)
       s_cand[k * nt + t] = u;
@@ -854,7 +962,6 @@ __global__ void __maxnreg__(64) k_density_list(
     if (k < CAND_SMEM) s_cand[k * nt + t] = u;
     cl[(size_t)k * n + i] = u;
   };
-  auto lget = [&](int k) -> unsigned { return cl[(size_t)k * n + i]; };
   D4 xi = D4{0.0, 0.0, 0.0, 0.0};
   if (valid) xi = x[i];
   const int ei = (int)xi.w;
@@ -871,8 +978,8 @@ __global__ void __maxnreg__(64) k_density_list(
     // the candidates inside the cut-off first, the shell out to r_list after
     // them: the shell's pairs mostly fail the exact test, and at the end of
     // the lists whole warps skip them
-    nc = collect_candidates<true>(P, i, active, Bi, oi, bin_count, bins, err, lget, lset, P.rc2_band, P.lcap);
-    nc = collect_candidates<true>(P, i, active, Bi, oi, bin_count, bins, err, lget, lset, P.rl2_band, P.lcap,
+    nc = collect_candidates(P, i, active, Bi, oi, bin_count, bins, err, lset, P.rc2_band, P.lcap);
+    nc = collect_candidates(P, i, active, Bi, oi, bin_count, bins, err, lset, P.rl2_band, P.lcap,
                                   nullptr, P.rc2_band, nc);
     if (valid) cl_n[i] = nc;
   } else {
@@ -889,7 +996,7 @@ __global__ void __maxnreg__(64) k_density_list(
           oi = atom_off[i];
         }
       }
-      nc = collect_candidates<true, true>(P, i, fresh, Bi, oi, bin_count, bins, err, sget, sset, P.rl2_band, P.kcap,
+      nc = collect_candidates<true>(P, i, fresh, Bi, oi, bin_count, bins, err, sset, P.rl2_band, P.kcap,
                                           state);
       // the moved atoms near enough (a widened test; pass 2 decides)
       const int nf = rb[1];  // <= LIST_FMAX on a step without a build
@@ -939,7 +1046,7 @@ __global__ void __maxnreg__(64) k_density_list(
       const double r2 = dot3_fma(ex, ey, ez, ex, ey, ez);
       if (below(r2, P.rc2)) {
         if (ns < P.kcap)
-          density_pair<true, MULTI, true>(P, ei, j | (code << IDX_BITS), (int)xj.w, ex, ey, ez, r2,
+          density_pair<MULTI, true>(P, ei, j | (code << IDX_BITS), (int)xj.w, ex, ey, ez, r2,
                                           (size_t)ns * n + i, pj, pe, pg, v, err, rho, mxx, mxy, mxz, myy, myz, mzz,
                                           Sx, Sy, Sz);
         else
@@ -1180,37 +1287,86 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
 
 // -------------------------------------------------------- friction sweep 1
 
+// The EXACT sweeps over the pairs: several lanes of a warp per atom make the
+// terms of as many pairs at once, and the sums still run one pair after the
+// other in ascending neighbour index, as the reference's do: the terms of a
+// chunk go through shared memory, where each of an atom's first lanes adds
+// one component's.  A pair that does not count leaves -0.0, which changes no
+// sum.  (One lane per atom left the SMs few warps with chains of FP64
+// latency, and everything else waiting for it.)
+constexpr int EX_THREADS = 128;
+constexpr int EX_ROW = EX_THREADS + 1;  // row of one component: distinct banks for the adding lanes
+
+// dot3 with its products on the integer units
+__device__ __forceinline__ double soft_dot3(const D4 &e, double x, double y, double z) {
+  return soft::mul(e.x, x) + soft::mul(e.y, y) + soft::mul(e.z, z);
+}
+
 // force_prl stage 1 (fix_eph.cpp:699-741) in the reference's expression order
 // (EXACT mode; FAST mode folds it into the density sweep):
 // w_i = sum_j p_ij [(e.v_i) - (e.v_j)] e,  p_ij = alpha_i rho_j(r^2) / (rho_i r^2)
-__global__ void __launch_bounds__(128) k_friction_w(StepParams P, const int *__restrict__ mask,
-                                                     const D4 *__restrict__ v, const unsigned *__restrict__ pj,
-                                                     const D4 *__restrict__ pe, const double2 *__restrict__ pg,
-                                                     const int *__restrict__ nshort, const D4 *__restrict__ A,
-                                                     D4 *__restrict__ Bw) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P.n) return;
-  const D4 Ai = A[i];
-  if (!(mask[i] & P.groupbit) || !pos_double(Ai.x)) return;  // Bw[i].yzw stays 0
-  const D4 vi = v[i];
-  const int ns = nshort[i];
-  double wx = 0.0, wy = 0.0, wz = 0.0;
-  for (int k = 0; k < ns; ++k) {
-    const size_t slot = (size_t)k * P.n + i;
-    const unsigned j = pj[slot] & IDX_MASK;
-    const D4 e = pe[slot];
-    const D4 vj = v[j];
-    const double rji = pg[slot].x;
-    const double prescaler = Ai.y * rji / (Ai.x * e.w);
-    const double var1 = prescaler * dot3(e.x, e.y, e.z, vi.x, vi.y, vi.z);
-    const double var2 = prescaler * dot3(e.x, e.y, e.z, vj.x, vj.y, vj.z);
-    const double dvar = var1 - var2;
-    wx += dvar * e.x;
-    wy += dvar * e.y;
-    wz += dvar * e.z;
+// FP64 issue binds it: what a pair leaves to the FP64 pipe is 12 operations,
+// the quotient and ten of the 13 products run on the integer units.  GB300, us
+// per step at 62,500 atoms: 186 with one lane per atom and the hardware's
+// operations; 145 with the quotients here; 127 with four lanes; 82 with the
+// products.
+template <int L>
+__global__ void __launch_bounds__(EX_THREADS) k_friction_w(StepParams P, const int *__restrict__ mask,
+                                                            const D4 *__restrict__ v, const unsigned *__restrict__ pj,
+                                                            const D4 *__restrict__ pe, const double2 *__restrict__ pg,
+                                                            const int *__restrict__ nshort, const D4 *__restrict__ A,
+                                                            D4 *__restrict__ Bw) {
+  __shared__ double s_term[3 * EX_ROW];
+  const int t = threadIdx.x, g = t & (L - 1), i = blockIdx.x * (EX_THREADS / L) + t / L;
+  D4 Ai{0.0, 0.0, 0.0, 0.0}, vi{0.0, 0.0, 0.0, 0.0};
+  int ns = 0;
+  if (i < P.n && (mask[i] & P.groupbit)) {
+    Ai = A[i];
+    if (pos_double(Ai.x)) {  // otherwise Bw[i].yzw stays 0
+      vi = v[i];
+      ns = nshort[i];
+    }
   }
-  const double xiz = Bw[i].x;
-  Bw[i] = D4{xiz, wx, wy, wz};
+  constexpr int OWN = (3 + L - 1) / L;  // components g, g + L, ...
+  double w[OWN];
+#pragma unroll
+  for (int c = 0; c < OWN; ++c) w[c] = 0.0;
+  const int nmax = __reduce_max_sync(0xffffffffu, ns);
+  for (int k = g; k - g < nmax; k += L) {
+    double tx = -0.0, ty = -0.0, tz = -0.0;
+    if (k < ns) {
+      const size_t slot = (size_t)k * P.n + i;
+      const unsigned j = pj[slot] & IDX_MASK;
+      const D4 e = pe[slot];
+      const D4 vj = v[j];
+      const double rji = pg[slot].x;
+      const double prescaler = soft::div(soft::mul(Ai.y, rji), soft::divisor(soft::mul(Ai.x, e.w)));
+      const double var1 = soft::mul(prescaler, dot3(e.x, e.y, e.z, vi.x, vi.y, vi.z));
+      const double var2 = soft::mul(prescaler, soft_dot3(e, vj.x, vj.y, vj.z));
+      const double dvar = var1 - var2;
+      tx = soft::mul(dvar, e.x);
+      ty = soft::mul(dvar, e.y);
+      tz = soft::mul(dvar, e.z);
+    }
+    s_term[t] = tx;
+    s_term[EX_ROW + t] = ty;
+    s_term[2 * EX_ROW + t] = tz;
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < OWN; ++c) {
+      const int q = g + c * L;
+      if (q < 3) {
+        const double *term = s_term + q * EX_ROW + (t - g);
+#pragma unroll
+        for (int m = 0; m < L; ++m) w[c] += term[m];
+      }
+    }
+    __syncwarp();
+  }
+  if (ns == 0) return;
+#pragma unroll
+  for (int c = 0; c < OWN; ++c)
+    if (g + c * L < 3) reinterpret_cast<double *>(Bw + i)[1 + g + c * L] = w[c];
 }
 
 // ------------------------------------------------ friction + random sweep
@@ -1263,10 +1419,10 @@ __device__ __forceinline__ void store_forces(const StepParams &P, int i, bool li
 }
 
 // force_prl stages 2 and 3 (fix_eph.cpp:748-836) in one pass over the pairs,
-// then the force update of post_force (fix_eph.cpp:892-906):
+// then the force update of post_force (fix_eph.cpp:892-906), FAST mode:
 //   f_EPH_i -= sum_j [a_i rho_j(r^2) (e.w_i)/(rho_i r^2) - a_j rho_i(r^2) (e.w_j)/(rho_j r^2)] e
 //   f_RNG_i  = eta sqrt(T_e(x_i)) sum_j [same with xi] e
-template <bool FAST, bool MULTI, bool FRIC, bool RAND>
+template <bool MULTI, bool FRIC, bool RAND>
 __global__ void __launch_bounds__(128) k_forces(StepParams P, const int *__restrict__ mask,
                                                 const unsigned *__restrict__ pj, const D4 *__restrict__ pe,
                                                 const double2 *__restrict__ pg, const int *__restrict__ nshort,
@@ -1289,49 +1445,26 @@ __global__ void __launch_bounds__(128) k_forces(StepParams P, const int *__restr
       const D4 Aj = A[j];
       if (!pos_double(Aj.x)) continue;
       const D4 e = pe[slot];
-      // FAST mode with one element has no pg rows (the buffer is not allocated)
-      const double2 g = (FAST && !MULTI) ? make_double2(0.0, 0.0) : pg[slot];
+      // one element has no pg rows (the buffer is not allocated)
+      const double2 g = MULTI ? pg[slot] : make_double2(0.0, 0.0);
       const D4 Bj = Bw[j];
-      if (FAST) {
-        const double a = Ai.y * e.w;                  // alpha_i/rho_i * rho_j(r^2)/r^2
-        const double b = Aj.y * (MULTI ? g.x : e.w);  // alpha_j/rho_j * rho_i(r^2)/r^2
-        if (FRIC) {
-          const double di = dot3_fma(e.x, e.y, e.z, Bi.y, Bi.z, Bi.w);
-          const double dj = dot3_fma(e.x, e.y, e.z, Bj.y, Bj.z, Bj.w);
-          const double dvar = fma(a, di, -(b * dj));
-          fex = fma(-dvar, e.x, fex);
-          fey = fma(-dvar, e.y, fey);
-          fez = fma(-dvar, e.z, fez);
-        }
-        if (RAND) {
-          const double di = dot3_fma(e.x, e.y, e.z, xix, xiy, xiz);
-          const double dj = dot3_fma(e.x, e.y, e.z, Aj.z, Aj.w, Bj.x);
-          const double dvar = fma(a, di, -(b * dj));
-          frx = fma(dvar, e.x, frx);
-          fry = fma(dvar, e.y, fry);
-          frz = fma(dvar, e.z, frz);
-        }
-      } else {
-        const double r2 = e.w;
-        const double ai = Ai.y * g.x;                 // alpha_i * rho_j(r^2)
-        const double aj = Aj.y * (MULTI ? g.y : g.x);  // alpha_j * rho_i(r^2)
-        const double den_i = Ai.x * r2, den_j = Aj.x * r2;
-        if (FRIC) {
-          const double var1 = ai * dot3(e.x, e.y, e.z, Bi.y, Bi.z, Bi.w) / den_i;
-          const double var2 = aj * dot3(e.x, e.y, e.z, Bj.y, Bj.z, Bj.w) / den_j;
-          const double dvar = var1 - var2;
-          fex -= dvar * e.x;
-          fey -= dvar * e.y;
-          fez -= dvar * e.z;
-        }
-        if (RAND) {
-          const double var1 = ai * dot3(e.x, e.y, e.z, xix, xiy, xiz) / den_i;
-          const double var2 = aj * dot3(e.x, e.y, e.z, Aj.z, Aj.w, Bj.x) / den_j;
-          const double dvar = var1 - var2;
-          frx += dvar * e.x;
-          fry += dvar * e.y;
-          frz += dvar * e.z;
-        }
+      const double a = Ai.y * e.w;                  // alpha_i/rho_i * rho_j(r^2)/r^2
+      const double b = Aj.y * (MULTI ? g.x : e.w);  // alpha_j/rho_j * rho_i(r^2)/r^2
+      if (FRIC) {
+        const double di = dot3_fma(e.x, e.y, e.z, Bi.y, Bi.z, Bi.w);
+        const double dj = dot3_fma(e.x, e.y, e.z, Bj.y, Bj.z, Bj.w);
+        const double dvar = fma(a, di, -(b * dj));
+        fex = fma(-dvar, e.x, fex);
+        fey = fma(-dvar, e.y, fey);
+        fez = fma(-dvar, e.z, fez);
+      }
+      if (RAND) {
+        const double di = dot3_fma(e.x, e.y, e.z, xix, xiy, xiz);
+        const double dj = dot3_fma(e.x, e.y, e.z, Aj.z, Aj.w, Bj.x);
+        const double dvar = fma(a, di, -(b * dj));
+        frx = fma(dvar, e.x, frx);
+        fry = fma(dvar, e.y, fry);
+        frz = fma(dvar, e.z, frz);
       }
     }
     if (RAND) {
@@ -1342,6 +1475,108 @@ __global__ void __launch_bounds__(128) k_forces(StepParams P, const int *__restr
     }
   }
   store_forces<FRIC, RAND>(P, i, live, fex, fey, fez, frx, fry, frz, f, f_eph, f_rng, f_dis, f_sto);
+}
+
+// The same in the reference's expression order (EXACT mode).  FP64 issue
+// and integer issue bind it: per pair 32 operations stay on the FP64 pipe (the
+// four scalar products and the sums; with these products on the integer units
+// too it took 240), beside two divisors, four quotients and ten products on
+// the integer units.  GB300, us per step at 62,500 atoms: 459 with one lane
+// per atom and the hardware's operations; 277 with the quotients here; 226 with
+// four lanes and the products.
+template <bool MULTI, bool FRIC, bool RAND, int L>
+__global__ void __launch_bounds__(EX_THREADS) k_forces_exact(StepParams P, const int *__restrict__ mask,
+                                                              const unsigned *__restrict__ pj,
+                                                              const D4 *__restrict__ pe,
+                                                              const double2 *__restrict__ pg,
+                                                              const int *__restrict__ nshort,
+                                                              const D4 *__restrict__ A, const D4 *__restrict__ Bw,
+                                                              const double *__restrict__ Te_i, D4 *__restrict__ f,
+                                                              D4 *__restrict__ f_eph, D4 *__restrict__ f_rng,
+                                                              D4 *__restrict__ f_dis, D4 *__restrict__ f_sto) {
+  constexpr int NA = EX_THREADS / L;
+  __shared__ double s_term[6 * EX_ROW];
+  const int t = threadIdx.x, g = t & (L - 1), i = blockIdx.x * NA + t / L;
+  D4 Ai{0.0, 0.0, 0.0, 0.0}, Bi{0.0, 0.0, 0.0, 0.0};
+  int ns = 0;
+  if (i < P.n && (mask[i] & P.groupbit)) {
+    Ai = A[i];
+    if (pos_double(Ai.x)) {
+      Bi = Bw[i];
+      ns = nshort[i];
+    }
+  }
+  // components g, g + L, ... of friction x, y, z, random x, y, z
+  constexpr int OWN = (6 + L - 1) / L;
+  double sum[OWN];
+#pragma unroll
+  for (int c = 0; c < OWN; ++c) sum[c] = 0.0;
+  const int nmax = FRIC || RAND ? __reduce_max_sync(0xffffffffu, ns) : 0;
+  for (int k = g; k - g < nmax; k += L) {
+    double term[6] = {-0.0, -0.0, -0.0, -0.0, -0.0, -0.0};
+    if (k < ns) {
+      const size_t slot = (size_t)k * P.n + i;
+      const unsigned j = pj[slot] & IDX_MASK;
+      const D4 Aj = A[j];
+      if (pos_double(Aj.x)) {
+        const D4 e = pe[slot];
+        const double2 q = pg[slot];
+        const D4 Bj = Bw[j];
+        const double ai = soft::mul(Ai.y, q.x);                  // alpha_i * rho_j(r^2)
+        const double aj = soft::mul(Aj.y, MULTI ? q.y : q.x);  // alpha_j * rho_i(r^2)
+        const soft::Divisor den_i = soft::divisor(soft::mul(Ai.x, e.w)), den_j = soft::divisor(soft::mul(Aj.x, e.w));
+        if (FRIC) {
+          const double var1 = soft::div(ai * dot3(e.x, e.y, e.z, Bi.y, Bi.z, Bi.w), den_i);
+          const double var2 = soft::div(aj * dot3(e.x, e.y, e.z, Bj.y, Bj.z, Bj.w), den_j);
+          const double dvar = var1 - var2;
+          term[0] = -soft::mul(dvar, e.x);
+          term[1] = -soft::mul(dvar, e.y);
+          term[2] = -soft::mul(dvar, e.z);
+        }
+        if (RAND) {
+          const double var1 = soft::div(ai * dot3(e.x, e.y, e.z, Ai.z, Ai.w, Bi.x), den_i);
+          const double var2 = soft::div(aj * dot3(e.x, e.y, e.z, Aj.z, Aj.w, Bj.x), den_j);
+          const double dvar = var1 - var2;
+          term[3] = soft::mul(dvar, e.x);
+          term[4] = soft::mul(dvar, e.y);
+          term[5] = soft::mul(dvar, e.z);
+        }
+      }
+    }
+#pragma unroll
+    for (int q = FRIC ? 0 : 3; q < (RAND ? 6 : 3); ++q) s_term[q * EX_ROW + t] = term[q];
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < OWN; ++c) {
+      const int q = g + c * L;
+      if (q >= (FRIC ? 0 : 3) && q < (RAND ? 6 : 3)) {
+        const double *p = s_term + q * EX_ROW + (t - g);
+#pragma unroll
+        for (int m = 0; m < L; ++m) sum[c] += p[m];
+      }
+    }
+    __syncwarp();
+  }
+  // a thread per atom finishes, in the block's first threads
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < OWN; ++c)
+    if (g + c * L < 6) s_term[(g + c * L) * EX_ROW + t / L] = sum[c];
+  __syncthreads();
+  if (t >= NA) return;
+  const int o = blockIdx.x * NA + t;
+  if (o >= P.n) return;
+  double r[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) r[q] = s_term[q * EX_ROW + t];
+  const bool live = (mask[o] & P.groupbit) && pos_double(A[o].x);
+  if (RAND && live) {
+    const double var = P.eta * sqrt(Te_i[o]);
+    r[3] *= var;
+    r[4] *= var;
+    r[5] *= var;
+  }
+  store_forces<FRIC, RAND>(P, o, live, r[0], r[1], r[2], r[3], r[4], r[5], f, f_eph, f_rng, f_dis, f_sto);
 }
 
 // Stages 2 and 3 in FAST mode after k_density<.., true> (same sums as
@@ -1894,18 +2129,16 @@ __global__ void k_fdm_bounds(long ncells, const double *__restrict__ C, const do
 // periodic wrap and ZERO_DERIVATIVE walls, then T += (ddT + dT + S)/(rho_e C_e)
 // dt' on DYNAMIC cells and the clamp at T = 0.  FAST: ih2 = 1/h^2 per axis and
 // irhoC = 1/(rho_e C_e) per cell come precomputed (the same correctly rounded
-// quotients as 1.0 / x here).  CG: read the temperatures through L2 only
-// (other blocks wrote them in the substep before).
-template <bool FAST, bool CG>
+// quotients as 1.0 / x here).
+template <bool FAST>
 __device__ __forceinline__ double fdm_cell(long r, long nx, long ny, long nz, double dx, double dy, double dz,
                                            double inner_dt, const double *__restrict__ T,
                                            const double *__restrict__ kappa, const double *__restrict__ rhoC,
                                            const double *__restrict__ S, const signed char *__restrict__ flag,
                                            double dTr, unsigned long long *__restrict__ counters,
                                            const TdynTables &td, double3 ih2, const double *__restrict__ irhoC) {
-  auto ldT = [&](long k) -> double { return CG ? __ldcg(T + k) : T[k]; };
   const long i = r % nx, j = (r / nx) % ny, k = r / (nx * ny);
-  const double Tr = ldT(r);
+  const double Tr = T[r];
   double ddT = 0.0;
   if (flag[r] != 2) {
     long p, q;
@@ -1921,14 +2154,15 @@ __device__ __forceinline__ double fdm_cell(long r, long nx, long ny, long nz, do
       q = qr[a];
       if (flag[q] == 2) q = r;
       else if (flag[p] == 2) p = r;
-      const double Tq = ldT(q), Tp = ldT(p);
+      const double Tq = T[q], Tp = T[p];
       if (FAST) {  // reciprocals instead of the reference's divisions (within 1e-15 of them)
         const double ih2v = ih2s[a];
         ddT = fma((kappa[q] - kappa[p]) * (Tq - Tp), 0.25 * ih2v, ddT);
         ddT = fma(kappa[r] * ih2v, Tq + Tp - 2.0 * Tr, ddT);
       } else {
-        ddT += (kappa[q] - kappa[p]) * (Tq - Tp) / h[a] / h[a] / 4.0;
-        ddT += kappa[r] * ((Tq + Tp - 2.0 * Tr) / h[a] / h[a]);
+        const soft::Divisor hd = soft::divisor(h[a]);
+        ddT += soft::div(soft::div((kappa[q] - kappa[p]) * (Tq - Tp), hd), hd) * 0.25;
+        ddT += kappa[r] * soft::div(soft::div(Tq + Tp - 2.0 * Tr, hd), hd);
       }
     }
   }
@@ -1941,7 +2175,7 @@ __device__ __forceinline__ double fdm_cell(long r, long nx, long ny, long nz, do
       E += (ddT + dTr + S[r]) / td.rho[r] * inner_dt;
       t = linear_reverse(td, E);
     } else {
-      t += (ddT + dTr + S[r]) / rhoC[r] * inner_dt;
+      t += soft::div(ddT + dTr + S[r], soft::divisor(rhoC[r])) * inner_dt;
     }
   }
   if (t < 0.0) {
@@ -1977,50 +2211,8 @@ __global__ void k_fdm_substep(long nx, long ny, long nz, double dx, double dy, d
   } else {
     dTr = dT[r];
   }
-  Tout[r] = fdm_cell<FAST, false>(r, nx, ny, nz, dx, dy, dz, inner_dt, T, kappa, rhoC, S, flag, dTr, counters, td,
+  Tout[r] = fdm_cell<FAST>(r, nx, ny, nz, dx, dy, dz, inner_dt, T, kappa, rhoC, S, flag, dTr, counters, td,
                                   ih2, irhoC);
-}
-
-// All substeps of a small grid (EXACT) in one launch of one thread-block cluster of
-// FDM_CLUSTER blocks (one per SM), block b holding the cells
-// [b * blockDim, (b + 1) * blockDim) (one cell per thread).  Substeps are
-// separated by a device-scope fence and the cluster's hardware barrier,
-// which every thread of every block reaches the same number of times (the
-// loop bound is a launch argument).  Substep s reads src, writes dst as the
-// per-substep launches do (rec: substep s writes rec + s * ncells);
-// temperatures are read through L2.  Results are those of nsub launches of
-// k_fdm_substep.
-constexpr int FDM_CLUSTER = 8;
-__global__ void __launch_bounds__(1024, 1)
-    k_fdm_cluster(long nx, long ny, long nz, double dx, double dy, double dz, double inner_dt, unsigned nsub,
-                  double *__restrict__ T0, double *__restrict__ T1, double *__restrict__ rec,
-                  const double *__restrict__ kappa, const double *__restrict__ rhoC, const double *__restrict__ S,
-                  const signed char *__restrict__ flag, double *__restrict__ dT, U128 *__restrict__ acc,
-                  unsigned long long *__restrict__ counters, TdynTables td, double3 ih2,
-                  const double *__restrict__ irhoC) {
-  const long ntotal = nx * ny * nz;
-  const long r = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool mine = r < ntotal;
-  double dTr = 0.0;
-  if (mine) {
-    U128 a = acc[r];
-    dTr = from_fixed(a);
-    dT[r] = dTr;
-    acc[r] = U128{0ull, 0ull};
-  }
-  const double *src = T0;
-  double *dst = T1;
-  for (unsigned s = 0; s < nsub; ++s) {
-    if (rec) dst = rec + (size_t)s * (size_t)ntotal;
-    if (mine)
-      dst[r] = fdm_cell<false, true>(r, nx, ny, nz, dx, dy, dz, inner_dt, src, kappa, rhoC, S, flag, dTr, counters,
-                                    td, ih2, irhoC);
-    __threadfence();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    double *next = rec ? nullptr : const_cast<double *>(src);
-    src = dst;
-    if (!rec) dst = next;
-  }
 }
 
 // ------------------------------------------------ FAST grid substeps
@@ -2206,6 +2398,84 @@ __global__ void __launch_bounds__(FDM_CLUSTER_CELLS)
       for (int q = 0; q < 6; ++q)
         asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(Tm[q]) : "r"(at[q] + cur) : "memory");
       T = fdm_next<UNIFORM>(T, Tm, w, src, counters);
+      s_T[(cur ? 0 : nt) + t] = T;
+      if (rec) rec[(size_t)s * (size_t)F.nc + r] = T;
+    }
+    cur = half - cur;
+  }
+  if (mine) T0[r] = T;
+  // no block leaves while another may still read its buffers
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The EXACT substeps of a small grid the same way, in fdm_cell's expressions
+// (no cell with a temperature-dependent C_e).  The quotients' latency binds it:
+// 13 per cell and substep, of which three follow one another.  GB300, us per
+// step: 8^3 cells 116 -> 33, 20^3 cells 134 -> 73.
+constexpr int FDM_EXACT_CELLS = 512;  // cells per block at most
+__global__ void __launch_bounds__(FDM_EXACT_CELLS)
+    k_fdm_cluster_exact(FdmFast F, double3 h, double inner_dt, unsigned nsub, double *__restrict__ T0,
+                        double *__restrict__ rec, const double *__restrict__ kappa, const double *__restrict__ rhoC,
+                        const double *__restrict__ S, const signed char *__restrict__ flag, double *__restrict__ dT,
+                        U128 *__restrict__ acc, unsigned long long *__restrict__ counters) {
+  extern __shared__ double s_T[];  // [2][blockDim]
+  const int t = (int)threadIdx.x, nt = (int)blockDim.x;
+  const int r = (int)blockIdx.x * nt + t;
+  const bool mine = r < F.nc;
+  const soft::Divisor hd[3] = {soft::divisor(h.x), soft::divisor(h.y), soft::divisor(h.z)};
+  soft::Divisor rc = hd[0];
+  double T = 0.0, dTr = 0.0, Sr = 0.0, kr = 0.0, kd[3] = {0.0, 0.0, 0.0};
+  int fl = 0;
+  unsigned at[6];
+  if (mine) {
+    int m[6];
+    fdm_neighbours(F, r, m);
+    fl = flag[r];
+    kr = kappa[r];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      int &p = m[2 * a], &q = m[2 * a + 1];
+      if (flag[q] == 2) q = r;
+      else if (flag[p] == 2) p = r;
+      kd[a] = kappa[q] - kappa[p];
+    }
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      const int owner = m[q] / nt;
+      const unsigned local = (unsigned)__cvta_generic_to_shared(s_T + (m[q] - owner * nt));
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at[q]) : "r"(local), "r"(owner));
+    }
+    T = T0[r];
+    s_T[t] = T;
+    rc = soft::divisor(rhoC[r]);
+    Sr = S[r];
+    dTr = from_fixed(acc[r]);
+    dT[r] = dTr;
+    acc[r] = U128{0ull, 0ull};
+  }
+  unsigned cur = 0;
+  const unsigned half = (unsigned)(nt * sizeof(double));
+  for (unsigned s = 0; s < nsub; ++s) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (mine) {
+      double Tm[6];
+#pragma unroll
+      for (int q = 0; q < 6; ++q)
+        asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(Tm[q]) : "r"(at[q] + cur) : "memory");
+      double ddT = 0.0;
+      if (fl != 2) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          const double Tp = Tm[2 * a], Tq = Tm[2 * a + 1];
+          ddT += soft::div(soft::div(kd[a] * (Tq - Tp), hd[a]), hd[a]) * 0.25;
+          ddT += kr * soft::div(soft::div(Tq + Tp - 2.0 * T, hd[a]), hd[a]);
+        }
+      }
+      if (fl == 1) T += soft::div(ddT + dTr + Sr, rc) * inner_dt;
+      if (T < 0.0) {
+        T = 0.0;
+        atomicAdd(&counters[CNT_T_CLAMP], 1ull);
+      }
       s_T[(cur ? 0 : nt) + t] = T;
       if (rec) rec[(size_t)s * (size_t)F.nc + r] = T;
     }
