@@ -422,12 +422,13 @@ void launch_density_df(eph_ctx *c, int xi_mode) {
   C.pj = c->pj.p;
   C.kcap = c->P.kcap;
   C.band = c->P.rc2_band;
-  C.rc2 = c->P.rc2;
   C.cl = c->cl.p;
   C.cl_n = c->cl_n.p;
   C.state = c->state.p;
   C.rb = c->rb.p;
   C.flist = c->flist.p;
+  C.fpos = c->fpos.p;
+  C.far2 = far_cutoff2(c, c->P.rc2);
   C.xref = c->xref.p;
   D.mask = c->mask.p;
   D.v = c->v.p;
@@ -674,6 +675,7 @@ void drop_list(eph_ctx *c) {
   c->state.free();
   c->rb.free();
   c->flist.free();
+  c->fpos.free();
   c->xref.free();
 }
 
@@ -708,12 +710,17 @@ int configure_list(eph_ctx *c) {
   if (c->xref.n != N) CUDA_TRY(c, c->xref.alloc(N));
   if (!c->rb.p) CUDA_TRY(c, c->rb.alloc(4));
   if (!c->flist.p) CUDA_TRY(c, c->flist.alloc(LIST_FMAX));
+  if (!c->fpos.p) CUDA_TRY(c, c->fpos.alloc(LIST_FMAX));
   CUDA_TRY(c, cudaMemsetAsync(c->rb.p, 0, 4 * sizeof(int), c->stream));
   CUDA_TRY(c, cudaMemsetAsync(c->rb.p, 0x01, 1, c->stream));  // rb[0] = 1: the next step builds
   c->P.lcap = lcap;
   c->P.rl2_band = (float)(rl * rl * (1.0 + 1e-4));
   c->P.rmark2_band = (float)(rm * rm * (1.0 + 1e-4));
   c->P.lslow2 = 0.25 * c->lskin * c->lskin;
+  // an FP32 displacement is off by a few units of 2^-24 of the box edge where
+  // an image is taken off, of its own size elsewhere
+  const double slow = 0.5 * c->lskin * (1.0 - 1e-5) - std::ldexp(std::max({c->prd[0], c->prd[1], c->prd[2]}), -21);
+  c->P.lslow2_band = slow > 0.0 ? (float)(slow * slow) : 0.0f;
   for (int k = 0; k < 3; ++k) {
     c->P.half_prd[k] = 0.5 * c->prd[k];
     c->P.half_prdf[k] = (float)c->P.half_prd[k];
@@ -792,18 +799,20 @@ int launch_bin(eph_ctx *c) {
     int *rb = c->rb.p;
     CUDA_TRY(c, cudaMemsetAsync(rb + 1, 0, sizeof(int), c->stream));
     const bool df = df_records_wanted(c);
-    k_list_check<<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->xref.p, c->state.p, rb,
-                                              c->flist.p, c->counters.p, df ? c->dfrec.p : nullptr,
-                                              c->v.p);
+    if (df)
+      k_list_check<true><<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->xref.p, c->state.p,
+                                                      rb, c->flist.p, c->counters.p, c->dfrec.p, c->v.p);
+    else
+      k_list_check<false><<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->xref.p, c->state.p,
+                                                       rb, c->flist.p, c->counters.p, nullptr, nullptr);
     k_list_decide<<<1, 32, 0, c->stream>>>(rb, c->flist.p, c->counters.p);
-    k_list_mark<<<LIST_FMAX, BLOCK, 0, c->stream>>>(c->P, c->x.p, rb, c->flist.p, c->bin_count.p, c->bins.p,
-                                                    c->state.p);
-    k_zero_if<<<nblocks(c->nbins), BLOCK, 0, c->stream>>>(c->bin_count.p, c->nbins, rb + 2);
+    k_list_mark<<<std::max(LIST_FMAX, nblocks(c->nbins, 512)), 512, 0, c->stream>>>(
+        c->P, c->x.p, rb, c->flist.p, c->bin_count.p, c->nbins, c->bins.p, c->state.p, c->fpos.p);
     k_bin<<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->bin_count.p, c->bins.p,
                                        c->atom_bin.p, c->atom_off.p, c->d_err.p, c->counters.p, 0, rb + 2,
                                        c->xref.p, df ? c->dfrec.p : nullptr, c->v.p);
     launch_bin_sort(c, rb + 2);
-    ps.launched(6);
+    ps.launched(5);
     CUDA_TRY(c, cudaGetLastError());
     return EPH_OK;
   }

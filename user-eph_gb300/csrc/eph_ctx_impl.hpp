@@ -3,6 +3,8 @@
 // eph_adjoint.cu (the reverse-mode gradient).  Not part of the public ABI.
 #pragma once
 
+#include <algorithm>
+#include <cmath>
 #include <string>
 #include <vector>
 
@@ -110,6 +112,7 @@ struct eph_ctx {
   DevBuf<unsigned> cl;  // [lcap][n] candidates
   DevBuf<int> cl_n, state, rb, flist;
   DevBuf<D4> xref;  // positions at the last build
+  DevBuf<D4> fpos;  // the moved atoms' positions wrapped into the box
 
   DevBuf<D4> tab_rho_r_sq, tab_beta, tab_alpha;
   // FAST pair sums in df64 (eph_set_pair_arithmetic, on by default): the
@@ -210,6 +213,14 @@ bool eam_pair_list(const eph_ctx *c, const unsigned **pj, const int **ns, const 
 double eam_cutoff(const eph_ctx *c);  // its cut-off, 0 without one
 int eam_resize(eph_ctx *c);  // per-atom buffers of the pair force for c->n atoms
 void eam_free(eph_ctx *c);
+
+// squared distance within which a moved atom is a candidate: the cut-off
+// widened by the error of an FP32 distance across the box
+inline float far_cutoff2(const eph_ctx *c, double rc2) {
+  const double r = std::sqrt(rc2) * (1.0 + 5e-5) +
+                   std::ldexp(std::max(c->prd[0], std::max(c->prd[1], c->prd[2])), -21);
+  return (float)(r * r);
+}
 
 inline cudaEvent_t take_event(eph_ctx *c) {
   if (!c->event_pool.empty()) {

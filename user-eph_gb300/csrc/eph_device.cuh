@@ -59,6 +59,7 @@ struct StepParams {
   float rl2_band;     // r_list^2 (1 + 1e-4): candidates kept in the list
   float rmark2_band;  // (r_cutoff + s/2)^2 (1 + 1e-4): atoms this close to a moved atom search afresh
   double lslow2;      // (s/2)^2: squared displacement from which an atom counts as moved
+  float lslow2_band;  // the same less the error of an FP32 displacement across the box
   double half_prd[3];
   float half_prdf[3];
   int lcap;           // rows of the candidate list

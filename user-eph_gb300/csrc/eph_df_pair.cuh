@@ -190,17 +190,23 @@ __device__ __forceinline__ void own_fixed(const int4 *__restrict__ rec, int i, l
 // The record of atom i for the df64 pair sums, one 64-byte line half: {x lo,
 // x hi, y lo, y hi}, {z lo, z hi, element, moved}, velocity hi parts, velocity
 // lo parts.  Position in fixed point plus `image` boxes.
-__device__ __forceinline__ void df_record(const StepParams &P, int i, const D4 &x, const int *image, bool moved,
-                                          const D4 &v, int4 *__restrict__ rec) {
-  long long f[3] = {to_fixed_coord(x.x, P.fix_q), to_fixed_coord(x.y, P.fix_q), to_fixed_coord(x.z, P.fix_q)};
+__device__ __forceinline__ void df_record_fixed(const StepParams &P, int i, const long long *at, int element,
+                                                const int *image, bool moved, const D4 &v, int4 *__restrict__ rec) {
+  long long f[3];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) f[k] += (long long)image[k] * P.fix_prd[k];
+  for (int k = 0; k < 3; ++k) f[k] = at[k] + (long long)image[k] * P.fix_prd[k];
   const df64::df vx = df64::from_double(v.x), vy = df64::from_double(v.y), vz = df64::from_double(v.z);
   int4 *r = rec + 4 * (size_t)i;
   r[0] = make_int4((int)f[0], (int)(f[0] >> 32), (int)f[1], (int)(f[1] >> 32));
-  r[1] = make_int4((int)f[2], (int)(f[2] >> 32), (int)x.w, moved ? 1 : 0);
+  r[1] = make_int4((int)f[2], (int)(f[2] >> 32), element, moved ? 1 : 0);
   r[2] = make_int4(__float_as_int(vx.hi), __float_as_int(vy.hi), __float_as_int(vz.hi), 0);
   r[3] = make_int4(__float_as_int(vx.lo), __float_as_int(vy.lo), __float_as_int(vz.lo), 0);
+}
+
+__device__ __forceinline__ void df_record(const StepParams &P, int i, const D4 &x, const int *image, bool moved,
+                                          const D4 &v, int4 *__restrict__ rec) {
+  const long long f[3] = {to_fixed_coord(x.x, P.fix_q), to_fixed_coord(x.y, P.fix_q), to_fixed_coord(x.z, P.fix_q)};
+  df_record_fixed(P, i, f, (int)trunc_index(x.w), image, moved, v, rec);
 }
 
 }  // namespace ephgb

@@ -326,8 +326,8 @@ __global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
   long long xi[3] = {0, 0, 0};
   if (valid) own_fixed(C.rec, i, xi);
   const unsigned *tail;
-  bool fresh;
-  const int nc = pair_candidates<LANES, LIST, CAP>(P, C, i, g, valid, valid, at, tail, fresh);
+  int first;
+  const int nc = pair_candidates<LANES, LIST, CAP>(P, C, i, g, valid, valid, at, tail, first);
   __syncwarp();
   const df rc2{E.rc2_hi, E.rc2_lo}, inv_dr{E.inv_dr_hi, E.inv_dr_lo};
   bsum rs = bsum_zero();
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
              ez = fixed_df(ef[2], P.fix_hi, P.fix_lo);
     const df r2 = dot3(ex, ey, ez, ex, ey, ez);
     bool in = k < nc && lt(r2, rc2);
-    if (LIST) in = in && (fresh || cb.w == 0);  // a moved atom in a kept list is out of reach
+    if (LIST) in = in && (k >= first || cb.w == 0);  // a moved atom in a kept list is out of reach
     const unsigned who = __ballot_sync(FULL, in);
     if (who == 0u) continue;  // the lists' shell, together at their ends
     // the pair's row: from the front, in lane order; with kept lists the pairs
@@ -665,12 +665,13 @@ int launch_eam(eph_ctx *c) {
     C.pj = d->pj.p;
     C.kcap = d->kcap;
     C.band = E.rc2_band;
-    C.rc2 = E.rc2;
     C.cl = c->cl.p;
     C.cl_n = c->cl_n.p;
     C.state = c->state.p;
     C.rb = c->rb.p;
     C.flist = c->flist.p;
+    C.fpos = c->fpos.p;
+    C.far2 = far_cutoff2(c, E.rc2);
     C.xref = c->xref.p;
     const int lanes = eam_lanes(c);
     if (E.one >= 0) {

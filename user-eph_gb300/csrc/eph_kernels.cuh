@@ -811,9 +811,9 @@ __global__ void __launch_bounds__(tpa_threads(TPA)) k_density_tpa(
 // i and j both moved less than s/2 since the build, |x_i - x_j| < r_cutoff
 // implies that j is in i's list.  Atoms that moved farther ("moved", at most
 // LIST_FMAX of them) are handled every step instead: they and every atom
-// within r_cutoff + s/2 of one of them (from the bins of the build) search
-// the bins afresh, leave moved atoms' bin entries out and take the moved
-// atoms as extra candidates.  More moved atoms, or a request from the host,
+// within r_cutoff + s/2 of one of them search the bins of the build afresh
+// (the df64 sweeps: see pair_candidates), leave moved atoms' bin entries out
+// and take the moved atoms as extra candidates.  More moved atoms, or a request from the host,
 // make the step a build step.  Decisions live on the device (rb[0] build
 // requested, rb[1] moved atoms this step, rb[2] this step builds), so a
 // captured step replays them.  Lists hold atom indices; the periodic image of
@@ -824,13 +824,21 @@ __global__ void __launch_bounds__(tpa_threads(TPA)) k_density_tpa(
 
 // First kernel of a step with list reuse: the engine's wrap (as k_bin does
 // it), then each atom's displacement since the list build; moved atoms get
-// state 2 and join the list of moved atoms (state 0 otherwise).  With rec
-// (the df64 sweeps), also every atom's record for them (record_image) and
-// whether it moved.
+// state 2 and join the list of moved atoms (state 0 otherwise).  With RECORDS
+// (the df64 sweeps), also every atom's record for them and whether it moved.
+// The boxes added to a record's position are those of the image next to the
+// position at the build (so the image codes of the lists' entries stay what
+// they were), or, for an atom that moved, of the image in the box (the codes
+// of the searches around it are found there).  With RECORDS the displacement's
+// images and square are FP32 work, against a threshold lowered by their error
+// (an atom may count as moved a hair early, never late): three differences
+// and the velocities' split are all that is left in FP64.  FP64 issue bound it before (83%
+// of that pipe), memory does now: GB300, 2,048,000 atoms: 169 -> 76 us.
+template <bool RECORDS>
 __global__ void k_list_check(StepParams P, D4 *__restrict__ x, D4 *__restrict__ xhold,
                              const int *__restrict__ wrapflag, const D4 *__restrict__ xref, int *__restrict__ state,
                              int *__restrict__ rb, int *__restrict__ flist, unsigned long long *__restrict__ counters,
-                             int4 *__restrict__ rec = nullptr, const D4 *__restrict__ v = nullptr) {
+                             int4 *__restrict__ rec, const D4 *__restrict__ v) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *P.step += 1ull;  // read by the density sweep that follows
   bool moved = false;
@@ -843,16 +851,35 @@ __global__ void k_list_check(StepParams P, D4 *__restrict__ x, D4 *__restrict__ 
       if (i == 0) atomicAdd(&counters[CNT_WRAP], 1ull);
     }
     const D4 r = xref[i];
-    const double d[3] = {xi.x - r.x, xi.y - r.y, xi.z - r.z};
-    const double dx = min_image(d[0], P.prd[0], P.half_prd[0]), dy = min_image(d[1], P.prd[1], P.half_prd[1]),
-                 dz = min_image(d[2], P.prd[2], P.half_prd[2]);
-    moved = dx * dx + dy * dy + dz * dz >= P.lslow2;
-    state[i] = moved ? 2 : 0;
-    if (rec) {
+    if (RECORDS) {
+      const double now[3] = {xi.x, xi.y, xi.z}, d[3] = {xi.x - r.x, xi.y - r.y, xi.z - r.z};
+      long long f[3];
       int image[3];
-      record_image(P, xi, d, moved, image);
-      df_record(P, i, xi, image, moved, v[i], rec);
+      float r2 = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        f[k] = to_fixed_coord(now[k], P.fix_q);
+        const float df = float_bits(d[k]), half = P.half_prdf[k];
+        image[k] = df > half ? -1 : (df < -half ? 1 : 0);
+        const float e = df + (float)(2 * image[k]) * half;
+        r2 += e * e;
+      }
+      moved = !(r2 < P.lslow2_band);
+      if (moved) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          double q;
+          image[k] = wrap_image(P, k, now[k], q);
+        }
+      }
+      df_record_fixed(P, i, f, (int)trunc_index(xi.w), image, moved, v[i], rec);
+    } else {
+      const double dx = min_image(xi.x - r.x, P.prd[0], P.half_prd[0]),
+                   dy = min_image(xi.y - r.y, P.prd[1], P.half_prd[1]),
+                   dz = min_image(xi.z - r.z, P.prd[2], P.half_prd[2]);
+      moved = dx * dx + dy * dy + dz * dz >= P.lslow2;
     }
+    state[i] = moved ? 2 : 0;
   }
   // one atomic per warp (after a long run without a build most atoms move)
   const unsigned mv = __ballot_sync(0xffffffffu, moved);
@@ -888,23 +915,36 @@ __global__ void k_list_decide(int *__restrict__ rb, int *__restrict__ flist,
   }
 }
 
-__global__ void k_zero_if(int *__restrict__ p, int n, const int *__restrict__ gate) {
-  if (!*gate) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = 0;
-}
-
-// Block b: moved atom flist[b] flags (state |= 1) every atom whose position
-// at the build lies within r_cutoff + s/2 of its current position — the
-// only unmoved atoms it can now be within r_cutoff of.
-__global__ void k_list_mark(StepParams P, const D4 *__restrict__ x, const int *__restrict__ rb,
-                            const int *__restrict__ flist, const int *__restrict__ bin_count,
-                            const BinEntry *__restrict__ bins, int *__restrict__ state) {
-  if (rb[2] || (int)blockIdx.x >= rb[1]) return;
-  const int f = flist[blockIdx.x];
-  int4 B;
-  float4 o;
-  current_bin(P, x[f], B, o);
+// On a build step: clears the bins.  Otherwise block b: moved atom flist[b]
+// flags (state |= 1) every atom whose position at the build lies within
+// r_cutoff + s/2 of its current position -- the only unmoved atoms it can now
+// be within r_cutoff of -- and leaves its position wrapped into the box, which
+// those atoms compare with.  One thread wraps (a division per axis: FP64 issue,
+// 16 cycles for each warp that would repeat it).
+__global__ void __launch_bounds__(512) k_list_mark(StepParams P, const D4 *__restrict__ x, const int *__restrict__ rb,
+                                                   const int *__restrict__ flist, int *__restrict__ bin_count,
+                                                   int nbins, const BinEntry *__restrict__ bins,
+                                                   int *__restrict__ state, D4 *__restrict__ fpos) {
+  if (rb[2]) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q < nbins) bin_count[q] = 0;
+    return;
+  }
+  if ((int)blockIdx.x >= rb[1]) return;
+  __shared__ int4 s_B;
+  __shared__ float4 s_o;
+  if (threadIdx.x == 0) {
+    double wrapped[3];
+    int4 B;
+    float4 o;
+    current_bin(P, x[flist[blockIdx.x]], B, o, wrapped);
+    fpos[blockIdx.x] = D4{wrapped[0], wrapped[1], wrapped[2], 0.0};
+    s_B = B;
+    s_o = o;
+  }
+  __syncthreads();
+  const int4 B = s_B;
+  const float4 o = s_o;
   const int per = 27 * P.bcap;
   for (int q = threadIdx.x; q < per; q += blockDim.x) {
     const int slot = q % P.bcap, b = q / P.bcap;
@@ -1063,14 +1103,11 @@ __global__ void __maxnreg__(64) k_density_list(
 // ------------------------------------------- FAST density sweep in df64
 //
 // calculate_environment (fix_eph.cpp:431-466), stage 1 and M_i in one pass
-// (the FAST density sweep of k_density<true, MULTI, true>) with every
+// (the FAST density sweep of k_density<MULTI, true>) with every
 // per-pair operation in df64 on the FP32 pipe and LANES lanes per atom.
 //   pass 1 gathers the atom's candidates into shared memory (its lanes share
 //     one list): DF_BINS searches the 27 bins of the step, DF_EAM takes them
-//     from the EAM engine's pair list, DF_LIST keeps lists (build steps search
-//     the bins within r_cutoff + s and write them; atoms flagged by
-//     k_list_check / k_list_mark search the bins of the build afresh, leave
-//     moved atoms' entries out and add the moved atoms);
+//     from the EAM engine's pair list, DF_LIST keeps lists (pair_candidates);
 //   pass 2 forms e from the fixed-point positions (pair_fixed, fixed_df), r^2,
 //     the cut-off test, rho_j(r^2) (spline_rho_df), H = rho_j(r^2) / r^2 and the
 //     sums of M_i and S_i (blocked df64 sums: 8 products, then a Dekker
@@ -1153,7 +1190,7 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
     ei = rb.z;
   }
   int nc = 0;
-  bool fresh = true;
+  int first = 0;
   const unsigned *tail = pj;
   if (SRC == DF_EAM && D.ens_in) {  // the list has them apart
     tail = D.elist;
@@ -1162,7 +1199,7 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
     auto set = [&](int k, unsigned u) { pj[(size_t)k * n + i] = u; };
     list_candidates<LANES>(P, i, active, xi, D.elist, D.ens, D.C.rec, D.C.err, nc, P.kcap, set, P.rc2_band);
   } else {
-    nc = pair_candidates<LANES, SRC == DF_LIST, CAP>(P, D.C, i, g, valid, active, at, tail, fresh);
+    nc = pair_candidates<LANES, SRC == DF_LIST, CAP>(P, D.C, i, g, valid, active, at, tail, first);
   }
   __syncwarp();
   // pass 2; the next candidate's position is loaded while this one is summed,
@@ -1196,7 +1233,7 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
     // a moved atom in a kept list is out of the cut-off of every atom that
     // reads its list (it may even be outside the integers' range)
     bool in = k < nc && lt(r2, rc2);
-    if (SRC == DF_LIST) in = in && (fresh || cb.w == 0);
+    if (SRC == DF_LIST) in = in && (k >= first || cb.w == 0);
     // the shell beyond the cut-off sits at the end of the lists: where no
     // lane of the warp has a pair inside, the iteration would add only zeros
     const unsigned who = __ballot_sync(0xffffffffu, in);
@@ -2017,6 +2054,9 @@ __global__ void k_forces_ttm(StepParams P, const int *__restrict__ mask, const D
 // (2^-64 units) and integer addition is order-free, so the grid and the
 // energy total are the same whatever order the atoms arrive in; the block
 // totals of the energy go to `part` and are summed by k_energy_total.
+// The quotients and half of the products run on the integer units (the same
+// bits): FP64 issue bound it (83% of that pipe), GB300, 2,048,000 atoms: 137 ->
+// 78 us.
 template <bool FRIC, bool RAND, bool GRID>
 __global__ void __launch_bounds__(256) k_deposit(StepParams P, const int *__restrict__ mask,
                                                  const D4 *__restrict__ v, const D4 *__restrict__ f_eph,
@@ -2028,23 +2068,24 @@ __global__ void __launch_bounds__(256) k_deposit(StepParams P, const int *__rest
   if (i < P.n && (mask[i] & P.groupbit)) {
     const D4 vi = v[i];
     U128 g{0ull, 0ull};
+    const soft::Divisor prescale = soft::divisor(P.prescale);
     if (FRIC) {
       const D4 fe = f_eph[i];
       double dE = 0.0;
-      dE -= fe.x * vi.x * P.dt;
-      dE -= fe.y * vi.y * P.dt;
-      dE -= fe.z * vi.z * P.dt;
+      dE -= soft::mul(fe.x * vi.x, P.dt);
+      dE -= soft::mul(fe.y * vi.y, P.dt);
+      dE -= soft::mul(fe.z * vi.z, P.dt);
       e = add128(e, to_fixed(dE, err));
-      if (GRID) g = add128(g, to_fixed(dE / P.prescale, err));
+      if (GRID) g = add128(g, to_fixed(soft::div(dE, prescale), err));
     }
     if (RAND) {
       const D4 fr = f_rng[i];
       double dE = 0.0;
-      dE -= fr.x * vi.x * P.dt;
-      dE -= fr.y * vi.y * P.dt;
-      dE -= fr.z * vi.z * P.dt;
+      dE -= soft::mul(fr.x * vi.x, P.dt);
+      dE -= soft::mul(fr.y * vi.y, P.dt);
+      dE -= soft::mul(fr.z * vi.z, P.dt);
       e = add128(e, to_fixed(dE, err));
-      if (GRID) g = add128(g, to_fixed(dE / P.prescale, err));
+      if (GRID) g = add128(g, to_fixed(soft::div(dE, prescale), err));
     }
     if (GRID && (g.lo | g.hi)) atomic_add128(acc + cell[i], g);
   }
