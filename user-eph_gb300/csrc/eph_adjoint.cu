@@ -1279,11 +1279,7 @@ int run_step(eph_adjoint *a, int s) {
   const size_t N = (size_t)a->n;
   const long before = c->launches;
   int r;
-  if ((r = ctxi::launch_initial(c, 1))) return from_ctx(a, r);
-  if (c->have_fext)
-    ADJ_TRY(a, d2d(c->f.p, c->fext.p, N, c->stream));
-  else
-    ADJ_TRY(a, cudaMemsetAsync(c->f.p, 0, sizeof(D4) * N, c->stream));
+  if ((r = ctxi::launch_initial(c, 1, true))) return from_ctx(a, r);
   if ((r = ctxi::launch_post_force(c, 0))) return from_ctx(a, r);
   const size_t o = (size_t)std::max(s, 0) * N, og = (size_t)std::max(s, 0) * (size_t)a->nc;
   const int rb = nb_of(std::max((long)a->n, a->nc));
@@ -1294,9 +1290,8 @@ int run_step(eph_adjoint *a, int s) {
     k_adj_record_mid<<<dim3((unsigned)rb, 8), ABLOCK, 0, c->stream>>>(R, a->n, a->nc, a->kcap);
     a->launches += 1;
   }
-  if ((r = ctxi::launch_final(c))) return from_ctx(a, r);
   if (s >= 0 && a->fdm) c->fdm_rec = a->r_Tsub.p + (size_t)s * a->nsub * (size_t)a->nc;
-  r = ctxi::launch_end_of_step(c);
+  r = ctxi::launch_end_of_step(c, true);
   c->fdm_rec = nullptr;
   if (r) return from_ctx(a, r);
   if (s >= 0) {

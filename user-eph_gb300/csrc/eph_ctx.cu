@@ -344,16 +344,18 @@ int require_atoms(eph_ctx *c) {
 
 // --------------------------------------------------------------- launches
 
-int launch_initial(eph_ctx *c, int check_wrap) {
+int launch_initial(eph_ctx *c, int check_wrap, bool clear) {
   PhaseScope ps(c, EPH_PHASE_INTEGRATE);
   ps.launched();
   const int nb = nblocks(c->n);
   if (c->mode == EPH_MODE_FAST)
     k_initial_integrate<true><<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->v.p, c->f.p, c->type.p, c->mask.p,
-                                                           c->xhold.p, check_wrap, c->wrapflag.p);
+                                                           c->xhold.p, check_wrap, c->wrapflag.p, clear,
+                                                           c->have_fext ? c->fext.p : nullptr);
   else
     k_initial_integrate<false><<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->v.p, c->f.p, c->type.p, c->mask.p,
-                                                            c->xhold.p, check_wrap, c->wrapflag.p);
+                                                            c->xhold.p, check_wrap, c->wrapflag.p, clear,
+                                                           c->have_fext ? c->fext.p : nullptr);
   CUDA_TRY(c, cudaGetLastError());
   return EPH_OK;
 }
@@ -879,28 +881,38 @@ int launch_pair_sweeps(eph_ctx *c, int xi_mode) {
 }
 
 template <bool FRIC, bool RAND, bool GRID>
-void launch_deposit_t(eph_ctx *c) {
-  k_deposit<FRIC, RAND, GRID><<<nblocks(c->n, 256), 256, 0, c->stream>>>(
-      c->P, c->mask.p, c->v.p, c->f_eph.p, c->f_rng.p, c->cell.p, c->acc.p, c->part.p, c->d_err.p);
+void launch_deposit_t(eph_ctx *c, bool kick) {
+#define EPH_DEPOSIT(K)                                                                                            \
+  k_deposit<FRIC, RAND, GRID, K><<<nblocks(c->n, 256), 256, 0, c->stream>>>(                                        \
+      c->P, c->mask.p, c->v.p, c->f_eph.p, c->f_rng.p, c->cell.p, c->acc.p, c->part.p, c->d_err.p, c->f.p,        \
+      c->type.p, c->deposit_left.p, c->scal.p + 1, c->scal.p + 0)
+  if (!kick) EPH_DEPOSIT(0);
+  else if (c->mode == EPH_MODE_FAST) EPH_DEPOSIT(2);
+  else EPH_DEPOSIT(1);
+#undef EPH_DEPOSIT
 }
 
-// end_of_step: deposits, FDM substeps, energy total
-int launch_end_of_step(eph_ctx *c) {
+// final_integrate (with_final) and end_of_step: deposits and the energy total,
+// FDM substeps
+int launch_end_of_step(eph_ctx *c, bool with_final) {
   const bool fr = c->P.flags & FLAG_FRICTION, ra = c->P.flags & FLAG_RANDOM, gr = c->P.flags & FLAG_FDM;
+  if (with_final && !fr && !ra) {
+    int r = launch_final(c);
+    if (r) return r;
+  }
   if (fr || ra) {
     PhaseScope ps(c, EPH_PHASE_DEPOSIT);
-    ps.launched(2);
+    ps.launched();
     if (fr && ra) {
-      if (gr) launch_deposit_t<true, true, true>(c);
-      else launch_deposit_t<true, true, false>(c);
+      if (gr) launch_deposit_t<true, true, true>(c, with_final);
+      else launch_deposit_t<true, true, false>(c, with_final);
     } else if (fr) {
-      if (gr) launch_deposit_t<true, false, true>(c);
-      else launch_deposit_t<true, false, false>(c);
+      if (gr) launch_deposit_t<true, false, true>(c, with_final);
+      else launch_deposit_t<true, false, false>(c, with_final);
     } else {
-      if (gr) launch_deposit_t<false, true, true>(c);
-      else launch_deposit_t<false, true, false>(c);
+      if (gr) launch_deposit_t<false, true, true>(c, with_final);
+      else launch_deposit_t<false, true, false>(c, with_final);
     }
-    k_energy_total<<<1, 1024, 0, c->stream>>>(c->part.p, nblocks(c->n, 256), c->scal.p + 1, c->scal.p + 0);
   }
   if (gr) {
     PhaseScope ps(c, EPH_PHASE_FDM);
@@ -1004,21 +1016,12 @@ int write_T_output(eph_ctx *c) {
 // same sequence is executed directly or captured into a graph.
 int record_step(eph_ctx *c, int xi_mode) {
   int r;
-  if ((r = launch_initial(c, 1))) return r;
-  if (c->eam) {
-    // the engine's pair force on this step's positions (Verlet: after the
-    // wrap and the neighbour bins, before post_force)
-    if ((r = launch_bin(c)) || (r = launch_eam(c)) || (r = launch_pair_sweeps(c, xi_mode))) return r;
-  } else {
-    // force clear + the external (pair) force
-    if (c->have_fext)
-      CUDA_TRY(c, cudaMemcpyAsync(c->f.p, c->fext.p, sizeof(D4) * (size_t)c->n, cudaMemcpyDeviceToDevice, c->stream));
-    else
-      CUDA_TRY(c, cudaMemsetAsync(c->f.p, 0, sizeof(D4) * (size_t)c->n, c->stream));
-    if ((r = launch_post_force(c, xi_mode))) return r;
-  }
-  if ((r = launch_final(c))) return r;
-  return launch_end_of_step(c);
+  // the force cleared to the external (pair) force, unless the EAM engine sets it
+  if ((r = launch_initial(c, 1, !c->eam))) return r;
+  // with EAM the engine's pair force on this step's positions (Verlet: after
+  // the wrap and the neighbour bins, before post_force)
+  if ((r = launch_bin(c)) || (c->eam && (r = launch_eam(c))) || (r = launch_pair_sweeps(c, xi_mode))) return r;
+  return launch_end_of_step(c, true);
 }
 
 void drop_graph(eph_ctx *c) {
@@ -1166,6 +1169,8 @@ int eph_create(int narg, const char *const *arg, const eph_md *md, eph_ctx **out
   CUDA_TRY(c, c->step_ctr.alloc(1));
   CUDA_TRY(c, cudaMemset(c->step_ctr.p, 0, sizeof(unsigned long long)));
   CUDA_TRY(c, c->scal.alloc(4));
+  CUDA_TRY(c, c->deposit_left.alloc(1));
+  CUDA_TRY(c, cudaMemset(c->deposit_left.p, 0, sizeof(unsigned)));
   CUDA_TRY(c, c->gsum.alloc(1));
   CUDA_TRY(c, cudaMemset(c->d_err.p, 0, sizeof(unsigned)));
   CUDA_TRY(c, cudaMemset(c->counters.p, 0, sizeof(unsigned long long) * NCOUNTERS));
@@ -1701,7 +1706,7 @@ int eph_initial_integrate(eph_ctx *c) {
   if (!c) return EPH_ERR_ARG;
   int r = require_atoms(c);
   if (r) return r;
-  return launch_initial(c, 0);
+  return launch_initial(c, 0, false);
 }
 
 int eph_post_force(eph_ctx *c, int xi_source) {
@@ -1726,7 +1731,7 @@ int eph_end_of_step(eph_ctx *c) {
   if (!c) return EPH_ERR_ARG;
   int r = require_atoms(c);
   if (r) return r;
-  r = launch_end_of_step(c);
+  r = launch_end_of_step(c, false);
   if (r) return r;
   if (c->arr_pending) {  // the per-atom array eph_post_force_host sent out
     CUDA_TRY(c, cudaEventSynchronize(c->arr_done));

@@ -167,6 +167,7 @@ struct eph_ctx {
   long graph_launches = 0;  // kernels in one replay
 
   DevBuf<double> scal;  // 0 Ee, 1 E_local, 2 T_total
+  DevBuf<unsigned> deposit_left;  // blocks of k_deposit done so far
   DevBuf<unsigned> d_err;
   DevBuf<unsigned long long> counters;
   DevBuf<int> wrapflag;
@@ -186,10 +187,11 @@ int upload_grid(eph_ctx *c);
 void set_time_params(eph_ctx *c);
 void drop_graph(eph_ctx *c);
 // the four phases of one engine step on the context's stream
-int launch_initial(eph_ctx *c, int check_wrap);
+// (clear: the force set to the external one for the step to come)
+int launch_initial(eph_ctx *c, int check_wrap, bool clear);
 int launch_post_force(eph_ctx *c, int xi_mode);
 int launch_final(eph_ctx *c);
-int launch_end_of_step(eph_ctx *c);
+int launch_end_of_step(eph_ctx *c, bool with_final);
 // post_force in two parts: spatial binning (and the wrap), then the sweeps
 int launch_bin(eph_ctx *c);
 // candidate-list reuse on or off as the context's settings allow (bins,

@@ -60,12 +60,14 @@ __device__ __forceinline__ void kick(double dtfm, const D4 &fi, D4 &vi) {
 }
 
 // FixEPH::initial_integrate (fix_eph.cpp:305-328) and the engine's rebuild
-// test (an atom moved more than skin/2 since the last wrap).
+// test (an atom moved more than skin/2 since the last wrap).  With `clear`, also
+// the engine's force of the step to come: the external one, or zero (a
+// memset or copy of its own before).
 template <bool FAST>
-__global__ void k_initial_integrate(StepParams P, D4 *__restrict__ x, D4 *__restrict__ v,
-                                    const D4 *__restrict__ f, const int *__restrict__ type,
-                                    const int *__restrict__ mask, const D4 *__restrict__ xhold, int check_wrap,
-                                    int *__restrict__ wrapflag) {
+__global__ void k_initial_integrate(StepParams P, D4 *__restrict__ x, D4 *__restrict__ v, D4 *__restrict__ f,
+                                    const int *__restrict__ type, const int *__restrict__ mask,
+                                    const D4 *__restrict__ xhold, int check_wrap, int *__restrict__ wrapflag,
+                                    int clear, const D4 *__restrict__ fext) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool moved = false;
   if (i < P.n) {
@@ -76,6 +78,7 @@ __global__ void k_initial_integrate(StepParams P, D4 *__restrict__ x, D4 *__rest
       v[i] = vi;
       x[i] = xi;
     }
+    if (clear) f[i] = fext ? fext[i] : D4{0.0, 0.0, 0.0, 0.0};
     if (check_wrap) {
       const D4 h = xhold[i];
       const double dx = xi.x - h.x, dy = xi.y - h.y, dz = xi.z - h.z;
@@ -2053,20 +2056,32 @@ __global__ void k_forces_ttm(StepParams P, const int *__restrict__ mask, const D
 // The grid sums are exact: every term becomes a 128-bit fixed-point integer
 // (2^-64 units) and integer addition is order-free, so the grid and the
 // energy total are the same whatever order the atoms arrive in; the block
-// totals of the energy go to `part` and are summed by k_energy_total.
+// totals of the energy go to `part`, and the last block to leave its own
+// (`left` counts them, and is 0 again afterwards) adds them up and adds the
+// step's exchange to Ee (fix_eph.cpp:402-404): integers, so the sum does not
+// depend on which block that is.
+// KICK: final_integrate in the same pass (0: not here, 1: EXACT, 2: FAST).
+// (A launch of its own for each of the two took 3.7 and 3.3 us more of a step of
+// 110 us at 4,000 atoms on GB300.)
 // The quotients and half of the products run on the integer units (the same
 // bits): FP64 issue bound it (83% of that pipe), GB300, 2,048,000 atoms: 137 ->
 // 78 us.
-template <bool FRIC, bool RAND, bool GRID>
+template <bool FRIC, bool RAND, bool GRID, int KICK>
 __global__ void __launch_bounds__(256) k_deposit(StepParams P, const int *__restrict__ mask,
-                                                 const D4 *__restrict__ v, const D4 *__restrict__ f_eph,
+                                                 D4 *__restrict__ v, const D4 *__restrict__ f_eph,
                                                  const D4 *__restrict__ f_rng, const int *__restrict__ cell,
                                                  U128 *__restrict__ acc, U128 *__restrict__ part,
-                                                 unsigned *__restrict__ err) {
+                                                 unsigned *__restrict__ err, const D4 *__restrict__ f,
+                                                 const int *__restrict__ type, unsigned *__restrict__ left,
+                                                 double *__restrict__ E_local, double *__restrict__ Ee) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   U128 e{0ull, 0ull};
   if (i < P.n && (mask[i] & P.groupbit)) {
-    const D4 vi = v[i];
+    D4 vi = v[i];
+    if (KICK && !(P.flags & 0x08)) {
+      kick<KICK == 2>(P.dtfm[type[i]], f[i], vi);
+      v[i] = vi;
+    }
     U128 g{0ull, 0ull};
     const soft::Divisor prescale = soft::divisor(P.prescale);
     if (FRIC) {
@@ -2095,28 +2110,33 @@ __global__ void __launch_bounds__(256) k_deposit(StepParams P, const int *__rest
   __shared__ U128 warp_tot[8];
   if ((threadIdx.x & 31) == 0) warp_tot[threadIdx.x >> 5] = e;
   __syncthreads();
+  __shared__ bool s_last;
   if (threadIdx.x == 0) {
     U128 t{0ull, 0ull};
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t = add128(t, warp_tot[w]);
     part[blockIdx.x] = t;
+    __threadfence();
+    s_last = atomicAdd(left, 1u) == gridDim.x - 1;
   }
-}
-
-// Sum the block totals, add the step's exchange to Ee (fix_eph.cpp:402-404).
-__global__ void k_energy_total(const U128 *__restrict__ part, int nparts, double *__restrict__ E_local,
-                               double *__restrict__ Ee) {
-  U128 t{0ull, 0ull};
-  for (int b = threadIdx.x; b < nparts; b += blockDim.x) t = add128(t, part[b]);
-  for (int d = 16; d > 0; d >>= 1) t = add128(t, shfl_down128(t, d));
-  __shared__ U128 warp_tot[32];
-  if ((threadIdx.x & 31) == 0) warp_tot[threadIdx.x >> 5] = t;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  e = U128{0ull, 0ull};
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
+    const ulonglong2 t = __ldcg(reinterpret_cast<const ulonglong2 *>(part + b));
+    e = add128(e, U128{t.x, t.y});
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) e = add128(e, shfl_down128(e, d));
+  if ((threadIdx.x & 31) == 0) warp_tot[threadIdx.x >> 5] = e;
   __syncthreads();
   if (threadIdx.x == 0) {
-    U128 s{0ull, 0ull};
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s = add128(s, warp_tot[w]);
-    const double e = from_fixed(s);
-    *E_local = e;
-    *Ee += e;
+    U128 t{0ull, 0ull};
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t = add128(t, warp_tot[w]);
+    const double step = from_fixed(t);
+    *E_local = step;
+    *Ee += step;
+    *left = 0u;
   }
 }
 
