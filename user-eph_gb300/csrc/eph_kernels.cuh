@@ -666,12 +666,12 @@ __global__ void __launch_bounds__(EXD_THREADS, 4) k_density_exact(
 // resident blocks of 128 threads per SM the df64 sweeps are compiled for
 // (their register budget: 65,536 / (128 x blocks)); measured on GB300 at
 // 2,048,000 atoms: density 6 / 7 / 8 blocks 1.44 / 1.36 / 1.69 ms (8 spills),
-// forces 7 / 8 / 9 blocks 0.84 / 0.84 / 0.89 ms (9 spills)
+// forces 8 / 9 blocks 0.86 / 0.80 ms
 #ifndef EPH_DF_DENSITY_BLOCKS
 #define EPH_DF_DENSITY_BLOCKS 7
 #endif
 #ifndef EPH_DF_FORCES_BLOCKS
-#define EPH_DF_FORCES_BLOCKS 8
+#define EPH_DF_FORCES_BLOCKS 9
 #endif
 
 // The FAST density sweep with TPA lanes per atom for small systems (FP64 pair
@@ -1627,7 +1627,12 @@ __global__ void __launch_bounds__(EX_THREADS) k_forces_exact(StepParams P, const
 //   f_EPH_i = -M_i W_i + sum_{j live} H_ji (e.W_j) e + sum_{j not live} H_ij (e.W_i) e
 //   f_RNG_i = eta sqrt(T_e) [M_i X_i - sum_{j live} H_ji (e.X_j) e - sum_{j not live} H_ij (e.X_i) e]
 // ("live": rho_j > 0, the reference's test; the last sums take back the
-// pairs it skips).  Per pair 14 FP64 instructions instead of 24.
+// pairs it skips).  Per pair 14 FP64 instructions instead of 24.  A skipped
+// pair is the same term with the atom's own record and H_ij, so it takes its
+// turn in the loop (with part of the atoms outside the group every atom has
+// some: a second pass over the pairs for them, by one lane per atom, made the
+// sweep of 9,724 atoms, a fifth of them outside, 53 us instead of 23 on
+// GB300, and that of 32,000 atoms in df64 187 instead of 35).
 template <bool MULTI, bool RAND, int TPA = 1>
 __global__ void __launch_bounds__(128) k_forces_m(StepParams P, const unsigned *__restrict__ pj,
                                                   const D4 *__restrict__ pe, const double2 *__restrict__ pg,
@@ -1641,7 +1646,7 @@ __global__ void __launch_bounds__(128) k_forces_m(StepParams P, const unsigned *
   if (TPA == 1 && i >= P.n) return;  // with TPA > 1 every lane joins the sums
   double fex = 0.0, fey = 0.0, fez = 0.0, frx = 0.0, fry = 0.0, frz = 0.0;
   bool live = false;
-  int ns = 0, skipped = 0;
+  int ns = 0;
   if (i < P.n) {
     live = pos_double(G[2 * (size_t)i + 1].z);  // rho_i > 0 (0 outside the group)
     if (live) ns = nshort[i];
@@ -1652,13 +1657,14 @@ __global__ void __launch_bounds__(128) k_forces_m(StepParams P, const unsigned *
     const unsigned j = j_next;
     if (k + TPA < ns) j_next = pj[slot + (size_t)TPA * P.n] & IDX_MASK;
     const D4 e = pe[slot];
-    const D4 Gj1 = G[2 * (size_t)j], Gj2 = G[2 * (size_t)j + 1];
-    if (!pos_double(Gj2.z)) {  // a pair the reference skips (handled below)
-      skipped = 1;
-      continue;
+    D4 Gj1 = G[2 * (size_t)j], Gj2 = G[2 * (size_t)j + 1];
+    const bool skip = !pos_double(Gj2.z);
+    if (skip) {  // a pair the reference skips: its share of M_i comes back out
+      Gj1 = G[2 * (size_t)i];
+      Gj2 = G[2 * (size_t)i + 1];
     }
     if (MULTI) {
-      const double Hji = pg[slot].x;  // rho_i(r^2)/r^2
+      const double Hji = skip ? e.w : pg[slot].x;  // rho_i(r^2)/r^2 (H_ij)
       const double sw = Hji * dot3_fma(e.x, e.y, e.z, Gj1.x, Gj1.y, Gj1.z);
       fex = fma(sw, e.x, fex);
       fey = fma(sw, e.y, fey);
@@ -1688,7 +1694,6 @@ __global__ void __launch_bounds__(128) k_forces_m(StepParams P, const unsigned *
     // an atom each
     constexpr int NA = 128 / TPA, NSUM = RAND ? 6 : 3;
     __shared__ double s_sum[NSUM * 128], s_tot[NSUM * NA];
-    __shared__ int s_skip[128];
     const int t = threadIdx.x, at = g * NA + t / TPA;
     s_sum[at] = fex;
     s_sum[128 + at] = fey;
@@ -1698,7 +1703,6 @@ __global__ void __launch_bounds__(128) k_forces_m(StepParams P, const unsigned *
       s_sum[(NSUM - 2) * 128 + at] = fry;
       s_sum[(NSUM - 1) * 128 + at] = frz;
     }
-    s_skip[at] = skipped;
     __syncthreads();
     for (int q = t; q < NSUM * NA; q += 128) {
       const double *w = s_sum + q / NA * 128 + q % NA;
@@ -1718,52 +1722,19 @@ __global__ void __launch_bounds__(128) k_forces_m(StepParams P, const unsigned *
       fry = s_tot[(NSUM - 2) * NA + t];
       frz = s_tot[(NSUM - 1) * NA + t];
     }
-    skipped = 0;
-#pragma unroll
-    for (int l = 0; l < TPA; ++l) skipped |= s_skip[l * NA + t];
     live = pos_double(G[2 * (size_t)i + 1].z);
-    ns = live ? nshort[i] : 0;
   }
   if (live) {
-    double cex = 0.0, cey = 0.0, cez = 0.0, crx = 0.0, cry = 0.0, crz = 0.0;
     const D4 Gi1 = G[2 * (size_t)i], Gi2 = G[2 * (size_t)i + 1];
-    if (skipped) {  // rare: the skipped pairs' shares of M_i come back out (a second
-                    // pass keeps this work out of the main loop's instruction stream)
-      for (int k = 0; k < ns; ++k) {
-        const size_t slot = (size_t)k * P.n + i;
-        const unsigned j = pj[slot] & IDX_MASK;
-        if (pos_double(G[2 * (size_t)j + 1].z)) continue;
-        const D4 e = pe[slot];
-        // H_ij e: {H e.x, e.y, e.z} with several elements, {e.w, pg} with one
-        double hx = e.x, hy = e.y, hz = e.z, H = e.w;
-        if (!MULTI) {
-          const double2 h = pg[slot];
-          hx = e.w;
-          hy = h.x;
-          hz = h.y;
-          H = 1.0;
-        }
-        const double sw = H * dot3_fma(e.x, e.y, e.z, Gi1.x, Gi1.y, Gi1.z);
-        cex = fma(sw, hx, cex);
-        cey = fma(sw, hy, cey);
-        cez = fma(sw, hz, cez);
-        if (RAND) {
-          const double sx = H * dot3_fma(e.x, e.y, e.z, Gi1.w, Gi2.x, Gi2.y);
-          crx = fma(sx, hx, crx);
-          cry = fma(sx, hy, cry);
-          crz = fma(sx, hz, crz);
-        }
-      }
-    }
     const D4 M1 = Mm[i], M2 = Mm[(size_t)P.n + i];  // {xx, xy, xz, yy}, {yz, zz}
-    fex += cex - fma(M1.x, Gi1.x, fma(M1.y, Gi1.y, M1.z * Gi1.z));
-    fey += cey - fma(M1.y, Gi1.x, fma(M1.w, Gi1.y, M2.x * Gi1.z));
-    fez += cez - fma(M1.z, Gi1.x, fma(M2.x, Gi1.y, M2.y * Gi1.z));
+    fex -= fma(M1.x, Gi1.x, fma(M1.y, Gi1.y, M1.z * Gi1.z));
+    fey -= fma(M1.y, Gi1.x, fma(M1.w, Gi1.y, M2.x * Gi1.z));
+    fez -= fma(M1.z, Gi1.x, fma(M2.x, Gi1.y, M2.y * Gi1.z));
     if (RAND) {
       const double var = P.eta * sqrt(Te_i[i]);
-      frx = var * (fma(M1.x, Gi1.w, fma(M1.y, Gi2.x, M1.z * Gi2.y)) - crx - frx);
-      fry = var * (fma(M1.y, Gi1.w, fma(M1.w, Gi2.x, M2.x * Gi2.y)) - cry - fry);
-      frz = var * (fma(M1.z, Gi1.w, fma(M2.x, Gi2.x, M2.y * Gi2.y)) - crz - frz);
+      frx = var * (fma(M1.x, Gi1.w, fma(M1.y, Gi2.x, M1.z * Gi2.y)) - frx);
+      fry = var * (fma(M1.y, Gi1.w, fma(M1.w, Gi2.x, M2.x * Gi2.y)) - fry);
+      frz = var * (fma(M1.z, Gi1.w, fma(M2.x, Gi2.x, M2.y * Gi2.y)) - frz);
     }
   }
   store_forces<true, RAND>(P, i, live, fex, fey, fez, frx, fry, frz, f, f_eph, f_rng, f_dis, f_sto);
@@ -1778,9 +1749,10 @@ __global__ void __launch_bounds__(128) k_forces_m(StepParams P, const unsigned *
 // record's first word.
 // It streams the pair cache (36 B per pair) and gathers a 48 B record per pair
 // from L2; on GB300 the latency of those loads bounds it, so the totals live
-// in shared memory (64 registers, 8 blocks per SM) and the next neighbour's
+// in shared memory (56 registers, 9 blocks per SM) and the next neighbour's
 // index is loaded one pair ahead.  2,048,000 atoms: 1.18 ms with 52 B per pair
-// and 16-byte loads; 1.10 with 36 B; 0.84 with 256-bit loads and 8 blocks.
+// and 16-byte loads; 1.10 with 36 B; 0.84 with 256-bit loads and 8 blocks; 0.80
+// with the skipped pairs in the loop and 9.
 template <bool MULTI, bool RAND, int TPA = 1>
 __global__ void __launch_bounds__(128, EPH_DF_FORCES_BLOCKS)
     k_forces_df(StepParams P, const unsigned *__restrict__ pj, const float4 *__restrict__ pe,
@@ -1823,28 +1795,81 @@ __global__ void __launch_bounds__(128, EPH_DF_FORCES_BLOCKS)
     const size_t slot = (size_t)k * P.n + i;
     const unsigned j = jn;
     if (k + TPA < ns) jn = pj[slot + (size_t)TPA * P.n] & IDX_MASK;
-    float4 a, b, G0, G1;
+    float4 a, b, G0, G1, G2;
     load_row(Gf + 4 * (size_t)j, G0, G1);
     load_row_once(pe + 2 * slot, a, b);
-    if (G0.x != G0.x) {  // a pair the reference skips (handled below)
-      skipped = 1;
-    } else {
-      const df ex{a.x, b.x}, ey{a.y, b.y}, ez{a.z, b.z}, Hji{a.w, b.w};
-      const df sw = mul(Hji, dot3(ex, ey, ez, df{G0.x, G1.x}, df{G0.y, G1.y}, df{G0.z, G1.z}));
-      acc_fma(sm[0], sw, ex);
-      acc_fma(sm[1], sw, ey);
-      acc_fma(sm[2], sw, ez);
-      if (RAND) {
-        const float4 G2 = Gf[4 * (size_t)j + 2];
-        const df sx = mul(Hji, dot3(ex, ey, ez, df{G0.w, G1.w}, df{G2.x, G2.z}, df{G2.y, G2.w}));
-        acc_fma(sm[NS - 3], sx, ex);
-        acc_fma(sm[NS - 2], sx, ey);
-        acc_fma(sm[NS - 1], sx, ez);
+    if (RAND) G2 = Gf[4 * (size_t)j + 2];
+    const df ex{a.x, b.x}, ey{a.y, b.y}, ez{a.z, b.z};
+    df H{a.w, b.w};  // H_ji
+    if (G0.x != G0.x) {  // a pair the reference skips: its share of M_i comes back out
+      ++skipped;
+      load_row(Gf + 4 * (size_t)i, G0, G1);
+      if (RAND) G2 = Gf[4 * (size_t)i + 2];
+      if (MULTI) {  // H_ij: the cached H_ji with one element
+        const int ej = rec[4 * (size_t)j + 1].z;
+        if (ej != rec[4 * (size_t)i + 1].z) {
+          const df r2 = dot3(ex, ey, ez, ex, ey, ez);
+          H = mul(spline_rho_df(P, ej, r2, err), recip(r2, rcp_estimate(r2.hi)));
+        }
       }
+    }
+    const df sw = mul(H, dot3(ex, ey, ez, df{G0.x, G1.x}, df{G0.y, G1.y}, df{G0.z, G1.z}));
+    acc_fma(sm[0], sw, ex);
+    acc_fma(sm[1], sw, ey);
+    acc_fma(sm[2], sw, ez);
+    if (RAND) {
+      const df sx = mul(H, dot3(ex, ey, ez, df{G0.w, G1.w}, df{G2.x, G2.z}, df{G2.y, G2.w}));
+      acc_fma(sm[NS - 3], sx, ex);
+      acc_fma(sm[NS - 2], sx, ey);
+      acc_fma(sm[NS - 1], sx, ez);
     }
     if ((m & 7) == 7) fold();
   }
   fold();
+  // More than half of the pairs skipped: -M_i W_i and what comes back out nearly
+  // cancel, so the live pairs (the fewer ones) are summed alone, both terms of
+  // each.  All lanes of an atom decide alike.
+#pragma unroll
+  for (int o = TPA / 2; o > 0; o >>= 1) skipped += __shfl_xor_sync(0xffffffffu, skipped, o);
+  const bool direct = 2 * skipped > ns;
+  if (direct) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) s_tot[q * 128 + t] = make_float2(0.f, 0.f);
+    m = 0;
+    for (int k = g; k < ns; k += TPA) {
+      const size_t slot = (size_t)k * P.n + i;
+      const unsigned j = pj[slot] & IDX_MASK;
+      float4 a, b, G0, G1, O0, O1;
+      load_row(Gf + 4 * (size_t)j, G0, G1);
+      if (G0.x != G0.x) continue;
+      load_row(Gf + 4 * (size_t)i, O0, O1);
+      load_row(pe + 2 * slot, a, b);
+      const df ex{a.x, b.x}, ey{a.y, b.y}, ez{a.z, b.z}, Hji{a.w, b.w};
+      df Hij = Hji;
+      if (MULTI) {
+        const int ej = rec[4 * (size_t)j + 1].z;
+        if (ej != rec[4 * (size_t)i + 1].z) {
+          const df r2 = dot3(ex, ey, ez, ex, ey, ez);
+          Hij = mul(spline_rho_df(P, ej, r2, err), recip(r2, rcp_estimate(r2.hi)));
+        }
+      }
+      const df sw = sub(mul(Hji, dot3(ex, ey, ez, df{G0.x, G1.x}, df{G0.y, G1.y}, df{G0.z, G1.z})),
+                        mul(Hij, dot3(ex, ey, ez, df{O0.x, O1.x}, df{O0.y, O1.y}, df{O0.z, O1.z})));
+      acc_fma(sm[0], sw, ex);
+      acc_fma(sm[1], sw, ey);
+      acc_fma(sm[2], sw, ez);
+      if (RAND) {
+        const float4 G2 = Gf[4 * (size_t)j + 2], O2 = Gf[4 * (size_t)i + 2];
+        const df sx = sub(mul(Hji, dot3(ex, ey, ez, df{G0.w, G1.w}, df{G2.x, G2.z}, df{G2.y, G2.w})),
+                          mul(Hij, dot3(ex, ey, ez, df{O0.w, O1.w}, df{O2.x, O2.z}, df{O2.y, O2.w})));
+        acc_fma(sm[NS - 3], sx, ex);
+        acc_fma(sm[NS - 2], sx, ey);
+        acc_fma(sm[NS - 1], sx, ez);
+      }
+      if ((++m & 7) == 0) fold();
+    }
+    fold();
+  }
   double tot[6];
 #pragma unroll
   for (int q = 0; q < NS; ++q) {
@@ -1869,55 +1894,24 @@ __global__ void __launch_bounds__(128, EPH_DF_FORCES_BLOCKS)
         fry += __shfl_xor_sync(0xffffffffu, fry, o);
         frz += __shfl_xor_sync(0xffffffffu, frz, o);
       }
-      skipped |= __shfl_xor_sync(0xffffffffu, skipped, o);
     }
     if (i >= P.n || g != 0) return;
   }
   if (live) {
-    double cex = 0.0, cey = 0.0, cez = 0.0, crx = 0.0, cry = 0.0, crz = 0.0;
     const D4 Ai = A[i], Bi = Bw[i];
     const double a = Ai.y;  // alpha_i / rho_i
     const double Wx = a * Bi.y, Wy = a * Bi.z, Wz = a * Bi.w;
     const double Xx = a * Ai.z, Xy = a * Ai.w, Xz = a * Bi.x;
-    if (skipped) {  // rare: the skipped pairs' shares of M_i come back out
-      for (int k = 0; k < ns; ++k) {
-        const size_t slot = (size_t)k * P.n + i;
-        const unsigned j = pj[slot] & IDX_MASK;
-        const float g0 = Gf[4 * (size_t)j].x;
-        if (g0 == g0) continue;
-        const float4 hi = pe[2 * slot], lo = pe[2 * slot + 1];
-        const df dx{hi.x, lo.x}, dy{hi.y, lo.y}, dz{hi.z, lo.z};
-        df H{hi.w, lo.w};  // H_ij: the cached H_ji with one element
-        if (MULTI) {
-          const int ej = rec[4 * (size_t)j + 1].z;
-          if (ej != rec[4 * (size_t)i + 1].z) {
-            const df r2 = dot3(dx, dy, dz, dx, dy, dz);
-            H = mul(spline_rho_df(P, ej, r2, err), recip(r2, rcp_estimate(r2.hi)));
-          }
-        }
-        const double ex = to_double(dx), ey = to_double(dy), ez = to_double(dz);
-        const double hx = to_double(mul(H, dx)), hy = to_double(mul(H, dy)), hz = to_double(mul(H, dz));
-        const double sw = dot3_fma(ex, ey, ez, Wx, Wy, Wz);
-        cex = fma(sw, hx, cex);
-        cey = fma(sw, hy, cey);
-        cez = fma(sw, hz, cez);
-        if (RAND) {
-          const double sx = dot3_fma(ex, ey, ez, Xx, Xy, Xz);
-          crx = fma(sx, hx, crx);
-          cry = fma(sx, hy, cry);
-          crz = fma(sx, hz, crz);
-        }
-      }
-    }
-    const D4 M1 = Mm[i], M2 = Mm[(size_t)P.n + i];  // {xx, xy, xz, yy}, {yz, zz}
-    fex += cex - fma(M1.x, Wx, fma(M1.y, Wy, M1.z * Wz));
-    fey += cey - fma(M1.y, Wx, fma(M1.w, Wy, M2.x * Wz));
-    fez += cez - fma(M1.z, Wx, fma(M2.x, Wy, M2.y * Wz));
+    D4 M1 = Mm[i], M2 = Mm[(size_t)P.n + i];  // {xx, xy, xz, yy}, {yz, zz}
+    if (direct) M1 = M2 = D4{0.0, 0.0, 0.0, 0.0};
+    fex -= fma(M1.x, Wx, fma(M1.y, Wy, M1.z * Wz));
+    fey -= fma(M1.y, Wx, fma(M1.w, Wy, M2.x * Wz));
+    fez -= fma(M1.z, Wx, fma(M2.x, Wy, M2.y * Wz));
     if (RAND) {
       const double var = P.eta * sqrt(Te_i[i]);
-      frx = var * (fma(M1.x, Xx, fma(M1.y, Xy, M1.z * Xz)) - crx - frx);
-      fry = var * (fma(M1.y, Xx, fma(M1.w, Xy, M2.x * Xz)) - cry - fry);
-      frz = var * (fma(M1.z, Xx, fma(M2.x, Xy, M2.y * Xz)) - crz - frz);
+      frx = var * (fma(M1.x, Xx, fma(M1.y, Xy, M1.z * Xz)) - frx);
+      fry = var * (fma(M1.y, Xx, fma(M1.w, Xy, M2.x * Xz)) - fry);
+      frz = var * (fma(M1.z, Xx, fma(M2.x, Xy, M2.y * Xz)) - frz);
     }
   }
   store_forces<true, RAND>(P, i, live, fex, fey, fez, frx, fry, frz, f, f_eph, f_rng, f_dis, f_sto);
