@@ -150,12 +150,12 @@ def forces_bytes(n_atoms, n_pairs):
 # lists, 42.0 pairs per atom, like the bench workload); the bench's traffic figure is this ratio times the algorithmic
 # bytes at its own size.  Under 1: part of a sweep's pair-cache writes is
 # still in L2 when it ends.
-DENSITY_DRAM_OVER_ALGORITHMIC = 0.858
-FORCES_DRAM_OVER_ALGORITHMIC = 0.987
+DENSITY_DRAM_OVER_ALGORITHMIC = 0.793
+FORCES_DRAM_OVER_ALGORITHMIC = 0.998
 # pipe and issue figures of the two sweeps (ncu, the same captures)
-DENSITY_PIPES = {"issue_active": 0.469, "fma_pipe": 0.332, "alu_pipe": 0.144, "fp64_pipe": 0.294,
+DENSITY_PIPES = {"issue_active": 0.557, "fma_pipe": 0.414, "alu_pipe": 0.221, "fp64_pipe": 0.372,
                  "top_stall": "long_scoreboard"}
-FORCES_PIPES = {"issue_active": 0.379, "fma_pipe": 0.298, "alu_pipe": 0.083, "fp64_pipe": 0.157,
+FORCES_PIPES = {"issue_active": 0.418, "fma_pipe": 0.359, "alu_pipe": 0.112, "fp64_pipe": 0.174,
                 "top_stall": "long_scoreboard"}
 
 
@@ -819,15 +819,15 @@ def main():
         return {"bound": "hbm", "kernel": kernel, "achieved": achieved, "peak": hbm, "unit": "GB/s",
                 "frac": achieved / hbm, "peak_source": peak_src, "traffic": dram_ratio * nbytes,
                 "algorithmic_bytes": nbytes, "launch_ms": t_launch * 1000.0, "pipes_ncu_131k": pipes,
-                "note": "df64 pair arithmetic on the FP32 pipe; latency-bound on the neighbours' records "
-                        "(ncu: long-scoreboard stalls first)"}
+                "note": "df64 pair arithmetic on the FP32 pipe; bound by issue and by the L1 wavefronts of "
+                        "the neighbours' scattered records (ncu: 0.56-0.59 of the wavefront rate)"}
     line = {
         "metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": res["ms"] / args.steps, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64 (pair terms df64)", "data": "synthetic",
         "config": {"workload": WORKLOAD, "atoms_per_gpu": n, "grid": list(GRID), "dt_ps": DT,
                    "parallelism": f"replicas x{world}" if world > 1 else "single GPU",
-                   "l2": "inputs larger than L2 (pair cache ~%d MB)" % (res["n_pairs"] * 52 // 2 ** 20),
+                   "l2": "inputs larger than L2 (pair cache ~%d MB)" % (res["n_pairs"] * 36 // 2 ** 20),
                    "mode": "fast", "pair_arithmetic": "df64", "xi": "device Philox4x32-10"},
         "gpu_launches": res["launches"],
         "roofline": roofline("density", "k_density_df", density_bytes(n, res["n_pairs"]),

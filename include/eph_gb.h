@@ -250,10 +250,11 @@ int eph_set_pair_arithmetic(eph_ctx *ctx, int which);
  * the lists off).  The reference takes its pairs from the engine's Verlet list
  * (fix_eph.cpp:273-275: a full list with cutoff r_cutoff, padded by the
  * engine's skin and rebuilt when an atom moved half of it); here the list is
- * the context's own.  In FAST mode (model 4, the one-lane density sweep) the
+ * the context's own (with eph_set_pair_eam, of the pair force's list).  In FAST
+ * mode (model 4, the df64 or the one-lane FP64 density sweep) the
  * candidates within r_cutoff + s are found by a bin search on build steps
  * only; in between, up to 32 atoms that moved more than s/2 (and the atoms
- * near them) search afresh every step, and more of them make the step a
+ * near them) are handled every step, and more of them make the step a
  * build step (counter 2 counts the builds).  Pairs and results are those of
  * a search every step, up to the order of the sums.  *active reports whether
  * the context uses it (either pointer may be NULL). */
