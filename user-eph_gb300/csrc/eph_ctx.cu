@@ -1343,7 +1343,7 @@ int eph_autotune(eph_ctx *c, int *chosen) {
   if (r) return r;
   if (c->mode != EPH_MODE_FAST || c->args.model != 4) {
     if (chosen) *chosen = 1;
-    return EPH_OK;  // EXACT keeps the reference's order: one lane per atom
+    return EPH_OK;  // EXACT keeps the reference's order: its lanes follow the atom count
   }
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   // the sweeps need a step's pairs

@@ -464,10 +464,9 @@ __device__ __forceinline__ void density_epilogue(
 // instruction costs the same whether 1 or 32 lanes are active, so the FP64
 // work must run in lockstep.
 //   pass 1 (FP32/integer): candidates from the 27 bins around the atom with an
-//     FP32 distance test padded by 1e-4 of rc^2, kept in shared memory; EXACT
-//     mode keeps them in ascending neighbour index (the order of the
-//     reference's list, so sums round identically), FAST mode in the fixed
-//     bin-stencil order of index-sorted bins
+//     FP32 distance test padded by 1e-4 of rc^2, kept in shared memory in the
+//     fixed bin-stencil order of index-sorted bins (EXACT: k_density_exact, in
+//     ascending neighbour index, the order of the reference's list)
 //   pass 2 (FP64): the exact test r^2 < rc^2 with e = (x_j + image) - x_i, the
 //     density sum, and the pair cache of the in-cutoff pairs
 // Pair cache row k of atom i sits at k*n + i (coalesced across the warp):
