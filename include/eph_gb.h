@@ -202,7 +202,7 @@ int eph_pair_energy(eph_ctx *ctx, double *E);
  * counterpart): 0 = chosen from the atom count (the default), or 1, 2, 4, 8.
  * More lanes keep small systems (tens of thousands of atoms) from waiting on
  * their loads; the sums' order, and so the last bits, depend on it (EXACT
- * mode always uses one lane). */
+ * mode has lanes of its own, and the reference's order of the sums). */
 int eph_set_threads_per_atom(eph_ctx *ctx, int tpa);
 int eph_get_threads_per_atom(eph_ctx *ctx, int *tpa);
 /* Time the sweeps with 1, 2, 4 and 8 lanes per atom on the current pairs
