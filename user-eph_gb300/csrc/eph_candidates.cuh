@@ -284,10 +284,12 @@ struct CandidateArgs {
   const D4 *xref;
   const D4 *fpos;  // the moved atoms' positions wrapped into the box
   float far2;      // the moved atoms' widened cut-off (far_cutoff2)
+  int list_all;    // a build makes every atom's list, whether this sweep reads it or not
 };
 
 // The candidates of atom i from the bins of this step or the kept lists,
-// LANES lanes to an atom (g: the lane's number).  `at(k)`, k < CAP, is the
+// LANES lanes to an atom (g: the lane's number); none where it is not active
+// (valid: i is an atom).  `at(k)`, k < CAP, is the
 // shared-memory place of candidate k; further ones go to the atom's rows of
 // pj, or stay in the list (`tail`: where to read them).  Of the candidates
 // before number `first` those flagged as moved do not count: a list's entries
@@ -324,9 +326,12 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
     return nc;
   }
   if (C.rb[2] != 0) {  // a build step
+    // the EAM engine's sweep reads the lists of the atoms outside the group
+    // too, whichever sweep made them
+    const bool listed = C.list_all ? valid : active;
     int4 Bi = make_int4(0, 0, 0, 0);
     float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (active) {
+    if (listed) {
       Bi = C.atom_bin[i];
       oi = C.atom_off[i];
     }
@@ -338,17 +343,17 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
     // them: the shell's pairs mostly fail the exact test, and at the end of
     // the lists whole warps skip them
     if (LANES == 1) {
-      nc = collect_candidates(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, lset, C.band, P.lcap);
-      nc = collect_candidates(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, lset, P.rl2_band, P.lcap,
+      nc = collect_candidates(P, i, listed, Bi, oi, C.bin_count, C.bins, C.err, lset, C.band, P.lcap);
+      nc = collect_candidates(P, i, listed, Bi, oi, C.bin_count, C.bins, C.err, lset, P.rl2_band, P.lcap,
                               nullptr, C.band, nc);
     } else {
-      shared_candidates<LANES>(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, nc, P.lcap, lset, C.band);
-      shared_candidates<LANES>(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, nc, P.lcap, lset, P.rl2_band, nullptr,
+      shared_candidates<LANES>(P, i, listed, Bi, oi, C.bin_count, C.bins, C.err, nc, P.lcap, lset, C.band);
+      shared_candidates<LANES>(P, i, listed, Bi, oi, C.bin_count, C.bins, C.err, nc, P.lcap, lset, P.rl2_band, nullptr,
                                C.band);
     }
     tail = C.cl;
     if (valid && g == 0) C.cl_n[i] = nc;
-    return nc;
+    return active ? nc : 0;
   }
   const int st = active ? C.state[i] : 0;
   const bool near = st != 0;

@@ -432,6 +432,7 @@ void launch_density_df(eph_ctx *c, int xi_mode) {
   C.fpos = c->fpos.p;
   C.far2 = far_cutoff2(c, c->P.rc2);
   C.xref = c->xref.p;
+  C.list_all = c->eam != nullptr;
   D.mask = c->mask.p;
   D.v = c->v.p;
   D.xi_given = c->xi.p;

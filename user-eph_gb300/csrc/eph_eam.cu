@@ -673,6 +673,7 @@ int launch_eam(eph_ctx *c) {
     C.fpos = c->fpos.p;
     C.far2 = far_cutoff2(c, E.rc2);
     C.xref = c->xref.p;
+    C.list_all = 1;
     const int lanes = eam_lanes(c);
     if (E.one >= 0) {
       if (lanes == 2) launch_eam_df<true, 2>(c, E, C, fext);
