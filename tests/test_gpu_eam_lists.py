@@ -62,3 +62,39 @@ def test_atoms_outside_the_group_keep_their_lists(built, beta_file, tmp_path, bu
         for f in (got, ref):
             f.step(1, xi=xi)
         agree(got, ref)
+
+
+def hot_atoms(at, count, speed, seed):
+    rng = np.random.default_rng(seed)
+    hot = rng.choice(at.n, count, replace=False)
+    u = rng.standard_normal((count, 3))
+    at.v[hot] = speed * u / np.sqrt((u * u).sum(1))[:, None]
+
+
+# 8 and 4 lanes per atom; half the box empty (the row capacities, which follow
+# the box's mean density, are then those of half the atoms' neighbours); pair
+# forces longer and shorter than the fix's cut-off; a skin that puts more
+# candidates than rows around an atom
+MOVED = [((17, 16, 17), 2.0, "ni", 0.3), ((21, 20, 20), 2.0, "ni", 0.3), ((17, 16, 17), 1.0, "short", 0.6),
+         ((17, 16, 17), 1.0, "ni", 2.0), ((17, 16, 17), 1.0, "hook", 0.3)]
+
+
+@pytest.mark.parametrize("cells,stretch,eam,skin", MOVED)
+def test_moved_atoms_find_every_neighbour(built, beta_file, tmp_path, cells, stretch, eam, skin):
+    at = W.fcc_lattice(cells, seed=62)
+    at.boxhi = at.boxhi * np.array([1.0, 1.0, stretch])
+    hot_atoms(at, 12, 900.0 if skin < 1.0 else 2200.0, 3)
+    words = W.fix_args(beta_file, grid=(9, 8, 10), T_e=900.0)
+    path = W.write_eam_sutton_chen(str(tmp_path / "short.eam"), rc=2.7, r_on=2.55) if eam == "short" else ni_eam(tmp_path)
+    got, ref = with_and_without_lists(words, at, path, skin)
+    rng = np.random.default_rng(12)
+    builds = []
+    for _ in range(4):
+        xi = rng.standard_normal((at.n, 3))
+        for f in (got, ref):
+            f.step(1, xi=xi)
+            if eam == "hook":
+                f.post_force(xi)
+        agree(got, ref)
+        builds.append(got.counter("build"))
+    assert builds[-1] == builds[0]  # the atoms moved between builds

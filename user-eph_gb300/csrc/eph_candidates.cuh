@@ -230,6 +230,19 @@ __device__ __forceinline__ int collect_candidates(const StepParams &P, int i, bo
   return nc;
 }
 
+// the FP32 r^2 of candidate u from position xi, by the high words of the
+// fixed-point positions of this step
+__device__ __forceinline__ float pair_r2(const StepParams &P, const int4 *__restrict__ rec, unsigned u,
+                                         const long long *xi) {
+  long long e[3];
+  int4 ra, rb;
+  load_record(rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
+  pair_fixed(P, ra, rb, u >> IDX_BITS, xi, e);
+  const float ex = (float)(int)(e[0] >> 32) * P.fix_hi, ey = (float)(int)(e[1] >> 32) * P.fix_hi,
+              ez = (float)(int)(e[2] >> 32) * P.fix_hi;
+  return ex * ex + ey * ey + ez * ez;
+}
+
 // Pass 1 from the standalone engine's EAM pair list of this step
 // (k_eam_density's rows: every pair within the EAM cut-off, which exceeds
 // r2band): its entries within the FP32 threshold r2band, from the high words
@@ -249,13 +262,7 @@ __device__ __forceinline__ void list_candidates(const StepParams &P, int i, bool
     unsigned u = 0;
     if (k < ne) {
       u = elist[(size_t)k * P.n + i];
-      long long e[3];
-      int4 ra, rb;
-      load_record(rec + 4 * (size_t)(u & IDX_MASK), ra, rb);
-      pair_fixed(P, ra, rb, u >> IDX_BITS, xi, e);
-      const float ex = (float)(int)(e[0] >> 32) * P.fix_hi, ey = (float)(int)(e[1] >> 32) * P.fix_hi,
-                  ez = (float)(int)(e[2] >> 32) * P.fix_hi;
-      const float r2 = ex * ex + ey * ey + ez * ez;
+      const float r2 = pair_r2(P, rec, u, xi);
       take = r2 < r2band && keep(u, r2);
     }
     append_candidate<LANES>(take, u, nc, cap, cset, err);
@@ -272,8 +279,8 @@ struct CandidateArgs {
   const D4 *x;
   unsigned *err;
   // rows of the sweep's own pair list (kcap of them), which also hold the
-  // candidates that have no room in shared memory: a row is written only
-  // after the candidate there is read
+  // candidates that have no room in shared memory (and a moved atom's, without
+  // `moved`): a row is written only after the candidate there is read
   unsigned *pj;
   int kcap;
   float band;  // FP32 threshold of the cut-off
@@ -285,29 +292,42 @@ struct CandidateArgs {
   const D4 *fpos;  // the moved atoms' positions wrapped into the box
   float far2;      // the moved atoms' widened cut-off (far_cutoff2)
   int list_all;    // a build makes every atom's list, whether this sweep reads it or not
+  // candidates of the moved atoms, mcap each (all that their bins can hold, and
+  // every moved atom), for a sweep that keeps other pairs in their rows of pj
+  unsigned *moved;
+  int mcap;
 };
 
 // The candidates of atom i from the bins of this step or the kept lists,
 // LANES lanes to an atom (g: the lane's number); none where it is not active
 // (valid: i is an atom).  `at(k)`, k < CAP, is the
 // shared-memory place of candidate k; further ones go to the atom's rows of
-// pj, or stay in the list (`tail`: where to read them).  Of the candidates
+// pj, or stay in the list (`tail`: where number 0 would be; number k is k `step`
+// on, which is n but for a moved atom's with MOVED_ROWS).  Of the candidates
 // before number `first` those flagged as moved do not count: a list's entries
 // for them are of the build.
 // Kept lists: build steps search the bins within r_list and write the lists;
 // atoms that moved (k_list_check) search the bins of the build, atoms near one
-// (k_list_mark) take their list, and both then add the moved atoms.  A cascade's few hundred such atoms sit in a few
+// (k_list_mark) take their list, and both then add the moved atoms.  What a moved
+// atom finds is tested with the positions of this step, so that it needs no more
+// rows than a search of this step's bins; it waits in the atom's rows of pj, or
+// with MOVED_ROWS in rows of its own (C.moved), where the sweep writes pairs to
+// the far end of pj's rows: nothing would keep those off candidates not read
+// yet, and with half the box empty, rows for half the neighbours, they were lost.
+// A cascade's few hundred such atoms sit in a few
 // warps, whose latency is the sweep's tail: searching bin after bin with the
 // one lane, for both kinds, made the sweep 215 us at 131,072 atoms of two
 // elements on GB300; 154 now, as without moved atoms.
 // Every lane of the warp calls it.
-template <int LANES, bool LIST, int CAP, class At>
+template <int LANES, bool LIST, bool MOVED_ROWS, int CAP, class At>
 __device__ __forceinline__ int pair_candidates(const StepParams &P, const CandidateArgs &C, int i, int g, bool valid,
-                                               bool active, At at, const unsigned *&tail, int &first) {
+                                               bool active, At at, const unsigned *&tail, unsigned &step,
+                                               int &first) {
   const size_t n = (size_t)P.n;
   int nc = 0;
   first = 0;
-  tail = C.pj;
+  step = (unsigned)P.n;
+  tail = C.pj + i;
   auto set = [&](int k, unsigned u) {
     if (k < CAP) at(k) = u;
     else C.pj[(size_t)k * n + i] = u;
@@ -351,7 +371,7 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
       shared_candidates<LANES>(P, i, listed, Bi, oi, C.bin_count, C.bins, C.err, nc, P.lcap, lset, P.rl2_band, nullptr,
                                C.band);
     }
-    tail = C.cl;
+    tail = C.cl + i;
     if (valid && g == 0) C.cl_n[i] = nc;
     return active ? nc : 0;
   }
@@ -373,7 +393,10 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
       }
     }
     // an atom that moved searches the bins of the build, the whole warp for one
-    // such atom after the other, into its rows of pj
+    // such atom after the other
+    const int nf = C.rb[1];  // <= LIST_FMAX on a step without a build
+    int room = C.kcap;
+    unsigned *rows = C.pj + i;
     for (unsigned todo = __ballot_sync(0xffffffffu, (st & 2) != 0 && g == 0); todo; todo &= todo - 1) {
       const int src = __ffs(todo) - 1;
       const int is = __shfl_sync(0xffffffffu, i, src);
@@ -382,23 +405,40 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
       const float4 os = make_float4(__shfl_sync(0xffffffffu, oi.x, src), __shfl_sync(0xffffffffu, oi.y, src),
                                     __shfl_sync(0xffffffffu, oi.z, src), 0.f);
       int found = 0;
-      auto row = [&](int k, unsigned u) { C.pj[(size_t)k * n + is] = u; };
-      shared_candidates<32, true>(P, is, true, Bs, os, C.bin_count, C.bins, C.err, found, C.kcap, row, P.rl2_band,
-                                  C.state);
-      if (i == is) nc = found;
+      unsigned *own = C.pj + is;
+      if (MOVED_ROWS) {  // the moved atoms' order in flist
+        const int lane = (int)threadIdx.x & 31;
+        own = C.moved + (size_t)(__ffs(__ballot_sync(0xffffffffu, lane < nf && C.flist[lane] == is)) - 1) * C.mcap;
+      }
+      const size_t next = MOVED_ROWS ? 1 : n;
+      const int most = MOVED_ROWS ? C.mcap : C.kcap;
+      long long xs[3];
+      own_fixed(C.rec, is, xs);
+      auto row = [&](int k, unsigned u) { own[(size_t)k * next] = u; };
+      auto near_now = [&](unsigned u, float) { return pair_r2(P, C.rec, u, xs) < C.band; };
+      shared_candidates<32, true>(P, is, true, Bs, os, C.bin_count, C.bins, C.err, found, most, row, P.rl2_band,
+                                  C.state, -1.f, near_now);
+      if (i == is) {
+        nc = found;
+        if (MOVED_ROWS) {
+          rows = own;
+          step = 1;
+          room = most;
+        }
+      }
     }
     // one that did not, but is near one that did, has the unmoved ones in its
     // list, whose rows past the end take the moved ones
     if (st == 1) {
       nc = first = C.cl_n[i];
-      tail = C.cl;
+      rows = C.cl + i;
+      room = P.lcap;
     }
-    const int room = st == 1 ? P.lcap : C.kcap;
-    unsigned *rows = st == 1 ? C.cl : C.pj;
-    auto add = [&](int k, unsigned u) { rows[(size_t)k * n + i] = u; };
+    tail = rows;
+    const size_t next = MOVED_ROWS ? step : n;
+    auto add = [&](int k, unsigned u) { rows[(size_t)k * next] = u; };
     // the moved atoms near enough (a widened FP32 test; the exact one decides),
     // their image next to the position above; the atom's lanes take turns
-    const int nf = C.rb[1];  // <= LIST_FMAX on a step without a build
     for (int q = g; q - g < nf; q += LANES) {
       bool take = false;
       unsigned u = 0;
@@ -424,7 +464,7 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
     }
   }
   if (!near) {
-    tail = C.cl;
+    tail = C.cl + i;
     nc = active ? C.cl_n[i] : 0;
     first = nc;
   }

@@ -679,6 +679,8 @@ void drop_list(eph_ctx *c) {
   c->rb.free();
   c->flist.free();
   c->fpos.free();
+  c->mcand.free();
+  c->mcap = 0;
   c->xref.free();
 }
 
@@ -714,6 +716,9 @@ int configure_list(eph_ctx *c) {
   if (!c->rb.p) CUDA_TRY(c, c->rb.alloc(4));
   if (!c->flist.p) CUDA_TRY(c, c->flist.alloc(LIST_FMAX));
   if (!c->fpos.p) CUDA_TRY(c, c->fpos.alloc(LIST_FMAX));
+  const int mcap = 27 * c->bcap + LIST_FMAX;
+  if (mcap != c->mcap) CUDA_TRY(c, c->mcand.alloc((size_t)LIST_FMAX * mcap));
+  c->mcap = mcap;
   CUDA_TRY(c, cudaMemsetAsync(c->rb.p, 0, 4 * sizeof(int), c->stream));
   CUDA_TRY(c, cudaMemsetAsync(c->rb.p, 0x01, 1, c->stream));  // rb[0] = 1: the next step builds
   c->P.lcap = lcap;

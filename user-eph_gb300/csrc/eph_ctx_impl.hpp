@@ -113,6 +113,8 @@ struct eph_ctx {
   DevBuf<int> cl_n, state, rb, flist;
   DevBuf<D4> xref;  // positions at the last build
   DevBuf<D4> fpos;  // the moved atoms' positions wrapped into the box
+  DevBuf<unsigned> mcand;  // [LIST_FMAX][mcap] their candidates
+  int mcap = 0;
 
   DevBuf<D4> tab_rho_r_sq, tab_beta, tab_alpha;
   // FAST pair sums in df64 (eph_set_pair_arithmetic, on by default): the

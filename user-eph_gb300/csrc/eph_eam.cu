@@ -326,8 +326,9 @@ __global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
   long long xi[3] = {0, 0, 0};
   if (valid) own_fixed(C.rec, i, xi);
   const unsigned *tail;
+  unsigned step;
   int first;
-  const int nc = pair_candidates<LANES, LIST, CAP>(P, C, i, g, valid, valid, at, tail, first);
+  const int nc = pair_candidates<LANES, LIST, LIST, CAP>(P, C, i, g, valid, valid, at, tail, step, first);
   __syncwarp();
   const df rc2{E.rc2_hi, E.rc2_lo}, inv_dr{E.inv_dr_hi, E.inv_dr_lo};
   bsum rs = bsum_zero();
@@ -335,7 +336,7 @@ __global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
   const int nmax = __reduce_max_sync(FULL, nc);
   auto cand = [&](int k) -> unsigned {
     if (k >= nc) return CODE_NOSHIFT << IDX_BITS;  // atom 0, not counted
-    return k < CAP ? at(k) : tail[(size_t)k * n + i];
+    return k < CAP ? at(k) : tail[(size_t)k * step];
   };
   unsigned u = cand(g), u2 = cand(g + LANES);
   int4 ra, rb;
@@ -375,7 +376,9 @@ __global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
     }
     if (in) {
       const int row = out ? C.kcap - 1 - back : slot;
-      if (ns + far <= C.kcap) C.pj[(size_t)row * n + i] = uc;  // front rows <= k: the candidate there is consumed
+      // with kept lists no candidate waits in these rows; else row <= k, and the
+      // candidate there is consumed
+      if (ns + far <= C.kcap) C.pj[(size_t)row * n + i] = uc;
       else atomicOr(C.err, ERR_PAIR_OVERFLOW);
       const df r = mul(r2, rsqrt(r2, rsqrt_estimate(r2.hi)));
       int mk;
@@ -673,6 +676,8 @@ int launch_eam(eph_ctx *c) {
     C.fpos = c->fpos.p;
     C.far2 = far_cutoff2(c, E.rc2);
     C.xref = c->xref.p;
+    C.moved = c->mcand.p;
+    C.mcap = c->mcap;
     C.list_all = 1;
     const int lanes = eam_lanes(c);
     if (E.one >= 0) {

@@ -1181,6 +1181,23 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
   unsigned *__restrict__ pj = D.C.pj;
 #pragma unroll
   for (int q = 0; q < 9; ++q) s_tot[q * 128 + t] = make_float2(0.f, 0.f);
+  int nc = 0;
+  int first = 0;
+  const unsigned *tail = pj + i;
+  if (SRC == DF_EAM && D.ens_in) {  // the list has them apart
+    tail = D.elist + i;
+    nc = active ? D.ens_in[i] : 0;
+  } else if (SRC == DF_EAM) {
+    auto set = [&](int k, unsigned u) { pj[(size_t)k * n + i] = u; };
+    long long xi[3] = {0, 0, 0};
+    if (valid) own_fixed(D.C.rec, i, xi);
+    list_candidates<LANES>(P, i, active, xi, D.elist, D.ens, D.C.rec, D.C.err, nc, P.kcap, set, P.rc2_band);
+  } else {
+    unsigned step;  // n: a moved atom's candidates wait in its rows of pj
+    nc = pair_candidates<LANES, SRC == DF_LIST, false, CAP>(P, D.C, i, g, valid, active, at, tail, step, first);
+  }
+  __syncwarp();
+  // after the candidates: their searches need the registers
   long long xi[3] = {0, 0, 0};
   int ei = 0;
   if (valid) {
@@ -1191,19 +1208,6 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
     xi[2] = ((long long)rb.y << 32) | (unsigned)rb.x;
     ei = rb.z;
   }
-  int nc = 0;
-  int first = 0;
-  const unsigned *tail = pj;
-  if (SRC == DF_EAM && D.ens_in) {  // the list has them apart
-    tail = D.elist;
-    nc = active ? D.ens_in[i] : 0;
-  } else if (SRC == DF_EAM) {
-    auto set = [&](int k, unsigned u) { pj[(size_t)k * n + i] = u; };
-    list_candidates<LANES>(P, i, active, xi, D.elist, D.ens, D.C.rec, D.C.err, nc, P.kcap, set, P.rc2_band);
-  } else {
-    nc = pair_candidates<LANES, SRC == DF_LIST, CAP>(P, D.C, i, g, valid, active, at, tail, first);
-  }
-  __syncwarp();
   // pass 2; the next candidate's position is loaded while this one is summed,
   // each half of a record in one 256-bit load (load_row)
   acc sm[9];
@@ -1214,7 +1218,7 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
   int ns = 0;
   auto cand = [&](int k) -> unsigned {
     if (k >= nc) return CODE_NOSHIFT << IDX_BITS;  // atom 0, not counted
-    return k < CAP ? at(k) : tail[(size_t)k * n + i];
+    return k < CAP ? at(k) : tail[(size_t)k * n];
   };
   unsigned u = cand(g), u2 = cand(g + LANES);
   int4 ra, rb;
