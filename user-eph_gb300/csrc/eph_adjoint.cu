@@ -1742,7 +1742,7 @@ int bwd_finish(eph_adjoint *a, bool skip_last, cudaStream_t st) {
   ADJ_TRY(a, cudaStreamSynchronize(st));
   if ((r = ctxi::check_device(c))) return from_ctx(a, r);
   if (herr) {
-    cudaMemset(a->d_err.p, 0, sizeof(unsigned));
+    cudaMemsetAsync(a->d_err.p, 0, sizeof(unsigned), c->stream);
     return afail(a, EPH_ERR_RANGE, "device: a grid cotangent sum left the fixed-point range");
   }
   a->grad_rho.assign(B.n_elements, std::vector<double>(B.n_rho, 0.0));
@@ -1802,9 +1802,9 @@ int eph_adjoint_create(eph_ctx *c, int checkpoint_every, eph_adjoint **out) {
   ADJ_TRY(a, a->tbc.alloc(N));
   ADJ_TRY(a, a->tb_acc.alloc(nc));
   ADJ_TRY(a, a->d_err.alloc(1));
-  ADJ_TRY(a, cudaMemset(a->tb_acc.p, 0, sizeof(U128) * nc));
-  ADJ_TRY(a, cudaMemset(a->d_err.p, 0, sizeof(unsigned)));
-  ADJ_TRY(a, cudaMemcpy(a->rho_e.p, c->grid.rho.data(), nc * sizeof(double), cudaMemcpyHostToDevice));
+  ADJ_TRY(a, cudaMemsetAsync(a->tb_acc.p, 0, sizeof(U128) * nc, c->stream));
+  ADJ_TRY(a, cudaMemsetAsync(a->d_err.p, 0, sizeof(unsigned), c->stream));
+  ADJ_TRY(a, ctxi::upload(c, a->rho_e.p, c->grid.rho.data(), nc * sizeof(double)));
   const Beta &B = c->beta;
   a->nt4_rho = 4 * B.n_elements * (int)B.n_rho;
   a->nt4_alpha = 4 * B.n_elements * (int)B.n_beta;

@@ -60,7 +60,7 @@ int upload_tables(eph_ctx *c) {
       cudaError_t r = dst.alloc((size_t)b.n_elements * nk);
       if (r != cudaSuccess) return r;
     }
-    return cudaMemcpy(dst.p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
+    return upload(c, dst.p, h.data(), h.size() * sizeof(double));
   };
   CUDA_TRY(c, up(c->tab_rho_r_sq, EPH_SPLINE_RHO_R_SQ, b.n_rho));
   CUDA_TRY(c, up(c->tab_beta, EPH_SPLINE_BETA, b.n_beta));
@@ -101,7 +101,7 @@ int upload_tables(eph_ctx *c) {
       c->buf_gen += 1;
       CUDA_TRY(c, c->tab_rho_df.alloc(h.size()));
     }
-    CUDA_TRY(c, cudaMemcpy(c->tab_rho_df.p, h.data(), h.size() * sizeof(float4), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, upload(c, c->tab_rho_df.p, h.data(), h.size() * sizeof(float4)));
     c->P.tab_rho_df = c->tab_rho_df.p;
   }
   return EPH_OK;
@@ -111,7 +111,7 @@ int upload_tables(eph_ctx *c) {
 cudaError_t upload_inverse(eph_ctx *c, const std::vector<double> &rc) {
   std::vector<double> inv(rc.size());
   for (size_t i = 0; i < rc.size(); ++i) inv[i] = 1.0 / rc[i];
-  return cudaMemcpy(c->irhoC.p, inv.data(), inv.size() * 8, cudaMemcpyHostToDevice);
+  return upload(c, c->irhoC.p, inv.data(), inv.size() * 8);
 }
 
 int upload_grid(eph_ctx *c) {
@@ -133,14 +133,14 @@ int upload_grid(eph_ctx *c) {
     rc[i] = g.rho[i] * g.C[i];  // eph_fdm.h:372 prescaler
     fl[i] = (signed char)g.flag[i];
   }
-  CUDA_TRY(c, cudaMemcpy(c->T0.p, g.T.data(), nc * 8, cudaMemcpyHostToDevice));
-  CUDA_TRY(c, cudaMemcpy(c->kappa.p, g.kappa.data(), nc * 8, cudaMemcpyHostToDevice));
-  CUDA_TRY(c, cudaMemcpy(c->rhoC.p, rc.data(), nc * 8, cudaMemcpyHostToDevice));
+  CUDA_TRY(c, upload(c, c->T0.p, g.T.data(), nc * 8));
+  CUDA_TRY(c, upload(c, c->kappa.p, g.kappa.data(), nc * 8));
+  CUDA_TRY(c, upload(c, c->rhoC.p, rc.data(), nc * 8));
   CUDA_TRY(c, upload_inverse(c, rc));
-  CUDA_TRY(c, cudaMemcpy(c->S.p, g.S.data(), nc * 8, cudaMemcpyHostToDevice));
-  CUDA_TRY(c, cudaMemcpy(c->gflag.p, fl.data(), nc, cudaMemcpyHostToDevice));
-  CUDA_TRY(c, cudaMemset(c->dT.p, 0, nc * 8));
-  CUDA_TRY(c, cudaMemset(c->acc.p, 0, nc * sizeof(U128)));
+  CUDA_TRY(c, upload(c, c->S.p, g.S.data(), nc * 8));
+  CUDA_TRY(c, upload(c, c->gflag.p, fl.data(), nc));
+  CUDA_TRY(c, cudaMemsetAsync(c->dT.p, 0, nc * 8, c->stream));
+  CUDA_TRY(c, cudaMemsetAsync(c->acc.p, 0, nc * sizeof(U128), c->stream));
   c->td = TdynTables{};
   bool any = false;
   for (size_t i = 0; i < nc; ++i) any = any || g.T_dynamic[i];
@@ -156,13 +156,13 @@ int upload_grid(eph_ctx *c) {
     CUDA_TRY(c, c->C_T.alloc(nt));
     CUDA_TRY(c, c->K_T.alloc(nt));
     CUDA_TRY(c, c->bounds.alloc(4));
-    CUDA_TRY(c, cudaMemcpy(c->tdyn.p, td.data(), nc, cudaMemcpyHostToDevice));
-    CUDA_TRY(c, cudaMemcpy(c->gC.p, g.C.data(), nc * 8, cudaMemcpyHostToDevice));
-    CUDA_TRY(c, cudaMemcpy(c->grho.p, g.rho.data(), nc * 8, cudaMemcpyHostToDevice));
-    CUDA_TRY(c, cudaMemcpy(c->E_y.p, g.E_T.y.data(), nt * 8, cudaMemcpyHostToDevice));
-    CUDA_TRY(c, cudaMemcpy(c->E_dy.p, g.E_T.dy.data(), nt * 8, cudaMemcpyHostToDevice));
-    CUDA_TRY(c, cudaMemcpy(c->C_T.p, g.C_T.c.data(), nt * sizeof(D4), cudaMemcpyHostToDevice));
-    CUDA_TRY(c, cudaMemcpy(c->K_T.p, g.kappa_T.c.data(), nt * sizeof(D4), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, upload(c, c->tdyn.p, td.data(), nc));
+    CUDA_TRY(c, upload(c, c->gC.p, g.C.data(), nc * 8));
+    CUDA_TRY(c, upload(c, c->grho.p, g.rho.data(), nc * 8));
+    CUDA_TRY(c, upload(c, c->E_y.p, g.E_T.y.data(), nt * 8));
+    CUDA_TRY(c, upload(c, c->E_dy.p, g.E_T.dy.data(), nt * 8));
+    CUDA_TRY(c, upload(c, c->C_T.p, g.C_T.c.data(), nt * sizeof(D4)));
+    CUDA_TRY(c, upload(c, c->K_T.p, g.kappa_T.c.data(), nt * sizeof(D4)));
     if (!c->h_bounds) CUDA_TRY(c, cudaMallocHost(&c->h_bounds, 4 * sizeof(double)));
     c->td = TdynTables{c->tdyn.p, c->C_T.p, c->K_T.p, c->E_y.p, c->E_dy.p, c->grho.p, g.E_T.dx, g.C_T.inv_dx, (int)nt};
   }
@@ -1173,15 +1173,15 @@ int eph_create(int narg, const char *const *arg, const eph_md *md, eph_ctx **out
   CUDA_TRY(c, c->counters.alloc(NCOUNTERS));
   CUDA_TRY(c, c->wrapflag.alloc(1));
   CUDA_TRY(c, c->step_ctr.alloc(1));
-  CUDA_TRY(c, cudaMemset(c->step_ctr.p, 0, sizeof(unsigned long long)));
+  CUDA_TRY(c, cudaMemsetAsync(c->step_ctr.p, 0, sizeof(unsigned long long), c->stream));
   CUDA_TRY(c, c->scal.alloc(4));
   CUDA_TRY(c, c->deposit_left.alloc(1));
-  CUDA_TRY(c, cudaMemset(c->deposit_left.p, 0, sizeof(unsigned)));
+  CUDA_TRY(c, cudaMemsetAsync(c->deposit_left.p, 0, sizeof(unsigned), c->stream));
   CUDA_TRY(c, c->gsum.alloc(1));
-  CUDA_TRY(c, cudaMemset(c->d_err.p, 0, sizeof(unsigned)));
-  CUDA_TRY(c, cudaMemset(c->counters.p, 0, sizeof(unsigned long long) * NCOUNTERS));
-  CUDA_TRY(c, cudaMemset(c->wrapflag.p, 0, sizeof(int)));
-  CUDA_TRY(c, cudaMemset(c->scal.p, 0, sizeof(double) * 4));
+  CUDA_TRY(c, cudaMemsetAsync(c->d_err.p, 0, sizeof(unsigned), c->stream));
+  CUDA_TRY(c, cudaMemsetAsync(c->counters.p, 0, sizeof(unsigned long long) * NCOUNTERS, c->stream));
+  CUDA_TRY(c, cudaMemsetAsync(c->wrapflag.p, 0, sizeof(int), c->stream));
+  CUDA_TRY(c, cudaMemsetAsync(c->scal.p, 0, sizeof(double) * 4, c->stream));
   r = upload_tables(c);
   if (r) return r;
   r = upload_grid(c);
@@ -1233,7 +1233,7 @@ int eph_create(int narg, const char *const *arg, const eph_md *md, eph_ctx **out
   if ((r = build_fdm_coef(c))) return r;
   // bins: edge >= rc (1 + 5e-5), at least 3 per axis
   if ((r = set_bin_geometry(c, c->beta.r_cutoff))) return r;
-  CUDA_TRY(c, cudaDeviceSynchronize());  // the set-up copies and memsets above ran on the default stream
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   return EPH_OK;
 }
 
@@ -1605,9 +1605,9 @@ int eph_set_atoms(eph_ctx *c, int n, const double *hx, const double *hv, const i
   // atoms
   std::vector<int> m(N, 1);
   if (hmask) std::memcpy(m.data(), hmask, sizeof(int) * N);
-  CUDA_TRY(c, cudaMemcpy(c->type.p, htype, sizeof(int) * N, cudaMemcpyHostToDevice));
-  CUDA_TRY(c, cudaMemcpy(c->mask.p, m.data(), sizeof(int) * N, cudaMemcpyHostToDevice));
-  CUDA_TRY(c, cudaMemcpy(c->tmap.p, c->P.type_map, sizeof(int) * 65, cudaMemcpyHostToDevice));
+  CUDA_TRY(c, upload(c, c->type.p, htype, sizeof(int) * N));
+  CUDA_TRY(c, upload(c, c->mask.p, m.data(), sizeof(int) * N));
+  CUDA_TRY(c, upload(c, c->tmap.p, c->P.type_map, sizeof(int) * 65));
   for (DevBuf<D4> *b : {&c->x, &c->v, &c->f, &c->xhold, &c->f_eph, &c->f_rng, &c->xi, &c->A, &c->Bw})
     CUDA_TRY(c, cudaMemsetAsync(b->p, 0, sizeof(D4) * N, c->stream));
   int r = eph_put(c, EPH_FIELD_X, hx, EPH_HOST);
@@ -2338,9 +2338,9 @@ int eph_set_grid_constants(eph_ctx *c, double C_e, double kappa_e) {
   for (size_t i = 0; i < nc; ++i) rc[i] = g.rho[i] * g.C[i];
   CUDA_TRY(c, cudaSetDevice(c->device));
   CUDA_TRY(c, cudaStreamSynchronize(c->stream));
-  CUDA_TRY(c, cudaMemcpy(c->rhoC.p, rc.data(), nc * 8, cudaMemcpyHostToDevice));
+  CUDA_TRY(c, upload(c, c->rhoC.p, rc.data(), nc * 8));
   CUDA_TRY(c, upload_inverse(c, rc));
-  CUDA_TRY(c, cudaMemcpy(c->kappa.p, g.kappa.data(), nc * 8, cudaMemcpyHostToDevice));
+  CUDA_TRY(c, upload(c, c->kappa.p, g.kappa.data(), nc * 8));
   drop_graph(c);  // the substep count may change
   const unsigned nsub = c->nsub;
   set_time_params(c);

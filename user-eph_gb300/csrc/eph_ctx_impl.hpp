@@ -226,6 +226,14 @@ inline float far_cutoff2(const eph_ctx *c, double rc2) {
   return (float)(r * r);
 }
 
+// A set-up copy from pageable host memory, on the context's stream: what the
+// stream does next finds it done (cudaMemcpy on the default stream is not
+// ordered with it, and may return before the device has the data).
+inline cudaError_t upload(eph_ctx *c, void *dst, const void *src, size_t bytes) {
+  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;  // src may be a local of the caller's
+}
+
 inline cudaEvent_t take_event(eph_ctx *c) {
   if (!c->event_pool.empty()) {
     cudaEvent_t e = c->event_pool.back();

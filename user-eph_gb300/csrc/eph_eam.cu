@@ -566,7 +566,7 @@ int upload_table(eph_ctx *c, DevBuf<D4> &dst, const std::vector<std::vector<doub
     all.insert(all.end(), coef.begin(), coef.end());
   }
   CUDA_TRY(c, dst.alloc(all.size() / 4));
-  CUDA_TRY(c, cudaMemcpy(dst.p, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CUDA_TRY(c, ctxi::upload(c, dst.p, all.data(), all.size() * sizeof(double)));
   if (dfo) {
     std::vector<float> split(2 * all.size());
     for (size_t m = 0; m < all.size() / 4; ++m)
@@ -576,7 +576,7 @@ int upload_table(eph_ctx *c, DevBuf<D4> &dst, const std::vector<std::vector<doub
         split[8 * m + 4 + k] = v.lo;
       }
     CUDA_TRY(c, dfo->alloc(all.size() / 2));
-    CUDA_TRY(c, cudaMemcpy(dfo->p, split.data(), split.size() * sizeof(float), cudaMemcpyHostToDevice));
+    CUDA_TRY(c, ctxi::upload(c, dfo->p, split.data(), split.size() * sizeof(float)));
   }
   return EPH_OK;
 }
@@ -627,7 +627,7 @@ int eam_resize(eph_ctx *c) {
   CUDA_TRY(c, d->ns.alloc(N));
   CUDA_TRY(c, d->ns_in.alloc(N));
   CUDA_TRY(c, d->fpd.alloc(N));
-  CUDA_TRY(c, cudaMemset(d->energy.p, 0, sizeof(double) * N));
+  CUDA_TRY(c, cudaMemsetAsync(d->energy.p, 0, sizeof(double) * N, c->stream));
   // pair rows from the number density: twice the cut-off sphere, plus slack
   const double dens = (double)c->n / (c->prd[0] * c->prd[1] * c->prd[2]);
   const double rc = d->host.rc;
