@@ -52,3 +52,27 @@ fix.step(1)
 """)
     assert sum("k_fdm_coef" in words[-1] for words in log) == 1
     assert [words for words in log if words[0] == "default"] == []
+
+
+@pytest.mark.parametrize("change", ["reset_dt(0.0005)", "set_grid_constants(3e-6, 0.2)",
+                                    "set_beta_knots(0, np.linspace(1.0, 0.0, 2000), np.full(2000, 0.05))"])
+def test_a_replica_changes_after_the_queued_steps(logged, beta_file, change):
+    """A batch's steps run on its own stream: a replica's new time step, grid
+    constants or tables wait for those queued before."""
+    log = logged(f"""
+import numpy as np
+import sys
+import ephgb
+from ephgb import workloads as W
+at = W.fcc_lattice(5)
+batch = ephgb.Batch([(W.fix_args({beta_file!r}), at)] * 2)
+batch.step(3)
+fix = batch.replicas[1]
+sys.stderr.write("mark change\\n")
+fix.{change}
+""")
+    last = max(i for i, words in enumerate(log) if words[-1] == "cudaGraphLaunch")
+    stream = log[last][1]
+    after = log[log.index(["mark", "change"]):]
+    first_work = next(i for i, words in enumerate(after) if words[0] in ("stream", "default"))
+    assert ["wait", stream] in after[:first_work]

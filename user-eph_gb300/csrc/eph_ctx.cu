@@ -233,6 +233,7 @@ int build_fdm_coef(eph_ctx *c) {
                                                          c->irhoC.p, c->S.p, c->gflag.p, c->fdm_coef.p,
                                                          c->fdm_coef.p + 6 * nc, c->fdm_coef.p + 7 * nc);
   CUDA_TRY(c, cudaGetLastError());
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));  // a batch steps on a stream of its own
   return EPH_OK;
 }
 
@@ -1991,6 +1992,7 @@ int eph_compute_vector(eph_ctx *c, int i, double *out) {
 
 int eph_reset_dt(eph_ctx *c, double dt) {
   if (!c || !(dt > 0)) return EPH_ERR_ARG;
+  CUDA_TRY(c, settle(c));  // queued steps read the old coefficients
   drop_graph(c);
   c->buf_gen += 1;  // graphs captured elsewhere hold the old step constants
   c->dt = dt;
@@ -2131,6 +2133,7 @@ int eph_batch_create(int nrep, const int *narg, const char *const *const *arg, c
     b->err = "cannot create the batch stream";
     return EPH_ERR_CUDA;
   }
+  for (eph_ctx *c : b->reps) c->batch = b->main;
   b->joins.assign(nrep, nullptr);
   for (auto &e : b->joins)
     if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return EPH_ERR_CUDA;
@@ -2319,7 +2322,7 @@ int eph_set_beta_knots(eph_ctx *c, int elem, const double *rho_knots, long n_rho
   std::string e = c->beta.set_knots(elem, rho_knots, n_rho, beta_knots, n_beta);
   if (!e.empty()) return fail(c, EPH_ERR_ARG, e);
   CUDA_TRY(c, cudaSetDevice(c->device));
-  CUDA_TRY(c, cudaStreamSynchronize(c->stream));  // no kernel of the stream reads the tables meanwhile
+  CUDA_TRY(c, settle(c));  // no kernel reads the tables meanwhile
   return upload_tables(c);
 }
 
@@ -2337,7 +2340,7 @@ int eph_set_grid_constants(eph_ctx *c, double C_e, double kappa_e) {
   std::vector<double> rc(nc);
   for (size_t i = 0; i < nc; ++i) rc[i] = g.rho[i] * g.C[i];
   CUDA_TRY(c, cudaSetDevice(c->device));
-  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+  CUDA_TRY(c, settle(c));  // queued steps read the old constants
   CUDA_TRY(c, upload(c, c->rhoC.p, rc.data(), nc * 8));
   CUDA_TRY(c, upload_inverse(c, rc));
   CUDA_TRY(c, upload(c, c->kappa.p, g.kappa.data(), nc * 8));

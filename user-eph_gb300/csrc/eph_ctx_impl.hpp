@@ -49,6 +49,7 @@ struct eph_ctx {
   int device = 0;
   cudaStream_t stream = 0;
   bool own_stream = false;
+  cudaStream_t batch = nullptr;  // of a batch's replica: the stream its captured steps are queued on
 
   FixArgs args;
   Beta beta;
@@ -224,6 +225,13 @@ inline float far_cutoff2(const eph_ctx *c, double rc2) {
   const double r = std::sqrt(rc2) * (1.0 + 5e-5) +
                    std::ldexp(std::max(c->prd[0], std::max(c->prd[1], c->prd[2])), -21);
   return (float)(r * r);
+}
+
+// Wait for the steps queued so far, this context's and those of its batch:
+// before device data that they read is overwritten.
+inline cudaError_t settle(eph_ctx *c) {
+  const cudaError_t e = c->batch ? cudaStreamSynchronize(c->batch) : cudaSuccess;
+  return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
 }
 
 // A set-up copy from pageable host memory, on the context's stream: what the
