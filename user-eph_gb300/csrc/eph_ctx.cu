@@ -612,6 +612,11 @@ void launch_forces_t(eph_ctx *c) {
 int auto_tpa(long n) { return n <= 6144 ? 8 : (n <= 65536 ? 4 : 1); }
 
 // Bins of edge >= r (1 + 5e-5), at least three per axis; 0 or an error
+// bins along each axis for a search radius r
+void bins_along(const eph_ctx *c, double r, int *nb) {
+  for (int k = 0; k < 3; ++k) nb[k] = (int)(c->prd[k] / (r * (1.0 + 5e-5)));
+}
+
 int set_bin_geometry(eph_ctx *c, double r) {
   const double edge = r * (1.0 + 5e-5);
   int nb[3];
@@ -643,6 +648,23 @@ int auto_bcap(const eph_ctx *c) {
   const double dens = c->n / (c->prd[0] * c->prd[1] * c->prd[2]);
   const double per_bin = dens * c->P.w[0] * c->P.w[1] * c->P.w[2];
   return ((int)std::ceil(2.0 * per_bin + 16.0) + 7) / 8 * 8;
+}
+
+// The same for the lists' wider bins, which must hold what the cut-off's bins
+// hold without lists.  Where the box is mostly empty that is not given by the
+// mean density: there the capacity grows with the bin's volume (and a fifth, for
+// the lattice planes that a wider bin may take in), up to 0.25 atoms per A^3, which
+// is denser than any solid and leaves a full box's capacity as it is.
+int list_bcap(const eph_ctx *c, double rc) {
+  int nb[3];
+  bins_along(c, rc, nb);
+  const double vol = c->P.w[0] * c->P.w[1] * c->P.w[2];
+  const double plain = c->prd[0] * c->prd[1] * c->prd[2] / ((double)nb[0] * nb[1] * nb[2]);
+  auto round8 = [](double v) { return ((int)std::ceil(v) + 7) / 8 * 8; };
+  if (c->bcap_user) return std::max(c->bcap_set, (int)std::ceil(1.2 * c->bcap_set * vol / plain));
+  const double dens = c->n / (c->prd[0] * c->prd[1] * c->prd[2]);
+  const double grown = 1.2 * round8(2.0 * dens * plain + 16.0) * vol / plain;
+  return std::max(auto_bcap(c), round8(std::min(grown, 0.25 * vol)));
 }
 
 // Kept candidate lists: FAST mode, model 4 with friction, the one-lane
@@ -692,7 +714,7 @@ int configure_list(eph_ctx *c) {
   const int nbins_was = c->nbins, bcap_was = c->bcap;
   int r = set_bin_geometry(c, want ? rc + c->lskin : rc);
   if (r) return r;
-  if (!c->bcap_user) c->bcap = auto_bcap(c);
+  c->bcap = want ? list_bcap(c, rc) : (c->bcap_user ? c->bcap_set : auto_bcap(c));
   c->P.bcap = c->bcap;
   if (c->nbins != nbins_was || c->bcap != bcap_was || !c->bins.p) {
     CUDA_TRY(c, c->bins.alloc((size_t)c->nbins * c->bcap));
@@ -708,7 +730,14 @@ int configure_list(eph_ctx *c) {
   const size_t N = (size_t)c->n;
   const double rl = rc + c->lskin, rm = rc + 0.5 * c->lskin;
   const double dens = c->n / (c->prd[0] * c->prd[1] * c->prd[2]);
-  const int lcap = std::min(c->eam ? 512 : 256, ((int)std::ceil(2.0 * dens * 4.18879020478639 * rl * rl * rl + 24.0) + 7) / 8 * 8);
+  // rows for the candidates out to r_list: by the mean density, but also for all
+  // that fit the pair rows without lists, grown with the sphere, and a lattice
+  // shell more (in a box that is mostly empty the mean density says little: a
+  // third full of Ni at 6.5 A, 104 pair rows and 91 candidates, 134 out to 6.8 A)
+  const int kcap = c->beta.r_cutoff >= eam_cutoff(c) ? c->kcap : eam_rows(c);
+  const double rows = std::max(2.0 * dens * 4.18879020478639 * rl * rl * rl + 24.0,
+                               kcap * (rl * rl * rl) / (rc * rc * rc) + 48.0);
+  const int lcap = std::min(c->eam ? 1 << 16 : 256, ((int)std::ceil(rows) + 7) / 8 * 8);
   if (lcap != c->lcap || c->cl.n != (size_t)lcap * N) CUDA_TRY(c, c->cl.alloc((size_t)lcap * N));
   c->lcap = lcap;
   for (DevBuf<int> *b : {&c->cl_n, &c->state})
@@ -1264,7 +1293,7 @@ int eph_set_capacity(eph_ctx *c, int bin_capacity, int pair_capacity) {
   drop_graph(c);
   if (pair_capacity > KMAX) return fail(c, EPH_ERR_ARG, "pair capacity above the compiled maximum");
   c->buf_gen += 1;
-  if (bin_capacity > 0) c->bcap = bin_capacity, c->bcap_user = true;
+  if (bin_capacity > 0) c->bcap = c->bcap_set = bin_capacity, c->bcap_user = true;
   if (pair_capacity > 0) c->kcap = pair_capacity;
   if (c->n > 0) {
     c->P.bcap = c->bcap;
@@ -1316,7 +1345,7 @@ int apply_list_skin(eph_ctx *c, double skin, bool user) {
   if (r) return r;
   if (was && !c->reuse) {  // back to the cutoff's bins
     if ((r = set_bin_geometry(c, pair_radius(c)))) return r;
-    if (!c->bcap_user) c->bcap = auto_bcap(c);
+    c->bcap = c->bcap_user ? c->bcap_set : auto_bcap(c);
     c->P.bcap = c->bcap;
     CUDA_TRY(c, c->bins.alloc((size_t)c->nbins * c->bcap));
     CUDA_TRY(c, c->bin_count.alloc((size_t)c->nbins));

@@ -101,7 +101,8 @@ struct eph_ctx {
   DevBuf<D4> pe;
   DevBuf<double2> pg;
   int nbins = 0, bcap = 0, kcap = 0;
-  bool bcap_user = false;  // bin capacity set by eph_set_capacity
+  bool bcap_user = false;  // bin capacity set by eph_set_capacity, to bcap_set
+  int bcap_set = 0;
   // candidate-list reuse (FAST mode, one lane per atom, model 4 with
   // friction): the list skin s (0: search the bins every step), whether it is
   // on, and whether an adjoint keeps it off (its recomputed segments must
@@ -216,6 +217,7 @@ int launch_eam(eph_ctx *c);
 // front of the rows, where the list puts them apart (else null)
 bool eam_pair_list(const eph_ctx *c, const unsigned **pj, const int **ns, const int **inner);
 double eam_cutoff(const eph_ctx *c);  // its cut-off, 0 without one
+int eam_rows(const eph_ctx *c);       // rows of its pair list, 0 without one
 int eam_resize(eph_ctx *c);  // per-atom buffers of the pair force for c->n atoms
 void eam_free(eph_ctx *c);
 

@@ -613,6 +613,8 @@ namespace ctxi {
 
 double eam_cutoff(const eph_ctx *c) { return c->eam ? c->eam->host.rc : 0.0; }
 
+int eam_rows(const eph_ctx *c) { return c->eam ? c->eam->kcap : 0; }
+
 void eam_free(eph_ctx *c) {
   delete c->eam;
   c->eam = nullptr;
