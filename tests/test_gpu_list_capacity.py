@@ -42,3 +42,19 @@ def test_lists_take_what_a_search_takes(built, tmp_path, cells, stretch, eam, cu
         f.set_atoms(at.x, at.v, at.type, at.mask)
     assert got.list_skin()[1] and not ref.list_skin()[1]
     compare(got, ref, at.n)
+
+
+@pytest.mark.parametrize("change", [dict(bins=48), dict(pairs=112), dict(bins=40, pairs=120)])
+def test_a_new_capacity_starts_new_lists(built, beta_file, change):
+    """eph_set_capacity gives the bins that the lists and moved atoms read anew."""
+    at = W.fcc_lattice((17, 16, 17), seed=62)
+    at.v[::1500] *= 300.0  # a few atoms that move between builds
+    words = W.fix_args(beta_file, grid=(9, 8, 10), T_e=900.0)
+    got, ref = (ephgb.FixEPH(words, at, dt=0.0005) for _ in range(2))
+    got.set_list_skin(0.3)
+    ref.set_list_skin(0.0)
+    compare(got, ref, at.n)
+    builds = got.counter("build")
+    got.set_capacity(**change)
+    compare(got, ref, at.n, seed=13)
+    assert got.counter("build") == builds + 1

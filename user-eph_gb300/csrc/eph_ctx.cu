@@ -1302,6 +1302,9 @@ int eph_set_capacity(eph_ctx *c, int bin_capacity, int pair_capacity) {
     CUDA_TRY(c, c->pj.alloc((size_t)c->kcap * c->n));
     CUDA_TRY(c, c->pe.alloc((size_t)c->kcap * c->n));
     CUDA_TRY(c, alloc_pg(c));
+    // kept lists: their capacities follow, and the bins of the last build are
+    // gone, so the next step builds
+    return configure_list(c);
   }
   return EPH_OK;
 }
