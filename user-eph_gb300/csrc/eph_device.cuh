@@ -184,16 +184,6 @@ __device__ __forceinline__ double recip_nr(double x) {
   return fma(r, fma(-x, r, 1.0), r);
 }
 
-// 1/x for x > 0 to ~1 ulp: recip_nr's FP32-seeded Newton step and one more
-// (its 2^-44 squared is below FP64's last bit), four FP64 instructions and
-// none of them a conversion; outside the FP32 exponent range, the division.
-__device__ __forceinline__ double inv_positive(double x) {
-  const unsigned e = (unsigned)((unsigned long long)__double_as_longlong(x) >> 52);  // with the sign bit
-  if (e < 1023 - 100 || e > 1023 + 100) return 1.0 / x;
-  const double r = recip_nr(x);
-  return fma(r, fma(-x, r, 1.0), r);
-}
-
 __device__ __forceinline__ double dot3(double ax, double ay, double az, double bx, double by, double bz) {
   return ax * bx + ay * by + az * bz;  // ((ax bx + ay by) + az bz), fix_eph.h:160-163
 }

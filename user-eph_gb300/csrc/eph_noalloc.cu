@@ -23,6 +23,7 @@
 
 #include "eph_device.cuh"
 #include "eph_gb.h"
+#include "eph_softfp.cuh"
 
 using namespace ephgb;
 
@@ -87,18 +88,26 @@ __global__ void k_noalloc_bounds_of(const double *__restrict__ parts, double *__
   block_bounds(p[0], p[1], p[2], out);
 }
 
-// One substep of EPH_FDM::solve (eph_fdm.h:315-396): T_out from T_in.
-// Bound by FP64 issue (2 lanes per SM and clock): the reference's twelve
-// divisions by the spacings become products with 1/h^2 from the host, the
-// division by rho_e C_e one FP32-seeded Newton reciprocal (inv_positive), and
-// the cell's coordinates 32-bit divisions.  64^3 cells on GB300: 71 us per
-// substep before, 18 us now (at ~32 FP64 instructions per cell: 13 us).
-// The sum rounds within 1e-16 of itself, T itself at its own last bit as before.
+// x / 4 by the exponent
+__device__ __forceinline__ double quarter(double x) {
+  const unsigned e = soft::exponent(soft::bits(x));
+  return e - 3u < 0x7ffu - 3u ? soft::from_bits(soft::bits(x) - (2ull << 52)) : 0.25 * x;
+}
+
+// One substep of EPH_FDM::solve (eph_fdm.h:315-396) in the reference's
+// expression order, rounded as it rounds: T_out from T_in.
+// The hardware's thirteen quotients per cell made FP64 issue the bound (two
+// lanes per SM and clock).  Quotients and products run on the integer units
+// instead (the same bits), what the three spacings' quotients share comes from
+// the host, and the quarter is an exponent: 22 operations per cell are left to
+// the FP64 pipe.  64^3 cells on GB300, us per substep: 71 with the hardware's
+// operations, 18 with products by rounded reciprocals (other bits), 19 with the
+// quotients on the integer units, 16 with the products too.
 __global__ void __launch_bounds__(128)
-    k_noalloc_substep(int nx, int ny, int nz, double3 ih2, double3 ih2_4, double inner_dt, const double *__restrict__ T,
-                      double *__restrict__ Tout, const double *__restrict__ kappa, const double *__restrict__ rho,
-                      const double *__restrict__ C, const double *__restrict__ S, const double *__restrict__ dT,
-                      const signed char *__restrict__ flag) {
+    k_noalloc_substep(int nx, int ny, int nz, soft::Divisor hx, soft::Divisor hy, soft::Divisor hz, double inner_dt,
+                      const double *__restrict__ T, double *__restrict__ Tout, const double *__restrict__ kappa,
+                      const double *__restrict__ rho, const double *__restrict__ C, const double *__restrict__ S,
+                      const double *__restrict__ dT, const signed char *__restrict__ flag) {
   griddep_launch();
   griddep_wait();
   const int r = (int)(blockIdx.x * blockDim.x + threadIdx.x);
@@ -106,14 +115,12 @@ __global__ void __launch_bounds__(128)
   if (r >= nxy * nz) return;
   const int row = r / nx, i = r - row * nx, k = row / ny, j = row - k * ny;
   const double Tr = T[r];
-  const signed char fr = flag[r];
   double t = Tr;
-  if (fr == 1) {
+  if (flag[r] == 1) {
     const int p3[3] = {i > 0 ? r - 1 : r + (nx - 1), j > 0 ? r - nx : r + (nxy - nx),
                        k > 0 ? r - nxy : r + (nz - 1) * nxy};
     const int q3[3] = {i < nx - 1 ? r + 1 : r - (nx - 1), j < ny - 1 ? r + nx : r - (nxy - nx),
                        k < nz - 1 ? r + nxy : r - (nz - 1) * nxy};
-    const double ih[3] = {ih2.x, ih2.y, ih2.z}, ih4[3] = {ih2_4.x, ih2_4.y, ih2_4.z};
     // every load at once; the wall rule then selects values
     double Tq[3], Tp[3], kq[3], kp[3];
     bool wq[3], wp[3];
@@ -126,17 +133,18 @@ __global__ void __launch_bounds__(128)
       kq[a] = kappa[q3[a]];
       kp[a] = kappa[p3[a]];
     }
-    const double kr = kappa[r], source = dT[r] + S[r], inv = inv_positive(rho[r] * C[r]);
-    double grad = 0.0, lap = 0.0;  // sum of dk dT / 4 h^2, of the second differences
+    const double kr = kappa[r], add = dT[r], src = S[r], cap = soft::mul(rho[r], C[r]);
+    double ddT = 0.0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
+      const soft::Divisor &h = a == 0 ? hx : (a == 1 ? hy : hz);
       const bool sp = wp[a] && !wq[a];
       const double uq = wq[a] ? Tr : Tq[a], up = sp ? Tr : Tp[a];
       const double dk = (wq[a] ? kr : kq[a]) - (sp ? kr : kp[a]);
-      grad = fma(dk * (uq - up), ih4[a], grad);
-      lap = fma(ih[a], fma(-2.0, Tr, uq + up), lap);
+      ddT += quarter(soft::div(soft::div(soft::mul(dk, uq - up), h), h));
+      ddT += soft::mul(kr, soft::div(soft::div(fma(-2.0, Tr, uq + up), h), h));
     }
-    t = fma((fma(kr, lap, grad) + source) * inner_dt, inv, Tr);
+    t = Tr + soft::mul(soft::div(ddT + add + src, soft::divisor(cap)), inner_dt);
   }
   if (neg_double(t)) t = 0.0;
   Tout[r] = t;
@@ -194,8 +202,7 @@ extern "C" int eph_fdm_solve_noalloc(long nx, long ny, long nz, const double *lo
     inner_dt = dt / nsub;
   }
   const int threads = 128;
-  const double3 ih2 = make_double3(1.0 / (dx * dx), 1.0 / (dy * dy), 1.0 / (dz * dz));
-  const double3 ih2_4 = make_double3(0.25 * ih2.x, 0.25 * ih2.y, 0.25 * ih2.z);
+  const soft::Divisor hx = soft::divisor(dx), hy = soft::divisor(dy), hz = soft::divisor(dz);
   double *src = T, *dst = scratch;
   for (unsigned s = 0; s < nsub; ++s) {
     // each substep a programmatic dependent of the one before: its launch
@@ -209,8 +216,8 @@ extern "C" int eph_fdm_solve_noalloc(long nx, long ny, long nz, const double *lo
     at[0].val.programmaticStreamSerializationAllowed = s > 0 ? 1 : 0;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, k_noalloc_substep, (int)nx, (int)ny, (int)nz, ih2, ih2_4, inner_dt, (const double *)src, dst,
-                           kappa, rho_e, C_e, S, dT, flag) != cudaSuccess)
+    if (cudaLaunchKernelEx(&cfg, k_noalloc_substep, (int)nx, (int)ny, (int)nz, hx, hy, hz, inner_dt,
+                           (const double *)src, dst, kappa, rho_e, C_e, S, dT, flag) != cudaSuccess)
       return EPH_ERR_CUDA;
     double *t = src;
     src = dst;

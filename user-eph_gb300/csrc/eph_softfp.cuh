@@ -22,11 +22,12 @@
 // of the quotient.
 #pragma once
 
+#include <cstring>
+
 #ifdef __CUDACC__
 #define EPH_SOFT __host__ __device__ __forceinline__
 #else
 #include <cmath>
-#include <cstring>
 #define EPH_SOFT inline
 #endif
 
