@@ -1047,8 +1047,9 @@ __global__ void __launch_bounds__(ABLOCK)
     fb[i] = D4{dtfm * vbx, dtfm * vby, dtfm * vbz, 0.0};
   }
   if (RMODE == 0) {
-    // A warp takes 16 columns: a lane adds four of a column's 128 pairs, then
-    // the 32 lanes' sums in FP64, halving the columns a lane holds at every
+    // A warp takes 16 columns: a lane adds four of a column's 128 pairs (sum4:
+    // FP64's precision; as FP64 additions 1.7 % of a gradient pass more), then the
+    // 32 lanes' sums in FP64, halving the columns a lane holds at every
     // exchange (16 additions for 16 columns; a thread per column took 128 x 3
     // FP64 instructions of 16 cycles each)
     __syncthreads();
@@ -1057,15 +1058,17 @@ __global__ void __launch_bounds__(ABLOCK)
       double v[16];
 #pragma unroll
       for (int m = 0; m < 16; ++m) {
-        df64::df sum{0.0f, 0.0f};
+        v[m] = 0.0;
         if (q0 + m < nt4) {
+          df64::df cell[ABLOCK / 32];
 #pragma unroll
           for (int w = 0; w < ABLOCK / 32; ++w) {
-            const float2 cell = s_pf[(q0 + m) * nt + 32 * w + lane];
-            sum = df64::add(sum, df64::df{cell.x, cell.y});
+            const float2 c = s_pf[(q0 + m) * nt + 32 * w + lane];
+            cell[w] = df64::df{c.x, c.y};
           }
+          static_assert(ABLOCK == 128, "four pairs per lane");
+          v[m] = df64::sum4(cell[0], cell[1], cell[2], cell[3]);
         }
-        v[m] = df64::to_double(sum);
       }
 #pragma unroll
       for (int h = 8; h > 0; h >>= 1) {

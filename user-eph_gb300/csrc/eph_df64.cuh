@@ -106,6 +106,27 @@ DF_FN double to_double(df a) {
 #endif
 }
 
+// a + b + c + d in FP64, as good as FP64 additions: the high parts by TwoSum,
+// their errors and the low parts by TwoSum again, what that leaves plainly (some
+// 2^-70 of the largest term), and two FP64 additions where seven would stand
+DF_FN double sum4(df a, df b, df c, df d) {
+  float s, t, low[7] = {a.lo, b.lo, c.lo, d.lo, 0.0f, 0.0f, 0.0f};
+  two_sum(a.hi, b.hi, s, low[4]);
+  two_sum(s, c.hi, t, low[5]);
+  two_sum(t, d.hi, s, low[6]);
+  float m = low[0], rest = 0.0f;
+  for (int k = 1; k < 7; ++k) {
+    float e;
+    two_sum(m, low[k], m, e);
+    rest += e;
+  }
+#if defined(__CUDA_ARCH__)
+  return widen_bits(s) + (widen_bits(m) + widen_bits(rest));
+#else
+  return (double)s + ((double)m + (double)rest);
+#endif
+}
+
 DF_FN df neg(df a) { return df{-a.hi, -a.lo}; }
 
 // a + b within ~2 u of |a| + |b| (Dekker's add; the error relative to the sum
