@@ -2289,11 +2289,17 @@ struct FdmFast {
   int nx, ny, nz, nc;
   // uniform grid: kappa dt' / (rho_e C_e h^2) per axis and dt' / (rho_e C_e)
   const double *uni;
-  // per cell otherwise: 6 x nc weights (-x, +x, -y, +y, -z, +z; 0 where the
-  // stencil leaves a neighbour out or the cell does not change), the source
-  // weight and the constant source c_s S
+  // per cell otherwise: 6 x nc weights (-x, +x, -y, +y, -z, +z; -0.0 where the
+  // stencil leaves a neighbour out), the source weight (-0.0 where the cell does
+  // not change) and the constant source c_s S
   const double *coef, *src_w, *src0;
 };
+
+// the weight of what is left out: not merely multiplied by zero, since a wall's T
+// may be infinite or NaN.  By the high word: k_fdm_coef leaves no other weight
+// with this one (negative and below 2^-1042).
+__device__ __forceinline__ bool left_out(double w) { return __double2hiint(w) == (int)0x80000000; }
+__device__ __forceinline__ double not_left_out(double w) { return left_out(w) ? 0.0 : w; }
 
 // the neighbours of cell r in the order -x, +x, -y, +y, -z, +z (periodic)
 __device__ __forceinline__ void fdm_neighbours(const FdmFast &F, int r, int *m) {
@@ -2309,9 +2315,9 @@ __device__ __forceinline__ void fdm_neighbours(const FdmFast &F, int r, int *m) 
 
 // T of a cell after one substep from its own T, its neighbours' and its
 // source term `src` (c_s dT on a uniform grid, c_s (dT + S) otherwise); w: the
-// uniform grid's three coefficients or the cell's six weights
+// uniform grid's three coefficients or the cell's six weights; fixed: T stays
 template <bool UNIFORM>
-__device__ __forceinline__ double fdm_next(double T, const double *Tm, const double *w, double src,
+__device__ __forceinline__ double fdm_next(double T, const double *Tm, const double *w, double src, bool fixed,
                                            unsigned long long *__restrict__ counters) {
   double d;
   if (UNIFORM) {
@@ -2323,7 +2329,7 @@ __device__ __forceinline__ double fdm_next(double T, const double *Tm, const dou
 #pragma unroll
     for (int q = 0; q < 6; ++q) d = fma(w[q], Tm[q] - T, d);
   }
-  T += d;
+  if (UNIFORM || !fixed) T += d;
   if (neg_double(T)) {
     T = 0.0;
     atomicAdd(&counters[CNT_T_CLAMP], 1ull);
@@ -2367,10 +2373,10 @@ __global__ void k_fdm_coef(FdmFast F, double3 ih2, double inner_dt, const double
     if (wq) q = r;
     if (wp) p = r;
     const double d = 0.25 * (kappa[q] - kappa[p]), s = c * ih[a];
-    coef[(size_t)(2 * a) * F.nc + r] = wp ? 0.0 : s * (kr - d);
-    coef[(size_t)(2 * a + 1) * F.nc + r] = wq ? 0.0 : s * (kr + d);
+    coef[(size_t)(2 * a) * F.nc + r] = wp ? -0.0 : not_left_out(s * (kr - d));
+    coef[(size_t)(2 * a + 1) * F.nc + r] = wq ? -0.0 : not_left_out(s * (kr + d));
   }
-  src_w[r] = c;
+  src_w[r] = dyn ? not_left_out(c) : -0.0;
   src0[r] = dyn ? c * S[r] : 0.0;
 }
 
@@ -2389,6 +2395,9 @@ __global__ void __launch_bounds__(128)
   if (r < F.nc) {
     fdm_neighbours(F, r, m);
     fdm_weights<UNIFORM>(F, r, w, sw, s0);
+    if (!UNIFORM)
+#pragma unroll
+      for (int q = 0; q < 6; ++q) m[q] = left_out(w[q]) ? r : m[q];
   }
   griddep_wait();
   if (r >= F.nc) return;
@@ -2403,7 +2412,7 @@ __global__ void __launch_bounds__(128)
   double Tm[6];
 #pragma unroll
   for (int q = 0; q < 6; ++q) Tm[q] = T[m[q]];
-  Tout[r] = fdm_next<UNIFORM>(T[r], Tm, w, fma(sw, dTr, s0), counters);
+  Tout[r] = fdm_next<UNIFORM>(T[r], Tm, w, fma(sw, dTr, s0), left_out(sw), counters);
 }
 
 // All substeps of a small grid in one launch of one thread-block cluster
@@ -2428,9 +2437,16 @@ __global__ void __launch_bounds__(FDM_CLUSTER_CELLS)
   const bool mine = r < F.nc;
   double T = 0.0, src = 0.0, w[6];
   unsigned at[6];  // shared::cluster addresses of the neighbours in buffer 0
+  bool fixed = false;
   if (mine) {
     int m[6];
     fdm_neighbours(F, r, m);
+    double sw, s0;
+    fdm_weights<UNIFORM>(F, r, w, sw, s0);
+    fixed = left_out(sw);
+    if (!UNIFORM)
+#pragma unroll
+      for (int q = 0; q < 6; ++q) m[q] = left_out(w[q]) ? r : m[q];
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
       const int owner = m[q] / nt;
@@ -2439,8 +2455,6 @@ __global__ void __launch_bounds__(FDM_CLUSTER_CELLS)
     }
     T = T0[r];
     s_T[t] = T;
-    double sw, s0;
-    fdm_weights<UNIFORM>(F, r, w, sw, s0);
     const double dTr = from_fixed(acc[r]);
     dT[r] = dTr;
     acc[r] = U128{0ull, 0ull};
@@ -2455,7 +2469,7 @@ __global__ void __launch_bounds__(FDM_CLUSTER_CELLS)
 #pragma unroll
       for (int q = 0; q < 6; ++q)
         asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(Tm[q]) : "r"(at[q] + cur) : "memory");
-      T = fdm_next<UNIFORM>(T, Tm, w, src, counters);
+      T = fdm_next<UNIFORM>(T, Tm, w, src, fixed, counters);
       s_T[(cur ? 0 : nt) + t] = T;
       if (rec) rec[(size_t)s * (size_t)F.nc + r] = T;
     }
