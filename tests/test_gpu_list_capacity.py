@@ -58,3 +58,20 @@ def test_a_new_capacity_starts_new_lists(built, beta_file, change):
     got.set_capacity(**change)
     compare(got, ref, at.n, seed=13)
     assert got.counter("build") == builds + 1
+
+
+@pytest.mark.parametrize("skin", [0.0, 0.3])
+def test_more_pairs_than_rows_is_an_error(built, beta_file, tmp_path, skin):
+    """A fifth of the box full: 80 pair rows for 85 to 91 pairs of the pair force
+    (and room for their candidates in the lists).  An error, every step, and the
+    context still answers."""
+    at = W.fcc_lattice((17, 16, 17), seed=62, jitter=0.02)
+    at.boxhi = at.boxhi * np.array([1.0, 1.0, 5.0])
+    fix = ephgb.FixEPH(W.fix_args(beta_file, grid=(9, 8, 10)), at, dt=0.0005, eam=(ni_eam(tmp_path), ["Ni"]))
+    fix.set_list_skin(skin)
+    for _ in range(2):
+        fix.step(1)
+        with pytest.raises(ephgb.EphError) as e:
+            fix.synchronize()
+        assert e.value.status == 4  # EPH_ERR_CAPACITY
+    assert fix.get("T").size == 720

@@ -393,8 +393,10 @@ __global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
 #pragma unroll
   for (int o = LANES / 2; o > 0; o >>= 1) rho += __shfl_xor_sync(FULL, rho, o);
   if (!valid || g != 0) return;
-  ns = ns < C.kcap ? ns : C.kcap;
-  ens[i] = LIST ? (ns + far < C.kcap ? ns + far : C.kcap) : ns;
+  // more pairs than rows (the step ends in an error): some rows between those
+  // counted were never written, so none are read
+  if (ns + far > C.kcap) ns = far = 0;
+  ens[i] = ns + far;
   if (LIST) ens_in[i] = ns;
   const int el = ONE ? E.one : E.map[type[i]];
   double F, dF;
