@@ -355,39 +355,40 @@ __global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
     bool in = k < nc && lt(r2, rc2);
     if (LIST) in = in && (k >= first || cb.w == 0);  // a moved atom in a kept list is out of reach
     const unsigned who = __ballot_sync(FULL, in);
-    if (who == 0u) continue;  // the lists' shell, together at their ends
-    // the pair's row: from the front, in lane order; with kept lists the pairs
-    // the fix's density sweep does not need go to the row's back
-    const bool out = LIST && in && !(r2.hi < P.rc2_band);
-    int slot = ns, back = far;
-    if (LANES > 1) {
-      const unsigned lane = t & 31, below = (1u << lane) - 1u;
-      const unsigned group = ((1u << LANES) - 1u) << (lane & ~(LANES - 1));
-      const unsigned outs = LIST ? __ballot_sync(FULL, out) & group : 0u, ins = who & group & ~outs;
-      slot += __popc(ins & below);
-      ns += __popc(ins);
-      if (LIST) {
-        back += __popc(outs & below);
-        far += __popc(outs);
+    if (who != 0u) {  // else the lists' shell, together at their ends
+      // the pair's row: from the front, in lane order; with kept lists the pairs
+      // the fix's density sweep does not need go to the row's back
+      const bool out = LIST && in && !(r2.hi < P.rc2_band);
+      int slot = ns, back = far;
+      if (LANES > 1) {
+        const unsigned lane = t & 31, below = (1u << lane) - 1u;
+        const unsigned group = ((1u << LANES) - 1u) << (lane & ~(LANES - 1));
+        const unsigned outs = LIST ? __ballot_sync(FULL, out) & group : 0u, ins = who & group & ~outs;
+        slot += __popc(ins & below);
+        ns += __popc(ins);
+        if (LIST) {
+          back += __popc(outs & below);
+          far += __popc(outs);
+        }
+      } else {
+        ns += in && !out;
+        far += out;
       }
-    } else {
-      ns += in && !out;
-      far += out;
+      if (in) {
+        const int row = out ? C.kcap - 1 - back : slot;
+        // with kept lists no candidate waits in these rows; else row <= k, and the
+        // candidate there is consumed
+        if (ns + far <= C.kcap) C.pj[(size_t)row * n + i] = uc;
+        else atomicOr(C.err, ERR_PAIR_OVERFLOW);
+        const df r = mul(r2, rsqrt(r2, rsqrt_estimate(r2.hi)));
+        int mk;
+        df p;
+        herm_place(E.nr, mul(r, inv_dr), mk, p);
+        const int b = ONE ? E.one : E.map[type[uc & IDX_MASK]];
+        acc_add(rs.blk, herm_value(E.fd + 2 * (size_t)b * E.nr, mk, p));
+      }
     }
-    if (in) {
-      const int row = out ? C.kcap - 1 - back : slot;
-      // with kept lists no candidate waits in these rows; else row <= k, and the
-      // candidate there is consumed
-      if (ns + far <= C.kcap) C.pj[(size_t)row * n + i] = uc;
-      else atomicOr(C.err, ERR_PAIR_OVERFLOW);
-      const df r = mul(r2, rsqrt(r2, rsqrt_estimate(r2.hi)));
-      int mk;
-      df p;
-      herm_place(E.nr, mul(r, inv_dr), mk, p);
-      const int b = ONE ? E.one : E.map[type[uc & IDX_MASK]];
-      acc_add(rs.blk, herm_value(E.fd + 2 * (size_t)b * E.nr, mk, p));
-    }
-    if ((m & 7) == 7) bsum_fold(rs);
+    if ((m & 7) == 7) bsum_fold(rs);  // at most 8 terms to a block, skipped iterations or not
   }
   double rho = to_double(bsum_value(rs));
 #pragma unroll
