@@ -223,6 +223,19 @@ DF_FN df rsqrt(df a, float y) {
   return r;
 }
 
+// sqrt(a) from s ~ sqrt(a) to ~2^-45 (a times rsqrt(a, y)): s + y (a - s^2) / 2,
+// the residual without s.lo^2 (2^-49 of the root).  a.hi - s.hi^2 is exact by
+// TwoProd and so, but for one rounding, is what 2 s.hi s.lo leaves of it: within
+// 2^-47, 2^-50 in the mean (sqrt below 2^-49.6, the product alone 2^-47.4).
+DF_FN df sqrt_near(df a, df s, float y) {
+  float p, pe;
+  two_prod(s.hi, s.hi, p, pe);
+  const float res = (fmaf(-2.0f * s.hi, s.lo, a.hi - p) - pe) + a.lo;
+  df r;
+  fast_two_sum(s.hi, fmaf(0.5f * y, res, s.lo), r.hi, r.lo);
+  return r;
+}
+
 // sqrt(a) for a > 0 in the FP32 normal range from y ~ 1/sqrt(a.hi): the
 // estimate s0 = a.hi y, then twice s + y (a - s^2) / 2 (Karp and Markstein's
 // form of Newton's iteration, "High-precision division and square root",

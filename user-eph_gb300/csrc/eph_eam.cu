@@ -411,7 +411,8 @@ __global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
 }
 
 // k_eam_force with the pair arithmetic in double-float and LANES lanes per
-// atom: per pair 1/r (a Newton step on the FP32 estimate), r = r^2 / r, the
+// atom: per pair 1/r (a Newton step on the FP32 estimate), r = r^2 / r and a
+// residual step (the steep tables need r to the last bits), the
 // Hermite tables f_b, f_a and z2r = r phi at one interval and offset, dE/dr and
 // (dE/dr / r) e in df64, the force and 1/2 sum phi in blocked sums.  Bound by
 // FP32 issue: ~700 instructions per pair before (an interval and a scaled
@@ -463,10 +464,11 @@ __global__ void __launch_bounds__(128, EPH_EAM_FORCE_BLOCKS)
     const df ex = fixed_df(ef[0], P.fix_hi, P.fix_lo), ey = fixed_df(ef[1], P.fix_hi, P.fix_lo),
              ez = fixed_df(ef[2], P.fix_hi, P.fix_lo);
     const df r2 = dot3(ex, ey, ez, ex, ey, ez);
-    const df rinv = rsqrt(r2, rsqrt_estimate(r2.hi));
+    const float y = rsqrt_estimate(r2.hi);
+    const df rinv = rsqrt(r2, y);
     int mk;
     df p;
-    herm_place(E.nr, mul(mul(r2, rinv), inv_dr), mk, p);
+    herm_place(E.nr, mul(sqrt_near(r2, mul(r2, rinv), y), inv_dr), mk, p);
     const int b = ONE ? el : E.map[type[uc & IDX_MASK]];
     df fb, dfb, z, dz;
     herm_both(E.fd + 2 * (size_t)b * E.nr, mk, p, fb, dfb);
