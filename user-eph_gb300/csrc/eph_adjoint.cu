@@ -1406,6 +1406,13 @@ void launch_sweeps(eph_adjoint *a, const Slot &S) {
   a->launches += 1;
 }
 
+// the reverse of a step's grid solve of ns substeps in one cluster launch
+// (k_adj_fdm_cluster), which needs 17 B more per substep and cell
+bool reverse_in_cluster(const eph_adjoint *a, unsigned ns) {
+  const int most = a->c->fdm_fast_cluster;
+  return most && a->nc <= (long)ADJ_CLUSTER_CELLS * most && ns <= 65535u;
+}
+
 // reverse of the recorded step in slot s; eb, tau: device addresses of
 // dL/dE and dL/dT_mean / ncells of the step
 int reverse_step(eph_adjoint *a, int s, const double *eb, const double *tau) {
@@ -1420,7 +1427,7 @@ int reverse_step(eph_adjoint *a, int s, const double *eb, const double *tau) {
     auto Tat = [&](unsigned m) -> const double * {
       return m == 0 ? a->r_T0.p + (size_t)s * nc : a->r_Tsub.p + ((size_t)s * ns + (m - 1)) * (size_t)nc;
     };
-    if (c->fdm_fast_cluster && nc <= (long)ADJ_CLUSTER_CELLS * c->fdm_fast_cluster && ns <= 65535u) {
+    if (reverse_in_cluster(a, ns)) {
       k_adj_fdm_rates<<<dim3((unsigned)nb_of(nc, 64), ns), 64, 0, c->stream>>>(
           G, Tat(0), a->r_Tsub.p + (size_t)s * ns * nc, src, a->fdm_rates.p, a->fdm_kept.p);
       int blocks = 1;
@@ -1652,8 +1659,9 @@ int ensure_records(eph_adjoint *a) {
   if ((r = ensure(a, a->r_pj, K * (size_t)a->kcap * N))) return r;
   if ((r = ensure(a, a->r_T0, K * (size_t)a->nc)) || (r = ensure(a, a->r_src, K * (size_t)a->nc))) return r;
   if ((r = ensure(a, a->r_Tsub, K * (size_t)a->nsub * (size_t)a->nc))) return r;
-  if ((r = ensure(a, a->fdm_rates, (size_t)a->nsub * (size_t)a->nc)) ||
-      (r = ensure(a, a->fdm_kept, (size_t)a->nsub * (size_t)a->nc)))
+  if (a->fdm && reverse_in_cluster(a, a->nsub) &&
+      ((r = ensure(a, a->fdm_rates, (size_t)a->nsub * (size_t)a->nc)) ||
+       (r = ensure(a, a->fdm_kept, (size_t)a->nsub * (size_t)a->nc))))
     return r;
   return EPH_OK;
 }
