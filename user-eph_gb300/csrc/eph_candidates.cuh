@@ -289,9 +289,9 @@ struct CandidateArgs {
   int *cl_n;
   const int *state, *rb, *flist;
   const D4 *xref;
+  int *partial;    // set by a build that leaves the atoms outside the group without lists of this build (or null)
   const D4 *fpos;  // the moved atoms' positions wrapped into the box
   float far2;      // the moved atoms' widened cut-off (far_cutoff2)
-  int list_all;    // a build makes every atom's list, whether this sweep reads it or not
   // candidates of the moved atoms, mcap each (all that their bins can hold, and
   // every moved atom), for a sweep that keeps other pairs in their rows of pj
   unsigned *moved;
@@ -299,8 +299,8 @@ struct CandidateArgs {
 };
 
 // The candidates of atom i from the bins of this step or the kept lists,
-// LANES lanes to an atom (g: the lane's number); none where it is not active
-// (valid: i is an atom).  `at(k)`, k < CAP, is the
+// LANES lanes to an atom (g: the lane's number); none where it is not active.
+// `at(k)`, k < CAP, is the
 // shared-memory place of candidate k; further ones go to the atom's rows of
 // pj, or stay in the list (`tail`: where number 0 would be; number k is k `step`
 // on, which is n but for a moved atom's with MOVED_ROWS).  Of the candidates
@@ -320,9 +320,8 @@ struct CandidateArgs {
 // elements on GB300; 154 now, as without moved atoms.
 // Every lane of the warp calls it.
 template <int LANES, bool LIST, bool MOVED_ROWS, int CAP, class At>
-__device__ __forceinline__ int pair_candidates(const StepParams &P, const CandidateArgs &C, int i, int g, bool valid,
-                                               bool active, At at, const unsigned *&tail, unsigned &step,
-                                               int &first) {
+__device__ __forceinline__ int pair_candidates(const StepParams &P, const CandidateArgs &C, int i, int g, bool active, At at,
+                                               const unsigned *&tail, unsigned &step, int &first) {
   const size_t n = (size_t)P.n;
   int nc = 0;
   first = 0;
@@ -346,12 +345,9 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
     return nc;
   }
   if (C.rb[2] != 0) {  // a build step
-    // the EAM engine's sweep reads the lists of the atoms outside the group
-    // too, whichever sweep made them
-    const bool listed = C.list_all ? valid : active;
     int4 Bi = make_int4(0, 0, 0, 0);
     float4 oi = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (listed) {
+    if (active) {
       Bi = C.atom_bin[i];
       oi = C.atom_off[i];
     }
@@ -363,17 +359,19 @@ __device__ __forceinline__ int pair_candidates(const StepParams &P, const Candid
     // them: the shell's pairs mostly fail the exact test, and at the end of
     // the lists whole warps skip them
     if (LANES == 1) {
-      nc = collect_candidates(P, i, listed, Bi, oi, C.bin_count, C.bins, C.err, lset, C.band, P.lcap);
-      nc = collect_candidates(P, i, listed, Bi, oi, C.bin_count, C.bins, C.err, lset, P.rl2_band, P.lcap,
+      nc = collect_candidates(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, lset, C.band, P.lcap);
+      nc = collect_candidates(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, lset, P.rl2_band, P.lcap,
                               nullptr, C.band, nc);
     } else {
-      shared_candidates<LANES>(P, i, listed, Bi, oi, C.bin_count, C.bins, C.err, nc, P.lcap, lset, C.band);
-      shared_candidates<LANES>(P, i, listed, Bi, oi, C.bin_count, C.bins, C.err, nc, P.lcap, lset, P.rl2_band, nullptr,
+      shared_candidates<LANES>(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, nc, P.lcap, lset, C.band);
+      shared_candidates<LANES>(P, i, active, Bi, oi, C.bin_count, C.bins, C.err, nc, P.lcap, lset, P.rl2_band, nullptr,
                                C.band);
     }
     tail = C.cl + i;
-    if (valid && g == 0) C.cl_n[i] = nc;
-    return active ? nc : 0;
+    // an atom that is not active keeps the list that another sweep made
+    if (active && g == 0) C.cl_n[i] = nc;
+    if (C.partial && i == 0 && g == 0) *C.partial = 1;
+    return nc;
   }
   const int st = active ? C.state[i] : 0;
   const bool near = st != 0;

@@ -433,7 +433,6 @@ void launch_density_df(eph_ctx *c, int xi_mode) {
   C.fpos = c->fpos.p;
   C.far2 = far_cutoff2(c, c->P.rc2);
   C.xref = c->xref.p;
-  C.list_all = c->eam != nullptr;
   D.mask = c->mask.p;
   D.v = c->v.p;
   D.xi_given = c->xi.p;
@@ -454,6 +453,8 @@ void launch_density_df(eph_ctx *c, int xi_mode) {
   // with the standalone engine's EAM force the candidates come from its pair
   // list of this step (no bin scan)
   if (!(c->eam_list_fresh && eam_pair_list(c, &D.elist, &D.ens, &D.ens_in))) D.elist = nullptr;
+  // post_force by itself beside an EAM engine lists the group's atoms only
+  if (c->reuse && c->eam && !c->eam_list_fresh) C.partial = c->rb.p + 3;
   c->eam_list_fresh = false;
   switch (density_lanes(c)) {
     case 1: launch_density_df_l<MULTI, 1>(c, D); break;
@@ -827,7 +828,7 @@ void launch_bin_sort(eph_ctx *c, const int *gate) {
   }
 }
 
-int launch_bin(eph_ctx *c) {
+int launch_bin(eph_ctx *c, bool pair_force) {
   const int nb = nblocks(c->n);
   PhaseScope ps(c, EPH_PHASE_BIN);
   if (c->reuse) {
@@ -843,7 +844,7 @@ int launch_bin(eph_ctx *c) {
     else
       k_list_check<false><<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->xref.p, c->state.p,
                                                        rb, c->flist.p, c->counters.p, nullptr, nullptr);
-    k_list_decide<<<1, 32, 0, c->stream>>>(rb, c->flist.p, c->counters.p);
+    k_list_decide<<<1, 32, 0, c->stream>>>(rb, c->flist.p, c->counters.p, pair_force);
     k_list_mark<<<std::max(LIST_FMAX, nblocks(c->nbins, 512)), 512, 0, c->stream>>>(
         c->P, c->x.p, rb, c->flist.p, c->bin_count.p, c->nbins, c->bins.p, c->state.p, c->fpos.p);
     k_bin<<<nb, BLOCK, 0, c->stream>>>(c->P, c->x.p, c->xhold.p, c->wrapflag.p, c->bin_count.p, c->bins.p,
@@ -1056,7 +1057,7 @@ int record_step(eph_ctx *c, int xi_mode) {
   if ((r = launch_initial(c, 1, !c->eam))) return r;
   // with EAM the engine's pair force on this step's positions (Verlet: after
   // the wrap and the neighbour bins, before post_force)
-  if ((r = launch_bin(c)) || (c->eam && (r = launch_eam(c))) || (r = launch_pair_sweeps(c, xi_mode))) return r;
+  if ((r = launch_bin(c, c->eam)) || (c->eam && (r = launch_eam(c))) || (r = launch_pair_sweeps(c, xi_mode))) return r;
   return launch_end_of_step(c, true);
 }
 

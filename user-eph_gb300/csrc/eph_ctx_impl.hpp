@@ -197,7 +197,8 @@ int launch_post_force(eph_ctx *c, int xi_mode);
 int launch_final(eph_ctx *c);
 int launch_end_of_step(eph_ctx *c, bool with_final);
 // post_force in two parts: spatial binning (and the wrap), then the sweeps
-int launch_bin(eph_ctx *c);
+// (pair_force: launch_eam follows)
+int launch_bin(eph_ctx *c, bool pair_force = false);
 // candidate-list reuse on or off as the context's settings allow (bins,
 // list buffers), and a build requested for the next step; drop_list turns it off
 int configure_list(eph_ctx *c);

@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
   const unsigned *tail;
   unsigned step;
   int first;
-  const int nc = pair_candidates<LANES, LIST, LIST, CAP>(P, C, i, g, valid, valid, at, tail, step, first);
+  const int nc = pair_candidates<LANES, LIST, LIST, CAP>(P, C, i, g, valid, at, tail, step, first);
   __syncwarp();
   const df rc2{E.rc2_hi, E.rc2_lo}, inv_dr{E.inv_dr_hi, E.inv_dr_lo};
   bsum rs = bsum_zero();
@@ -685,7 +685,6 @@ int launch_eam(eph_ctx *c) {
     C.xref = c->xref.p;
     C.moved = c->mcand.p;
     C.mcap = c->mcap;
-    C.list_all = 1;
     const int lanes = eam_lanes(c);
     if (E.one >= 0) {
       if (lanes == 2) launch_eam_df<true, 2>(c, E, C, fext);

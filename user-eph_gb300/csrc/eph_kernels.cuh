@@ -817,7 +817,8 @@ __global__ void __launch_bounds__(tpa_threads(TPA)) k_density_tpa(
 // (the df64 sweeps: see pair_candidates), leave moved atoms' bin entries out
 // and take the moved atoms as extra candidates.  More moved atoms, or a request from the host,
 // make the step a build step.  Decisions live on the device (rb[0] build
-// requested, rb[1] moved atoms this step, rb[2] this step builds), so a
+// requested, rb[1] moved atoms this step, rb[2] this step builds, rb[3] the lists
+// are of the group's atoms only, which a step with a pair force makes anew), so a
 // captured step replays them.  Lists hold atom indices; the periodic image of
 // a pair is the minimum image of the current positions, decided in FP32 (the
 // box is at least three list radii wide, so it is the image within the
@@ -899,10 +900,10 @@ __global__ void k_list_check(StepParams P, D4 *__restrict__ x, D4 *__restrict__ 
 // appended in any order; the order of the extra candidates must not change
 // from run to run).
 __global__ void k_list_decide(int *__restrict__ rb, int *__restrict__ flist,
-                              unsigned long long *__restrict__ counters) {
+                              unsigned long long *__restrict__ counters, bool pair_force) {
   const int lane = threadIdx.x;
   const int cnt = rb[1];
-  const bool build = rb[0] != 0 || cnt > LIST_FMAX;
+  const bool build = rb[0] != 0 || (pair_force && rb[3] != 0) || cnt > LIST_FMAX;
   if (!build && cnt > 1) {
     const int v = lane < cnt ? flist[lane] : 0x7fffffff;
     int rank = 0;
@@ -913,7 +914,10 @@ __global__ void k_list_decide(int *__restrict__ rb, int *__restrict__ flist,
   if (lane == 0) {
     rb[2] = build ? 1 : 0;
     rb[0] = 0;
-    if (build) atomicAdd(&counters[CNT_BUILD], 1ull);
+    if (build) {
+      rb[3] = 0;
+      atomicAdd(&counters[CNT_BUILD], 1ull);
+    }
   }
 }
 
@@ -1194,7 +1198,7 @@ __global__ void __launch_bounds__(128, EPH_DF_DENSITY_BLOCKS) k_density_df(StepP
     list_candidates<LANES>(P, i, active, xi, D.elist, D.ens, D.C.rec, D.C.err, nc, P.kcap, set, P.rc2_band);
   } else {
     unsigned step;  // n: a moved atom's candidates wait in its rows of pj
-    nc = pair_candidates<LANES, SRC == DF_LIST, false, CAP>(P, D.C, i, g, valid, active, at, tail, step, first);
+    nc = pair_candidates<LANES, SRC == DF_LIST, false, CAP>(P, D.C, i, g, active, at, tail, step, first);
   }
   __syncwarp();
   // after the candidates: their searches need the registers
