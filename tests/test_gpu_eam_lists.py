@@ -1,5 +1,5 @@
 """Kept candidate lists that the EAM engine's pair force shares with the fix's
-density sweep, against a bin search every step (list skin 0).
+density sweep, against a bin search every step (list skin 0, or FP64 pair terms).
 
 Tolerance: the bars of tests/test_gpu_eam.py, forces 1e-11 and energy 1e-12;
 rho 2e-12 (either arithmetic is within 1e-12 of the reference)."""
@@ -98,3 +98,27 @@ def test_moved_atoms_find_every_neighbour(built, beta_file, tmp_path, cells, str
         agree(got, ref)
         builds.append(got.counter("build"))
     assert builds[-1] == builds[0]  # the atoms moved between builds
+
+
+@pytest.mark.parametrize("cells", [(17, 16, 17), (21, 20, 20)])
+def test_two_elements_over_lists(built, beta_file, tmp_path, cells):
+    """Unlike pairs (f_a and f_b tables apart) at 8 and 4 lanes per atom, against
+    FP64 pair terms and a search every step."""
+    from test_gpu_df_sweeps import write_two_element_setfl
+
+    at = W.fcc_lattice(cells, seed=63)
+    at.type = np.where(np.random.default_rng(2).random(at.n) < 0.4, 2, 1).astype(np.int32)
+    at.mass = np.array([0.0, W.NI_MASS, W.NI_MASS])
+    hot_atoms(at, 6, 700.0, 3)
+    words = W.fix_args(beta_file, grid=(9, 8, 10), T_e=900.0, elements=("Ni", "Ni"))
+    pair = (write_two_element_setfl(str(tmp_path / "two.eam")), ["Ni", "Xx"])
+    got, ref = (ephgb.FixEPH(words, at, dt=0.0005, eam=pair) for _ in range(2))
+    assert got.list_skin()[1]
+    ref.set_pair_arithmetic(ephgb.PAIRS_FP64)
+    assert not ref.list_skin()[1]
+    rng = np.random.default_rng(13)
+    for _ in range(3):
+        xi = rng.standard_normal((at.n, 3))
+        for f in (got, ref):
+            f.step(1, xi=xi)
+        agree(got, ref)
