@@ -49,8 +49,10 @@ int fail(eph_ctx *c, int code, const std::string &msg) {
 
 int upload_tables(eph_ctx *c) {
   const Beta &b = c->beta;
+  std::vector<std::vector<double>> sources;  // until the copies are done
   auto up = [&](DevBuf<D4> &dst, int which, long nk) -> cudaError_t {
-    std::vector<double> h((size_t)b.n_elements * nk * 4);
+    sources.emplace_back((size_t)b.n_elements * nk * 4);
+    std::vector<double> &h = sources.back();
     for (int e = 0; e < b.n_elements; ++e) {
       const Spline &s = b.table(which, e);
       std::memcpy(&h[(size_t)e * nk * 4], s.c.data(), sizeof(double) * 4 * nk);
@@ -102,16 +104,19 @@ int upload_tables(eph_ctx *c) {
       CUDA_TRY(c, c->tab_rho_df.alloc(h.size()));
     }
     CUDA_TRY(c, upload(c, c->tab_rho_df.p, h.data(), h.size() * sizeof(float4)));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     c->P.tab_rho_df = c->tab_rho_df.p;
   }
   return EPH_OK;
 }
 
-// 1/(rho_e C_e) per cell for the FAST substeps (IEEE quotients, as on the device)
+// 1/(rho_e C_e) per cell for the FAST substeps (IEEE quotients, as on the device);
+// done, as every copy of the stream before it, on return
 cudaError_t upload_inverse(eph_ctx *c, const std::vector<double> &rc) {
   std::vector<double> inv(rc.size());
   for (size_t i = 0; i < rc.size(); ++i) inv[i] = 1.0 / rc[i];
-  return upload(c, c->irhoC.p, inv.data(), inv.size() * 8);
+  const cudaError_t e = upload(c, c->irhoC.p, inv.data(), inv.size() * 8);
+  return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;
 }
 
 int upload_grid(eph_ctx *c) {
@@ -136,9 +141,9 @@ int upload_grid(eph_ctx *c) {
   CUDA_TRY(c, upload(c, c->T0.p, g.T.data(), nc * 8));
   CUDA_TRY(c, upload(c, c->kappa.p, g.kappa.data(), nc * 8));
   CUDA_TRY(c, upload(c, c->rhoC.p, rc.data(), nc * 8));
-  CUDA_TRY(c, upload_inverse(c, rc));
   CUDA_TRY(c, upload(c, c->S.p, g.S.data(), nc * 8));
   CUDA_TRY(c, upload(c, c->gflag.p, fl.data(), nc));
+  CUDA_TRY(c, upload_inverse(c, rc));
   CUDA_TRY(c, cudaMemsetAsync(c->dT.p, 0, nc * 8, c->stream));
   CUDA_TRY(c, cudaMemsetAsync(c->acc.p, 0, nc * sizeof(U128), c->stream));
   c->td = TdynTables{};
@@ -163,6 +168,7 @@ int upload_grid(eph_ctx *c) {
     CUDA_TRY(c, upload(c, c->E_dy.p, g.E_T.dy.data(), nt * 8));
     CUDA_TRY(c, upload(c, c->C_T.p, g.C_T.c.data(), nt * sizeof(D4)));
     CUDA_TRY(c, upload(c, c->K_T.p, g.kappa_T.c.data(), nt * sizeof(D4)));
+    CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     if (!c->h_bounds) CUDA_TRY(c, cudaMallocHost(&c->h_bounds, 4 * sizeof(double)));
     c->td = TdynTables{c->tdyn.p, c->C_T.p, c->K_T.p, c->E_y.p, c->E_dy.p, c->grho.p, g.E_T.dx, g.C_T.inv_dx, (int)nt};
   }
@@ -380,9 +386,9 @@ bool fused_friction(const eph_ctx *c) {
   return c->mode == EPH_MODE_FAST && c->args.model == 4 && (c->P.flags & FLAG_FRICTION) && c->fuse_w;
 }
 
-// FAST pair sums in df64: the one-lane density sweep with stage 1 folded,
-// over the bin search (k_density_df) or the kept lists (k_density_list_df),
-// then k_forces_df at any lanes per atom
+// FAST pair sums in df64: k_density_df with stage 1 folded (over the bin search,
+// the kept lists or the EAM engine's pair list), then k_forces_df; below 16,384
+// atoms only where the caller chose one lane per atom
 bool df_active(const eph_ctx *c) {
   return c->pair_arith == EPH_PAIRS_DF64 && c->mode == EPH_MODE_FAST && fused_friction(c) &&
          !(c->tpa > 1 && c->n < 16384);
@@ -488,11 +494,10 @@ constexpr int EXACT_WIDE = 16384;
 
 template <bool FAST, bool MULTI, bool FUSE>
 void launch_density_f(eph_ctx *c, int xi_mode) {
-  // several lanes per atom in the density sweep too below 16,384 atoms, where
-  // one lane per atom leaves it latency bound (measured on GB300: 4,000 atoms
-  // 0.289 -> 0.210 ms per step; from 16,384 atoms on the extra exact-test pass
-  // and lane sums cost more than they hide: 32,000 atoms 71 -> 81 ms per 200
-  // steps, so the one-lane sweep stays there)
+  // below 16,384 atoms FP64 pair terms over many lanes per atom (k_density_tpa,
+  // density_tpa), where one lane per atom leaves the sweep latency bound; from
+  // there on the df64 sweep with lanes of its own (density_lanes), or with FP64
+  // pair sums the one-lane sweep
   if constexpr (FAST) {
     if (c->tpa > 1 && c->n < 16384) {
       // with the EAM engine the pairs come from its list of this step
@@ -668,10 +673,11 @@ int list_bcap(const eph_ctx *c, double rc) {
   return std::max(auto_bcap(c), round8(std::min(grown, 0.25 * vol)));
 }
 
-// Kept candidate lists: FAST mode, model 4 with friction, the one-lane
-// density sweep (one lane per atom, or 16,384 atoms and more), no pair force
-// of the engine (it needs bins every step) and no adjoint.  With FP64 pair
-// sums by default from 2^15 to 2^20 atoms: the lists save the bin search, which the density
+// Kept candidate lists: FAST mode, model 4 with friction, the df64 density
+// sweep or the one-lane FP64 one (one lane per atom, or 16,384 atoms and more),
+// no adjoint; beside an EAM engine, whose pair force shares them, with df64 pair
+// sums only (its FP64 sweeps search the bins every step).  With FP64 pair sums
+// by default from 2^15 to 2^20 atoms: the lists save the bin search, which the density
 // sweep's FP64 pass hides less well in small systems, and cost four small
 // launches a step plus the atoms near moved ones (measured on GB300 with a
 // 0.3 A skin, step time: 16,384 atoms +18 %, 62,500 atoms -8 %, 131,072 atoms
@@ -1642,6 +1648,7 @@ int eph_set_atoms(eph_ctx *c, int n, const double *hx, const double *hv, const i
   CUDA_TRY(c, upload(c, c->type.p, htype, sizeof(int) * N));
   CUDA_TRY(c, upload(c, c->mask.p, m.data(), sizeof(int) * N));
   CUDA_TRY(c, upload(c, c->tmap.p, c->P.type_map, sizeof(int) * 65));
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   for (DevBuf<D4> *b : {&c->x, &c->v, &c->f, &c->xhold, &c->f_eph, &c->f_rng, &c->xi, &c->A, &c->Bw})
     CUDA_TRY(c, cudaMemsetAsync(b->p, 0, sizeof(D4) * N, c->stream));
   int r = eph_put(c, EPH_FIELD_X, hx, EPH_HOST);
@@ -2375,8 +2382,8 @@ int eph_set_grid_constants(eph_ctx *c, double C_e, double kappa_e) {
   CUDA_TRY(c, cudaSetDevice(c->device));
   CUDA_TRY(c, settle(c));  // queued steps read the old constants
   CUDA_TRY(c, upload(c, c->rhoC.p, rc.data(), nc * 8));
-  CUDA_TRY(c, upload_inverse(c, rc));
   CUDA_TRY(c, upload(c, c->kappa.p, g.kappa.data(), nc * 8));
+  CUDA_TRY(c, upload_inverse(c, rc));
   drop_graph(c);  // the substep count may change
   const unsigned nsub = c->nsub;
   set_time_params(c);

@@ -239,10 +239,10 @@ inline cudaError_t settle(eph_ctx *c) {
 
 // A set-up copy from pageable host memory, on the context's stream: what the
 // stream does next finds it done (cudaMemcpy on the default stream is not
-// ordered with it, and may return before the device has the data).
+// ordered with it, and may return before the device has the data).  The caller
+// waits for the stream before src goes.
 inline cudaError_t upload(eph_ctx *c, void *dst, const void *src, size_t bytes) {
-  const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream);
-  return e == cudaSuccess ? cudaStreamSynchronize(c->stream) : e;  // src may be a local of the caller's
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream);
 }
 
 inline cudaEvent_t take_event(eph_ctx *c) {

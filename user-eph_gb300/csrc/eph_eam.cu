@@ -309,7 +309,7 @@ __device__ __forceinline__ void herm_both(const float4 *__restrict__ t, int m, d
 // What bounds it: the candidates.  The 27 bins of 6.5 A hold 675 of them per
 // atom, of which 78-85 are pairs; the bins' search took two thirds of the
 // instructions (73,000 a warp), the kept lists leave 121 per atom.
-// GB300, 256,000 atoms: 989 us -> 285 (kept lists); where the bins are searched
+// GB300, 256,000 atoms: 989 us -> 273 (kept lists); where the bins are searched
 // every step, 16,384 atoms took both sweeps 536 us, now 100 (8 lanes).
 template <bool ONE, int LANES, bool LIST>
 __global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(128, EPH_EAM_DENSITY_BLOCKS)
 // (dE/dr / r) e in df64, the force and 1/2 sum phi in blocked sums.  Bound by
 // FP32 issue: ~700 instructions per pair before (an interval and a scaled
 // derivative per table, square root and reciprocal apart), ~430 now.
-// GB300, 256,000 atoms: 596 -> 361 us.
+// GB300, 256,000 atoms: 596 -> 366 us (361 without the residual step).
 template <bool ONE, int LANES>
 __global__ void __launch_bounds__(128, EPH_EAM_FORCE_BLOCKS)
     k_eam_force_df(StepParams P, EamParams E, const int *__restrict__ type, const unsigned *__restrict__ epj,
@@ -572,8 +572,9 @@ int upload_table(eph_ctx *c, DevBuf<D4> &dst, const std::vector<std::vector<doub
   }
   CUDA_TRY(c, dst.alloc(all.size() / 4));
   CUDA_TRY(c, ctxi::upload(c, dst.p, all.data(), all.size() * sizeof(double)));
+  std::vector<float> split;
   if (dfo) {
-    std::vector<float> split(2 * all.size());
+    split.resize(2 * all.size());
     for (size_t m = 0; m < all.size() / 4; ++m)
       for (int k = 0; k < 4; ++k) {
         const df64::df v = df64::from_double(all[4 * m + k]);
@@ -583,6 +584,7 @@ int upload_table(eph_ctx *c, DevBuf<D4> &dst, const std::vector<std::vector<doub
     CUDA_TRY(c, dfo->alloc(all.size() / 2));
     CUDA_TRY(c, ctxi::upload(c, dfo->p, split.data(), split.size() * sizeof(float)));
   }
+  CUDA_TRY(c, cudaStreamSynchronize(c->stream));
   return EPH_OK;
 }
 
