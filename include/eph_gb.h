@@ -165,7 +165,8 @@ int eph_set_graph(eph_ctx *ctx, int on);
  * transferred to the electrons, 1 -> mean electronic temperature
  * (eph_fdm.h:189-196). */
 int eph_compute_vector(eph_ctx *ctx, int i, double *out);
-/* FixEPH::reset_dt (fix_eph.cpp:909-916). */
+/* FixEPH::reset_dt (fix_eph.cpp:909-916).  Waits for the steps queued so far, a
+ * batch's included. */
 int eph_reset_dt(eph_ctx *ctx, double dt);
 /* EPH_FDM::save_state (eph_fdm.h:226-265) and save_temperature
  * (eph_fdm.h:198-224) of the current grid. */
@@ -184,7 +185,9 @@ int eph_synchronize(eph_ctx *ctx);
  * once, eph_beta.h:174-180), 1 grid cells clamped at T = 0 (eph_fdm.h:391-394),
  * 2 neighbour-list builds, 3 position wraps. */
 int eph_get_counter(eph_ctx *ctx, int which, long *out);
-/* Capacity of a spatial bin and of a per-atom pair list (0 keeps a value). */
+/* Capacity of a spatial bin and of a per-atom pair list (0 keeps a value).  The
+ * bin capacity is that of bins of the cut-off; the wider ones of kept lists
+ * (eph_set_list_skin) grow with their volume. */
 int eph_set_capacity(eph_ctx *ctx, int bin_capacity, int pair_capacity);
 
 /* Pair force of the standalone engine (eph_step, batches): eam/alloy from a

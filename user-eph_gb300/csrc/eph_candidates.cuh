@@ -13,9 +13,6 @@ __device__ __forceinline__ double min_image(double d, double L, double h) {
   return d > h ? d - L : (d < -h ? d + L : d);
 }
 
-// the boxes min_image adds to d
-__device__ __forceinline__ int image_count(double d, double h) { return d > h ? -1 : (d < -h ? 1 : 0); }
-
 // The 3x3x3 image code of x_j seen from x_i: the image of x_j within half a
 // box of x_i on every axis, decided in FP32 (the box is at least three list
 // radii wide, so a pair within the list radius is far from the threshold).

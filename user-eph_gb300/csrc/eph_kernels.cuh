@@ -1,8 +1,9 @@
 // sm_103a kernels of the fix-eph hot path.
 //
-// One thread per atom for every per-atom sweep.  The FP64 pipe of GB300
-// issues about two instructions per clock per SM, so these kernels are bound
-// by FP64 instruction issue, not by HBM: the design removes FP64 work
+// One to 32 lanes per atom by size, one thread per atom for what is done once
+// per atom.  The FP64 pipe of GB300 issues about two instructions per clock per
+// SM, so the kernels with FP64 pair terms are bound by FP64 instruction issue,
+// not by HBM (those with df64 terms: see k_density_df): the design removes FP64 work
 // (in-cutoff pairs compacted per step so the warps sweep them in lockstep,
 // pair geometry and rho(r^2) cached once per step, alpha/beta per atom once)
 // and keeps integer/FP32 work (binning, candidate tests, sorting) off the
@@ -1137,8 +1138,8 @@ __global__ void __maxnreg__(64) k_density_list(
 // record halves and table rows: 1.84; lists read from global memory two
 // candidates ahead, so that the L1 keeps the table and records: 1.47; the
 // division-free grid cell: 1.44; 7 blocks per SM, which the totals' place in
-// shared memory allows: 1.36.  Now the issue slots, the L1 and (in the
-// epilogues) the FP64 pipe are each 60-65 % busy.  Cooperative asynchronous
+// shared memory allows: 1.36 (1.375 since moved atoms test what they find).  Now
+// the issue slots, the L1 and (in the epilogues) the FP64 pipe are each 60-65 % busy.  Cooperative asynchronous
 // copies of whole records to shared memory took 1.69 and were not kept.
 enum : int { DF_BINS = 0, DF_LIST = 1, DF_EAM = 2 };
 
@@ -1629,7 +1630,7 @@ __global__ void __launch_bounds__(EX_THREADS) k_forces_exact(StepParams P, const
 // Stages 2 and 3 in FAST mode after k_density<.., true> (same sums as
 // k_forces, split into the atom's own part and the neighbours' part); TPA
 // lanes per atom take rows g, g + TPA, ... of the neighbours' part and
-// combine by a butterfly, as k_forces_tpa does.  With W_i = a_i w_i, X_i = a_i xi_i (a_i = alpha_i/rho_i)
+// their sums meet in shared memory, where one thread per atom finishes.  With W_i = a_i w_i, X_i = a_i xi_i (a_i = alpha_i/rho_i)
 // and M_i = sum_j H_ij e e^T over all of the atom's pairs:
 //   f_EPH_i = -M_i W_i + sum_{j live} H_ji (e.W_j) e + sum_{j not live} H_ij (e.W_i) e
 //   f_RNG_i = eta sqrt(T_e) [M_i X_i - sum_{j live} H_ji (e.X_j) e - sum_{j not live} H_ij (e.X_i) e]
